@@ -134,6 +134,16 @@ __device__ __forceinline__ void philox_normal4(uint64_t seed, uint32_t group,
   box_muller(r.z, r.w, out[2], out[3]);
 }
 
+// Uniform in (0, 1) with 53 random bits from Philox (seed, counter (pair,
+// step, 0, GBSGMC_TAG_SWAP)).
+__device__ __forceinline__ double swap_uniform(uint64_t seed, uint32_t pair, uint32_t step) {
+  const U32x4 r = philox4x32_10(U32x4{pair, step, 0u, GBSGMC_TAG_SWAP},
+                                static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+  const uint64_t bits = ((static_cast<uint64_t>(r.x) >> 5) << 26) |
+                        (static_cast<uint64_t>(r.y) >> 6);
+  return (static_cast<double>(bits) + 0.5) * (1.0 / 9007199254740992.0);
+}
+
 struct Noise {
   const float* buf;
   int64_t stride;

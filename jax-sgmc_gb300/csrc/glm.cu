@@ -37,70 +37,33 @@
 #include <tuple>
 
 #include "common.cuh"
+#include "glm.cuh"
 #include "internal.h"
 
 namespace gbsgmc {
+int glm_sm_count() {
+  static int cached = 0;
+  if (cached == 0) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) ==
+            cudaSuccess &&
+        n > 0)
+      cached = n;
+    else
+      cached = 152;
+  }
+  return cached;
+}
+
 namespace {
 
 constexpr int kMaxWarps = 16;   // warps per CTA: 8 or 16 (a kernel parameter)
 constexpr int kMaxRowsPerSlice = 1024;
 constexpr int kMinSlicesAlloc = 16;
 
-enum Mode { kValueGrad = 0, kSgldStep = 1 };
-
-struct GlmArgs {
-  int family, d, dq;
-  int y_inline;
-  int64_t n_obs, n_rows, ld;
-  const float* X;
-  const float* y;
-  float inv_s2;     // 1/sigma^2 (linear-Gaussian)
-  float log_norm;   // log sigma + 0.5 log 2 pi (linear-Gaussian)
-  float inv_p2;     // 1/prior_scale^2, 0 for a flat prior
-  double prior_const;  // d * (log s + 0.5 log 2 pi), 0 for a flat prior
-  float inv_temp;
-  int chains, n, slices, rows_per_slice;
-  const int32_t* idx;
-  int64_t idx_stride;
-  int steps;                // SGLD steps per launch (> 1: one CTA per chain)
-  int64_t idx_step_stride;  // elements between the index sets of two steps
-  const float* mask;
-  int mode;
-  float* w;
-  float* v;
-  float alpha, lmbd;
-  Sched sched;
-  Noise noise;
-  double* U;
-  float* grad;
-  float* lk;
-  double* lk_var;
-  float* samples;
-  double* sample_lik;
-  float4* ws_part;
-  double* ws_sums;
-  unsigned* ws_ticket;
-  void* ws_base;
-  size_t ws_size;
-  int slices_fixed;   // > 0: slices per chain chosen by the caller
-  int rw_fixed;       // > 0: rows per warp chosen by the caller
-  int warps_fixed;    // > 0: warps per CTA chosen by the caller
-  int pf_fixed;       // 1: prefetching variant, -1: not, 0: library choice
-  int dyn_fixed;      // 1: dynamically scheduled kernel, -1: not, 0: library choice
-  int* status;
-  int vec4;   // rows are 16-byte aligned: 128-bit loads
-  // Replica exchange: chain c's index row and noise stream belong to chain
-  // ident[c] (the states that moved into c with an exchange); NULL: c itself.
-  const int32_t* ident;
-};
-
-// The chain whose index row and noise stream chain (slot) c uses.
-__device__ __forceinline__ int ident_of(const GlmArgs& a, int c) {
-  return a.ident != nullptr ? __ldg(a.ident + c) : c;
-}
-
 struct SmemLayout {
-  size_t flags, idx, idx2, m, red, sums, wbuf, total;
+  size_t flags, idx, idx2, m, red, sums, lanes, wbuf, total;
 };
 
 __host__ __device__ inline size_t align_up(size_t x, size_t a) {
@@ -126,83 +89,14 @@ __host__ __device__ inline SmemLayout smem_layout(int rows_per_slice, int dq,
   o += static_cast<size_t>(warps) * dq * 16;
   o = align_up(o, 16);
   L.sums = o;
-  o += sizeof(double) * 4 * (warps + 1);
+  o += sizeof(double) * 4;
+  L.lanes = o;  // the row-owning lanes' sums, at most eight per warp
+  o += sizeof(LaneSums) * 8 * warps;
   o = align_up(o, 16);
   L.wbuf = o;  // w between the steps of a multi-step launch
   o += static_cast<size_t>(dq) * 16;
   L.total = o;
   return L;
-}
-
-// Bernoulli-logit log-likelihood y z - softplus(z) and its derivative
-// y - sigmoid(z), from one exponential: e = exp(-|z|),
-// softplus(z) = max(z, 0) + log1p(e), sigmoid(z) = 1/(1+e) or e/(1+e).
-__device__ __forceinline__ void logistic_link(float z, float y, float& lk,
-                                              float& dz) {
-  const float e = expf(-fabsf(z));
-  const float r = 1.0f / (1.0f + e);
-  lk = y * z - (fmaxf(z, 0.0f) + log1pf(e));
-  dz = y - (z >= 0.0f ? r : e * r);
-}
-
-// 128-bit read-only load that does not allocate in L1 (rows are read once).
-__device__ __forceinline__ float4 ld_row4(const float* p) {
-  float4 v;
-  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p));
-  return v;
-}
-
-__device__ __forceinline__ float ld_row1(const float* p) {
-  float v;
-  asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-  return v;
-}
-
-// 4-byte asynchronous copy global -> shared (completes in the background;
-// cp_async_wait_all waits for the calling thread's copies).
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-  const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gmem_src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-template <int RW>
-struct Log2;
-template <>
-struct Log2<1> { static constexpr int v = 0; };
-template <>
-struct Log2<2> { static constexpr int v = 1; };
-template <>
-struct Log2<4> { static constexpr int v = 2; };
-template <>
-struct Log2<8> { static constexpr int v = 3; };
-
-// Sum of p[r] over the 32 lanes for RW rows at once.  Returns, in every lane
-// of group g = lane >> (5 - log2 RW), the full sum of row g.
-template <int RW>
-__device__ __forceinline__ float transposed_warp_sum(float (&p)[RW], int lane) {
-  constexpr int LOG = Log2<RW>::v;
-#pragma unroll
-  for (int t = 0; t < LOG; ++t) {
-    const int o = 16 >> t;
-    const int half = RW >> (t + 1);
-    const bool upper = (lane & o) != 0;
-#pragma unroll
-    for (int i = 0; i < half; ++i) {
-      const float send = upper ? p[i] : p[i + half];
-      const float keep = upper ? p[i + half] : p[i];
-      p[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-    }
-  }
-  float z = p[0];
-#pragma unroll
-  for (int o = 16 >> LOG; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-  return z;
 }
 
 // Issues every load of the tile of rows [r0, r0 + RW): x of the RW rows and
@@ -246,95 +140,6 @@ __device__ __forceinline__ void load_tile(const GlmArgs& a, const int32_t* idx_s
   }
 }
 
-// Per-lane accumulators of one CTA row stream.  The likelihood sums stay in
-// fp32 per lane (a lane sees a few dozen rows); they are widened to fp64 for
-// the warp and block reductions.  GB300's fp64 pipe runs at a small fraction
-// of the fp32 rate, so per-row fp64 arithmetic would throttle the kernel.
-//
-// The sum of the (masked) likelihoods that makes U is compensated: each
-// addition's rounding error is carried in mlk_c (Neumaier's variant of
-// Kahan summation, A. Neumaier 1974), so a lane's sum is good to about one
-// rounding of its total whatever its row count.  Once the sum overflows the
-// correction is dropped, so an infinite likelihood sum stays infinite (the
-// MH tests reject such a proposal) instead of turning into inf - inf.
-//
-// The variance needs E[lk^2] - E[lk]^2, which cancels badly when |lk| is
-// large, so each lane sums around its first value K: s1 = sum(lk - K),
-// s2 = sum((lk - K)^2); the widening to fp64 restores sum(lk) and sum(lk^2).
-template <int QPL>
-struct Accum {
-  float4 acc[QPL];
-  float mlk, mlk_c, K, s1, s2;
-  int cnt;
-};
-
-__device__ __forceinline__ void neumaier_add(float& sum, float& comp, float x) {
-  const float t = sum + x;
-  const float e = fabsf(sum) >= fabsf(x) ? (sum - t) + x : (x - t) + sum;
-  comp += isfinite(t) ? e : 0.0f;
-  sum = t;
-}
-
-// Likelihood, adjoint and accumulation for a loaded tile (see load_tile).
-template <int QPL, int RW>
-__device__ __forceinline__ void consume_tile(const GlmArgs& a, const float* m_s,
-                                             float* lk_out, int r0, int lane,
-                                             int g, bool leader,
-                                             const float4 (&wq)[QPL],
-                                             const float4 (&xv)[RW][QPL],
-                                             float yv, int og, Accum<QPL>& A) {
-  constexpr int GROUP = 32 / RW;
-  float p[RW];
-#pragma unroll
-  for (int r = 0; r < RW; ++r) {
-    float z = 0.0f;
-#pragma unroll
-    for (int k = 0; k < QPL; ++k) {
-      z = fmaf(xv[r][k].x, wq[k].x, z);
-      z = fmaf(xv[r][k].y, wq[k].y, z);
-      z = fmaf(xv[r][k].z, wq[k].z, z);
-      z = fmaf(xv[r][k].w, wq[k].w, z);
-    }
-    p[r] = z;
-  }
-  const float z = transposed_warp_sum<RW>(p, lane);
-  const bool ok = og >= 0;
-  const int row = r0 + g;
-  const float mw = (ok && a.mask != nullptr) ? m_s[row] : 1.0f;
-  float lkv, dz;
-  if (a.family == GBSGMC_GLM_LOGISTIC) {
-    logistic_link(z, yv, lkv, dz);
-  } else if (a.family == GBSGMC_GLM_LINEAR) {
-    lkv = z;
-    dz = 1.0f;
-  } else {
-    const float res = yv - z;
-    lkv = -0.5f * res * res * a.inv_s2 - a.log_norm;
-    dz = res * a.inv_s2;
-  }
-  const float coef = ok ? mw * dz : 0.0f;
-  if (ok && leader) {
-    neumaier_add(A.mlk, A.mlk_c, mw * lkv);
-    if (A.cnt == 0) A.K = lkv;
-    const float dk = lkv - A.K;
-    A.s1 += dk;
-    A.s2 = fmaf(dk, dk, A.s2);
-    A.cnt += 1;
-    if (lk_out != nullptr) lk_out[row] = lkv;
-  }
-#pragma unroll
-  for (int r = 0; r < RW; ++r) {
-    const float cr = __shfl_sync(0xffffffffu, coef, r * GROUP);
-#pragma unroll
-    for (int k = 0; k < QPL; ++k) {
-      A.acc[k].x = fmaf(cr, xv[r][k].x, A.acc[k].x);
-      A.acc[k].y = fmaf(cr, xv[r][k].y, A.acc[k].y);
-      A.acc[k].z = fmaf(cr, xv[r][k].z, A.acc[k].z);
-      A.acc[k].w = fmaf(cr, xv[r][k].w, A.acc[k].w);
-    }
-  }
-}
-
 // Step j of a launch (see glm_kernel): indices at idx + j * idx_step_stride,
 // schedule step counter + offset + j.
 template <int QPL, int RW, bool PF, int WARPS>
@@ -352,6 +157,7 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
   float* m_s = reinterpret_cast<float*>(smem + L.m);
   float4* red = reinterpret_cast<float4*>(smem + L.red);
   double* sums = reinterpret_cast<double*>(smem + L.sums);
+  LaneSums* lsum = reinterpret_cast<LaneSums*>(smem + L.lanes);
   float4* w_s = reinterpret_cast<float4*>(smem + L.wbuf);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -436,16 +242,12 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
       vq.w = e0 + 3 < a.d ? vc[3] : 0.0f;
     }
   }
-  if (a.inv_p2 > 0.0f && warp == 0) {
-    double ww = 0.0;
-#pragma unroll
-    for (int k = 0; k < QPL; ++k) {
-      const double e[4] = {wq[k].x, wq[k].y, wq[k].z, wq[k].w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ww += e[i] * e[i];
-    }
-    ww = warp_sum(ww);
-    if (lane == 0) sums[WARPS * 4 + 3] = ww;
+  // U and var(lk) are wanted of an evaluation, of a launch's last step and of
+  // a kept step; in between only their finiteness is checked.
+  const bool want_u = a.mode == kValueGrad || j + 1 == a.steps || slot >= 0;
+  if (want_u && a.inv_p2 > 0.0f && warp == WARPS - 1) {
+    const double ww = warp_sum(lane_sum_squares<QPL>(wq));
+    if (lane == 0) sums[3] = ww;
   }
   const int g = lane >> (5 - LOG);           // my row in the link phase
   const bool leader = (lane & (GROUP - 1)) == 0;
@@ -478,23 +280,14 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
       consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, wq, xv, yv, og, A);
     }
   }
-  // Widen once: sum(lk) = s1 + n K, sum(lk^2) = s2 + 2 K s1 + n K^2.
-  const double K = A.K, n_l = A.cnt;
-  double my_mlk = static_cast<double>(A.mlk) + A.mlk_c;
-  double my_lk = static_cast<double>(A.s1) + n_l * K;
-  double my_lk2 = static_cast<double>(A.s2) + 2.0 * K * A.s1 + n_l * K * K;
-  my_mlk = warp_sum(my_mlk);
-  my_lk = warp_sum(my_lk);
-  my_lk2 = warp_sum(my_lk2);
+  if (leader) {
+    if (want_u) lsum[warp * RW + g] = lane_sums<QPL>(A);
+    else if (!isfinite(A.mlk)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+  }
 #pragma unroll
   for (int k = 0; k < QPL; ++k) {
     const int q = lane + 32 * k;
     if (q < dq) red[warp * dq + q] = A.acc[k];
-  }
-  if (lane == 0) {
-    sums[warp * 4 + 0] = my_mlk;
-    sums[warp * 4 + 1] = my_lk;
-    sums[warp * 4 + 2] = my_lk2;
   }
   __syncthreads();
 
@@ -510,27 +303,18 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
     }
     red[q] = t;
   }
-  if (tid == 0) {
-    double t0 = 0.0, t1 = 0.0, t2 = 0.0;
-    for (int w = 0; w < WARPS; ++w) {
-      t0 += sums[w * 4 + 0];
-      t1 += sums[w * 4 + 1];
-      t2 += sums[w * 4 + 2];
-    }
-    sums[WARPS * 4 + 0] = t0;
-    sums[WARPS * 4 + 1] = t1;
-    sums[WARPS * 4 + 2] = t2;
-  }
+  // The last warp alone carries the FP64 work (the sums here, U and var(lk)
+  // in the epilogue); the others go on with the gradient and the update.
+  const bool clerk = warp == WARPS - 1;
+  double tot[3] = {0.0, 0.0, 0.0};
+  if (clerk && want_u) reduce_lane_sums(lsum, WARPS * RW, lane, tot);
   __syncthreads();
 
   if (a.slices > 1) {
     const int64_t pc = static_cast<int64_t>(c) * a.slices + s;
     for (int q = tid; q < dq; q += (WARPS * 32)) a.ws_part[pc * dq + q] = red[q];
-    if (tid == 0) {
-      a.ws_sums[pc * 4 + 0] = sums[WARPS * 4 + 0];
-      a.ws_sums[pc * 4 + 1] = sums[WARPS * 4 + 1];
-      a.ws_sums[pc * 4 + 2] = sums[WARPS * 4 + 2];
-    }
+    if (clerk && lane < 3)
+      a.ws_sums[pc * 4 + lane] = lane == 0 ? tot[0] : (lane == 1 ? tot[1] : tot[2]);
     __threadfence();
     __syncthreads();
     if (tid == 0) {
@@ -554,39 +338,22 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
       }
       red[q] = t;
     }
-    if (tid == 0) {
+    if (clerk) {
       const double* ps = a.ws_sums + static_cast<int64_t>(c) * a.slices * 4;
-      double t0 = 0.0, t1 = 0.0, t2 = 0.0;
-      for (int k = 0; k < a.slices; ++k) {
-        t0 += __ldcg(ps + k * 4 + 0);
-        t1 += __ldcg(ps + k * 4 + 1);
-        t2 += __ldcg(ps + k * 4 + 2);
-      }
-      sums[WARPS * 4 + 0] = t0;
-      sums[WARPS * 4 + 1] = t1;
-      sums[WARPS * 4 + 2] = t2;
+      sum_slices(ps, a.slices, lane, tot);
     }
     __syncthreads();
   }
 
   // ------------------------------ epilogue ---------------------------------
-  const double sum_mlk = sums[WARPS * 4 + 0];
-  const double sum_lk = sums[WARPS * 4 + 1];
-  const double sum_lk2 = sums[WARPS * 4 + 2];
   float* wc = a.w + static_cast<int64_t>(c) * a.d;
-  const float scale = static_cast<float>(static_cast<double>(a.n_obs) / a.n);
-
-  const double ww = a.inv_p2 > 0.0f ? sums[WARPS * 4 + 3] : 0.0;
-  const double log_prior = -0.5 * ww * a.inv_p2 - a.prior_const;
-  // -N * mean(lk) without a mask, -N/n * (lk . mask) with one, as written in
-  // potential.py:183-185 (the unmasked form is exact for integer sums).
-  const double lik = a.mask == nullptr
-                         ? -static_cast<double>(a.n_obs) * (sum_mlk / a.n)
-                         : -(static_cast<double>(a.n_obs) / a.n) * sum_mlk;
-  const double U = (lik - log_prior) * a.inv_temp;
-  const double mean_lk = sum_lk / a.n;
-  const double var_lk = fmax(sum_lk2 / a.n - mean_lk * mean_lk, 0.0);
-  if (!isfinite(U)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+  const float scale = a.scale;
+  double U = 0.0, var_lk = 0.0;
+  if (want_u && clerk && lane == 0) {
+    U = glm_potential(a, tot[0], a.inv_p2 > 0.0f ? sums[3] : 0.0);
+    var_lk = glm_variance(a, tot[1], tot[2]);
+    if (!isfinite(U)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+  }
 
   const float* gl = reinterpret_cast<const float*>(red);
   if (a.mode == kValueGrad) {
@@ -595,7 +362,7 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
       for (int j = tid; j < a.d; j += (WARPS * 32))
         gc[j] = (-scale * gl[j] + wc[j] * a.inv_p2) * a.inv_temp;
     }
-    if (tid == 0) {
+    if (clerk && lane == 0) {
       a.U[c] = U;
       if (a.lk_var != nullptr) a.lk_var[c] = var_lk;
     }
@@ -647,7 +414,7 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
     if (multi) w_s[q] = make_float4(xn[0], xn[1], xn[2], xn[3]);
   }
   if (bad) raise_status(a.status, GBSGMC_ERR_NONFINITE);
-  if (tid == 0) {
+  if (want_u && clerk && lane == 0) {
     if (a.U != nullptr) a.U[c] = U;
     if (a.lk_var != nullptr) a.lk_var[c] = var_lk;
     if (slot >= 0 && a.sample_lik != nullptr)
@@ -734,7 +501,7 @@ __device__ __forceinline__ void dyn_epilogue(const GlmArgs& a, int c, int lane,
   ww = warp_sum(ww);
 
   float* wc = a.w + static_cast<int64_t>(c) * a.d;
-  const float scale = static_cast<float>(static_cast<double>(a.n_obs) / a.n);
+  const float scale = a.scale;
   const double log_prior = -0.5 * ww * a.inv_p2 - a.prior_const;
   const double lik = a.mask == nullptr
                          ? -static_cast<double>(a.n_obs) * (sum_mlk / a.n)
@@ -960,21 +727,6 @@ WsView ws_view(void* ws, int chains, int n, int d) {
   return v;
 }
 
-int sm_count() {
-  static int cached = 0;
-  if (cached == 0) {
-    int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) ==
-            cudaSuccess &&
-        n > 0)
-      cached = n;
-    else
-      cached = 152;
-  }
-  return cached;
-}
-
 // Rows a warp holds at once, and the CTAs per SM the register budget is set
 // for, per float4-column count QPL.  More rows per warp cut the per-row
 // instruction count (one transposed reduction and one link evaluation per
@@ -1007,8 +759,8 @@ int choose_slices(int chains, int n, int row_bytes) {
   if (forced > 0) return clamp_slices(forced, n);
   const double target = 384.0 * 1024.0;
   int s = static_cast<int>(std::ceil(static_cast<double>(n) * row_bytes / target));
-  if (static_cast<int64_t>(chains) * s < sm_count())
-    s = std::max(s, std::min(ceil_div(sm_count(), std::max(chains, 1)), n / 32));
+  if (static_cast<int64_t>(chains) * s < glm_sm_count())
+    s = std::max(s, std::min(ceil_div(glm_sm_count(), std::max(chains, 1)), n / 32));
   return clamp_slices(std::max(s, 1), n);
 }
 
@@ -1129,7 +881,7 @@ struct DynVariant {
     const int64_t need = (items + WARPS - 1) / WARPS;
     const int grid = static_cast<int>(
         std::max<int64_t>(1, std::min<int64_t>(need,
-                                               static_cast<int64_t>(sm_count()) *
+                                               static_cast<int64_t>(glm_sm_count()) *
                                                    occupancy(smem))));
     GlmArgs b = a;
     b.steps = 1;
@@ -1208,9 +960,21 @@ int launch_glm(GlmArgs& a, cudaStream_t st) {
   return launch_q<8>(a, L.total, st);
 }
 
-int fill_common(GlmArgs& a, const gbsgmc_glm* m, int chains, int n,
+struct TuneKey {
+  int chains, n, d;
+  int64_t ld;
+  bool operator<(const TuneKey& o) const {
+    return std::tie(chains, n, d, ld) < std::tie(o.chains, o.n, o.d, o.ld);
+  }
+};
+std::mutex g_tune_mutex;
+std::map<TuneKey, GlmTune> g_tune_cache;
+
+}  // namespace
+
+int glm_fill_args(GlmArgs& a, const gbsgmc_glm* m, int chains, int n,
                 const int32_t* idx, int64_t idx_stride, const float* mask,
-                void* ws, size_t ws_size, int* status, GlmTune tune = GlmTune{}) {
+                void* ws, size_t ws_size, int* status, GlmTune tune) {
   if (m == nullptr || m->X == nullptr || idx == nullptr ||
       (m->y == nullptr && !m->y_inline && m->family != GBSGMC_GLM_LINEAR))
     return set_error(GBSGMC_ERR_ARG, "glm: null model, data or index pointer");
@@ -1252,6 +1016,7 @@ int fill_common(GlmArgs& a, const gbsgmc_glm* m, int chains, int n,
     a.prior_const = 0.0;
   }
   a.inv_temp = 1.0f / m->temperature;
+  a.scale = n > 0 ? static_cast<float>(static_cast<double>(m->n_obs) / n) : 0.0f;
   a.chains = chains;
   a.n = n;
   a.slices = 0;
@@ -1291,18 +1056,6 @@ int fill_common(GlmArgs& a, const gbsgmc_glm* m, int chains, int n,
   return GBSGMC_OK;
 }
 
-struct TuneKey {
-  int chains, n, d;
-  int64_t ld;
-  bool operator<(const TuneKey& o) const {
-    return std::tie(chains, n, d, ld) < std::tie(o.chains, o.n, o.d, o.ld);
-  }
-};
-std::mutex g_tune_mutex;
-std::map<TuneKey, GlmTune> g_tune_cache;
-
-}  // namespace
-
 bool glm_tune_lookup(int chains, int n, int d, int64_t ld, GlmTune* out) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   auto it = g_tune_cache.find(TuneKey{chains, n, d, ld});
@@ -1314,6 +1067,14 @@ bool glm_tune_lookup(int chains, int n, int d, int64_t ld, GlmTune* out) {
 void glm_tune_store(int chains, int n, int d, int64_t ld, GlmTune t) {
   std::lock_guard<std::mutex> lock(g_tune_mutex);
   g_tune_cache[TuneKey{chains, n, d, ld}] = t;
+}
+
+int glm_qpl(int dq) { return qpl_for(dq); }
+int glm_rows_per_warp(int dq) {
+  const int qpl = qpl_for(dq);
+  const int forced = rows_override();
+  return qpl <= 2 && (forced == 2 || forced == 4 || forced == 8) ? forced
+                                                                 : default_rows_per_warp(qpl);
 }
 
 // Shared with the plan implementation.
@@ -1348,6 +1109,7 @@ int glm_prepare() {
   if (rc == GBSGMC_OK) rc = DynVariant<2, 8, 2, 8>::prepare();
   if (rc == GBSGMC_OK) rc = DynVariant<2, 4, 3, 8>::prepare();
   if (rc == GBSGMC_OK) rc = DynVariant<2, 2, 4, 8>::prepare();
+  if (rc == GBSGMC_OK) rc = glm_loop_prepare();
   return rc;
 }
 
@@ -1360,7 +1122,7 @@ int glm_sgld_step(const gbsgmc_glm* model, int chains, int n,
                   int* status_dev, cudaStream_t stream, GlmTune tune, int steps,
                   int64_t idx_step_stride, const int32_t* ident_dev) {
   GlmArgs a;
-  int rc = fill_common(a, model, chains, n, idx_dev, idx_stride, nullptr, ws,
+  int rc = glm_fill_args(a, model, chains, n, idx_dev, idx_stride, nullptr, ws,
                        ws_size, status_dev, tune);
   if (rc != GBSGMC_OK) return rc;
   if (w_dev == nullptr || sched == nullptr || noise == nullptr)
@@ -1411,8 +1173,8 @@ extern "C" int gbsgmc_glm_value_and_grad(
     void* workspace_dev, size_t workspace_bytes, int* status_dev,
     gbsgmc_stream_t stream) {
   GlmArgs a;
-  int rc = fill_common(a, model, chains, n, idx_dev, idx_stride, mask_dev,
-                       workspace_dev, workspace_bytes, status_dev);
+  int rc = glm_fill_args(a, model, chains, n, idx_dev, idx_stride, mask_dev,
+                       workspace_dev, workspace_bytes, status_dev, GlmTune{});
   if (rc != GBSGMC_OK) return rc;
   if (w_dev == nullptr || U_dev == nullptr)
     return set_error(GBSGMC_ERR_ARG, "glm_value_and_grad: null w or U");

@@ -21,7 +21,53 @@ struct GlmTune {
   int prefetch = 0;       // 1: two register tiles in flight per warp
   int dynamic = 0;        // 1: warps claim items of `slices` per chain
   int multistep = 0;      // 1: plans run a block of steps in one launch
+  int loop = 0;           // > 0: that launch is glm_loop with `loop` CTAs per chain
 };
+
+// glm_loop.cu: a block of integrator steps of all chains in one launch.
+enum GlmLoopKind {
+  kLoopSgld = 0,     // SGLD, with RMSprop when aux is given
+  kLoopObabo = 1,    // two minibatches per step
+  kLoopSghmc = 2,    // momentum resample every `leapfrog` steps
+  kLoopLeapfrog = 3, // AMAGOLD's reversible leapfrog: one trajectory
+  kLoopPairs = 4,    // reSGLD (normal, hot) pairs: rows p and pairs + p
+};
+struct GlmLoopCall {
+  const gbsgmc_glm* model = nullptr;
+  int kind = kLoopSgld, chains = 0, n = 0, steps = 0, leapfrog = 1;
+  int ctas = 1;            // CTAs per chain (glm_loop_ctas)
+  int rows_per_warp = 0;   // 0: the library's choice
+  const int32_t* idx = nullptr;          // step j, chain c: idx + j idx_step_stride
+  int64_t idx_stride = 0, idx_step_stride = 0;  //   + c idx_stride, [draws n]
+  float* x = nullptr;
+  float* aux = nullptr;    // RMSprop state (may be null) or momentum
+  float alpha = 0.9f, lmbd = 1e-5f, friction = 0.f;
+  const float* mass = nullptr;
+  const gbsgmc_sched* sched = nullptr;
+  const gbsgmc_noise* noise = nullptr;
+  double *U = nullptr, *lk_var = nullptr;  // of the last step
+  double* ke = nullptr;        // OBABO: kinetic energies [2, chains], added to
+  double* energy = nullptr;    // leapfrog: energies [chains], added to
+  float* samples = nullptr;    // kept steps (the schedule's keep slots)
+  double* sample_lik = nullptr;
+  // pairs
+  double F = 1.0;
+  uint64_t swap_seed = 0;
+  const int32_t* pair_chain = nullptr;
+  int32_t* ident = nullptr;
+  double* ssq = nullptr;
+  int64_t* k = nullptr;
+  int32_t* counts = nullptr;
+  int* status = nullptr;
+};
+int glm_loop_ctas(int units, int chains_per_unit, int n, int d);
+int glm_loop_prepare();
+int glm_loop(const GlmLoopCall& c, cudaStream_t st);
+// glm.cu: the float4 columns per lane and default rows per warp of a row of
+// dq float4, and the device's SM count.
+int glm_qpl(int dq);
+int glm_rows_per_warp(int dq);
+int glm_sm_count();
 
 size_t glm_ws_bytes(int chains, int n, int d);
 // Launch shapes chosen by the plan autotuner, per problem shape.

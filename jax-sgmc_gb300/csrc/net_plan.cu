@@ -55,6 +55,12 @@ struct NetPlan final : gbsgmc_plan {
   UpdateFusion fz;          // the mirror and squares of the new positions
   float pf = 0.f;           // 1 / (s^2 T) of the prior, 0 for a flat prior
   double* sq = nullptr;     // owned [chains, update_blocks]
+  // GLM families: a block's steps in one launch (glm_loop).
+  bool loop = false;
+  gbsgmc_glm glm{};
+  int ctas = 1;
+  float* samples = nullptr;      // kept steps (the schedule's keep slots)
+  double* sample_lik = nullptr;
 
   int draws() const { return integ.kind == GBSGMC_INTEGRATOR_OBABO ? 2 : 1; }
 
@@ -101,6 +107,7 @@ struct NetPlan final : gbsgmc_plan {
     // Every block: the index draw (unless external), the step counter and,
     // fused, the mirror.
     const int64_t fixed = (fused ? 3 : 2) - (isrc.external ? 1 : 0);
+    if (loop) return fixed + 1;
     switch (integ.kind) {
       case GBSGMC_INTEGRATOR_OBABO: return fixed + 2 + static_cast<int64_t>(g);
       case GBSGMC_INTEGRATOR_SGHMC:
@@ -124,6 +131,40 @@ struct NetPlan final : gbsgmc_plan {
                                rows, idx, per, cn, s);
     }
     if (rc != GBSGMC_OK) return rc;
+    if (loop) {
+      gbsgmc_sched s0 = sched;
+      s0.base_dev = base;
+      s0.offset = 0;
+      GlmLoopCall c;
+      c.model = &glm;
+      c.kind = integ.kind == GBSGMC_INTEGRATOR_OBABO   ? kLoopObabo
+               : integ.kind == GBSGMC_INTEGRATOR_SGHMC ? kLoopSghmc
+                                                       : kLoopSgld;
+      c.chains = chains;
+      c.n = n;
+      c.steps = g;
+      c.leapfrog = integ.kind == GBSGMC_INTEGRATOR_SGHMC ? integ.leapfrog_steps : 1;
+      c.ctas = ctas;
+      c.idx = idx;
+      c.idx_stride = per;
+      c.idx_step_stride = cn;
+      c.x = x;
+      c.aux = aux;
+      c.alpha = integ.alpha;
+      c.lmbd = integ.lmbd;
+      c.friction = integ.friction;
+      c.mass = integ.kind == GBSGMC_INTEGRATOR_SGLD ? nullptr : integ.mass_dev;
+      c.sched = &s0;
+      c.noise = &noise;
+      c.U = U;
+      c.lk_var = lk_var;
+      c.ke = ke;
+      c.samples = samples;
+      c.sample_lik = sample_lik;
+      c.status = status;
+      if ((rc = glm_loop(c, s))) return rc;
+      return plan_advance(this, g, s);
+    }
     if (integ.kind == GBSGMC_INTEGRATOR_OBABO) {
       if ((rc = enqueue_obabo(g, UpdateFusion{}, UpdateFusion{}, s))) return rc;
       return plan_advance(this, g, s);
@@ -749,16 +790,42 @@ extern "C" int gbsgmc_glm_plan_create(gbsgmc_plan** out, const gbsgmc_glm* model
                                       const gbsgmc_index_src* isrc, double* U_dev,
                                       double* lk_var_dev, double* ke_dev, int block_steps,
                                       int* status_dev) {
+  if (sched != nullptr && sched->keep_slot_dev != nullptr) {
+    if (out != nullptr) *out = nullptr;
+    return set_error(GBSGMC_ERR_UNSUPPORTED,
+                     "glm_plan_create: kept samples need gbsgmc_glm_plan_create_keep");
+  }
+  return gbsgmc_glm_plan_create_keep(out, model, chains, n, integ, x_dev, aux_dev, sched, noise,
+                                     isrc, U_dev, lk_var_dev, ke_dev, nullptr, nullptr,
+                                     block_steps, status_dev);
+}
+
+extern "C" int gbsgmc_glm_plan_create_keep(
+    gbsgmc_plan** out, const gbsgmc_glm* model, int chains, int n,
+    const gbsgmc_integrator* integ, float* x_dev, float* aux_dev, const gbsgmc_sched* sched,
+    const gbsgmc_noise* noise, const gbsgmc_index_src* isrc, double* U_dev, double* lk_var_dev,
+    double* ke_dev, float* samples_dev, double* sample_lik_dev, int block_steps,
+    int* status_dev) {
   if (out == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: null plan");
   *out = nullptr;
-  int rc = check_common(integ, chains, n, x_dev, aux_dev, sched, noise, isrc, U_dev,
-                        block_steps, status_dev);
+  gbsgmc_sched plain = {};
+  if (sched != nullptr) {
+    if (sched->keep_slot_dev != nullptr && samples_dev == nullptr)
+      return set_error(GBSGMC_ERR_ARG,
+                       "glm_plan_create: keep table given without sample buffer");
+    plain = *sched;
+    plain.keep_slot_dev = nullptr;  // taken inside the block's launch
+  }
+  int rc = check_common(integ, chains, n, x_dev, aux_dev, sched != nullptr ? &plain : nullptr,
+                        noise, isrc, U_dev, block_steps, status_dev);
   if (rc != GBSGMC_OK) return rc;
   if (model == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: null model");
-  const size_t ws = gbsgmc_glm_workspace_bytes(chains, n, model->d);
-  if (ws == 0) return set_error(GBSGMC_ERR_SHAPE, "glm_plan_create: bad shape");
+  if (gbsgmc_glm_workspace_bytes(chains, n, model->d) == 0)
+    return set_error(GBSGMC_ERR_SHAPE, "glm_plan_create: bad shape");
   NetPlan* p = new (std::nothrow) NetPlan();
   if (p == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: out of memory");
+  p->loop = true;
+  p->glm = *model;
   p->chains = chains;
   p->n = n;
   p->P = model->d;
@@ -772,30 +839,16 @@ extern "C" int gbsgmc_glm_plan_create(gbsgmc_plan** out, const gbsgmc_glm* model
   p->U = U_dev;
   p->lk_var = lk_var_dev;
   p->ke = ke_dev;
+  p->samples = samples_dev;
+  p->sample_lik = sample_lik_dev;
   p->status = status_dev;
-  p->ws_size = ws;
   do {
     if ((rc = plan_init(p, block_steps))) break;
     const size_t ibytes = sizeof(int32_t) * static_cast<size_t>(block_steps) * chains *
                           p->draws() * n;
-    if ((rc = p->alloc_grads("glm_plan_create: gradient"))) break;
-    if ((rc = plan_alloc(p, &p->U2, sizeof(double) * chains, "glm_plan_create: U")))
-      break;
     if ((rc = plan_alloc(p, &p->idx, ibytes, "glm_plan_create: index buffer"))) break;
-    if ((rc = plan_alloc(p, &p->ws, ws, "glm_plan_create: workspace"))) break;
-    // The GLM workspace's tickets start at zero and are left at zero.
-    if ((rc = cuda_err(cudaMemsetAsync(p->ws, 0, ws, p->stream), "glm_plan_create: memset")))
-      break;
     if ((rc = glm_prepare())) break;
-    const gbsgmc_glm m = *model;
-    void* wsp = p->ws;
-    const float* x = x_dev;
-    p->grad_fn = [m, chains, n, x, wsp, ws, status_dev](
-                     const int32_t* idx, int64_t stride, double* U, double* var, float* grad,
-                     cudaStream_t s) {
-      return gbsgmc_glm_value_and_grad(&m, chains, n, idx, stride, nullptr, x, U, grad,
-                                       nullptr, var, wsp, ws, status_dev, s);
-    };
+    p->ctas = glm_loop_ctas(chains, 1, n, model->d);
     if ((rc = p->setup_external("glm_plan_create: index memset"))) break;
     rc = plan_capture(p);
   } while (false);

@@ -286,6 +286,32 @@ int GlmPlan::steps_launch(int g, int32_t* buf, cudaStream_t s) {
   gbsgmc_sched s0 = sched;
   s0.base_dev = base;
   s0.offset = 0;
+  if (tune.loop > 0) {
+    GlmLoopCall c;
+    c.model = &model;
+    c.chains = chains;
+    c.n = n;
+    c.steps = g;
+    c.ctas = tune.loop;
+    c.rows_per_warp = tune.rows_per_warp;
+    c.idx = buf;
+    c.idx_stride = n;
+    c.idx_step_stride = cn;
+    c.x = w;
+    c.aux = v;
+    c.alpha = alpha;
+    c.lmbd = lmbd;
+    c.sched = &s0;
+    c.noise = &noise;
+    c.U = U;
+    c.lk_var = lk_var;
+    c.samples = samples;
+    c.sample_lik = sample_lik;
+    c.status = status;
+    const int rc = glm_loop(c, s);
+    if (rc != GBSGMC_OK) return rc;
+    return plan_advance(this, g, s);
+  }
   const int rc = glm_sgld_step(&model, chains, n, buf, n, w, v, alpha, lmbd, &s0,
                                &noise, U, lk_var, samples, sample_lik, ws,
                                ws_size, status, s, tune, g, cn);
@@ -413,6 +439,17 @@ int autotune(GlmPlan* p) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = GBSGMC_OK;
   std::vector<GlmTune> cands;
+  // With no more chains than half the SMs, blocks run as one glm_loop launch
+  // with a cluster per chain: every other form leaves SMs idle or pays a
+  // launch per step (one chain, n = 128, d = 32: 10.9 us a step against 4.0;
+  // 24 chains, n = 500, d = 101: 18.8 us a gradient against 8.2).
+  const int ctas = glm_loop_ctas(C, 1, n, d);
+  const GlmTune loop{ctas, glm_rows_per_warp((d + 3) / 4), 8, 0, 0, 1, ctas};
+  if (2 * C <= glm_sm_count()) {
+    p->tune = loop;
+    glm_tune_store(C, n, d, p->model.ld, loop);
+    return GBSGMC_OK;
+  }
   {
     const double rows_per_cta = (384.0 * 1024.0) / (4.0 * std::max<int64_t>(p->model.ld, 1));
     const int base = std::max(1, static_cast<int>(std::ceil(n / rows_per_cta)));
@@ -448,6 +485,7 @@ int autotune(GlmPlan* p) {
         cands.push_back(t);
       }
     }
+    if (p->G >= 6) cands.push_back(loop);
   }
   if (cands.size() <= 1) {
     if (!cands.empty()) p->tune = cands[0];
@@ -484,7 +522,25 @@ int autotune(GlmPlan* p) {
     const char* vb = std::getenv("GBSGMC_AUTOTUNE_VERBOSE");
     const bool verbose = vb != nullptr && vb[0] == '1';
     for (const GlmTune& t : cands) {
-      if (t.multistep) {
+      if (t.loop > 0) {
+        // A warm-up block, then six steps in one launch.
+        const GlmTune keep = p->tune;
+        p->tune = t;
+        float* const w0 = p->w;
+        float* const v0 = p->v;
+        const gbsgmc_sched s0 = p->sched;
+        p->w = w;
+        p->v = v0 != nullptr ? v : nullptr;
+        p->sched.keep_slot_dev = nullptr;
+        rc = p->steps_launch(6, p->idx, p->stream);
+        cudaEventRecord(e0, p->stream);
+        if (rc == GBSGMC_OK) rc = p->steps_launch(6, p->idx, p->stream);
+        p->tune = keep;
+        p->w = w0;
+        p->v = v0;
+        p->sched = s0;
+        if (rc == GBSGMC_OK) rc = plan_advance(p, -12, p->stream);
+      } else if (t.multistep) {
         // Two warm-up steps, then six steps in one launch.
         for (int rep = 0; rep < 2 && rc == GBSGMC_OK; ++rep)
           rc = glm_sgld_step(&p->model, C, n, p->idx, n, w,
@@ -601,7 +657,10 @@ extern "C" int gbsgmc_sgld_glm_plan_create(
     // GBSGMC_GLM_MULTISTEP=1/0 forces one launch per block of steps or one
     // launch per step, whatever the autotuner chose.
     if (const char* ms = std::getenv("GBSGMC_GLM_MULTISTEP"))
-      if (ms[0] == '0' || ms[0] == '1') p->tune.multistep = ms[0] == '1';
+      if (ms[0] == '0' || ms[0] == '1') {
+        p->tune.multistep = ms[0] == '1';
+        p->tune.loop = 0;
+      }
     if ((rc = plan_capture(p))) break;
     // GBSGMC_PLAN_PIPELINE=1 overlaps the next block's index draws with this
     // block's launch when the block is one launch and the draws carry state
@@ -628,7 +687,8 @@ namespace {
 // the pairs' exchange on the device.  The chains' index streams and noise
 // belong to chain identities that travel with exchanged states: identity i
 // draws its own indices (buffer [G, 2P, n] by identity) and its own noise
-// (chain id chain_base + i), and slot s runs identity ident[s].
+// (chain id chain_base + i), and slot s runs identity ident[s].  A block of
+// steps is one glm_loop launch, a cluster per pair.
 struct GlmPairsPlan final : gbsgmc_plan {
   gbsgmc_glm model;
   int pairs = 0, n = 0;
@@ -646,17 +706,15 @@ struct GlmPairsPlan final : gbsgmc_plan {
   float* samples = nullptr;
   double* sample_lik = nullptr;
   int* status = nullptr;
-  gbsgmc::GlmTune tune;
-  void* ws = nullptr;
-  size_t ws_size = 0;
+  int ctas = 1;  // CTAs per chain
   int32_t* idx = nullptr;
 
   ~GlmPairsPlan() override {
     if (stream != nullptr) cudaStreamSynchronize(stream);
-    gbsgmc::plan_free(this, ws);
     gbsgmc::plan_free(this, idx);
   }
-  int64_t launches_per_block(int g) const override { return 2 + 2 * static_cast<int64_t>(g); }
+  // The index draw, the block's steps, the step counter.
+  int64_t launches_per_block(int) const override { return 3; }
   int enqueue(int g, cudaStream_t s) override {
     using namespace gbsgmc;
     const int chains = 2 * pairs;
@@ -665,21 +723,38 @@ struct GlmPairsPlan final : gbsgmc_plan {
     int rc = gbsgmc_index_draw_pcg64(isrc.pcg_dev, chains, rows, static_cast<int64_t>(g) * n,
                                      n, idx, n, cn, status, s);
     if (rc != GBSGMC_OK) return rc;
-    for (int j = 0; j < g; ++j) {
-      gbsgmc_sched sj = sched;
-      sj.base_dev = base;
-      sj.offset = j;
-      gbsgmc_sched step_sched = sj;
-      step_sched.keep_slot_dev = nullptr;  // the exchange stores the samples
-      rc = glm_sgld_step(&model, chains, n, idx + j * cn, n, w, v, alpha, lmbd, &step_sched,
-                         &noise, U, lk_var, nullptr, nullptr, ws, ws_size, status, s, tune,
-                         1, 0, ident);
-      if (rc != GBSGMC_OK) return rc;
-      rc = resgld_pairs_exchange(pairs, model.d, w, v, U, lk_var, ident, &sj, temp.F,
-                                 temp.seed, pair_chain, temp.ssq_dev, temp.k_dev,
-                                 temp.counts_dev, samples, sample_lik, s);
-      if (rc != GBSGMC_OK) return rc;
-    }
+    gbsgmc_sched s0 = sched;
+    s0.base_dev = base;
+    s0.offset = 0;
+    GlmLoopCall c;
+    c.model = &model;
+    c.kind = kLoopPairs;
+    c.chains = chains;
+    c.n = n;
+    c.steps = g;
+    c.ctas = ctas;
+    c.idx = idx;
+    c.idx_stride = n;
+    c.idx_step_stride = cn;
+    c.x = w;
+    c.aux = v;
+    c.alpha = alpha;
+    c.lmbd = lmbd;
+    c.sched = &s0;
+    c.noise = &noise;
+    c.U = U;
+    c.lk_var = lk_var;
+    c.samples = samples;
+    c.sample_lik = sample_lik;
+    c.F = temp.F;
+    c.swap_seed = temp.seed;
+    c.pair_chain = pair_chain;
+    c.ident = ident;
+    c.ssq = temp.ssq_dev;
+    c.k = temp.k_dev;
+    c.counts = temp.counts_dev;
+    c.status = status;
+    if ((rc = glm_loop(c, s))) return rc;
     return plan_advance(this, g, s);
   }
 };
@@ -738,17 +813,12 @@ extern "C" int gbsgmc_glm_resgld_plan_create(
   do {
     if ((rc = plan_init(p, block_steps))) break;
     const int chains = 2 * pairs;
-    p->ws_size = glm_ws_bytes(chains, n, model->d);
-    if ((rc = plan_alloc(p, &p->ws, p->ws_size, "glm_resgld_plan_create: workspace"))) break;
     if ((rc = plan_alloc(p, &p->idx,
                          sizeof(int32_t) * static_cast<size_t>(block_steps) * chains * n,
                          "glm_resgld_plan_create: index buffer")))
       break;
     if ((rc = glm_prepare())) break;
-    // One launch per step (the exchange sits between steps): the cached
-    // launch shape of this problem, or the library's default.
-    glm_tune_lookup(chains, n, model->d, model->ld, &p->tune);
-    p->tune.multistep = 0;
+    p->ctas = glm_loop_ctas(pairs, 2, n, model->d);
     rc = plan_capture(p);
   } while (false);
   if (rc != GBSGMC_OK) {

@@ -403,16 +403,6 @@ __global__ void sghmc_momentum_kernel(int chains, int64_t P, const float* x, flo
   }
 }
 
-// Uniform in (0, 1) with 53 random bits from Philox (seed, counter (pair,
-// step, 0, GBSGMC_TAG_SWAP)).
-__device__ __forceinline__ double swap_uniform(uint64_t seed, uint32_t pair, uint32_t step) {
-  const U32x4 r = philox4x32_10(U32x4{pair, step, 0u, GBSGMC_TAG_SWAP},
-                                static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
-  const uint64_t bits = ((static_cast<uint64_t>(r.x) >> 5) << 26) |
-                        (static_cast<uint64_t>(r.y) >> 6);
-  return (static_cast<double>(bits) + 0.5) * (1.0 / 9007199254740992.0);
-}
-
 __global__ void resgld_swap_kernel(int pairs, const double* Un,
                                    const double* Uh, const double* var_n,
                                    const double* Tn, const double* Th,

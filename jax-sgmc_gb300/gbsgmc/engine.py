@@ -251,7 +251,8 @@ class NetPlan:
   def __init__(self, potential, dataset, X, AUX, n, kind, h_tab, t_tab,
                index_src, noise_seed, chain_base=0, block_steps=None,
                friction=0.0, leapfrog_steps=1, alpha=0.9, lmbd=1e-5,
-               mass=None, observation_count=None, feed=None):
+               mass=None, observation_count=None, feed=None, keep_tab=None,
+               n_kept=0):
     import torch
     C, P = X.shape
     self.C, self.P, self.n, self.kind = C, P, n, kind
@@ -261,9 +262,17 @@ class NetPlan:
     self.lk_var = torch.zeros(C, dtype=torch.float64, device="cuda")
     self.ke = torch.zeros(2 * C, dtype=torch.float64, device="cuda")
     self.status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    self.h_tab, self.t_tab = h_tab, t_tab
+    self.h_tab, self.t_tab, self.keep_tab = h_tab, t_tab, keep_tab
     self.index_src = index_src
-    self.sched = _lib.sched(step_size_dev=h_tab, temperature_dev=t_tab)
+    # Kept steps, taken inside the block's launch (GLM families only).
+    self.samples = self.sample_lik = None
+    if keep_tab is not None:
+      self.samples = torch.empty((max(int(n_kept), 1), C, P), dtype=torch.float32,
+                                 device="cuda")
+      self.sample_lik = torch.empty((max(int(n_kept), 1), C), dtype=torch.float64,
+                                    device="cuda")
+    self.sched = _lib.sched(step_size_dev=h_tab, temperature_dev=t_tab,
+                            keep_slot_dev=keep_tab)
     self.noise = _lib.noise(noise_seed, chain_base)
     lf = int(leapfrog_steps) if kind == "sghmc" else 1
     if block_steps is None:
@@ -277,14 +286,16 @@ class NetPlan:
     handle = _lib.C.c_void_p()
     # Kernel launches of one value-and-gradient call.
     self.launches_per_gradient = 30 if potential.is_cnn else \
-        10 if potential.is_mlp else 1
+        10 if potential.is_mlp else 0
     create = "gbsgmc_cnn_plan_create" if potential.is_cnn else \
         "gbsgmc_mlp_plan_create" if potential.is_mlp else \
-        "gbsgmc_glm_plan_create"
+        "gbsgmc_glm_plan_create_keep"
+    keep = () if potential.is_network else (_lib.ptr(self.samples),
+                                            _lib.ptr(self.sample_lik))
     _lib.call(create, _lib.C.byref(handle), self.model, C, n,
               self.integ, _lib.ptr(X), _lib.ptr(AUX), self.sched, self.noise,
               index_src.struct, _lib.ptr(self.U), _lib.ptr(self.lk_var),
-              _lib.ptr(self.ke), int(block_steps), _lib.ptr(self.status))
+              _lib.ptr(self.ke), *keep, int(block_steps), _lib.ptr(self.status))
     self.handle = handle
 
   def run(self, first_step, steps):
@@ -461,17 +472,28 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
   # One solver iteration is `steps` integrator steps with the same schedule.
   h_tab = torch.from_numpy(np.repeat(np.asarray(h, np.float32), steps)).cuda()
   t_tab = torch.from_numpy(np.repeat(np.asarray(t, np.float32), steps)).cuda()
+  C, P = len(states), X.shape[1]
+  kind_saving = saving.kind if saving is not None else "device"
+  # GLM chains keep their samples inside the blocks' launches, unless these
+  # go elsewhere during the run (moments, or a ring emptied to the host).
+  inside = not pot.is_network and kind_saving != "moments" and \
+      4 * C * P * max(n_kept, 1) <= RING_BYTES
+  if inside:
+    last = np.full(iterations * steps, -1, np.int32)
+    last[steps - 1::steps] = keep   # an iteration's state is its last step's
+    kw.update(keep_tab=torch.from_numpy(last).cuda(), n_kept=n_kept)
   plan = NetPlan(pot, dataset, X, AUX, rbf.mb_size, kind, h_tab, t_tab,
                  index_src, states[0].key, chain_ids[0], feed=feed, **kw)
-  C, P = len(states), X.shape[1]
-  extra = torch.empty((max(n_kept, 1), C), dtype=torch.float64, device="cuda")
+  extra = None if inside else \
+      torch.empty((max(n_kept, 1), C), dtype=torch.float64, device="cuda")
   # Kept samples: all on the device (device saving), streamed into FP64
   # moments (moments saving), or through a ring of device rows that a
   # SampleDrain empties to the host while the chains run (host saving).
   mom = drain = None
-  kind_saving = saving.kind if saving is not None else "device"
   ring = max(n_kept, 1)
-  if kind_saving == "moments":
+  if inside:
+    samples, extra = plan.samples, plan.sample_lik
+  elif kind_saving == "moments":
     mom = io.DeviceMoments(C, P)
     samples = None
   else:
@@ -485,7 +507,7 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
   try:
     done = 0
     try:
-      for k in np.nonzero(np.asarray(keep) >= 0)[0]:
+      for k in (() if inside else np.nonzero(np.asarray(keep) >= 0)[0]):
         plan.run(done * steps, (k + 1 - done) * steps)
         done = k + 1
         slot = int(keep[k])

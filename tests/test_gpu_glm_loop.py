@@ -1,0 +1,163 @@
+"""Blocks of integrator steps on the GLM potentials in one launch
+(glm_loop.cu) at the edges of its row tiles, chunks and clusters, against the
+oracle's trajectories on the same indices and Philox normals.
+
+Shapes: one feature (rows of 4 bytes: 4-byte copies), feature counts around
+the 128-column lanes and the 1,024 limit, minibatches below, at and above
+whole tiles of 32 rows and longer than the shared-memory ring, one chain (a
+cluster of up to eight CTAs), and more chains than SMs (one CTA each).
+
+Tolerance (as for the other K-step trajectories): 1e-4 relative plus 1e-5
+absolute; U within 1e-5 relative plus 1e-3 absolute.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import sgmc_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# (chains, n, d, family)
+SHAPES = [
+    (1, 1, 1, O.LINEAR_GAUSSIAN),
+    (1, 31, 7, O.LOGISTIC),
+    (2, 33, 33, O.LINEAR_GAUSSIAN),
+    (1, 257, 128, O.LOGISTIC),
+    (3, 500, 129, O.LOGISTIC),
+    (1, 6000, 40, O.LOGISTIC),
+    (2, 1100, 257, O.LOGISTIC),
+    (1, 300, 1021, O.LINEAR_GAUSSIAN),
+    (170, 65, 5, O.LOGISTIC),
+]
+K = 6
+
+
+def _cuda(a):
+  import torch
+  return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _words(C):
+  from gbsgmc.data.numpy_loader import pcg64_words
+  return np.array([pcg64_words(c) for c in range(C)], np.uint64).view(np.int64)
+
+
+def _setup(C, n, d, family):
+  from gbsgmc import data, likelihoods as L, potential
+  N = 7001
+  rng = np.random.default_rng(100 * d + n)
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  w = rng.normal(size=d) / np.sqrt(d)
+  if family == O.LOGISTIC:
+    y = (rng.random(N) < 1 / (1 + np.exp(-(X @ w)))).astype(np.float32)
+    lik = L.Logistic()
+  else:
+    y = (X @ w + 0.5 * rng.normal(size=N)).astype(np.float32)
+    lik = L.LinearGaussian(sigma=0.5)
+  loader = data.NumpyDataLoader(x=X, y=y)
+  pot = potential.minibatch_potential(L.GaussianPrior(3.0), lik)
+  x0 = (0.1 * rng.normal(size=(C, d))).astype(np.float32)
+  return X, y, loader.device_dataset(), pot, x0, N
+
+
+def _potential(X, y, w, idx, N, family):
+  return O.glm_potential(w, X, y, idx, N, family, 0.5, 3.0)
+
+
+@pytest.mark.parametrize("C,n,d,family", SHAPES)
+@pytest.mark.parametrize("kind", ["langevin", "obabo", "sghmc"])
+def test_block_matches_oracle(lib, kind, C, n, d, family):
+  import torch
+  from gbsgmc import engine
+  X, y, ds, pot, x0, N = _setup(C, n, d, family)
+  curvature = N * (4.0 if family == O.LINEAR_GAUSSIAN else 0.25) * \
+      max(1.0, 2.0 * d / n)   # of a minibatch, at most about (1 + sqrt(d/n))^2
+  h0 = 0.02 / curvature if kind == "langevin" else 0.02 / np.sqrt(curvature)
+  h = (h0 * 0.9 ** np.arange(K)).astype(np.float32)
+  T = np.ones(K, np.float32)
+  keep = np.array([-1, 0, -1, 1, -1, 2], np.int32)
+  draws = 2 if kind == "obabo" else 1
+  pcg = _cuda(_words(C))
+  x, aux = _cuda(x0), None if kind == "langevin" else _cuda(np.zeros_like(x0))
+  kw = {} if kind == "langevin" else dict(friction=2.0, leapfrog_steps=3)
+  plan = engine.NetPlan(pot, ds, x, aux, n, kind, _cuda(h), _cuda(T),
+                        engine.IndexSource(pcg=pcg), 11, block_steps=3,
+                        keep_tab=_cuda(keep), n_kept=3, **kw)
+  plan.run(0, K)
+  plan.check_status()
+  idx = np.stack([O.loader_draws(O.loader_rng(c), N, n, K * draws)
+                  for c in range(C)], 1)
+  xi = lambda tag, k: np.stack([O.philox_normals(11, c, k, tag, d)  # noqa: E731
+                                for c in range(C)]).astype(np.float32)
+  w, p, kept, lik = x0.copy(), np.zeros_like(x0), [], []
+  for k in range(K):
+    if kind == "langevin":
+      r = _potential(X, y, w, idx[k], N, family)
+      w, _ = O.sgld_step(w, r.grad.astype(np.float32), None, xi(0, k), h[k], 1.0,
+                         rms_prop=False)
+      U = -r.U
+    elif kind == "obabo":
+      a = _potential(X, y, w, idx[2 * k], N, family)
+      w, p, _ = O.obabo_first(w, p, a.grad.astype(np.float32), xi(1, k), h[k], 1.0, 2.0)
+      b = _potential(X, y, w, idx[2 * k + 1], N, family)
+      p, _ = O.obabo_second(p, b.grad.astype(np.float32), xi(2, k), h[k], 1.0, 2.0)
+      U = 0.5 * (a.U + b.U)
+    else:
+      if k % 3 == 0:
+        p = O.sghmc_resample(xi(3, k))
+      w, p = O.sghmc_position(w, p, h[k], 2.0)
+      r = _potential(X, y, w, idx[k], N, family)
+      p = O.sghmc_momentum(p, r.grad.astype(np.float32), xi(4, k), h[k], 2.0)
+      U = r.U
+    if keep[k] >= 0:
+      kept.append(w)
+      lik.append(U)
+  tol = dict(rtol=1e-4, atol=1e-5)
+  np.testing.assert_allclose(x.cpu().numpy(), w, **tol)
+  np.testing.assert_allclose(plan.samples.cpu().numpy(), np.stack(kept), **tol)
+  np.testing.assert_allclose(plan.sample_lik.cpu().numpy(), np.stack(lik), rtol=1e-5,
+                             atol=1e-3)
+  sign = -1.0 if kind == "langevin" else 1.0
+  np.testing.assert_allclose(plan.U.cpu().numpy(), sign * lik[-1], rtol=1e-5, atol=1e-3)
+  if kind != "langevin":
+    scale = np.abs(p).max()
+    np.testing.assert_allclose(aux.cpu().numpy(), p, rtol=1e-4, atol=1e-4 * scale)
+  # The streams stand where numpy's would.
+  for c in range(min(C, 3)):
+    rng = O.loader_rng(c)
+    O.loader_draws(rng, N, n, K * draws)
+    s = rng.bit_generator.state["state"]["state"]
+    got = pcg[c].cpu().numpy().view(np.uint64)
+    assert (int(got[0]) << 64) | int(got[1]) == s
+  assert torch.isfinite(plan.lk_var).all()
+
+
+@pytest.mark.parametrize("pairs,n,d", [(1, 33, 7), (2, 256, 64), (1, 900, 300), (90, 40, 12)])
+def test_pairs_match_the_per_pair_path(lib, pairs, n, d):
+  """alias.re_sgld through the block launches against one chain at a time
+  (other launch shapes, so other summation orders: 1e-4 relative)."""
+  from gbsgmc import alias, data, engine, likelihoods as L, potential
+  rng = np.random.default_rng(d)
+  N = 4000
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (X @ rng.normal(size=d) / np.sqrt(d) + 0.5 * rng.normal(size=N)).astype(np.float32)
+  pot = potential.minibatch_potential(L.GaussianPrior(10.0), L.LinearGaussian(sigma=0.5))
+  inits = [({"w": (0.1 * rng.normal(size=d)).astype(np.float32)},
+            {"w": (0.1 * rng.normal(size=d)).astype(np.float32)}) for _ in range(pairs)]
+  first = 0.05 / (4 * N * max(1.0, 2.0 * d / n))
+  outs = []
+  for fused in (True, False):
+    run = alias.re_sgld(pot, data.NumpyDataLoader(x=X, y=y), cache_size=7, batch_size=n,
+                        temperature=50.0, first_step_size=first,
+                        last_step_size=0.5 * first, burn_in=6, accepted_samples=6)
+    engine.FUSED_ENABLED = fused
+    try:
+      outs.append(run(*(inits if fused else inits[:2]), iterations=12))
+    finally:
+      engine.FUSED_ENABLED = True
+  for a, b in zip(*outs):
+    np.testing.assert_allclose(a["samples"]["variables"]["w"], b["samples"]["variables"]["w"],
+                               rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(a["samples"]["likelihood"], b["samples"]["likelihood"],
+                               rtol=1e-5, atol=1e-3)
