@@ -264,11 +264,11 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
     load_tile<QPL, RW>(a, idx_s, R, r0, lane, g, xa, ya, oa);
     while (r0 < R) {
       load_tile<QPL, RW>(a, idx_s, R, r0 + kStride, lane, g, xb, yb, ob);
-      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, wq, xa, ya, oa, A);
+      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, want_u, wq, xa, ya, oa, A);
       r0 += kStride;
       if (r0 >= R) break;
       load_tile<QPL, RW>(a, idx_s, R, r0 + kStride, lane, g, xa, ya, oa);
-      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, wq, xb, yb, ob, A);
+      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, want_u, wq, xb, yb, ob, A);
       r0 += kStride;
     }
   } else {
@@ -277,7 +277,7 @@ __device__ __forceinline__ void glm_step(const GlmArgs& a, int j, unsigned char*
       float yv;
       int og;
       load_tile<QPL, RW>(a, idx_s, R, r0, lane, g, xv, yv, og);
-      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, wq, xv, yv, og, A);
+      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, want_u, wq, xv, yv, og, A);
     }
   }
   if (leader) {
@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(WARPS * 32, MINB)
       float yv;
       int og;
       load_tile<QPL, RW>(a, idx_s, R, r0, lane, g, xv, yv, og);
-      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, wq, xv, yv, og, A);
+      consume_tile<QPL, RW>(a, m_s, lk_out, r0, lane, g, leader, true, wq, xv, yv, og, A);
     }
     const double K = A.K, n_l = A.cnt;
     const double my_mlk = warp_sum(static_cast<double>(A.mlk) + A.mlk_c);

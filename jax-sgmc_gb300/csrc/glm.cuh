@@ -74,11 +74,12 @@ __device__ __forceinline__ int ident_of(const GlmArgs& a, int c) {
 // Bernoulli-logit log-likelihood y z - softplus(z) and its derivative
 // y - sigmoid(z), from one exponential: e = exp(-|z|),
 // softplus(z) = max(z, 0) + log1p(e), sigmoid(z) = 1/(1+e) or e/(1+e).
-__device__ __forceinline__ void logistic_link(float z, float y, float& lk,
+// Without `want` lk is only a number that is finite where the likelihood is.
+__device__ __forceinline__ void logistic_link(float z, float y, bool want, float& lk,
                                               float& dz) {
   const float e = expf(-fabsf(z));
   const float r = 1.0f / (1.0f + e);
-  lk = y * z - (fmaxf(z, 0.0f) + log1pf(e));
+  lk = want ? y * z - (fmaxf(z, 0.0f) + log1pf(e)) : z * 1e-6f;
   dz = y - (z >= 0.0f ? r : e * r);
 }
 
@@ -118,6 +119,8 @@ template <>
 struct Log2<4> { static constexpr int v = 2; };
 template <>
 struct Log2<8> { static constexpr int v = 3; };
+template <>
+struct Log2<16> { static constexpr int v = 4; };
 
 // Sum of p[r] over the 32 lanes for RW rows at once.  Returns, in every lane
 // of group g = lane >> (5 - log2 RW), the full sum of row g.
@@ -172,10 +175,14 @@ __device__ __forceinline__ void neumaier_add(float& sum, float& comp, float x) {
 }
 
 // Likelihood, adjoint and accumulation for a loaded tile (see load_tile).
+// Without `want` (no U or var(lk) asked of this gradient) only what the
+// adjoint needs is computed, and A.mlk turns non-finite where a likelihood
+// would: about a third of the logistic link is its log1p and the
+// compensated sums.
 template <int QPL, int RW>
 __device__ __forceinline__ void consume_tile(const GlmArgs& a, const float* m_s,
                                              float* lk_out, int r0, int lane,
-                                             int g, bool leader,
+                                             int g, bool leader, bool want,
                                              const float4 (&wq)[QPL],
                                              const float4 (&xv)[RW][QPL],
                                              float yv, int og, Accum<QPL>& A) {
@@ -199,7 +206,7 @@ __device__ __forceinline__ void consume_tile(const GlmArgs& a, const float* m_s,
   const float mw = (ok && a.mask != nullptr) ? m_s[row] : 1.0f;
   float lkv, dz;
   if (a.family == GBSGMC_GLM_LOGISTIC) {
-    logistic_link(z, yv, lkv, dz);
+    logistic_link(z, yv, want, lkv, dz);
   } else if (a.family == GBSGMC_GLM_LINEAR) {
     lkv = z;
     dz = 1.0f;
@@ -210,13 +217,17 @@ __device__ __forceinline__ void consume_tile(const GlmArgs& a, const float* m_s,
   }
   const float coef = ok ? mw * dz : 0.0f;
   if (ok && leader) {
-    neumaier_add(A.mlk, A.mlk_c, mw * lkv);
-    if (A.cnt == 0) A.K = lkv;
-    const float dk = lkv - A.K;
-    A.s1 += dk;
-    A.s2 = fmaf(dk, dk, A.s2);
-    A.cnt += 1;
-    if (lk_out != nullptr) lk_out[row] = lkv;
+    if (want) {
+      neumaier_add(A.mlk, A.mlk_c, mw * lkv);
+      if (A.cnt == 0) A.K = lkv;
+      const float dk = lkv - A.K;
+      A.s1 += dk;
+      A.s2 = fmaf(dk, dk, A.s2);
+      A.cnt += 1;
+      if (lk_out != nullptr) lk_out[row] = lkv;
+    } else {
+      A.mlk += mw * lkv;
+    }
   }
 #pragma unroll
   for (int r = 0; r < RW; ++r) {
@@ -243,13 +254,65 @@ __device__ __forceinline__ LaneSums lane_sums(const Accum<QPL>& A) {
   return LaneSums{A.mlk, A.mlk_c, A.K, A.s1, A.s2, A.cnt};
 }
 
-// FP64 totals of `count` lanes' sums by one warp: t[0] = sum m lk, t[1] =
-// sum lk, t[2] = sum lk^2 (every lane gets them).  The widening restores
-// sum(lk) = s1 + n K and sum(lk^2) = s2 + 2 K s1 + n K^2.  FP64 runs at a
-// small fraction of the FP32 rate here, so it is done once per CTA, by one
-// warp, for the few lanes that hold sums, instead of by every warp.
+// An unevaluated sum of two floats, hi + lo (48 bits or more): exact sums and
+// products by the error-free transformations of Knuth and Dekker (FMA form).
+struct Float2Sum {
+  float hi, lo;
+};
+__device__ __forceinline__ Float2Sum two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  const float t = __fadd_rn(s, -a);
+  return {s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -t)), __fadd_rn(b, -t))};
+}
+__device__ __forceinline__ Float2Sum two_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return {p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ Float2Sum add2(Float2Sum a, Float2Sum b) {
+  const Float2Sum s = two_sum(a.hi, b.hi);
+  const Float2Sum t = two_sum(a.lo, b.lo);
+  const Float2Sum u = two_sum(s.hi, __fadd_rn(s.lo, t.hi));
+  return two_sum(u.hi, __fadd_rn(u.lo, t.lo));
+}
+
+// Totals of `count` lanes' sums by one warp: t[0] = sum m lk, t[1] = sum lk,
+// t[2] = sum lk^2 (every lane gets them).  The widening restores sum(lk) =
+// s1 + n K and sum(lk^2) = s2 + 2 K s1 + n K^2.  A warp's FP64 instruction
+// takes some 64 cycles here, so the lanes add pairs of floats and only the
+// totals become FP64 (16 tiles of 4 rows: 3,280 cycles in FP64); sums that
+// are not finite take the FP64 path, which keeps infinities what they are.
 __device__ __forceinline__ void reduce_lane_sums(const LaneSums* v, int count, int lane,
                                                  double (&t)[3]) {
+  Float2Sum f[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  bool fine = true;
+  for (int i = lane; i < count; i += 32) {
+    const LaneSums s = v[i];
+    const float n_l = static_cast<float>(s.cnt);   // exact: a lane's rows are few
+    const Float2Sum nk = two_prod(n_l, s.K);
+    const Float2Sum ks = two_prod(2.0f * s.K, s.s1);
+    Float2Sum nkk = two_prod(nk.hi, s.K);
+    nkk.lo = __fmaf_rn(nk.lo, s.K, nkk.lo);
+    f[0] = add2(f[0], two_sum(s.mlk, s.mlk_c));
+    f[1] = add2(f[1], add2(two_sum(s.s1, nk.hi), Float2Sum{nk.lo, 0.f}));
+    f[2] = add2(f[2], add2(add2(two_sum(s.s2, ks.hi), Float2Sum{ks.lo, 0.f}), nkk));
+    // Far from overflow: |values| below 2^96.
+    fine = fine && fabsf(s.mlk) < 7.9e28f && fabsf(nkk.hi) < 7.9e28f && fabsf(s.s2) < 7.9e28f &&
+           fabsf(ks.hi) < 7.9e28f;
+  }
+  if (__all_sync(0xffffffffu, fine)) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const Float2Sum u{__shfl_xor_sync(0xffffffffu, f[k].hi, o),
+                          __shfl_xor_sync(0xffffffffu, f[k].lo, o)};
+        // The same operand order in both lanes of a pair: the same bits.
+        f[k] = (lane & o) ? add2(u, f[k]) : add2(f[k], u);
+      }
+      t[k] = static_cast<double>(f[k].hi) + f[k].lo;
+    }
+    return;
+  }
   t[0] = t[1] = t[2] = 0.0;
   for (int i = lane; i < count; i += 32) {
     const LaneSums s = v[i];
@@ -291,17 +354,24 @@ __device__ __forceinline__ double lane_sum_squares(const float4 (&wq)[QPL]) {
 // U = (-N mean(lk) - log p(w)) / T, or (-(N/n) sum m lk - log p(w)) / T with
 // a mask, as written in potential.py:183-185 (the unmasked form is exact for
 // integer sums), and the biased variance of lk.
-__device__ __forceinline__ double glm_potential(const GlmArgs& a, double sum_mlk, double ww) {
+__device__ __forceinline__ double glm_potential_mean(const GlmArgs& a, double mean_lk,
+                                                     double ww) {
   const double log_prior = -0.5 * ww * a.inv_p2 - a.prior_const;
-  const double lik = a.mask == nullptr
-                         ? -static_cast<double>(a.n_obs) * (sum_mlk / a.n)
-                         : -(static_cast<double>(a.n_obs) / a.n) * sum_mlk;
+  const double lik = -static_cast<double>(a.n_obs) * mean_lk;
   return (lik - log_prior) * a.inv_temp;
+}
+__device__ __forceinline__ double glm_potential(const GlmArgs& a, double sum_mlk, double ww) {
+  if (a.mask == nullptr) return glm_potential_mean(a, sum_mlk / a.n, ww);
+  const double log_prior = -0.5 * ww * a.inv_p2 - a.prior_const;
+  const double lik = -(static_cast<double>(a.n_obs) / a.n) * sum_mlk;
+  return (lik - log_prior) * a.inv_temp;
+}
+__device__ __forceinline__ double glm_variance_mean(double mean_lk, double mean_lk2) {
+  return fmax(mean_lk2 - mean_lk * mean_lk, 0.0);
 }
 __device__ __forceinline__ double glm_variance(const GlmArgs& a, double sum_lk,
                                                double sum_lk2) {
-  const double mean_lk = sum_lk / a.n;
-  return fmax(sum_lk2 / a.n - mean_lk * mean_lk, 0.0);
+  return glm_variance_mean(sum_lk / a.n, sum_lk2 / a.n);
 }
 
 }  // namespace gbsgmc

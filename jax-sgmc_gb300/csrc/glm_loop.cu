@@ -6,28 +6,26 @@
 // rows of 32 features is 16 KB) but the chain of dependent latencies: index
 // load, row load, dot products, block reduction, update, next step; and, with
 // a launch per gradient and per update, the launches between them.  Here a
-// cluster of S CTAs owns a chain for the whole block:
-//   * CTA s holds rows [s R, (s + 1) R) of every minibatch.  The minibatches
-//     of a block are known before it starts, so indices and rows of the next
-//     chunks are copied to shared memory (cp.async, a ring of `depth` chunk
-//     buffers) while the current one is consumed: a step never waits for the
-//     row loads unless the memory system is the bound.
-//   * warps 0..7 take row tiles of the chunk exactly as glm_kernel does (same
-//     slices, warps, tiles and summation orders: the same bits), and the
-//     threads that own four parameters each keep x and v (or p) in registers.
-//   * every CTA writes its partial gradient into all CTAs of the cluster
-//     (distributed shared memory), one cluster barrier, and every CTA adds
-//     the partials in slice order and updates its own copy of x: no second
-//     exchange is needed.
-//   * warp 8 (the clerk) draws the update's Philox noise, reads the schedule
-//     and does the FP64 sums (U, var(lk), kinetic energies, the exchange
-//     decision) while the other warps stream rows.
+// cluster of S CTAs owns a chain for the whole block, and in each CTA
+//   * the copy warps run ahead: the minibatches of a block are known before it
+//     starts, so they gather the rows of the next chunks into a ring of shared
+//     memory buffers (cp.async, full / empty mbarriers), up to `depth` chunks
+//     before they are needed;
+//   * the row warps do what nothing else can do earlier: row tiles of the
+//     chunk exactly as glm_kernel takes them (same slices, warps, tiles and
+//     summation orders: the same bits), the reduction, the exchange and the
+//     update.  CTA s holds rows [s R, (s + 1) R) of every minibatch; it sends
+//     its partial gradient into all CTAs of the cluster (st.async, counted on
+//     the receivers' mbarriers), and every CTA adds the partials in slice
+//     order and updates its own copy of x, held in registers, so no second
+//     exchange is needed;
+//   * the noise warp draws the next gradient's Philox normals one gradient
+//     ahead, and the clerk warp reads the schedule and does the FP64 work (U,
+//     var(lk), kinetic energies, the exchange decision).
 // reSGLD pairs: both chains of a pair share a cluster (2 S CTAs).  An
 // exchange swaps the chains' roles (temperature, slot) instead of their
 // states; the rows are written to the slots they ended in when the block
 // ends.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -38,13 +36,17 @@
 namespace gbsgmc {
 namespace {
 
-namespace cg = cooperative_groups;
-
 constexpr int kRowWarps = 8;
 constexpr int kRowThreads = kRowWarps * 32;
-constexpr int kLoopThreads = kRowThreads + 32;  // + the clerk warp
+constexpr int kCopyWarps = 2;
+constexpr int kCopyThreads = kCopyWarps * 32;
+constexpr int kClerkWarp = kRowWarps;
+constexpr int kNoiseWarp = kRowWarps + 1;
+constexpr int kLoopThreads = kRowThreads + 64 + kCopyThreads;  // 168 registers a thread
+constexpr int kMaxOwned = 4;                    // parameters of a row thread: d <= 1024
 constexpr int kMaxCtas = 8;                     // portable cluster size
 constexpr int kMaxDepth = 4;
+constexpr int kCopyBatch = 8;                   // rows a lane group copies at once
 
 struct LoopArgs {
   GlmArgs g;
@@ -57,7 +59,7 @@ struct LoopArgs {
   double* ke;      // OBABO: kinetic energies [2, chains] to add to, or null
   double* energy;  // leapfrog: energies [chains] to add to
   int ctas;        // CTAs per chain
-  int chunk_rows, chunks, depth, idx_slots;
+  int chunk_rows, chunks, depth;
   int row_shift;   // log2 of the lanes that copy one row
   // pairs
   int pairs;
@@ -69,33 +71,88 @@ struct LoopArgs {
   int64_t* kc;
   int32_t* counts;
   // shared-memory offsets
-  unsigned o_y, o_idx, o_red, o_part, o_w, o_xi, o_xr, o_ke, o_lane, o_sums, o_step;
+  unsigned o_y, o_idx, o_red, o_part, o_w, o_xi, o_xr, o_ke, o_lane, o_sums, o_step, o_pair, o_bar;
 };
 
-// What the clerk hands the updating threads for one gradient.
+// What the clerk hands the row warps for one gradient.
 struct StepInfo {
   float h, T, h_next;
-  int slot, want_u, role;
+  int want_next;  // want_u of the next gradient
+  int slot;       // sample slot of this step, or -1
+  int prev_slot;  // pairs: the previous step's slot if this chain is to store it
+  int want_u;     // the clerk waits for this gradient's likelihood sums
 };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
-               "r"(ok ? 16 : 0)
+// Pairs: what a decision needs besides the sums.
+struct PairConsts {
+  double dbeta, sa, log_u, pad;
+};
+
+struct LoopBars {
+  uint64_t full[kMaxDepth], empty[kMaxDepth];
+  uint64_t part[2], sums[2];
+  int stop;  // a wait ran out: the remaining ones give up at once
+};
+
+__device__ __forceinline__ void cp16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
                : "memory");
 }
+// 4 bytes, or zeros when !ok.
 __device__ __forceinline__ void cp4(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src),
                "r"(ok ? 4 : 0)
                : "memory");
 }
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-// Waits until at most `pending` of this thread's newest groups are in flight.
-__device__ __forceinline__ void cp_wait(int pending) {
-  if (pending <= 0) asm volatile("cp.async.wait_group 0;" ::: "memory");
-  else if (pending == 1) asm volatile("cp.async.wait_group 1;" ::: "memory");
-  else asm volatile("cp.async.wait_group 2;" ::: "memory");
+// This thread's copies so far count as one arrival on `bar` when they land.
+__device__ __forceinline__ void cp_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
+               : "memory");
 }
+// Named barriers (ids below 16): sync waits, arrive does not.
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+constexpr int kBarRows = 1;   // the row warps among themselves
+constexpr int kBarStep = 2;   // + parity: partials, noise and the clerk's hand-over are ready
+constexpr int kBarSums = 4;   // + parity: rows -> clerk, the likelihood sums
+constexpr int kBarDone = 6;   // + parity: rows -> clerk, the update is done
+constexpr int kBarFree = 8;   // + parity: rows -> noise warp, the normals have been used
+constexpr int kBarEnd = 10;   // clerk -> rows, the last decision
+constexpr int kWithOne = kRowThreads + 32;
+constexpr int kWithBoth = kRowThreads + 64;
 
+// Address of `p` (this CTA's shared memory) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+  return a;
+}
+// 4 or 16 bytes to another CTA of the cluster, counted on that CTA's mbarrier.
+__device__ __forceinline__ void send4(uint32_t dst, uint32_t bar, float v) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(
+                   dst),
+               "r"(__float_as_uint(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void send16(uint32_t dst, uint32_t bar, uint32_t x, uint32_t y,
+                                       uint32_t z, uint32_t w) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+      ::"r"(dst), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
+      : "memory");
+}
+// Bounded wait for phase `phase` of a barrier.
+__device__ __forceinline__ void wait_phase(LoopBars* b, uint64_t* bar, int phase, int* status) {
+  if (mbar_try_wait(bar, phase & 1)) return;
+  if (!mbar_wait_bounded(bar, phase & 1, &b->stop)) {
+    b->stop = 1;
+    raise_status(status, GBSGMC_ERR_TIMEOUT);
+  }
+}
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
 }
@@ -113,19 +170,21 @@ struct ObaboStep {
     inject = sqrtf((1.0f - permanence) * T);
     half = 0.5f * h;
   }
-  __device__ __forceinline__ void first(float mi, float ms, float g, float xi, float& p, float& x,
-                                        float& ke) const {
+  // Each returns the factors of the parameter's kinetic energy.
+  __device__ __forceinline__ float2 first(float mi, float ms, float g, float xi, float& p,
+                                          float& x) const {
     float pj = __fmaf_rn(keep, p, __fmul_rn(inject, __fmul_rn(ms, xi)));
-    ke = __fmaf_rn(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj), ke);
+    const float2 ke = make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
     pj = __fmaf_rn(-half, g, pj);
     p = pj;
     x = __fmaf_rn(h, __fmul_rn(mi, pj), x);
+    return ke;
   }
-  __device__ __forceinline__ void second(float mi, float ms, float g, float xi, float& p,
-                                         float& ke) const {
+  __device__ __forceinline__ float2 second(float mi, float ms, float g, float xi,
+                                           float& p) const {
     const float pj = __fmaf_rn(-half, g, p);
-    ke = __fmaf_rn(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj), ke);
     p = __fmaf_rn(keep, pj, __fmul_rn(inject, __fmul_rn(ms, xi)));
+    return make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
   }
 };
 
@@ -149,17 +208,13 @@ __device__ __forceinline__ double slice_total(const SliceSums* s, int ctas, int 
 }
 
 template <int QPL, int RW>
-__global__ void __launch_bounds__(kLoopThreads, QPL <= 2 ? 2 : 1)
-    glm_loop_kernel(const LoopArgs L) {
+__global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArgs L) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int LOG = Log2<RW>::v;
   constexpr int GROUP = 32 >> LOG;
   constexpr int kStride = kRowWarps * RW;
   const GlmArgs& a = L.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const bool clerk = warp == kRowWarps;
-  const int g = lane >> (5 - LOG);
-  const bool leader = (lane & (GROUP - 1)) == 0;
   const int dq = a.dq, d = a.d, S = L.ctas, CH = L.chunk_rows, depth = L.depth;
   const bool pairs = L.kind == kLoopPairs;
   const bool moves = L.kind == kLoopSgld || pairs;  // aux is the RMSprop state
@@ -174,494 +229,334 @@ __global__ void __launch_bounds__(kLoopThreads, QPL <= 2 ? 2 : 1)
   const int row0 = slice * a.rows_per_slice;
   const int R = max(0, min(a.rows_per_slice, a.n - row0));
   const int events = a.steps * L.draws;
-  const int total = events * L.chunks;
 
   float4* rows_s = reinterpret_cast<float4*>(smem);
   float* y_s = reinterpret_cast<float*>(smem + L.o_y);
   int32_t* idx_s = reinterpret_cast<int32_t*>(smem + L.o_idx);
   float4* red = reinterpret_cast<float4*>(smem + L.o_red);
   float4* part = reinterpret_cast<float4*>(smem + L.o_part);   // [2][S][dq]
-  float4* w_s = reinterpret_cast<float4*>(smem + L.o_w);
-  float4* xi_s = reinterpret_cast<float4*>(smem + L.o_xi);
-  float4* xr_s = reinterpret_cast<float4*>(smem + L.o_xr);     // SGHMC resample
-  float* ke_s = reinterpret_cast<float*>(smem + L.o_ke);
-  LaneSums* lsum = reinterpret_cast<LaneSums*>(smem + L.o_lane);
+  float4* w_s = reinterpret_cast<float4*>(smem + L.o_w);       // [2][dq]
+  float4* xi_s = reinterpret_cast<float4*>(smem + L.o_xi);     // [2][dq]
+  float4* xr_s = reinterpret_cast<float4*>(smem + L.o_xr);     // [2][dq] (SGHMC resample)
+  float2* ke_s = reinterpret_cast<float2*>(smem + L.o_ke);     // [2][4 dq] energy factors
+  LaneSums* lsum = reinterpret_cast<LaneSums*>(smem + L.o_lane);    // [2][kRowWarps RW]
   SliceSums* sums = reinterpret_cast<SliceSums*>(smem + L.o_sums);  // [2][ncta]
-  StepInfo* info = reinterpret_cast<StepInfo*>(smem + L.o_step);
+  StepInfo* info = reinterpret_cast<StepInfo*>(smem + L.o_step);    // [2]
+  PairConsts* pair_c = reinterpret_cast<PairConsts*>(smem + L.o_pair);  // [4]
+  LoopBars* bars = reinterpret_cast<LoopBars*>(smem + L.o_bar);
 
-  // ---- copies ----------------------------------------------------------------
-  auto issue_idx = [&](int e, int q, int slot) {
-    const int cnt = min(CH, R - q * CH);
-    const int32_t* src = a.idx + (e / L.draws) * a.idx_step_stride +
-                         static_cast<int64_t>(who) * a.idx_stride + (e % L.draws) * a.n + row0 +
-                         q * CH;
-    for (int r = tid; r < cnt; r += kRowThreads) cp4(idx_s + slot * CH + r, src + r, true);
-  };
-  auto issue_rows = [&](int q, int slot, int buf) {
-    const int cnt = min(CH, R - q * CH);
-    const int32_t* ix = idx_s + slot * CH;
-    float4* dst = rows_s + static_cast<int64_t>(buf) * CH * dq;
-    const int per = 32 >> L.row_shift, sub = lane >> L.row_shift;
-    const int ql = lane & ((1 << L.row_shift) - 1);
-    for (int r = warp * per + sub; r < cnt; r += kRowWarps * per) {
-      const int o = ix[r];
-      const bool ok = o >= 0 && o < a.n_rows;
-      if (!ok && ql == 0) raise_status(a.status, GBSGMC_ERR_INDEX);
-      const float* src = a.X + (ok ? static_cast<int64_t>(o) * a.ld : 0);
-      if (a.vec4) {
-        for (int v = ql; v < dq; v += 32) cp16(dst + r * dq + v, src + 4 * v, ok);
-      } else {
-        float* out = reinterpret_cast<float*>(dst + r * dq);
-        for (int j = ql; j < 4 * dq; j += 1 << L.row_shift)
-          cp4(out + j, src + (j < d ? j : 0), ok && j < d);
-      }
+  if (tid == 0) {
+    for (int i = 0; i < depth; ++i) {
+      mbar_init(bars->full + i, 2 * kCopyThreads);
+      mbar_init(bars->empty + i, kRowWarps);
     }
-    if (a.y_inline || a.y != nullptr) {
-      for (int r = tid; r < cnt; r += kRowThreads) {
-        const int o = ix[r];
-        const bool ok = o >= 0 && o < a.n_rows;
-        const float* src = a.y_inline ? a.X + (ok ? static_cast<int64_t>(o) * a.ld + d : 0)
-                                      : a.y + (ok ? o : 0);
-        cp4(y_s + buf * CH + r, src, ok);
-      }
-    }
-  };
-
-  // Sequence numbers of the next index and row chunks to request.
-  int ie = 0, iq = 0, islot = 0;             // index chunk
-  int rs = 0, rq = 0, rslot = 0, rbuf = 0;   // row chunk
-  auto next_idx = [&]() {
-    if (ie < events && !clerk) issue_idx(ie, iq, islot);
-    if (++iq == L.chunks) iq = 0, ++ie;
-    if (++islot == L.idx_slots) islot = 0;
-  };
-  auto next_rows = [&]() {
-    if (rs < total && !clerk) issue_rows(rq, rslot, rbuf);
-    ++rs;
-    if (++rq == L.chunks) rq = 0;
-    if (++rslot == L.idx_slots) rslot = 0;
-    if (++rbuf == depth) rbuf = 0;
-  };
-
-  for (int i = 0; i < 2 * (depth - 1); ++i) next_idx();
-  cp_commit();
-  if (ncta > 1) cluster_arrive();  // every CTA runs before any remote write
-
-  // ---- state -----------------------------------------------------------------
-  const int64_t k0 = a.sched.step();
-  float* x_row = a.w + static_cast<int64_t>(row_in) * d;
-  float* aux_row = L.aux != nullptr ? L.aux + static_cast<int64_t>(row_in) * d : nullptr;
-  const bool owner = tid < dq;
-  float xs[4] = {0.f, 0.f, 0.f, 0.f}, as[4] = {0.f, 0.f, 0.f, 0.f};
-  float mi[4] = {1.f, 1.f, 1.f, 1.f}, ms[4] = {1.f, 1.f, 1.f, 1.f};
-  if (owner) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int j = 4 * tid + e;
-      if (j >= d) break;
-      xs[e] = x_row[j];
-      if (aux_row != nullptr) as[e] = aux_row[j];
-      if (L.mass != nullptr) {
-        const float m = __ldg(L.mass + j);
-        mi[e] = 1.0f / m;
-        ms[e] = sqrtf(m);
-      }
-    }
-    if (L.kind == kLoopSghmc) {
-      // A block starts at a resample (its steps are whole trajectories).
-      float xi[4];
-      noise4(a.noise, who, 4 * tid, d, k0, GBSGMC_TAG_SGHMC_RESAMPLE, xi);
-      const float h = a.sched.step_size(k0);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        as[e] = ms[e] * xi[e];
-        const float pj = as[e];
-        const float sm = mi[e] * pj;
-        xs[e] = xs[e] + h * sm;
-        as[e] = pj + (-h * L.friction) * sm;
-      }
-    } else if (L.kind == kLoopLeapfrog) {
-      const float s = 0.5f * a.sched.step_size(k0);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float sm = mi[e] * as[e];
-        xs[e] = xs[e] + s * sm;
-      }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (4 * tid + e >= d) xs[e] = as[e] = 0.f;
-    w_s[tid] = make_float4(xs[0], xs[1], xs[2], xs[3]);
-  }
-
-  // The clerk's running state.
-  double ke_acc[2] = {0.0, 0.0};
-  double U_first = 0.0;            // OBABO: the step's first minibatch
-  double U_mine = 0.0, var_mine = 0.0;
-  double ssq = 0.0;
-  int64_t kc = 0;
-  int exchanges = 0;
-  int role = half;                 // pairs: the slot this chain is in now
-  double U_pair[2] = {0.0, 0.0}, var_pair[2] = {0.0, 0.0};  // by chain (half)
-  if (clerk && pairs) {
-    ssq = L.ssq[unit];
-    kc = L.kc[unit];
-  }
-
-  // FP64 sum of the threads' kinetic-energy (or energy) parts of one update,
-  // in the order of update.cu's block sums.
-  auto energy_sum = [&]() {
-    double t = 0.0;
-    for (int w0 = 0; w0 < dq; w0 += 32) {
-      const double v = w0 + lane < dq ? static_cast<double>(ke_s[w0 + lane]) : 0.0;
-      t += warp_sum(v);
-    }
-    return t;
-  };
-  // The pair's decision after step k (gradient sums in buffer par): roles
-  // swap when log u >= log s.  Lanes 0 and 1 evaluate chain 0's and 1's U and
-  // var side by side.
-  auto decide = [&](int64_t k, int par) {
-    const int h = lane & 1;
-    const SliceSums* sp = sums + par * ncta + h * S;
-    const double U = glm_potential(a, slice_total(sp, S, 0), a.inv_p2 > 0.f ? sp[0].v[3] : 0.0);
-    const double var = glm_variance(a, slice_total(sp, S, 1), slice_total(sp, S, 2));
-#pragma unroll
     for (int i = 0; i < 2; ++i) {
-      U_pair[i] = __shfl_sync(0xffffffffu, U, i);
-      var_pair[i] = __shfl_sync(0xffffffffu, var, i);
+      mbar_init(bars->part + i, 1);
+      mbar_init(bars->sums + i, 1);
     }
-    const int n_chain = half ^ role;  // the chain in the normal slot
-    const double Un = U_pair[n_chain], Uh = U_pair[n_chain ^ 1];
-    kc += 1;
-    const double sa = 1.0 / static_cast<double>(kc);
-    ssq = (1.0 - sa) * ssq + sa * var_pair[n_chain];
-    const double Tn = a.sched.temperature(k, unit);
-    const double Th = a.sched.temperature(k, L.pairs + unit);
-    const double dbeta = 1.0 / Tn - 1.0 / Th;
-    const double log_s = dbeta * (Un - Uh - dbeta * ssq / L.F);
-    const uint64_t key = (L.swap_seed << 32) | static_cast<uint32_t>(__ldg(L.pair_chain + unit));
-    const double u = swap_uniform(key, 0u, static_cast<uint32_t>(k + 1));
-    // The reference keeps the pair when log u < log s (lax.cond true branch).
-    if (!(log(u) < log_s)) {
-      role ^= 1;
-      ++exchanges;
+    bars->stop = 0;
+    mbar_fence_init();
+    for (int i = 0; i < 2; ++i) {
+      mbar_arrive_expect_tx(bars->part + i, static_cast<uint32_t>(S) * d * 4);
+      mbar_arrive_expect_tx(bars->sums + i, static_cast<uint32_t>(ncta) * sizeof(SliceSums));
     }
-    const int slot = a.sched.keep_slot(k);
-    if (slot >= 0 && role == 0 && slice == 0) {
-      const int64_t at = static_cast<int64_t>(slot) * L.pairs + unit;
-      const float* x = reinterpret_cast<const float*>(w_s);
-      for (int j = lane; j < d; j += 32) a.samples[at * d + j] = x[j];
-      if (lane == 0 && a.sample_lik != nullptr) a.sample_lik[at] = -U_pair[half];
-    }
-  };
-
-  float4 wq[QPL];
-  Accum<QPL> A;
-
-  cp_wait(0);
+  }
   __syncthreads();
-  if (ncta > 1) cluster_wait();
-  for (int i = 0; i + 1 < depth; ++i) {
-    next_rows();
-    cp_commit();
+  if (ncta > 1) {  // every CTA runs, and its barriers exist, before any remote write
+    cluster_arrive();
+    cluster_wait();
   }
 
-  int e = 0, q = 0, slot_c = 0, buf_c = 0;
-  for (int s = 0; s < total; ++s) {
-    cp_wait(depth - 2);
-    __syncthreads();  // chunk s has arrived; the last update of w_s is visible
-    next_rows();
-    next_idx();
-    cp_commit();
-    const int j = L.draws == 2 ? e >> 1 : e;
-    const int par = e & 1;
-    if (q == 0) {
-      if (!clerk) {
+  // ============================== copy warps ====================================
+  if (warp > kNoiseWarp) {
+    const int cw = warp - kNoiseWarp - 1;
+    const int share = (CH + kCopyWarps - 1) / kCopyWarps;   // rows of a chunk per copy warp
+    const int sh = L.row_shift, per = 32 >> sh, sub = lane >> sh, ql = lane & ((1 << sh) - 1);
+    const float* X = a.X;
+    const float* yv = a.y;
+    const int64_t ld = a.ld, n_rows = a.n_rows;
+    const int vec4 = a.vec4, y_inline = a.y_inline, chunks = L.chunks;
+    int buf = 0, use = 0;  // ring position, times round the ring
+    for (int e = 0; e < events; ++e) {
+      const int32_t* src = a.idx + (L.draws == 2 ? e >> 1 : e) * a.idx_step_stride +
+                           static_cast<int64_t>(who) * a.idx_stride +
+                           (L.draws == 2 ? (e & 1) * a.n : 0) + row0;
+      for (int q = 0; q < chunks; ++q) {
+        const int cnt = min(CH, R - q * CH);
+        const int r_end = min(cnt, (cw + 1) * share);
+        int o = cw * share + lane < r_end ? __ldg(src + q * CH + cw * share + lane) : -1;
+        if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
+        float4* dst = rows_s + buf * CH * dq;
+        for (int r0 = cw * share; r0 < r_end; r0 += 32) {
+          const int r = r0 + lane;
+          if (r0 > cw * share) o = r < r_end ? __ldg(src + q * CH + r) : -1;
+          if (r < r_end) {
+            if (o < 0 || o >= n_rows) {
+              raise_status(a.status, GBSGMC_ERR_INDEX);
+              o = -1;
+            }
+            idx_s[buf * CH + r] = o;
+            if (o >= 0) {
+              if (y_inline) cp4(y_s + buf * CH + r, X + o * ld + d, true);
+              else if (yv != nullptr) cp4(y_s + buf * CH + r, yv + o, true);
+            }
+          }
+          // Rows with an invalid index are never read (idx_s is -1).  Eight
+          // rows per lane group are addressed before any copy is issued: one
+          // by one each row took 330 cycles of dependent instructions.
+          const int m = min(32, r_end - r0);
+          for (int i0 = 0; i0 < m; i0 += kCopyBatch * per) {
+            const float* from[kCopyBatch];
+            bool live[kCopyBatch];
 #pragma unroll
-        for (int k = 0; k < QPL; ++k) {
-          const int v = lane + 32 * k;
-          wq[k] = v < dq ? w_s[v] : make_float4(0.f, 0.f, 0.f, 0.f);
-          A.acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        A.mlk = A.mlk_c = A.K = A.s1 = A.s2 = 0.0f;
-        A.cnt = 0;
-      } else {
-        // The clerk: last step's decision and energies, this step's schedule,
-        // noise and, where U is wanted, the prior's sum(w^2).
-        const int64_t k = k0 + j;
-        if (pairs && e > 0) decide(k - 1, par ^ 1);
-        if (e > 0 && (L.energy != nullptr || L.ke != nullptr)) ke_acc[L.draws == 2 ? par ^ 1 : 0] += energy_sum();
-        const int keep = pairs ? -1 : a.sched.keep_slot(k);
-        const bool want = pairs || j + 1 == a.steps || keep >= 0;
-        if (lane == 0) {
-          StepInfo in;
-          in.h = a.sched.step_size(k);
-          in.T = a.sched.temperature(k, pairs ? (role ? L.pairs + unit : unit) : unit);
-          in.h_next = j + 1 < a.steps ? a.sched.step_size(k + 1) : in.h;
-          in.slot = keep;
-          in.want_u = want && L.kind != kLoopLeapfrog;
-          in.role = role;
-          *info = in;
-        }
-        const uint32_t tag = moves ? GBSGMC_TAG_SGLD
-                             : L.kind == kLoopObabo
-                                 ? (par == 0 ? GBSGMC_TAG_OBABO_1 : GBSGMC_TAG_OBABO_2)
-                                 : L.kind == kLoopSghmc ? GBSGMC_TAG_SGHMC_STEP
-                                                        : GBSGMC_TAG_AMAGOLD;
-        const bool resample = L.kind == kLoopSghmc && (j + 1) % L.leapfrog == 0 &&
-                              j + 1 < a.steps;
-        for (int v = lane; v < dq; v += 32) {
-          float xi[4];
-          noise4(a.noise, who, 4 * v, d, k, tag, xi);
-          xi_s[v] = make_float4(xi[0], xi[1], xi[2], xi[3]);
-          if (resample) {
-            noise4(a.noise, who, 4 * v, d, k + 1, GBSGMC_TAG_SGHMC_RESAMPLE, xi);
-            xr_s[v] = make_float4(xi[0], xi[1], xi[2], xi[3]);
+            for (int b = 0; b < kCopyBatch; ++b) {
+              const int i = i0 + b * per + sub;
+              const int oi = __shfl_sync(0xffffffffu, o, min(i, 31));
+              live[b] = i < m && oi >= 0;
+              from[b] = X + (live[b] ? oi * ld : 0);
+            }
+            float4* out = dst + (r0 + i0 + sub) * dq;
+            if (vec4) {
+              for (int v = ql; v < dq; v += 32) {
+#pragma unroll
+                for (int b = 0; b < kCopyBatch; ++b)
+                  if (live[b]) cp16(out + b * per * dq + v, from[b] + 4 * v);
+              }
+            } else {
+              for (int j = ql; j < 4 * dq; j += 1 << sh) {
+#pragma unroll
+                for (int b = 0; b < kCopyBatch; ++b)
+                  if (live[b])
+                    cp4(reinterpret_cast<float*>(out + b * per * dq) + j,
+                        from[b] + (j < d ? j : 0), j < d);
+              }
+            }
           }
         }
-        if (want && a.inv_p2 > 0.0f && L.kind != kLoopLeapfrog) {
-          float4 own[QPL];
-#pragma unroll
-          for (int i = 0; i < QPL; ++i) {
-            const int v = lane + 32 * i;
-            own[i] = v < dq ? w_s[v] : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-          const double ww = warp_sum(lane_sum_squares<QPL>(own));
-          if (lane == 0) sums[par * ncta + rank].v[3] = ww;
+        cp_arrive(bars->full + buf);
+        mbar_arrive(bars->full + buf);
+        if (++buf == depth) {
+          buf = 0;
+          ++use;
         }
       }
     }
-    if (!clerk) {
-      const int cnt = min(CH, R - q * CH);
-      const float4* rows = rows_s + static_cast<int64_t>(buf_c) * CH * dq;
-      const int32_t* ix = idx_s + slot_c * CH;
-      for (int r0 = warp * RW; r0 < cnt; r0 += kStride) {
-        float4 xv[RW][QPL];
-#pragma unroll
-        for (int r = 0; r < RW; ++r)
-#pragma unroll
-          for (int k = 0; k < QPL; ++k) {
-            const int v = lane + 32 * k;
-            xv[r][k] = r0 + r < cnt && v < dq ? rows[(r0 + r) * dq + v]
-                                              : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-        int og = r0 + g < cnt ? ix[r0 + g] : -1;
-        if (og >= a.n_rows) og = -1;
-        const float yv = og >= 0 ? y_s[buf_c * CH + r0 + g] : 0.0f;
-        consume_tile<QPL, RW>(a, nullptr, nullptr, r0, lane, g, leader, wq, xv, yv, og, A);
-      }
-    }
-    if (++slot_c == L.idx_slots) slot_c = 0;
-    if (++buf_c == depth) buf_c = 0;
-    if (++q < L.chunks) continue;
-    q = 0;
-
-    // ---- the gradient's reduction --------------------------------------------
-    if (!clerk) {
-#pragma unroll
-      for (int k = 0; k < QPL; ++k) {
-        const int v = lane + 32 * k;
-        if (v < dq) red[warp * dq + v] = A.acc[k];
-      }
-      if (leader) {
-        lsum[warp * RW + g] = lane_sums<QPL>(A);
-        if (!isfinite(A.mlk)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
-      }
-    }
-    __syncthreads();
-    const StepInfo in = *info;
-    float4 gs = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (owner) {
-      gs = red[tid];
-#pragma unroll
-      for (int w = 1; w < kRowWarps; ++w) {
-        const float4 u = red[w * dq + tid];
-        gs.x += u.x;
-        gs.y += u.y;
-        gs.z += u.z;
-        gs.w += u.w;
-      }
-    }
-    if (clerk && in.want_u) {
-      double t[3];
-      reduce_lane_sums(lsum, kRowWarps * RW, lane, t);
-      if (lane == 0) {
-        SliceSums* mine = sums + par * ncta + rank;
-        mine->v[0] = t[0];
-        mine->v[1] = t[1];
-        mine->v[2] = t[2];
-        if (ncta > 1) {
-          const SliceSums out = *mine;
-          const cg::cluster_group cl = cg::this_cluster();
-          for (int r = 0; r < ncta; ++r)
-            if (r != rank) *cl.map_shared_rank(mine, r) = out;
-        }
-      }
-    }
-    if (ncta > 1) {
-      const cg::cluster_group cl = cg::this_cluster();
-      if (owner && S > 1) {
-        float4* mine = part + (par * S + slice) * dq + tid;
-        for (int r = 0; r < S; ++r) *cl.map_shared_rank(mine, rank0 + r) = gs;
-      }
-      cluster_arrive();
-      cluster_wait();
-      if (owner && S > 1) {
-        const float4* all = part + par * S * dq + tid;
-        gs = all[0];
-        for (int r = 1; r < S; ++r) {
-          const float4 u = all[r * dq];
-          gs.x += u.x;
-          gs.y += u.y;
-          gs.z += u.z;
-          gs.w += u.w;
-        }
-      }
-    }
-
-    // ---- the update ------------------------------------------------------------
-    if (owner) {
-      const float gl[4] = {gs.x, gs.y, gs.z, gs.w};
-      const float4 x4 = xi_s[tid];
-      const float xi[4] = {x4.x, x4.y, x4.z, x4.w};
-      float gv[4];
-      bool bad = false;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        gv[i] = 4 * tid + i < d ? (-a.scale * gl[i] + xs[i] * a.inv_p2) * a.inv_temp : 0.0f;
-        bad |= !isfinite(gv[i]);
-      }
-      if (bad) raise_status(a.status, GBSGMC_ERR_NONFINITE);
-      if (moves) {
-        const float noise_scale = sqrtf(2.0f * in.T * in.h);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float x = xs[i];
-          const float scaled_gradient = -in.h * gv[i];
-          const float scaled_noise = noise_scale * xi[i];
-          if (aux_row != nullptr) {
-            const float vn = a.alpha * as[i] + (1.0f - a.alpha) * (gv[i] * gv[i]);
-            const float G = 1.0f / (a.lmbd + sqrtf(vn));
-            const float sG = sqrtf(G);
-            as[i] = vn;
-            xs[i] = x + ((0.0f + G * scaled_gradient) + sG * scaled_noise);
-          } else {
-            xs[i] = x + (scaled_gradient + scaled_noise);
-          }
-        }
-      } else if (L.kind == kLoopObabo) {
-        const ObaboStep ob(in.h, in.T, L.friction);
-        float ke = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (4 * tid + i >= d) break;
-          if (par == 0) ob.first(mi[i], ms[i], gv[i], xi[i], as[i], xs[i], ke);
-          else ob.second(mi[i], ms[i], gv[i], xi[i], as[i], ke);
-        }
-        ke_s[tid] = ke;
-      } else if (L.kind == kLoopSghmc) {
-        const float noise_scale = sqrtf(2.0f * in.h);
-        const bool more = j + 1 < a.steps;
-        const bool resample = more && (j + 1) % L.leapfrog == 0;
-        const float4 r4 = xr_s[tid];
-        const float xr[4] = {r4.x, r4.y, r4.z, r4.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float pj = as[i] + (-in.h) * gv[i];
-          pj = pj + L.friction * (noise_scale * xi[i]);
-          if (resample) pj = ms[i] * xr[i];
-          as[i] = pj;
-        }
-        // A kept step's state is this one, before the next step's position.
-        if (in.slot >= 0 && slice == 0) {
-          float* smp = a.samples + (static_cast<int64_t>(in.slot) * a.chains + unit) * d + 4 * tid;
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (4 * tid + i < d) smp[i] = xs[i];
-        }
-        if (more) {
-          const float h = in.h_next;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const float pj = as[i];
-            const float sm = mi[i] * pj;
-            xs[i] = xs[i] + h * sm;
-            as[i] = pj + (-h * L.friction) * sm;
-          }
-        }
-      } else {  // reversible leapfrog
-        const float decay = 1.0f - in.h * L.friction;
-        const float inv = 1.0f / (1.0f + in.h * L.friction);
-        const float ns = sqrtf(4.0f * L.friction * in.h);
-        const float s = (j + 1 < a.steps ? 1.0f : 0.5f) * in.h;
-        float en = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (4 * tid + i >= d) break;
-          const float pj = as[i], gj = gv[i];
-          const float noise_j = ns * (ms[i] * xi[i]);
-          const float pn = inv * ((decay * pj + (-in.h) * gj) + noise_j);
-          as[i] = pn;
-          en += (pj + pn) * (mi[i] * gj);
-          const float sm = mi[i] * pn;
-          xs[i] = xs[i] + s * sm;
-        }
-        ke_s[tid] = 0.5f * in.h * en;
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (4 * tid + i >= d) xs[i] = as[i] = 0.f;
-      w_s[tid] = make_float4(xs[0], xs[1], xs[2], xs[3]);
-      if (in.slot >= 0 && slice == 0 && L.kind != kLoopSghmc &&
-          (L.draws == 1 || par == 1)) {
-        float* smp = a.samples + (static_cast<int64_t>(in.slot) * a.chains + unit) * d + 4 * tid;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (4 * tid + i < d) smp[i] = xs[i];
-      }
-    }
-    if (clerk && in.want_u && !pairs) {
-      const SliceSums* sp = sums + par * ncta;
-      double U = glm_potential(a, slice_total(sp, S, 0), a.inv_p2 > 0.f ? sp[slice].v[3] : 0.0);
-      if (!isfinite(U) && lane == 0) raise_status(a.status, GBSGMC_ERR_NONFINITE);
-      if (L.kind == kLoopObabo) {
-        if (par == 0) U_first = U;
-        else U = 0.5 * (U_first + U);
-      }
-      U_mine = U;
-      var_mine = glm_variance(a, slice_total(sp, S, 1), slice_total(sp, S, 2));
-      if (in.slot >= 0 && a.sample_lik != nullptr && slice == 0 && lane == 0 &&
-          (L.draws == 1 || par == 1))
-        a.sample_lik[static_cast<int64_t>(in.slot) * a.chains + unit] = moves ? -U : U;
-    }
-    ++e;
+    return;
   }
 
-  // ---- the block's end -----------------------------------------------------------
-  cp_wait(0);
-  __syncthreads();
-  if (clerk) {
-    if (pairs) {
-      decide(k0 + a.steps - 1, (events - 1) & 1);
-      if (lane == 0) info->role = role;
+  const int64_t k0 = a.sched.step();
+
+  // ============================== the noise warp ================================
+  if (warp == kNoiseWarp) {
+    const uint32_t tag0 = moves ? GBSGMC_TAG_SGLD
+                          : L.kind == kLoopObabo ? GBSGMC_TAG_OBABO_1
+                          : L.kind == kLoopSghmc ? GBSGMC_TAG_SGHMC_STEP
+                                                 : GBSGMC_TAG_AMAGOLD;
+    const uint64_t key = pairs ? (L.swap_seed << 32) |
+                                     static_cast<uint32_t>(__ldg(L.pair_chain + unit))
+                               : 0;
+    int64_t kc = pairs ? L.kc[unit] : 0;
+    for (int e = 0; e < events; ++e) {
+      if (e > 1) bar_sync(kBarFree + (e & 1), kWithOne);  // update e - 2 is done
+      const int j = L.draws == 2 ? e >> 1 : e;
+      const int64_t k = k0 + j;
+      const uint32_t tag = L.draws == 2 ? tag0 + (e & 1) : tag0;
+      const bool resample =
+          L.kind == kLoopSghmc && (j + 1) % L.leapfrog == 0 && j + 1 < a.steps;
+      for (int v = lane; v < dq; v += 32) {
+        float xi[4];
+        noise4(a.noise, who, 4 * v, d, k, tag, xi);
+        xi_s[(e & 1) * dq + v] = make_float4(xi[0], xi[1], xi[2], xi[3]);
+        if (resample) {
+          noise4(a.noise, who, 4 * v, d, k + 1, GBSGMC_TAG_SGHMC_RESAMPLE, xi);
+          xr_s[(e & 1) * dq + v] = make_float4(xi[0], xi[1], xi[2], xi[3]);
+        }
+      }
+      if (pairs) {
+        const double T = a.sched.temperature(k, (lane & 1) ? L.pairs + unit : unit);
+        kc += 1;
+        // Lanes 0, 1: 1 / T of the normal and the hot slot; others: 1 / k.
+        const double inv = 1.0 / (lane < 2 ? T : static_cast<double>(kc));
+        const double b0 = __shfl_sync(0xffffffffu, inv, 0), b1 = __shfl_sync(0xffffffffu, inv, 1);
+        if (lane == 2)   // four steps deep: the clerk may lag two behind
+          pair_c[e & 3] = PairConsts{
+              b0 - b1, inv, log(swap_uniform(key, 0u, static_cast<uint32_t>(k + 1))), 0.0};
+        __syncwarp();
+      }
+      bar_arrive(kBarStep + (e & 1), kWithBoth);
     }
-    if (L.energy != nullptr || L.ke != nullptr) ke_acc[L.draws == 2 ? 1 : 0] += energy_sum();
+    // Each kBarFree generation that the rows complete is matched here.
+    for (int e = max(events - 2, 0); e < events; ++e) bar_sync(kBarFree + (e & 1), kWithOne);
+    return;
+  }
+
+  // ============================== the clerk =====================================
+  if (warp == kClerkWarp) {
+    double ke_acc[2] = {0.0, 0.0};
+    double U_first = 0.0, U_last = 0.0, var_last = 0.0;
+    double ssq = pairs ? L.ssq[unit] : 0.0;
+    int exchanges = 0, role = half, wants = 0;
+    int done_slot = -1;  // pairs: sample slot of the step last decided
+    const bool energies = L.energy != nullptr || L.ke != nullptr;
+    StepInfo in = {};
+    auto wanted = [&](int j, int slot) {
+      return L.kind != kLoopLeapfrog && (pairs || j + 1 == a.steps || slot >= 0);
+    };
+    // The schedule of gradient e (its temperature and role come when the
+    // previous step's exchange is decided).
+    auto prepare = [&](int e) {
+      const int j = L.draws == 2 ? e >> 1 : e;
+      const int jn = L.draws == 2 ? (e + 1) >> 1 : e + 1;
+      const int64_t k = k0 + j;
+      in.h = a.sched.step_size(k);
+      in.h_next = j + 1 < a.steps ? a.sched.step_size(k + 1) : in.h;
+      in.slot = a.sched.keep_slot(k);
+      in.want_u = wanted(j, in.slot);
+      in.want_next = jn < a.steps && wanted(jn, a.sched.keep_slot(k0 + jn));
+    };
+    auto hand_over = [&](int e) {
+      const int64_t k = k0 + (L.draws == 2 ? e >> 1 : e);
+      StepInfo out = in;
+      out.T = a.sched.temperature(k, pairs ? (role ? L.pairs + unit : unit) : unit);
+      out.prev_slot = -1;
+      if (pairs) {
+        out.prev_slot = role == 0 ? done_slot : -1;
+        out.slot = -1;
+      }
+      if (lane == 0) info[e & 1] = out;
+      __syncwarp();
+      bar_arrive(kBarStep + (e & 1), kWithBoth);
+    };
+    // FP64 sum of the energy parts of update e in the order of update.cu's
+    // kernels: a part is four parameters' products, added in turn in FP32.
+    auto take_energy = [&](int e) {
+      if (!energies) return;
+      const float2* p = ke_s + (e & 1) * 4 * dq;
+      const int64_t k = k0 + (L.draws == 2 ? e >> 1 : e);
+      const float half_h = L.kind == kLoopLeapfrog ? 0.5f * a.sched.step_size(k) : 0.f;
+      double t = 0.0;
+      for (int w0 = 0; w0 < dq; w0 += 32) {
+        float part = 0.f;
+        if (w0 + lane < dq) {
+          for (int i = 0; i < 4 && 4 * (w0 + lane) + i < d; ++i) {
+            const float2 f = p[4 * (w0 + lane) + i];
+            part = __fmaf_rn(f.x, f.y, part);
+          }
+          if (L.kind == kLoopLeapfrog) part = half_h * part;
+        }
+        t += warp_sum(static_cast<double>(part));
+      }
+      ke_acc[L.draws == 2 ? e & 1 : 0] += t;
+    };
+
+    prepare(0);
+    hand_over(0);
+    for (int e = 0; e < events; ++e) {
+      const int want = in.want_u, slot = in.slot;
+      if (e > 0) {
+        bar_sync(kBarDone + ((e - 1) & 1), kWithOne);
+        take_energy(e - 1);
+      }
+      double ww = 0.0;
+      if (want && a.inv_p2 > 0.0f) {
+        float4 own[QPL];
+#pragma unroll
+        for (int i = 0; i < QPL; ++i) {
+          const int v = lane + 32 * i;
+          own[i] = v < dq ? w_s[(e & 1) * dq + v] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        ww = warp_sum(lane_sum_squares<QPL>(own));
+      }
+      if (e + 1 < events) prepare(e + 1);
+      if (want) {
+        bar_sync(kBarSums + (e & 1), kWithOne);
+        double t[3];
+        reduce_lane_sums(lsum + (e & 1) * kRowWarps * RW, kRowWarps * RW, lane, t);
+        SliceSums* all = sums + (wants & 1) * ncta;
+        if (lane < ncta) {
+          const uint32_t dst = cluster_addr(all + rank, lane);
+          const uint32_t bar = cluster_addr(bars->sums + (wants & 1), lane);
+          const double v[4] = {t[0], t[1], t[2], ww};
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            send16(dst + 16 * i, bar, __double2loint(v[2 * i]), __double2hiint(v[2 * i]),
+                   __double2loint(v[2 * i + 1]), __double2hiint(v[2 * i + 1]));
+        }
+        wait_phase(bars, bars->sums + (wants & 1), wants >> 1, a.status);
+        if (lane == 0 && e + 1 < events)
+          mbar_arrive_expect_tx(bars->sums + (wants & 1),
+                                static_cast<uint32_t>(ncta) * sizeof(SliceSums));
+        ++wants;
+        // Means over the minibatch by chain (lane & 1) and sum (lane >> 1),
+        // so that their divisions run side by side.
+        const int h = pairs ? lane & 1 : 0, which = (lane >> 1) % 3;
+        const double mean = slice_total(all + h * S, S, which) / a.n;
+        const double prior = a.inv_p2 > 0.f ? all[h * S].v[3] : 0.0;
+        double U = glm_potential_mean(a, __shfl_sync(0xffffffffu, mean, lane & 1), prior);
+        double var = glm_variance_mean(__shfl_sync(0xffffffffu, mean, 2 + (lane & 1)),
+                                       __shfl_sync(0xffffffffu, mean, 4 + (lane & 1)));
+        if (!pairs) {
+          U = __shfl_sync(0xffffffffu, U, 0);
+          var = __shfl_sync(0xffffffffu, var, 0);
+          if (!isfinite(U) && lane == 0) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+          if (L.draws == 2) {
+            if ((e & 1) == 0) U_first = U;
+            else U = 0.5 * (U_first + U);
+          }
+          U_last = U;
+          var_last = var;
+          if (slot >= 0 && a.sample_lik != nullptr && slice == 0 && lane == 0 &&
+              (L.draws == 1 || (e & 1)))
+            a.sample_lik[static_cast<int64_t>(slot) * a.chains + unit] = moves ? -U : U;
+        } else {
+          // The exchange decision after step k: the roles swap when
+          // log u >= log s (the reference keeps the pair when log u < log s,
+          // lax.cond's true branch).
+          const double dbeta = pair_c[e & 3].dbeta, sa = pair_c[e & 3].sa;
+          const double log_u = pair_c[e & 3].log_u;
+          const int n_chain = half ^ role;  // the chain in the normal slot
+          const double Un = __shfl_sync(0xffffffffu, U, n_chain);
+          const double Uh = __shfl_sync(0xffffffffu, U, n_chain ^ 1);
+          ssq = (1.0 - sa) * ssq + sa * __shfl_sync(0xffffffffu, var, n_chain);
+          const double corr = dbeta * ssq;
+          const double log_s = dbeta * (Un - Uh - (L.F == 1.0 ? corr : corr / L.F));
+          if (!(log_u < log_s)) {
+            role ^= 1;
+            ++exchanges;
+          }
+          U_last = __shfl_sync(0xffffffffu, U, half);
+          var_last = __shfl_sync(0xffffffffu, var, half);
+          done_slot = slot;
+          if (slot >= 0 && role == 0 && slice == 0 && lane == 0 && a.sample_lik != nullptr)
+            a.sample_lik[static_cast<int64_t>(slot) * L.pairs + unit] = -U_last;
+        }
+      }
+      if (e + 1 < events) hand_over(e + 1);
+    }
+    bar_sync(kBarDone + ((events - 1) & 1), kWithOne);
+    take_energy(events - 1);
+    // The last decision, for the threads that write the rows back.
+    if (pairs && lane == 0) {
+      info[0].slot = role;
+      info[0].prev_slot = role == 0 ? done_slot : -1;
+    }
+    __syncwarp();
+    bar_arrive(kBarEnd, kWithOne);
     if (lane == 0 && slice == 0) {
       if (pairs) {
         const int row = role ? L.pairs + unit : unit;
-        a.U[row] = U_pair[half];
-        a.lk_var[row] = var_pair[half];
+        a.U[row] = U_last;
+        a.lk_var[row] = var_last;
         L.ident[row] = who;
         if (half == 0) {
           L.ssq[unit] = ssq;
-          L.kc[unit] = kc;
+          L.kc[unit] += a.steps;
           if (L.counts != nullptr) L.counts[unit] += exchanges;
         }
       } else {
         if (L.kind != kLoopLeapfrog) {
-          if (a.U != nullptr) a.U[unit] = U_mine;
-          if (a.lk_var != nullptr) a.lk_var[unit] = var_mine;
+          if (a.U != nullptr) a.U[unit] = U_last;
+          if (a.lk_var != nullptr) a.lk_var[unit] = var_last;
         }
         if (L.kind == kLoopObabo && L.ke != nullptr) {
           L.ke[unit] += ke_acc[0];
@@ -670,20 +565,248 @@ __global__ void __launch_bounds__(kLoopThreads, QPL <= 2 ? 2 : 1)
         if (L.kind == kLoopLeapfrog) L.energy[unit] += ke_acc[0];
       }
     }
+    return;
   }
-  __syncthreads();
-  if (owner && slice == 0) {
-    const int row = pairs ? (info->role ? L.pairs + unit : unit) : row_in;
+
+  // ============================== row warps =====================================
+  float* x_row = a.w + static_cast<int64_t>(row_in) * d;
+  float* aux_row = L.aux != nullptr ? L.aux + static_cast<int64_t>(row_in) * d : nullptr;
+  // Thread t owns the parameters t, t + 256, ...: one chain of square roots
+  // and divisions per thread where d allows.
+  const int owned = tid < d ? (d - tid + kRowThreads - 1) / kRowThreads : 0;
+  const int g = lane >> (5 - LOG);
+  const bool leader = (lane & (GROUP - 1)) == 0;
+  float xs[kMaxOwned], as[kMaxOwned], mi[kMaxOwned], ms[kMaxOwned];
+  float* wf = reinterpret_cast<float*>(w_s);
+#pragma unroll
+  for (int i = 0; i < kMaxOwned; ++i) {
+    xs[i] = as[i] = 0.f;
+    mi[i] = ms[i] = 1.f;
+    if (i >= owned) continue;
+    const int p = tid + i * kRowThreads;
+    xs[i] = x_row[p];
+    if (aux_row != nullptr) as[i] = aux_row[p];
+    if (L.mass != nullptr) {
+      const float m = __ldg(L.mass + p);
+      mi[i] = 1.0f / m;
+      ms[i] = sqrtf(m);
+    }
+    if (L.kind == kLoopSghmc) {
+      // A block starts at a resample (its steps are whole trajectories).
+      float xi[4];
+      noise4(a.noise, who, p & ~3, d, k0, GBSGMC_TAG_SGHMC_RESAMPLE, xi);
+      const float h = a.sched.step_size(k0);
+      const float z = (p & 2) ? ((p & 1) ? xi[3] : xi[2]) : ((p & 1) ? xi[1] : xi[0]);
+      as[i] = ms[i] * z;
+      const float pj = as[i];
+      const float sm = mi[i] * pj;
+      xs[i] = xs[i] + h * sm;
+      as[i] = pj + (-h * L.friction) * sm;
+    } else if (L.kind == kLoopLeapfrog) {
+      const float s = 0.5f * a.sched.step_size(k0);
+      const float sm = mi[i] * as[i];
+      xs[i] = xs[i] + s * sm;
+    }
+  }
+  // Columns d .. 4 dq stay zero in both copies of w.
+  for (int p = tid; p < 8 * dq; p += kRowThreads) wf[p] = 0.f;
+  bar_sync(kBarRows, kRowThreads);
+#pragma unroll
+  for (int i = 0; i < kMaxOwned; ++i)
+    if (i < owned) wf[tid + i * kRowThreads] = xs[i];
+  bar_sync(kBarRows, kRowThreads);
+
+  // Stores the thread's positions in sample row `at`.
+  auto keep_x = [&](int64_t at) {
+#pragma unroll
+    for (int i = 0; i < kMaxOwned; ++i)
+      if (i < owned) a.samples[at * d + tid + i * kRowThreads] = xs[i];
+  };
+
+  int want = pairs || (L.kind != kLoopLeapfrog &&
+                       (a.steps == 1 || a.sched.keep_slot(k0) >= 0));
+  int buf = 0, use = 0;
+  for (int e = 0; e < events; ++e) {
+    const int j = L.draws == 2 ? e >> 1 : e;
+    const int par = e & 1;
+    float4 wq[QPL];
+    Accum<QPL> A;
+#pragma unroll
+    for (int k = 0; k < QPL; ++k) {
+      const int v = lane + 32 * k;
+      wq[k] = v < dq ? w_s[par * dq + v] : make_float4(0.f, 0.f, 0.f, 0.f);
+      A.acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    A.mlk = A.mlk_c = A.K = A.s1 = A.s2 = 0.0f;
+    A.cnt = 0;
+    for (int q = 0; q < L.chunks; ++q) {
+      wait_phase(bars, bars->full + buf, use, a.status);
+      const int cnt = min(CH, R - q * CH);
+      const float4* rows = rows_s + buf * CH * dq;
+      const int32_t* ix = idx_s + buf * CH;
+      for (int r0 = warp * RW; r0 < cnt; r0 += kStride) {
+        const int og = r0 + g < cnt ? ix[r0 + g] : -1;
+        const float yv = og >= 0 ? y_s[buf * CH + r0 + g] : 0.0f;
+        float4 xv[RW][QPL];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+          const bool ok = __shfl_sync(0xffffffffu, og, r * GROUP) >= 0;
+#pragma unroll
+          for (int k = 0; k < QPL; ++k) {
+            const int v = lane + 32 * k;
+            xv[r][k] = ok && v < dq ? rows[(r0 + r) * dq + v]
+                                    : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+        }
+        consume_tile<QPL, RW>(a, nullptr, nullptr, r0, lane, g, leader, want, wq, xv, yv, og,
+                              A);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bars->empty + buf);
+      if (++buf == depth) {
+        buf = 0;
+        ++use;
+      }
+    }
+
+    // ---- the gradient's reduction ----------------------------------------------
+#pragma unroll
+    for (int k = 0; k < QPL; ++k) {
+      const int v = lane + 32 * k;
+      if (v < dq) red[warp * dq + v] = A.acc[k];
+    }
+    if (leader) {
+      lsum[(par * kRowWarps + warp) * RW + g] = lane_sums<QPL>(A);
+      if (!isfinite(A.mlk)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+    }
+    bar_sync(kBarStep + par, kWithBoth);
+    if (want) bar_arrive(kBarSums + par, kWithOne);
+    const StepInfo in = info[par];
+    want = in.want_next;
+    if (owned > 0) {
+      const float* redf = reinterpret_cast<const float*>(red);
+      float* partf = reinterpret_cast<float*>(part) + par * S * 4 * dq;
+      const float* xif = reinterpret_cast<const float*>(xi_s + par * dq);
+      const float* xrf = reinterpret_cast<const float*>(xr_s + par * dq);
+      float gl[kMaxOwned];
+#pragma unroll
+      for (int i = 0; i < kMaxOwned; ++i) {
+        gl[i] = 0.f;
+        if (i >= owned) continue;
+        const int p = tid + i * kRowThreads;
+        float t[kRowWarps];
+#pragma unroll
+        for (int w = 0; w < kRowWarps; ++w) t[w] = redf[w * 4 * dq + p];
+        gl[i] = t[0];
+#pragma unroll
+        for (int w = 1; w < kRowWarps; ++w) gl[i] += t[w];
+        if (S > 1) {
+          const float* mine = partf + slice * 4 * dq + p;
+          for (int r = 0; r < S; ++r)
+            send4(cluster_addr(mine, rank0 + r), cluster_addr(bars->part + par, rank0 + r), gl[i]);
+        }
+      }
+      if (S > 1) {
+        wait_phase(bars, bars->part + par, e >> 1, a.status);
+        if (tid == 0 && e + 2 < events)
+          mbar_arrive_expect_tx(bars->part + par, static_cast<uint32_t>(S) * d * 4);
+#pragma unroll
+        for (int i = 0; i < kMaxOwned; ++i) {
+          if (i >= owned) continue;
+          const float* all = partf + tid + i * kRowThreads;
+          gl[i] = all[0];
+          for (int r = 1; r < S; ++r) gl[i] += all[r * 4 * dq];
+        }
+      }
+
+      // ---- the update ------------------------------------------------------------
+      if (in.prev_slot >= 0 && slice == 0)
+        keep_x(static_cast<int64_t>(in.prev_slot) * L.pairs + unit);
+#pragma unroll
+      for (int i = 0; i < kMaxOwned; ++i) {
+        if (i >= owned) continue;
+        const int p = tid + i * kRowThreads;
+        const float xi = xif[p];
+        const float gv = (-a.scale * gl[i] + xs[i] * a.inv_p2) * a.inv_temp;
+        if (!isfinite(gv)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
+        if (moves) {
+          const float noise_scale = sqrtf(2.0f * in.T * in.h);
+          const float x = xs[i];
+          const float scaled_gradient = -in.h * gv;
+          const float scaled_noise = noise_scale * xi;
+          if (aux_row != nullptr) {
+            const float vn = a.alpha * as[i] + (1.0f - a.alpha) * (gv * gv);
+            const float G = 1.0f / (a.lmbd + sqrtf(vn));
+            const float sG = sqrtf(G);
+            as[i] = vn;
+            xs[i] = x + ((0.0f + G * scaled_gradient) + sG * scaled_noise);
+          } else {
+            xs[i] = x + (scaled_gradient + scaled_noise);
+          }
+        } else if (L.kind == kLoopObabo) {
+          const ObaboStep ob(in.h, in.T, L.friction);
+          if (par == 0) ke_s[p] = ob.first(mi[i], ms[i], gv, xi, as[i], xs[i]);
+          else ke_s[4 * dq + p] = ob.second(mi[i], ms[i], gv, xi, as[i]);
+        } else if (L.kind == kLoopSghmc) {
+          const float noise_scale = sqrtf(2.0f * in.h);
+          float pj = as[i] + (-in.h) * gv;
+          pj = pj + L.friction * (noise_scale * xi);
+          const bool more = j + 1 < a.steps;
+          if (more && (j + 1) % L.leapfrog == 0) pj = ms[i] * xrf[p];
+          as[i] = pj;
+          // A kept step's state is this one, before the next step's position.
+          if (in.slot >= 0 && slice == 0)
+            a.samples[(static_cast<int64_t>(in.slot) * a.chains + unit) * d + p] = xs[i];
+          if (more) {
+            const float h = in.h_next;
+            const float sm = mi[i] * pj;
+            xs[i] = xs[i] + h * sm;
+            as[i] = pj + (-h * L.friction) * sm;
+          }
+        } else {  // reversible leapfrog
+          const float decay = 1.0f - in.h * L.friction;
+          const float inv = 1.0f / (1.0f + in.h * L.friction);
+          const float ns = sqrtf(4.0f * L.friction * in.h);
+          const float s = (j + 1 < a.steps ? 1.0f : 0.5f) * in.h;
+          const float pj = as[i];
+          const float noise_j = ns * (ms[i] * xi);
+          const float pn = inv * ((decay * pj + (-in.h) * gv) + noise_j);
+          as[i] = pn;
+          ke_s[par * 4 * dq + p] = make_float2(pj + pn, mi[i] * gv);
+          const float sm = mi[i] * pn;
+          xs[i] = xs[i] + s * sm;
+        }
+        wf[(par ^ 1) * 4 * dq + p] = xs[i];
+      }
+      if (in.slot >= 0 && slice == 0 && L.kind != kLoopSghmc && (L.draws == 1 || par == 1))
+        keep_x(static_cast<int64_t>(in.slot) * a.chains + unit);
+    }
+    bar_arrive(kBarDone + par, kWithOne);
+    bar_arrive(kBarFree + par, kWithOne);
+    bar_sync(kBarRows, kRowThreads);  // the new w is visible; red is free
+  }
+
+  // ---- the block's end -----------------------------------------------------------
+  bar_sync(kBarEnd, kWithOne);
+  if (owned > 0 && slice == 0) {
+    int row = row_in;
+    if (pairs) {
+      row = info[0].slot ? L.pairs + unit : unit;
+      if (info[0].prev_slot >= 0)
+        keep_x(static_cast<int64_t>(info[0].prev_slot) * L.pairs + unit);
+    }
     float* xo = a.w + static_cast<int64_t>(row) * d;
     float* ao = L.aux != nullptr ? L.aux + static_cast<int64_t>(row) * d : nullptr;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if (4 * tid + i >= d) break;
-      xo[4 * tid + i] = xs[i];
-      if (ao != nullptr) ao[4 * tid + i] = as[i];
+    for (int i = 0; i < kMaxOwned; ++i) {
+      if (i >= owned) continue;
+      xo[tid + i * kRowThreads] = xs[i];
+      if (ao != nullptr) ao[tid + i * kRowThreads] = as[i];
     }
   }
 }
+
+constexpr size_t kLoopSmem = 220 * 1024;   // one CTA per SM
 
 size_t align16(size_t x) { return (x + 15) / 16 * 16; }
 
@@ -691,28 +814,28 @@ size_t align16(size_t x) { return (x + 15) / 16 * 16; }
 // shared memory, or 0 when no chunk fits.  A CTA's whole slice of a minibatch
 // is one chunk when three such chunks fit (two minibatches ahead of the one
 // being consumed); longer slices stream through up to four smaller chunks.
-size_t loop_layout(LoopArgs& L, int rw, int ncta, size_t limit) {
+size_t loop_layout(LoopArgs& L, int rw, int ncta) {
   const int dq = L.g.dq, stride = kRowWarps * rw, R = L.g.rows_per_slice;
   const size_t row = static_cast<size_t>(dq) * 16;
-  const auto fixed = [&]() {
-    return 16 + kRowWarps * row + (L.ctas > 1 ? 2 * L.ctas * row : 0) + 3 * row +
-           align16(4 * kRowThreads) + align16(sizeof(LaneSums) * kRowWarps * rw) +
-           sizeof(SliceSums) * 2 * ncta + align16(sizeof(StepInfo)) + 64;
-  };
+  const size_t n_red = kRowWarps * row, n_part = L.ctas > 1 ? 2 * L.ctas * row : 0;
+  const size_t n_ke = 4 * row, n_lane = 2 * sizeof(LaneSums) * kRowWarps * rw;
+  const size_t n_sums = 2 * sizeof(SliceSums) * ncta, n_step = 2 * sizeof(StepInfo);
+  const size_t n_pair = 4 * sizeof(PairConsts);
+  const size_t fixed = n_red + n_part + 6 * row + align16(n_ke) + align16(n_lane) +
+                       align16(n_sums) + align16(n_step) + n_pair + align16(sizeof(LoopBars)) + 64;
   const auto ring = [&](int depth, int rows) {
-    return depth * static_cast<size_t>(rows) * (row + 4) + (2 * depth - 1) * 4ull * rows;
+    return depth * static_cast<size_t>(rows) * (row + 8);
   };
-  if (fixed() >= limit) return 0;
-  const size_t room = limit - fixed();
-  const int whole = ceil_div(R, stride) * stride;
+  if (fixed >= kLoopSmem) return 0;
+  const size_t room = kLoopSmem - fixed;
+  const int whole = std::max(1, ceil_div(R, stride)) * stride;
   int depth = 0, rows = 0;
   if (ring(3, whole) <= room) {
     depth = 3;
     rows = whole;
   } else {
     for (int dp = kMaxDepth; dp >= 2 && depth == 0; --dp) {
-      const size_t per = ring(dp, stride);
-      const int m = static_cast<int>(room / per);
+      const int m = static_cast<int>(room / ring(dp, stride));
       if (m >= 1) {
         depth = dp;
         rows = std::min(m * stride, whole);
@@ -723,7 +846,6 @@ size_t loop_layout(LoopArgs& L, int rw, int ncta, size_t limit) {
   L.depth = depth;
   L.chunk_rows = rows;
   L.chunks = std::max(1, ceil_div(R, rows));
-  L.idx_slots = 2 * depth - 1;
   size_t o = static_cast<size_t>(depth) * rows * row;
   const auto take = [&](size_t bytes) {
     const size_t at = o;
@@ -731,21 +853,20 @@ size_t loop_layout(LoopArgs& L, int rw, int ncta, size_t limit) {
     return static_cast<unsigned>(at);
   };
   L.o_y = take(4ull * depth * rows);
-  L.o_idx = take(4ull * L.idx_slots * rows);
-  L.o_red = take(kRowWarps * row);
-  L.o_part = take(L.ctas > 1 ? 2 * L.ctas * row : 0);
-  L.o_w = take(row);
-  L.o_xi = take(row);
-  L.o_xr = take(row);
-  L.o_ke = take(4 * kRowThreads);
-  L.o_lane = take(sizeof(LaneSums) * kRowWarps * rw);
-  L.o_sums = take(sizeof(SliceSums) * 2 * ncta);
-  L.o_step = take(sizeof(StepInfo));
+  L.o_idx = take(4ull * depth * rows);
+  L.o_red = take(n_red);
+  L.o_part = take(n_part);
+  L.o_w = take(2 * row);
+  L.o_xi = take(2 * row);
+  L.o_xr = take(2 * row);
+  L.o_ke = take(n_ke);
+  L.o_lane = take(n_lane);
+  L.o_sums = take(n_sums);
+  L.o_step = take(n_step);
+  L.o_pair = take(n_pair);
+  L.o_bar = take(sizeof(LoopBars));
   return o;
 }
-
-constexpr size_t kSmemOne = 220 * 1024;   // one CTA per SM
-constexpr size_t kSmemTwo = 110 * 1024;   // two CTAs per SM
 
 template <int QPL, int RW>
 struct LoopVariant {
@@ -754,7 +875,7 @@ struct LoopVariant {
     if (done) return GBSGMC_OK;
     const cudaError_t e =
         cudaFuncSetAttribute(glm_loop_kernel<QPL, RW>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemOne);
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, kLoopSmem);
     if (e != cudaSuccess)
       return set_error(GBSGMC_ERR_CUDA, "glm_loop: cudaFuncSetAttribute: %s",
                        cudaGetErrorString(e));
@@ -764,8 +885,7 @@ struct LoopVariant {
   static int launch(LoopArgs& L, int units, int ncta, cudaStream_t st) {
     int rc = prepare();
     if (rc != GBSGMC_OK) return rc;
-    const bool sparse = static_cast<int64_t>(units) * ncta <= glm_sm_count();
-    const size_t smem = loop_layout(L, RW, ncta, sparse || QPL > 2 ? kSmemOne : kSmemTwo);
+    const size_t smem = loop_layout(L, RW, ncta);
     if (smem == 0)
       return set_error(GBSGMC_ERR_SHAPE, "glm_loop: shared memory too large");
     cudaLaunchConfig_t cfg = {};
@@ -807,14 +927,32 @@ int glm_loop_ctas(int units, int chains_per_unit, int n, int d) {
   return s;
 }
 
+namespace {
+
+// Rows a warp takes at once: its whole share of the slice where the registers
+// allow (a tile's latency is one dot product, reduction and link whatever its
+// rows: 125 rows of 101 features took 5,060 cycles in tiles of 4).
+int loop_rows_per_warp(int qpl, int rows_per_slice) {
+  const char* env = std::getenv("GBSGMC_GLM_RW");
+  const int forced = env != nullptr ? std::atoi(env) : 0;
+  const int least = qpl <= 2 ? 4 : (qpl == 4 ? 2 : 1);
+  const int most = qpl == 1 ? 16 : (qpl == 2 ? 8 : (qpl == 4 ? 4 : 1));
+  if (qpl <= 2 && (forced == 4 || forced == 8)) return forced;
+  int rw = least;
+  while (rw < most && rw * kRowWarps < rows_per_slice) rw *= 2;
+  return rw;
+}
+
+}  // namespace
+
 int glm_loop_prepare() {
-  int rc = LoopVariant<1, 2>::prepare();
-  if (rc == GBSGMC_OK) rc = LoopVariant<1, 4>::prepare();
+  int rc = LoopVariant<1, 4>::prepare();
   if (rc == GBSGMC_OK) rc = LoopVariant<1, 8>::prepare();
-  if (rc == GBSGMC_OK) rc = LoopVariant<2, 2>::prepare();
+  if (rc == GBSGMC_OK) rc = LoopVariant<1, 16>::prepare();
   if (rc == GBSGMC_OK) rc = LoopVariant<2, 4>::prepare();
   if (rc == GBSGMC_OK) rc = LoopVariant<2, 8>::prepare();
   if (rc == GBSGMC_OK) rc = LoopVariant<4, 2>::prepare();
+  if (rc == GBSGMC_OK) rc = LoopVariant<4, 4>::prepare();
   if (rc == GBSGMC_OK) rc = LoopVariant<8, 1>::prepare();
   return rc;
 }
@@ -877,16 +1015,17 @@ int glm_loop(const GlmLoopCall& c, cudaStream_t st) {
   }
   if (ncta > kMaxCtas) return set_error(GBSGMC_ERR_SHAPE, "glm_loop: too many CTAs per cluster");
   const int qpl = glm_qpl(L.g.dq);
-  const int rw = c.rows_per_warp > 0 ? c.rows_per_warp : glm_rows_per_warp(L.g.dq);
+  const int rw = loop_rows_per_warp(qpl, L.g.rows_per_slice);
   if (qpl == 1)
-    return rw == 8   ? LoopVariant<1, 8>::launch(L, units, ncta, st)
-           : rw == 4 ? LoopVariant<1, 4>::launch(L, units, ncta, st)
-                     : LoopVariant<1, 2>::launch(L, units, ncta, st);
+    return rw == 16  ? LoopVariant<1, 16>::launch(L, units, ncta, st)
+           : rw == 8 ? LoopVariant<1, 8>::launch(L, units, ncta, st)
+                     : LoopVariant<1, 4>::launch(L, units, ncta, st);
   if (qpl == 2)
-    return rw == 8   ? LoopVariant<2, 8>::launch(L, units, ncta, st)
-           : rw == 4 ? LoopVariant<2, 4>::launch(L, units, ncta, st)
-                     : LoopVariant<2, 2>::launch(L, units, ncta, st);
-  if (qpl == 4) return LoopVariant<4, 2>::launch(L, units, ncta, st);
+    return rw == 8 ? LoopVariant<2, 8>::launch(L, units, ncta, st)
+                   : LoopVariant<2, 4>::launch(L, units, ncta, st);
+  if (qpl == 4)
+    return rw == 4 ? LoopVariant<4, 4>::launch(L, units, ncta, st)
+                   : LoopVariant<4, 2>::launch(L, units, ncta, st);
   return LoopVariant<8, 1>::launch(L, units, ncta, st);
 }
 

@@ -36,7 +36,6 @@ struct GlmLoopCall {
   const gbsgmc_glm* model = nullptr;
   int kind = kLoopSgld, chains = 0, n = 0, steps = 0, leapfrog = 1;
   int ctas = 1;            // CTAs per chain (glm_loop_ctas)
-  int rows_per_warp = 0;   // 0: the library's choice
   const int32_t* idx = nullptr;          // step j, chain c: idx + j idx_step_stride
   int64_t idx_stride = 0, idx_step_stride = 0;  //   + c idx_stride, [draws n]
   float* x = nullptr;

@@ -293,7 +293,6 @@ int GlmPlan::steps_launch(int g, int32_t* buf, cudaStream_t s) {
     c.n = n;
     c.steps = g;
     c.ctas = tune.loop;
-    c.rows_per_warp = tune.rows_per_warp;
     c.idx = buf;
     c.idx_stride = n;
     c.idx_step_stride = cn;
