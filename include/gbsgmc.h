@@ -833,6 +833,38 @@ int gbsgmc_glm_plan_create_keep(gbsgmc_plan** plan, const gbsgmc_glm* model,
                                 double* sample_lik_dev, int block_steps,
                                 int* status_dev);
 
+/* The full-data potential of `chains` weight rows w_dev [chains, d]:
+ *   U_c = (-sum over all n_rows observations of lk_i(w_c) - log p(w_c)) / T
+ * with the model's prior and temperature; no gradient.  A chain's value does
+ * not depend on the other chains of the call.  Replaces
+ * jax_sgmc/potential.py:219-293. */
+size_t gbsgmc_glm_full_workspace_bytes(const gbsgmc_glm* model, int chains);
+int gbsgmc_glm_full_potential(const gbsgmc_glm* model, int chains, const float* w_dev,
+                              double* U_dev, void* workspace_dev, size_t workspace_bytes,
+                              int* status_dev, gbsgmc_stream_t stream);
+
+/* AMAGOLD (kind GBSGMC_MH_AMAGOLD: reversible leapfrog) and SGGMC
+ * (GBSGMC_MH_SGGMC: OBABO) chains on the generalised-linear families: per
+ * iteration integrator->leapfrog_steps integrator steps on `model`'s
+ * minibatches, the full-data potential of the proposals under `full`, and
+ * the decision of gbsgmc_mh_accept / _select (uniforms keyed by mh_seed,
+ * noise->chain_base + c and the iteration).  x_dev and p_dev [chains, d] and
+ * U_dev [chains] (the full potential of x) are updated in place.  The plan
+ * counts integrator steps: gbsgmc_plan_run takes multiples of
+ * leapfrog_steps, and the schedule's tables are per integrator step (the
+ * noise counter).  keep_dev [iterations] gives the sample slots: positions
+ * go to samples_dev [kept, chains, d], the AMAGOLD energy or the mean
+ * minibatch potential of the last step to stat_dev [kept, chains].  Replaces
+ * jax_sgmc/solver.py:301-577. */
+int gbsgmc_glm_mh_plan_create(gbsgmc_plan** plan, const gbsgmc_glm* model,
+                              const gbsgmc_glm* full, int kind, int chains, int n,
+                              const gbsgmc_integrator* integrator, float* x_dev,
+                              float* p_dev, double* U_dev, const gbsgmc_sched* sched,
+                              const gbsgmc_noise* noise, const gbsgmc_index_src* index_src,
+                              uint64_t mh_seed, const int32_t* keep_dev,
+                              float* samples_dev, double* stat_dev,
+                              int block_iterations, int* status_dev);
+
 /* Tempering of a network plan: replica r of R runs at the schedule's
  * temperature times chain_temperature_dev[r] (set in the plan's sched), and
  * every `every` steps adjacent replicas attempt an exchange

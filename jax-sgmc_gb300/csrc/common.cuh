@@ -144,6 +144,15 @@ __device__ __forceinline__ double swap_uniform(uint64_t seed, uint32_t pair, uin
   return (static_cast<double>(bits) + 0.5) * (1.0 / 9007199254740992.0);
 }
 
+// The same of Philox (seed, counter (chain, step, 0, GBSGMC_TAG_MH)).
+__device__ __forceinline__ double mh_uniform(uint64_t seed, uint32_t chain, uint32_t step) {
+  const U32x4 r = philox4x32_10(U32x4{chain, step, 0u, GBSGMC_TAG_MH},
+                                static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+  const uint64_t bits = ((static_cast<uint64_t>(r.x) >> 5) << 26) |
+                        (static_cast<uint64_t>(r.y) >> 6);
+  return (static_cast<double>(bits) + 0.5) * (1.0 / 9007199254740992.0);
+}
+
 struct Noise {
   const float* buf;
   int64_t stride;

@@ -660,13 +660,7 @@ __global__ void mh_accept_kernel(int chains, int kind, const double* U_old,
   if (u_in != nullptr) {
     u = u_in[c];
   } else {
-    const U32x4 r = philox4x32_10(
-        U32x4{static_cast<uint32_t>(chain_base + c), static_cast<uint32_t>(k), 0u,
-              GBSGMC_TAG_MH},
-        static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
-    const uint64_t bits = ((static_cast<uint64_t>(r.x) >> 5) << 26) |
-                          (static_cast<uint64_t>(r.y) >> 6);
-    u = (static_cast<double>(bits) + 0.5) * (1.0 / 9007199254740992.0);
+    u = mh_uniform(seed, static_cast<uint32_t>(chain_base + c), static_cast<uint32_t>(k));
   }
   const int acc = log(u) < la ? 1 : 0;
   accept[c] = acc;

@@ -216,6 +216,13 @@ SIGNATURES = {
                                          _vp, _vp, _P(Sched), _P(Noise),
                                          _P(IndexSrc), _vp, _vp, _vp, _vp, _vp, _i,
                                          _vp]),
+    "gbsgmc_glm_full_workspace_bytes": (C.c_size_t, [_P(Glm), _i]),
+    "gbsgmc_glm_full_potential": (_i, [_P(Glm), _i, _vp, _vp, _vp, C.c_size_t, _vp,
+                                       _vp]),
+    "gbsgmc_glm_mh_plan_create": (_i, [_P(_vp), _P(Glm), _P(Glm), _i, _i, _i,
+                                       _P(Integrator), _vp, _vp, _vp, _P(Sched),
+                                       _P(Noise), _P(IndexSrc), _u64, _vp, _vp, _vp,
+                                       _i, _vp]),
     "gbsgmc_resgld_sa_update": (_i, [_i, _vp, _vp, _vp, _vp]),
     "gbsgmc_resgld_exchange_adjacent": (_i, [_i, _i64, _vp, _vp, _vp, _vp,
                                              _P(Sched), _i, _vp, _d, _u64,

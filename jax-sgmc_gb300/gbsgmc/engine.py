@@ -846,6 +846,60 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
                                [s.normal.model_state for s in states])
 
 
+class MhPlan:
+  """Owns a ``gbsgmc_glm_mh_plan``: C AMAGOLD or SGGMC chains on a GLM
+  potential, per iteration one trajectory launch, one full-data pass and one
+  decision launch for all chains.  X, PM [C, d] and U [C] are updated in
+  place; ``samples`` and ``stat`` hold the kept iterations."""
+
+  def __init__(self, potential, full, dataset, X, PM, U, n, kind, steps, friction,
+               h_tab, t_tab, keep_tab, n_kept, pcg, mh_seed, noise_seed, chain_base,
+               observation_count):
+    import torch
+    C, P = X.shape
+    self.steps = int(steps)
+    self.model, self._keep_alive = potential.model(dataset, observation_count)
+    self.full, self._keep_full = full.model(dataset)
+    self.state = (X, PM, U, pcg, h_tab, t_tab, keep_tab)
+    self.samples = torch.empty((max(int(n_kept), 1), C, P), dtype=torch.float32,
+                               device="cuda")
+    self.stat = torch.empty((max(int(n_kept), 1), C), dtype=torch.float64, device="cuda")
+    self.status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    self.sched = _lib.sched(step_size_dev=h_tab, temperature_dev=t_tab)
+    self.noise = _lib.noise(noise_seed, chain_base)
+    self.isrc = _lib.IndexSrc(_lib.ptr(pcg), 0, int(chain_base), 0)
+    self.integ = _lib.Integrator(_lib.INTEGRATOR_OBABO, self.steps, float(friction),
+                                 0.9, 1e-5, 0, None)
+    handle = _lib.C.c_void_p()
+    _lib.call("gbsgmc_glm_mh_plan_create", _lib.C.byref(handle), self.model, self.full,
+              _lib.MH_AMAGOLD if kind == "amagold" else _lib.MH_SGGMC, C, int(n),
+              self.integ, _lib.ptr(X), _lib.ptr(PM), _lib.ptr(U), self.sched, self.noise,
+              self.isrc, int(mh_seed) & (2**64 - 1), _lib.ptr(keep_tab),
+              _lib.ptr(self.samples), _lib.ptr(self.stat),
+              max(1, DEFAULT_BLOCK_STEPS // self.steps), _lib.ptr(self.status))
+    self.handle = handle
+
+  def run(self, iterations):
+    _lib.call("gbsgmc_plan_run", self.handle, 0, int(iterations) * self.steps,
+              _lib.stream_handle())
+
+  def check_status(self):
+    code = int(self.status.item())
+    if code != 0:
+      raise _lib.GbsgmcError(code, "device status of the MH plan")
+
+  def close(self):
+    if getattr(self, "handle", None):
+      _lib.load().gbsgmc_plan_destroy(self.handle)
+      self.handle = None
+
+  def __del__(self):
+    try:
+      self.close()
+    except Exception:  # pragma: no cover - interpreter shutdown
+      pass
+
+
 def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   """Runs AMAGOLD / SGGMC chains batched (solver.py:301-577): each MH
   iteration proposes for all chains at once with the [C, P] kernels (the
@@ -858,7 +912,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   consecutive chain ids, fresh numpy PCG64 pipelines, no mass adaption, no
   constant mass or per-parameter friction, no injected noise."""
   import torch
-  from .potential import StochasticPotential
+  from .potential import FullPotential, StochasticPotential
   meta = getattr(solver, "meta", {})
   kind = meta.get("kind")
   if not FUSED_ENABLED or kind not in ("amagold", "sggmc") or schedulers:
@@ -913,6 +967,27 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   seed, noise_key = int(states[0].key), int(ists[0].key)
   noise = _lib.noise(noise_key, chain_ids[0])
   h, t, keep, n_kept, _ = sched_mod.tables(scheduler, iterations)
+  if not pot.is_network and isinstance(full, FullPotential) and \
+      steps * C * n <= 1 << 28:
+    # GLM chains: trajectories, full-data passes and decisions on the device.
+    tabs = [torch.from_numpy(np.repeat(np.asarray(a, np.float32), steps)).cuda()
+            for a in (h, t)]
+    plan = MhPlan(pot, full, ds, X, Pm, U_old.contiguous(), n, kind, steps, f, *tabs,
+                  torch.from_numpy(np.asarray(keep, np.int32)).cuda(), n_kept, pcg,
+                  seed, noise_key, chain_ids[0], N)
+    try:
+      if iterations:
+        plan.run(iterations)
+      plan.check_status()
+      samples, extra = plan.samples, plan.stat
+    finally:
+      plan.close()
+    host = pcg.cpu()   # the streams advanced on the device
+    for c, d in enumerate(ds_list):
+      d.state.copy_(pcg[c] if d.state.is_cuda else host[c])
+    return io.postprocess_chains(saving or io.no_save(), n_kept, samples[:n_kept],
+                                 [i.treedef for i in ists], {"energy": extra[:n_kept]},
+                                 [i.model_state for i in ists])
   per = steps * (2 if kind == "sggmc" else 1)
   idx = torch.empty((per, C, n), dtype=torch.int32, device="cuda")
   samples = torch.empty((max(n_kept, 1), C, P), dtype=torch.float32, device="cuda")

@@ -349,6 +349,29 @@ class FullPotential:
       g += r.grad
     return U / self.temperature, g / self.temperature
 
+  def model(self, dataset):
+    """``gbsgmc_glm`` of the full-data potential: the prior and this
+    potential's temperature."""
+    m, keep = self._unit.model(dataset)
+    m.temperature = self.temperature
+    return m, keep
+
+  def value_all(self, W, dataset):
+    """U [C] over all observations for C chains (GLM families): no gradient,
+    all chains in one pass over the data."""
+    import torch
+    C, d = W.shape
+    m, keep = self.model(dataset)
+    if m.d != d:
+      raise ValueError(f"parameters per chain {d} != features {m.d}")
+    W = W.to(torch.float32).contiguous()
+    U = torch.empty(C, dtype=torch.float64, device="cuda")
+    nbytes = int(_lib.load().gbsgmc_glm_full_workspace_bytes(m, C))
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    _lib.call("gbsgmc_glm_full_potential", m, C, _lib.ptr(W), _lib.ptr(U), _lib.ptr(ws),
+              nbytes, _lib.ptr(self._unit.status()), _lib.stream_handle())
+    return U
+
   def __call__(self, sample, data_state, full_data_map_fn, state=None):
     loader = getattr(full_data_map_fn, "loader", None)
     if loader is None:
@@ -357,7 +380,10 @@ class FullPotential:
     ds = loader.device_dataset()
     d = self._unit.dim(ds)
     w = _flat_device(sample, d).view(1, d)
-    U, _ = self.value_and_grad_all(w, ds)
+    if self._unit.is_network:
+      U, _ = self.value_and_grad_all(w, ds)
+    else:
+      U = self.value_all(w, ds)
     return U[0], (data_state, state)
 
 

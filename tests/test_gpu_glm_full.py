@@ -1,0 +1,55 @@
+"""The full-data potential of many chains (glm_full.cu) at the edges of its
+row tiles (256), feature panels (32) and chain groups (4 and 16), against the
+oracle in float64.
+
+Tolerance: each likelihood is an fp32 value of relative error about 1e-6 (its
+dot product over up to 1,021 features and its link), their sum is
+compensated: U within 1e-6 relative of the sum of the likelihoods' magnitudes.
+A chain's value must not depend on the other chains: bit for bit.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import sgmc_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,d,C,family", [
+    (1, 1, 1, O.LINEAR_GAUSSIAN),
+    (255, 7, 4, O.LOGISTIC),
+    (257, 33, 5, O.LINEAR_GAUSSIAN),
+    (5000, 64, 17, O.LOGISTIC),
+    (70001, 32, 3, O.LOGISTIC),
+    (600, 1021, 2, O.LOGISTIC),
+])
+def test_full_potential_matches_oracle(lib, N, d, C, family):
+  import torch
+  from gbsgmc import data, likelihoods as L, potential
+  rng = np.random.default_rng(N + d)
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  lik = L.Logistic() if family == O.LOGISTIC else L.LinearGaussian(sigma=0.5)
+  y = (rng.random(N) < 0.5 if family == O.LOGISTIC else rng.normal(size=N)).astype(np.float32)
+  W = (rng.normal(size=(C, d)) / np.sqrt(d)).astype(np.float32)
+  full = potential.full_potential(L.GaussianPrior(2.0), lik, temperature=1.5)
+  ds = data.NumpyDataLoader(x=X, y=y).device_dataset()
+  Wd = torch.from_numpy(W).cuda()
+  U = full.value_all(Wd, ds).cpu().numpy()
+  for c in range(C):
+    ref = O.glm_potential(W[c:c + 1], X, y, np.arange(N)[None], N, family, 0.5, 2.0, 1.5)
+    assert abs(U[c] - ref.U[0]) <= 1e-6 * (np.abs(ref.lk).sum() + 1.0)
+  one = torch.cat([full.value_all(Wd[c:c + 1], ds) for c in range(C)]).cpu().numpy()
+  np.testing.assert_array_equal(U, one)
+
+
+def test_infinite_likelihoods_stay_infinite(lib):
+  """A likelihood sum that overflows gives U = +inf (a proposal the MH
+  decision rejects), not NaN."""
+  import torch
+  from gbsgmc import data, likelihoods as L, potential
+  X = np.full((300, 2), 1e30, np.float32)
+  full = potential.full_potential(L.FlatPrior(), L.LinearGaussian(sigma=1.0))
+  ds = data.NumpyDataLoader(x=X, y=np.zeros(300, np.float32)).device_dataset()
+  U = full.value_all(torch.tensor([[1.0, 0.0], [0.0, 0.0]], device="cuda"), ds).cpu().numpy()
+  assert U[0] == np.inf and np.isfinite(U[1])
