@@ -122,6 +122,7 @@ constexpr int kBarSums = 4;   // + parity: rows -> clerk, the likelihood sums
 constexpr int kBarDone = 6;   // + parity: rows -> clerk, the update is done
 constexpr int kBarFree = 8;   // + parity: rows -> noise warp, the normals have been used
 constexpr int kBarEnd = 10;   // clerk -> rows, the last decision
+constexpr int kBarInit = 11;  // rows -> clerk, the first x is in shared memory
 constexpr int kWithOne = kRowThreads + 32;
 constexpr int kWithBoth = kRowThreads + 64;
 
@@ -451,6 +452,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
 
     prepare(0);
     hand_over(0);
+    bar_sync(kBarInit, kWithOne);
     for (int e = 0; e < events; ++e) {
       const int want = in.want_u, slot = in.slot;
       if (e > 0) {
@@ -614,6 +616,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
 #pragma unroll
   for (int i = 0; i < kMaxOwned; ++i)
     if (i < owned) wf[tid + i * kRowThreads] = xs[i];
+  bar_arrive(kBarInit, kWithOne);
   bar_sync(kBarRows, kRowThreads);
 
   // Stores the thread's positions in sample row `at`.
