@@ -90,9 +90,10 @@ def re_sgld(potential_fn, data_loader, cache_size: int = 512,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(resgld_solver[0], init_model_state=init_model_state)
-    states = [init(*pair) for pair in init_samples]
-    return mcmc(*states, iterations=iterations,
-                schedulers=[{'temperature': {'tau': temperature}}])
+    states = _init_states(resgld_solver[0], lambda pair: init(*pair), init_samples,
+                          init_model_state=init_model_state)
+    return mcmc.run_chains(states, iterations=iterations,
+                           schedulers=[{'temperature': {'tau': temperature}}])
 
   return run_fn
 
@@ -215,8 +216,9 @@ def sghmc(potential_fn, data_loader, cache_size: int = 512,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(sghmc_solver[0], init_model_state=init_model_state)
-    states = [init(s) for s in init_samples]
-    return mcmc(*states, iterations=iterations)
+    states = _init_states(sghmc_solver[0], init, init_samples,
+                          init_model_state=init_model_state)
+    return mcmc.run_chains(states, iterations=iterations)
 
   return run_fn
 
@@ -241,8 +243,9 @@ def obabo(potential_fn, data_loader, cache_size: int = 512,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(obabo_solver[0], init_model_state=init_model_state)
-    states = [init(s) for s in init_samples]
-    return mcmc(*states, iterations=iterations)
+    states = _init_states(obabo_solver[0], init, init_samples,
+                          init_model_state=init_model_state)
+    return mcmc.run_chains(states, iterations=iterations)
 
   return run_fn
 
@@ -297,8 +300,9 @@ def amagold(stochastic_potential_fn, full_potential_fn, data_loader,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(amagold_solver[0], init_model_state=init_model_state)
-    states = [init(s) for s in init_samples]
-    return mcmc(*states, iterations=iterations)
+    states = _init_states(amagold_solver[0], init, init_samples,
+                          init_model_state=init_model_state)
+    return mcmc.run_chains(states, iterations=iterations)
 
   return run_fn
 
@@ -330,7 +334,8 @@ def sggmc(stochastic_potential_fn, full_potential_fn, data_loader,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(sggmc_solver[0], init_model_state=init_model_state)
-    states = [init(s) for s in init_samples]
-    return mcmc(*states, iterations=iterations)
+    states = _init_states(sggmc_solver[0], init, init_samples,
+                          init_model_state=init_model_state)
+    return mcmc.run_chains(states, iterations=iterations)
 
   return run_fn

@@ -410,6 +410,7 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
   GLM families, whose SGLD has its own fused step); returns None when the
   chains do not qualify (the caller steps them one by one)."""
   import torch
+  from .integrator import ChainBatch, LangevinChains
   from .potential import StochasticPotential
   meta = getattr(solver, "meta", {})
   if not FUSED_ENABLED or meta.get("kind") != "sgmc" or schedulers:
@@ -422,51 +423,74 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
     return None
   pot = im.get("potential")
   bfn = im.get("batch_fn")
-  if not isinstance(pot, StochasticPotential) or not states:
+  if not isinstance(pot, StochasticPotential) or not len(states):
     return None
   if not isinstance(bfn, tuple) or not isinstance(bfn[1], RandomBatchFn):
     return None
   rbf = bfn[1]
-  if len({s.key for s in states}) != 1:
-    return None
-  chain_ids = [int(s.chain) for s in states]
-  if chain_ids != list(range(chain_ids[0], chain_ids[0] + len(states))):
-    return None
-  if rbf.kind != "host":
-    return None
-  ds_list = [s.data_state for s in states]
-  shuffled = ShuffledFeed.qualifies(rbf.loader, ds_list)
-  if not shuffled and any(d.state is None or d.cached_batches is not None
-                          for d in ds_list):
-    return None
   steps = int(im.get("steps", 1)) if kind != "langevin" else 1
-  if kind == "langevin":
-    adapt = [s.adapt_state for s in states]
-    if any(a is None for a in adapt) and not all(a is None for a in adapt):
-      return None
-    X = torch.stack([s.latent_variables for s in states]).contiguous().cuda()
-    AUX = torch.stack([a.v for a in adapt]).contiguous().cuda() \
-        if adapt[0] is not None else None
-    kw = dict(alpha=adapt[0].alpha, lmbd=adapt[0].lmbd) \
-        if adapt[0] is not None else {}
-    if any(int(s.step) != 0 for s in states):
-      return None
+  feed = pcg = pipelines = None
+  if isinstance(states, (ChainBatch, LangevinChains)) and rbf.kind == "host" and \
+      states.pipelines.loader is rbf.loader:
+    # Fresh chains made together: consecutive ids, one key, step 0.
+    pipelines = states.pipelines
+    key, chain_base = states.key, int(states.chain_ids[0])
+    X = states.positions.cuda()
+    if kind == "langevin":
+      AUX = None if states.rms_v is None else states.rms_v.cuda()
+      kw = {} if AUX is None else dict(alpha=states.alpha, lmbd=states.lmbd)
+    else:
+      if im.get("const_mass") is not None or not np.isscalar(im.get("friction")):
+        return None
+      AUX = states.momenta()
+      kw = dict(friction=float(im["friction"]), leapfrog_steps=steps)
+    pcg = pipelines.pcg.cuda()
+    index_src = IndexSource(pcg=pcg, chain_base=chain_base)
+    treedefs = [states.treedef] * len(states)
+    model_states = [states.model_state] * len(states)
   else:
-    X = torch.stack([s.positions for s in states]).contiguous()
-    AUX = torch.stack([s.momentum for s in states]).contiguous()
-    if im.get("const_mass") is not None or not np.isscalar(im.get("friction")):
+    if len({s.key for s in states}) != 1:
       return None
-    kw = dict(friction=float(im["friction"]), leapfrog_steps=steps)
-    if any(int(s.step) != 0 for s in states):
+    key = states[0].key
+    chain_ids = [int(s.chain) for s in states]
+    chain_base = chain_ids[0]
+    if chain_ids != list(range(chain_base, chain_base + len(states))):
       return None
-  feed = pcg = None
-  if shuffled:
-    # Shuffled streams: the host loader draws them, the plan reads them.
-    feed = ShuffledFeed(rbf.loader, ds_list, 2 if kind == "obabo" else 1)
-    index_src = IndexSource(chain_base=chain_ids[0], external=True)
-  else:
-    pcg = torch.stack([d.state for d in ds_list]).contiguous().cuda()
-    index_src = IndexSource(pcg=pcg, chain_base=chain_ids[0])
+    if rbf.kind != "host":
+      return None
+    ds_list = [s.data_state for s in states]
+    shuffled = ShuffledFeed.qualifies(rbf.loader, ds_list)
+    if not shuffled and any(d.state is None or d.cached_batches is not None
+                            for d in ds_list):
+      return None
+    if kind == "langevin":
+      adapt = [s.adapt_state for s in states]
+      if any(a is None for a in adapt) and not all(a is None for a in adapt):
+        return None
+      X = torch.stack([s.latent_variables for s in states]).contiguous().cuda()
+      AUX = torch.stack([a.v for a in adapt]).contiguous().cuda() \
+          if adapt[0] is not None else None
+      kw = dict(alpha=adapt[0].alpha, lmbd=adapt[0].lmbd) \
+          if adapt[0] is not None else {}
+      if any(int(s.step) != 0 for s in states):
+        return None
+    else:
+      X = torch.stack([s.positions for s in states]).contiguous()
+      AUX = torch.stack([s.momentum for s in states]).contiguous()
+      if im.get("const_mass") is not None or not np.isscalar(im.get("friction")):
+        return None
+      kw = dict(friction=float(im["friction"]), leapfrog_steps=steps)
+      if any(int(s.step) != 0 for s in states):
+        return None
+    if shuffled:
+      # Shuffled streams: the host loader draws them, the plan reads them.
+      feed = ShuffledFeed(rbf.loader, ds_list, 2 if kind == "obabo" else 1)
+      index_src = IndexSource(chain_base=chain_base, external=True)
+    else:
+      pcg = torch.stack([d.state for d in ds_list]).contiguous().cuda()
+      index_src = IndexSource(pcg=pcg, chain_base=chain_base)
+    treedefs = [s.treedef for s in states]
+    model_states = [s.model_state for s in states]
   dataset = rbf.loader.device_dataset()
   h, t, keep, n_kept, _ = sched_mod.tables(scheduler, iterations)
   # One solver iteration is `steps` integrator steps with the same schedule.
@@ -483,7 +507,7 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
     last[steps - 1::steps] = keep   # an iteration's state is its last step's
     kw.update(keep_tab=torch.from_numpy(last).cuda(), n_kept=n_kept)
   plan = NetPlan(pot, dataset, X, AUX, rbf.mb_size, kind, h_tab, t_tab,
-                 index_src, states[0].key, chain_ids[0], feed=feed, **kw)
+                 index_src, key, chain_base, feed=feed, **kw)
   extra = None if inside else \
       torch.empty((max(n_kept, 1), C), dtype=torch.float64, device="cuda")
   # Kept samples: all on the device (device saving), streamed into FP64
@@ -530,14 +554,14 @@ def try_fused_net(solver, scheduler, states, schedulers, iterations, saving):
     plan.close()
     if feed is not None:
       feed.close()
-  if pcg is not None:
-    host = pcg.cpu()   # the streams advanced on the device
+  if pipelines is not None:
+    pipelines.pcg.copy_(pcg)   # the streams advanced on the device
+  elif pcg is not None:
+    host = pcg.cpu()
     for c, s in enumerate(states):
       dst = s.data_state.state
       dst.copy_(pcg[c] if dst.is_cuda else host[c])
   key = "likelihood" if kind == "langevin" else "energy"
-  treedefs = [s.treedef for s in states]
-  model_states = [s.model_state for s in states]
   if mom is not None:
     return io.moment_results(n_kept, mom, treedefs, {key: extra[:n_kept]},
                              model_states)
@@ -755,6 +779,7 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
   import torch
   from .integrator import LangevinState, key_to_seed
   from .potential import StochasticPotential
+  from .solver import PairChains
   meta = getattr(solver, "meta", {})
   if not FUSED_ENABLED or meta.get("kind") != "parallel_tempering":
     return None
@@ -773,28 +798,6 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
   if pot.is_mlp and rbf.mb_size % 128 != 0:
     return None
   P = len(states)
-  chains = []
-  for s in states:
-    chains += [s.normal, s.hot]
-  if not all(isinstance(c, LangevinState) and c.step == 0 for c in chains):
-    return None
-  seeds = {int(s.seed) for s in states}
-  if len(seeds) != 1 or len({float(s.F) for s in states}) != 1:
-    return None
-  seed = seeds.pop()
-  if any(c.key != seed for c in chains):
-    return None
-  ids = [int(c.chain) for c in chains]
-  if ids != list(range(ids[0], ids[0] + 2 * P)):
-    return None
-  if any(int(s.pair_chain) != int(s.normal.chain) for s in states):
-    return None
-  ds = [c.data_state for c in chains]
-  if any(d.state is None or d.cached_batches is not None for d in ds):
-    return None
-  adapt = [c.adapt_state for c in chains]
-  if any(a is None for a in adapt) != all(a is None for a in adapt):
-    return None
   h, t, keep, n_kept, _ = sched_mod.tables(scheduler, iterations)
   h2, t2, _, _, _ = sched_mod.tables(scheduler, iterations, **schedulers[0])
   if not np.array_equal(h, h2) or iterations == 0 or not (t[0] > 0):
@@ -803,23 +806,65 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
   if not np.array_equal((t * f).astype(np.float32), t2):
     return None
   dataset = rbf.loader.device_dataset()
-  normals = [s.normal for s in states]
-  hots = [s.hot for s in states]
-  X = torch.stack([c.latent_variables for c in normals + hots]).contiguous().cuda()
-  if X.shape[1] != pot.dim(dataset):
-    return None
-  if adapt[0] is not None:
-    V = torch.stack([c.adapt_state.v for c in normals + hots]).contiguous().cuda()
-    alpha, lmbd = adapt[0].alpha, adapt[0].lmbd
+  if isinstance(states, PairChains) and states.chains.pipelines.loader is rbf.loader:
+    # Fresh pairs made together: consecutive ids, one key and F, step 0.
+    ch, seed, F = states.chains, states.seed, states.F
+    rows = [*range(0, 2 * P, 2), *range(1, 2 * P, 2)]   # normal chains, then hot
+    ids0 = int(ch.chain_ids[0])
+    X = ch.positions[rows].cuda()
+    if X.shape[1] != pot.dim(dataset):
+      return None
+    V = None if ch.rms_v is None else ch.rms_v[rows].cuda()
+    alpha, lmbd = ch.alpha, ch.lmbd
+    ds = None
+    pcg = ch.pipelines.pcg.cuda()   # by identity
+    pair_chain = torch.arange(ids0, ids0 + 2 * P, 2, dtype=torch.int32, device="cuda")
+    ssq = torch.full((P,), states.ssq_init, dtype=torch.float64, device="cuda")
+    k = torch.zeros(P, dtype=torch.int64, device="cuda")
+    treedefs, model_states = [ch.treedef] * P, [ch.model_state] * P
   else:
-    V, alpha, lmbd = None, 0.9, 1e-5
-  pcg = torch.stack([d.state for d in ds]).contiguous().cuda()   # by identity
+    chains = []
+    for s in states:
+      chains += [s.normal, s.hot]
+    if not all(isinstance(c, LangevinState) and c.step == 0 for c in chains):
+      return None
+    seeds = {int(s.seed) for s in states}
+    if len(seeds) != 1 or len({float(s.F) for s in states}) != 1:
+      return None
+    seed = seeds.pop()
+    if any(c.key != seed for c in chains):
+      return None
+    ids = [int(c.chain) for c in chains]
+    if ids != list(range(ids[0], ids[0] + 2 * P)):
+      return None
+    if any(int(s.pair_chain) != int(s.normal.chain) for s in states):
+      return None
+    ds = [c.data_state for c in chains]
+    if any(d.state is None or d.cached_batches is not None for d in ds):
+      return None
+    adapt = [c.adapt_state for c in chains]
+    if any(a is None for a in adapt) != all(a is None for a in adapt):
+      return None
+    normals = [s.normal for s in states]
+    hots = [s.hot for s in states]
+    X = torch.stack([c.latent_variables for c in normals + hots]).contiguous().cuda()
+    if X.shape[1] != pot.dim(dataset):
+      return None
+    if adapt[0] is not None:
+      V = torch.stack([c.adapt_state.v for c in normals + hots]).contiguous().cuda()
+      alpha, lmbd = adapt[0].alpha, adapt[0].lmbd
+    else:
+      V, alpha, lmbd = None, 0.9, 1e-5
+    pcg = torch.stack([d.state for d in ds]).contiguous().cuda()   # by identity
+    pair_chain = torch.tensor([int(s.pair_chain) for s in states], dtype=torch.int32,
+                              device="cuda")
+    ssq = torch.cat([s.ssq.reshape(1).to(torch.float64) for s in states]).cuda()
+    k = torch.cat([s.step.reshape(1).to(torch.int64) for s in states]).cuda()
+    ids0, F = ids[0], float(states[0].F)
+    treedefs = [s.normal.treedef for s in states]
+    model_states = [s.normal.model_state for s in states]
   ident = torch.from_numpy(np.concatenate([np.arange(0, 2 * P, 2),
                                            np.arange(1, 2 * P, 2)]).astype(np.int32)).cuda()
-  pair_chain = torch.tensor([int(s.pair_chain) for s in states], dtype=torch.int32,
-                            device="cuda")
-  ssq = torch.cat([s.ssq.reshape(1).to(torch.float64) for s in states]).cuda()
-  k = torch.cat([s.step.reshape(1).to(torch.int64) for s in states]).cuda()
   ladder = torch.from_numpy(np.concatenate([np.ones(P, np.float32),
                                             np.full(P, f, np.float32)])).cuda()
   tabs = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
@@ -827,8 +872,8 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
                     np.asarray(keep, np.int32))]
   block = min(rbf.cached_batches_count, DEFAULT_BLOCK_STEPS, max(iterations, 1))
   plan = ResgldPairsPlan(pot, dataset, X, V, alpha, lmbd, rbf.mb_size, *tabs, ladder,
-                         n_kept, pcg, ident, pair_chain, ssq, k, float(states[0].F),
-                         seed, seed, ids[0], block)
+                         n_kept, pcg, ident, pair_chain, ssq, k, F, seed, seed, ids0,
+                         block)
   global LAST_EXCHANGES
   try:
     plan.run(0, iterations)
@@ -837,13 +882,15 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
     LAST_EXCHANGES = plan.counts.cpu().numpy()
   finally:
     plan.close()
-  host = pcg.cpu()   # the identities' streams advanced on the device
-  for i, d in enumerate(ds):
-    d.state.copy_(pcg[i] if d.state.is_cuda else host[i])
-  return io.postprocess_chains(saving or io.no_save(), n_kept, samples,
-                               [s.normal.treedef for s in states],
-                               {"likelihood": lik},
-                               [s.normal.model_state for s in states])
+  # The identities' streams advanced on the device.
+  if ds is None:
+    states.chains.pipelines.pcg.copy_(pcg)
+  else:
+    host = pcg.cpu()
+    for i, d in enumerate(ds):
+      d.state.copy_(pcg[i] if d.state.is_cuda else host[i])
+  return io.postprocess_chains(saving or io.no_save(), n_kept, samples, treedefs,
+                               {"likelihood": lik}, model_states)
 
 
 class MhPlan:
@@ -913,6 +960,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   constant mass or per-parameter friction, no injected noise."""
   import torch
   from .potential import FullPotential, StochasticPotential
+  from .solver import MHChains
   meta = getattr(solver, "meta", {})
   kind = meta.get("kind")
   if not FUSED_ENABLED or kind not in ("amagold", "sggmc") or schedulers:
@@ -930,7 +978,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
     return None
   pot, bfn, full = im.get("potential"), im.get("batch_fn"), meta.get("full_potential")
   fmap = meta.get("full_data_map")
-  if not isinstance(pot, StochasticPotential) or full is None or not states:
+  if not isinstance(pot, StochasticPotential) or full is None or not len(states):
     return None
   if not isinstance(bfn, tuple) or not isinstance(bfn[1], RandomBatchFn) \
       or bfn[1].kind != "host":
@@ -938,17 +986,6 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   comps = getattr(scheduler, "components", None)
   if comps is None or any(getattr(comps[k], "table", None) is None
                           for k in ("step_size", "temperature", "burn_in", "thinning")):
-    return None
-  if len({int(s.key) for s in states}) != 1 or any(s.mh_step != 0 for s in states):
-    return None
-  ists = [s.integrator_state for s in states]
-  chain_ids = [int(i.chain) for i in ists]
-  if chain_ids != list(range(chain_ids[0], chain_ids[0] + len(states))):
-    return None
-  if any(int(i.step) != 0 for i in ists) or len({int(i.key) for i in ists}) != 1:
-    return None
-  ds_list = [i.data_state for i in ists]
-  if any(d.state is None or d.cached_batches is not None for d in ds_list):
     return None
   loader = getattr(fmap[1], "loader", None) if isinstance(fmap, tuple) else None
   if loader is None or loader is not bfn[1].loader:
@@ -958,14 +995,47 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   ds = loader.device_dataset()
   N = ds.observation_count
   steps, f = int(im["steps"]), float(im["friction"])
-  X = torch.stack([i.positions for i in ists]).contiguous()
-  Pm = torch.stack([i.momentum for i in ists]).contiguous()
+  pipelines = None
+  if isinstance(states, MHChains) and states.chains.pipelines.loader is loader:
+    # Fresh chains made together: consecutive ids, one key, step 0.
+    ch = states.chains
+    seed, noise_key, chain_base = states.seed, int(ch.key), int(ch.chain_ids[0])
+    X, Pm = ch.positions.cuda(), ch.momenta()
+    U_old = states.potential.clone()
+    pipelines = ch.pipelines
+    pcg = pipelines.pcg.cuda()
+    treedefs, model_states = [ch.treedef] * C, [ch.model_state] * C
+  else:
+    if len({int(s.key) for s in states}) != 1 or any(s.mh_step != 0 for s in states):
+      return None
+    ists = [s.integrator_state for s in states]
+    chain_ids = [int(i.chain) for i in ists]
+    if chain_ids != list(range(chain_ids[0], chain_ids[0] + C)):
+      return None
+    if any(int(i.step) != 0 for i in ists) or len({int(i.key) for i in ists}) != 1:
+      return None
+    ds_list = [i.data_state for i in ists]
+    if any(d.state is None or d.cached_batches is not None for d in ds_list):
+      return None
+    X = torch.stack([i.positions for i in ists]).contiguous()
+    Pm = torch.stack([i.momentum for i in ists]).contiguous()
+    U_old = torch.cat([s.potential.reshape(1) for s in states]).to(torch.float64)
+    pcg = torch.stack([d.state for d in ds_list]).contiguous().cuda()
+    seed, noise_key, chain_base = int(states[0].key), int(ists[0].key), chain_ids[0]
+    treedefs = [i.treedef for i in ists]
+    model_states = [i.model_state for i in ists]
+
+  def streams_back():
+    if pipelines is not None:
+      pipelines.pcg.copy_(pcg)   # the streams advanced on the device
+      return
+    host = pcg.cpu()
+    for c, d in enumerate(ds_list):
+      d.state.copy_(pcg[c] if d.state.is_cuda else host[c])
+
   P = X.shape[1]
-  U_old = torch.cat([s.potential.reshape(1) for s in states]).to(torch.float64)
-  pcg = torch.stack([d.state for d in ds_list]).contiguous().cuda()
   status = torch.zeros(1, dtype=torch.int32, device="cuda")
-  seed, noise_key = int(states[0].key), int(ists[0].key)
-  noise = _lib.noise(noise_key, chain_ids[0])
+  noise = _lib.noise(noise_key, chain_base)
   h, t, keep, n_kept, _ = sched_mod.tables(scheduler, iterations)
   if not pot.is_network and isinstance(full, FullPotential) and \
       steps * C * n <= 1 << 28:
@@ -974,7 +1044,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
             for a in (h, t)]
     plan = MhPlan(pot, full, ds, X, Pm, U_old.contiguous(), n, kind, steps, f, *tabs,
                   torch.from_numpy(np.asarray(keep, np.int32)).cuda(), n_kept, pcg,
-                  seed, noise_key, chain_ids[0], N)
+                  seed, noise_key, chain_base, N)
     try:
       if iterations:
         plan.run(iterations)
@@ -982,12 +1052,9 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
       samples, extra = plan.samples, plan.stat
     finally:
       plan.close()
-    host = pcg.cpu()   # the streams advanced on the device
-    for c, d in enumerate(ds_list):
-      d.state.copy_(pcg[c] if d.state.is_cuda else host[c])
+    streams_back()
     return io.postprocess_chains(saving or io.no_save(), n_kept, samples[:n_kept],
-                                 [i.treedef for i in ists], {"energy": extra[:n_kept]},
-                                 [i.model_state for i in ists])
+                                 treedefs, {"energy": extra[:n_kept]}, model_states)
   per = steps * (2 if kind == "sggmc" else 1)
   idx = torch.empty((per, C, n), dtype=torch.int32, device="cuda")
   samples = torch.empty((max(n_kept, 1), C, P), dtype=torch.float32, device="cuda")
@@ -1045,7 +1112,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
               _lib.MH_AMAGOLD if kind == "amagold" else _lib.MH_SGGMC,
               _lib.ptr(U_old), _lib.ptr(U_new), _lib.ptr(energy), _lib.ptr(ke0),
               _lib.ptr(ke1), _lib.sched(step_size=hk, temperature=tk, offset=k),
-              None, seed, chain_ids[0], _lib.ptr(accept), _lib.ptr(ratio),
+              None, seed, chain_base, _lib.ptr(accept), _lib.ptr(ratio),
               _lib.ptr(U_keep), s)
     _lib.call("gbsgmc_mh_select", C, P, _lib.ptr(accept), _lib.ptr(X),
               _lib.ptr(x_old), _lib.ptr(Pm), _lib.ptr(p_old),
@@ -1060,9 +1127,6 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   pot.check_status()
   full._unit.check_status()
   full._flat.check_status()
-  host = pcg.cpu()   # the streams advanced on the device
-  for c, d in enumerate(ds_list):
-    d.state.copy_(pcg[c] if d.state.is_cuda else host[c])
+  streams_back()
   return io.postprocess_chains(saving or io.no_save(), n_kept, samples[:n_kept],
-                               [i.treedef for i in ists], {"energy": extra[:n_kept]},
-                               [i.model_state for i in ists])
+                               treedefs, {"energy": extra[:n_kept]}, model_states)

@@ -305,6 +305,50 @@ def langevin_diffusion(potential_fn, batch_fn, adaption: AdaptionStrategy = None
                            adaption=adaption, noise_source=noise_source)
 
 
+class ChainBatch(Sequence):
+  """The initial states of C momentum chains (obabo, friction_leapfrog,
+  reversible_leapfrog) made together, as :class:`LangevinChains` for those:
+  host positions [C, P], the chains' pipelines, and ``momenta()`` for all
+  chains' initial momenta [C, P] on the device.  Indexing makes chain i's
+  state (``make(i)``, kept), so the sequence stands for the list of states;
+  the fused drivers move the whole tensors instead."""
+
+  def __init__(self, positions, pipelines, key, model_state, treedef, momenta, make):
+    self.positions, self.pipelines, self.key = positions, pipelines, key
+    self.model_state, self.treedef = model_state, treedef
+    self.momenta, self._make = momenta, make
+    self._states = [None] * int(positions.shape[0])
+
+  @property
+  def chain_ids(self):
+    return self.pipelines.chain_ids
+
+  def __len__(self):
+    return len(self._states)
+
+  def __getitem__(self, i):
+    if isinstance(i, slice):
+      return [self[j] for j in range(*i.indices(len(self)))]
+    if i < 0:
+      i += len(self)
+    st = self._states[i]   # raises IndexError past the end
+    if st is None:
+      st = self._states[i] = self._make(i)
+    return st
+
+
+def _bulk_chains(init_data, init_samples, batch_kwargs):
+  """(host positions [C, P], tree definition, pipelines) of chains made
+  together, or None when their pipelines must register one by one."""
+  import torch
+  many = getattr(init_data, "many", None)
+  if many is None:
+    return None
+  flat, tdef = util.ravel_many(init_samples)
+  pipelines = many(len(init_samples), **(batch_kwargs or {}))
+  return None if pipelines is None else (torch.from_numpy(flat), tdef, pipelines)
+
+
 def init_mass(mass) -> MassMatrix:
   """Diagonal mass (integrator.py:99-116): inverse and square root."""
   return MassMatrix(inv=1.0 / mass, sqrt=mass ** 0.5)
@@ -328,6 +372,30 @@ def obabo(potential_fn, batch_fn, steps=10, friction=1.0, const_mass=None,
         kinetic_energy_start=torch.zeros(1, dtype=torch.float64, device="cuda"),
         kinetic_energy_end=torch.zeros(1, dtype=torch.float64, device="cuda"),
         step=0, chain=int(data_state.chain_id or 0), treedef=tdef)
+
+  def init_many(init_samples, key=None, batch_kwargs=None, init_model_state=None):
+    """``[init_fn(s, key, ...) for s in init_samples]`` in bulk."""
+    import torch
+    got = _bulk_chains(init_data, init_samples, batch_kwargs)
+    if got is None:
+      return [init_fn(s, key, batch_kwargs, init_model_state) for s in init_samples]
+    W, tdef, pipelines = got
+    seed = key_to_seed(key)
+
+    def make(i):
+      w = W[i].cuda()
+      ke = torch.zeros(3, dtype=torch.float64, device="cuda")
+      return ObaboState(
+          positions=w, momentum=torch.zeros_like(w), potential=ke[0],
+          model_state=init_model_state, data_state=pipelines.state(i), key=seed,
+          kinetic_energy_start=ke[1:2], kinetic_energy_end=ke[2:3], step=0,
+          chain=int(pipelines.chain_ids[i]), treedef=tdef)
+
+    return ChainBatch(W, pipelines, seed, init_model_state, tdef,
+                      lambda: torch.zeros(W.shape, dtype=torch.float32, device="cuda"),
+                      make)
+
+  init_fn.many = init_many
 
   def integrate(state: ObaboState, parameters, mass=None):
     x, p = state.positions, state.momentum
@@ -405,6 +473,27 @@ def friction_leapfrog(potential_fn, batch_fn, steps=10, friction=0.25,
         model_state=init_model_state, data_state=data_state,
         key=key_to_seed(key), step=0, chain=int(data_state.chain_id or 0),
         treedef=tdef)
+
+  def init_many(init_samples, key=None, batch_kwargs=None, init_model_state=None):
+    """``[init_fn(s, key, ...) for s in init_samples]`` in bulk."""
+    import torch
+    got = _bulk_chains(init_data, init_samples, batch_kwargs)
+    if got is None:
+      return [init_fn(s, key, batch_kwargs, init_model_state) for s in init_samples]
+    W, tdef, pipelines = got
+    seed = key_to_seed(key)
+
+    def make(i):
+      w = W[i].cuda()
+      return LeapfrogState(
+          positions=w, momentum=w.clone(),
+          potential=torch.zeros((), dtype=torch.float64, device="cuda"),
+          model_state=init_model_state, data_state=pipelines.state(i), key=seed,
+          step=0, chain=int(pipelines.chain_ids[i]), treedef=tdef)
+
+    return ChainBatch(W, pipelines, seed, init_model_state, tdef, W.cuda, make)
+
+  init_fn.many = init_many
 
   def integrate(state: LeapfrogState, parameters, mass=None):
     x, p = state.positions, state.momentum
@@ -504,6 +593,37 @@ def reversible_leapfrog(potential_fn, batch_fn, steps: int = 10,
         potential=torch.zeros(1, dtype=torch.float64, device="cuda"),
         model_state=init_model_state, data_state=data_state, key=seed,
         step=0, chain=chain, treedef=tdef)
+
+  def init_many(init_samples, key=None, batch_kwargs=None, init_model_state=None):
+    """``[init_fn(s, key, ...) for s in init_samples]`` in bulk (unit mass, no
+    injected normals)."""
+    import torch
+    got = None
+    if const_mass is None and noise_source is None:
+      got = _bulk_chains(init_data, init_samples, batch_kwargs)
+    if got is None:
+      return [init_fn(s, key, batch_kwargs, init_model_state) for s in init_samples]
+    W, tdef, pipelines = got
+    seed = key_to_seed(key)
+
+    def momenta(first=0, count=None):
+      P = W.shape[1]
+      p = torch.empty((len(W) if count is None else count, P), dtype=torch.float32,
+                      device="cuda")
+      _lib.call("gbsgmc_philox_normal", seed, int(pipelines.chain_ids[first]), p.shape[0],
+                0, _lib.TAG_AMAGOLD_INIT, P, _lib.ptr(p), P, _lib.stream_handle())
+      return p
+
+    def make(i):
+      return LeapfrogState(
+          positions=W[i].cuda(), momentum=momenta(i, 1)[0],
+          potential=torch.zeros(1, dtype=torch.float64, device="cuda"),
+          model_state=init_model_state, data_state=pipelines.state(i), key=seed,
+          step=0, chain=int(pipelines.chain_ids[i]), treedef=tdef)
+
+    return ChainBatch(W, pipelines, seed, init_model_state, tdef, momenta, make)
+
+  init_fn.many = init_many
 
   def integrate(state: LeapfrogState, parameters, mass=None):
     import torch

@@ -11,6 +11,7 @@ the reference's per-chain format either way.
 
 from __future__ import annotations
 
+from collections.abc import Sequence
 from typing import Any, NamedTuple
 
 import numpy as np
@@ -57,6 +58,54 @@ class TemperingState(NamedTuple):
   pair_chain: int = 0   # chain id of the pair's first normal chain
 
 
+class PairChains(Sequence):
+  """The initial states of reSGLD pairs made together: ``chains`` are the
+  2P integrator states (normal, hot, normal, hot, ...) of a bulk
+  initialisation; indexing makes pair i's :class:`TemperingState`."""
+
+  def __init__(self, chains, ssq_init, F, seed, make):
+    self.chains, self.ssq_init, self.F, self.seed = chains, ssq_init, F, seed
+    self._make = make
+    self._states = [None] * (len(chains) // 2)
+
+  def __len__(self):
+    return len(self._states)
+
+  def __getitem__(self, i):
+    if isinstance(i, slice):
+      return [self[j] for j in range(*i.indices(len(self)))]
+    if i < 0:
+      i += len(self)
+    st = self._states[i]   # raises IndexError past the end
+    if st is None:
+      st = self._states[i] = self._make(self.chains[2 * i], self.chains[2 * i + 1])
+    return st
+
+
+class MHChains(Sequence):
+  """The initial states of MH chains made together: ``chains`` is the
+  integrator's bulk initialisation, ``potential`` [C] the full potentials of
+  the initial samples; indexing makes chain i's :class:`MHState`."""
+
+  def __init__(self, chains, potential, seed, make):
+    self.chains, self.potential, self.seed = chains, potential, seed
+    self._make = make
+    self._states = [None] * len(chains)
+
+  def __len__(self):
+    return len(self._states)
+
+  def __getitem__(self, i):
+    if isinstance(i, slice):
+      return [self[j] for j in range(*i.indices(len(self)))]
+    if i < 0:
+      i += len(self)
+    st = self._states[i]   # raises IndexError past the end
+    if st is None:
+      st = self._states[i] = self._make(i)
+    return st
+
+
 def parallel_tempering(integrator, sa_schedule=None):
   """reSGLD: a normal and a hot chain exchanging states (solver.py:220-299).
 
@@ -73,8 +122,6 @@ def parallel_tempering(integrator, sa_schedule=None):
 
   def init(normal_sample, tempered_sample, ssq_init=0.0, key=0, F=1.0,
            **kwargs):
-    import torch
-    from .integrator import key_to_seed
     seed = int(np.asarray(key).ravel()[-1]) if key is not None else 0
     # Both chains draw their noise with the pair's key; their own chain ids
     # (their data pipelines') keep the streams apart, and the streams move
@@ -82,6 +129,11 @@ def parallel_tempering(integrator, sa_schedule=None):
     # ids (pipelines that carry none) get distinct keys instead.
     normal = init_integrator(normal_sample, key=seed, **kwargs)
     hot = init_integrator(tempered_sample, key=seed, **kwargs)
+    return pair_state(normal, hot, ssq_init, seed, F)
+
+  def pair_state(normal, hot, ssq_init, seed, F):
+    import torch
+    from .integrator import key_to_seed
     if normal.chain == hot.chain:
       normal = normal._replace(key=key_to_seed((seed, 1)))
       hot = hot._replace(key=key_to_seed((seed, 2)))
@@ -90,6 +142,20 @@ def parallel_tempering(integrator, sa_schedule=None):
         torch.full((1,), float(ssq_init), dtype=torch.float64, device="cuda"),
         float(F), torch.zeros(1, dtype=torch.int64, device="cuda"),
         key_to_seed((seed, normal.chain)), seed, int(normal.chain))
+
+  def init_many(pairs, ssq_init=0.0, key=0, F=1.0, **kwargs):
+    """``[init(*pair, ...) for pair in pairs]`` in bulk."""
+    from .integrator import LangevinChains
+    seed = int(np.asarray(key).ravel()[-1]) if key is not None else 0
+    chains = init_integrator.many([s for pair in pairs for s in pair], key=seed,
+                                  **kwargs)
+    make = lambda normal, hot: pair_state(normal, hot, ssq_init, seed, F)  # noqa: E731
+    if not isinstance(chains, LangevinChains):
+      return [make(n, h) for n, h in zip(chains[0::2], chains[1::2])]
+    return PairChains(chains, float(ssq_init), float(F), seed, make)
+
+  if getattr(init_integrator, "many", None) is not None:
+    init.many = init_many
 
   def update(state: TemperingState, normal_schedule, hot_schedule,
              uniform=None):
@@ -178,6 +244,37 @@ def _mh_solver(kind, integrator, full_potential_fn, full_data_map,
                    acceptance_ratio=torch.zeros(1, dtype=torch.float64,
                                                 device="cuda"),
                    step_size=0.0, mh_step=0, mass_state=mass_state)
+
+  def init_many(init_samples, key=0, init_model_state=None, **kwargs):
+    """``[init(s, key, ...) for s in init_samples]`` in bulk, the full
+    potentials of the samples in one pass over the data."""
+    import torch
+    from .integrator import ChainBatch
+    loader = getattr(full_data_map_fn, "loader", None)
+    unit = getattr(full_potential_fn, "_unit", None)
+    if mass_adaption is not None or kwargs or loader is None or unit is None or \
+        unit.is_network or len(init_samples) < 2:
+      return [init(s, key, init_model_state=init_model_state, **kwargs)
+              for s in init_samples]
+    seed = int(np.asarray(key).ravel()[-1]) if key is not None else 0
+    chains = init_integrator.many(init_samples, key=(seed, 1),
+                                  init_model_state=init_model_state)
+
+    def state(ist, U):
+      return MHState(integrator_state=ist, potential=U, full_data_state=init_full_data(),
+                     key=seed, acceptance_ratio=torch.zeros(1, dtype=torch.float64,
+                                                            device="cuda"),
+                     step_size=0.0, mh_step=0, mass_state=None)
+
+    X = chains.positions.cuda() if isinstance(chains, ChainBatch) else \
+        torch.stack([c.positions for c in chains])
+    U = full_potential_fn.value_all(X, loader.device_dataset())
+    if not isinstance(chains, ChainBatch):
+      return [state(c, U[i:i + 1].clone()) for i, c in enumerate(chains)]
+    return MHChains(chains, U, seed, lambda i: state(chains[i], U[i:i + 1].clone()))
+
+  if getattr(init_integrator, "many", None) is not None:
+    init.many = init_many
 
   def update(state: MHState, schedule):
     import torch
