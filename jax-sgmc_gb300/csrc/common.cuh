@@ -320,6 +320,39 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// An unevaluated sum of two floats, hi + lo (48 bits or more): exact sums and
+// products by the error-free transformations of Knuth and Dekker (FMA form).
+struct Float2Sum {
+  float hi, lo;
+};
+__device__ __forceinline__ Float2Sum two_sum(float a, float b) {
+  const float s = __fadd_rn(a, b);
+  const float t = __fadd_rn(s, -a);
+  return {s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -t)), __fadd_rn(b, -t))};
+}
+__device__ __forceinline__ Float2Sum two_prod(float a, float b) {
+  const float p = __fmul_rn(a, b);
+  return {p, __fmaf_rn(a, b, -p)};
+}
+__device__ __forceinline__ Float2Sum add2(Float2Sum a, Float2Sum b) {
+  const Float2Sum s = two_sum(a.hi, b.hi);
+  const Float2Sum t = two_sum(a.lo, b.lo);
+  const Float2Sum u = two_sum(s.hi, __fadd_rn(s.lo, t.hi));
+  return two_sum(u.hi, __fadd_rn(u.lo, t.lo));
+}
+// Sum over the warp of pairs of floats, the same in every lane.
+__device__ __forceinline__ Float2Sum warp_sum(Float2Sum f) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const Float2Sum u{__shfl_xor_sync(0xffffffffu, f.hi, o),
+                      __shfl_xor_sync(0xffffffffu, f.lo, o)};
+    // The same operand order in both lanes of a pair: the same bits.
+    f = (lane & o) ? add2(u, f) : add2(f, u);
+  }
+  return f;
+}
+
 // Sum over the block; every thread receives the result.  `scratch` holds at
 // least blockDim.x / 32 doubles.  Contains __syncthreads.
 __device__ __forceinline__ double block_sum(double v, double* scratch) {

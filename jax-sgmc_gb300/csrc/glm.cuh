@@ -254,27 +254,6 @@ __device__ __forceinline__ LaneSums lane_sums(const Accum<QPL>& A) {
   return LaneSums{A.mlk, A.mlk_c, A.K, A.s1, A.s2, A.cnt};
 }
 
-// An unevaluated sum of two floats, hi + lo (48 bits or more): exact sums and
-// products by the error-free transformations of Knuth and Dekker (FMA form).
-struct Float2Sum {
-  float hi, lo;
-};
-__device__ __forceinline__ Float2Sum two_sum(float a, float b) {
-  const float s = __fadd_rn(a, b);
-  const float t = __fadd_rn(s, -a);
-  return {s, __fadd_rn(__fadd_rn(a, -__fadd_rn(s, -t)), __fadd_rn(b, -t))};
-}
-__device__ __forceinline__ Float2Sum two_prod(float a, float b) {
-  const float p = __fmul_rn(a, b);
-  return {p, __fmaf_rn(a, b, -p)};
-}
-__device__ __forceinline__ Float2Sum add2(Float2Sum a, Float2Sum b) {
-  const Float2Sum s = two_sum(a.hi, b.hi);
-  const Float2Sum t = two_sum(a.lo, b.lo);
-  const Float2Sum u = two_sum(s.hi, __fadd_rn(s.lo, t.hi));
-  return two_sum(u.hi, __fadd_rn(u.lo, t.lo));
-}
-
 // Totals of `count` lanes' sums by one warp: t[0] = sum m lk, t[1] = sum lk,
 // t[2] = sum lk^2 (every lane gets them).  The widening restores sum(lk) =
 // s1 + n K and sum(lk^2) = s2 + 2 K s1 + n K^2.  A warp's FP64 instruction
@@ -302,13 +281,7 @@ __device__ __forceinline__ void reduce_lane_sums(const LaneSums* v, int count, i
   if (__all_sync(0xffffffffu, fine)) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const Float2Sum u{__shfl_xor_sync(0xffffffffu, f[k].hi, o),
-                          __shfl_xor_sync(0xffffffffu, f[k].lo, o)};
-        // The same operand order in both lanes of a pair: the same bits.
-        f[k] = (lane & o) ? add2(u, f[k]) : add2(f[k], u);
-      }
+      f[k] = warp_sum(f[k]);
       t[k] = static_cast<double>(f[k].hi) + f[k].lo;
     }
     return;

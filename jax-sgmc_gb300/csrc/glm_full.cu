@@ -162,13 +162,7 @@ __global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a,
   for (int c = 0; c < CB; ++c) {
     double s;
     if (__all_sync(0xffffffffu, fabsf(sum[c]) < 7.9e28f)) {
-      Float2Sum f = two_sum(sum[c], comp[c]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const Float2Sum u{__shfl_xor_sync(0xffffffffu, f.hi, o),
-                          __shfl_xor_sync(0xffffffffu, f.lo, o)};
-        f = (lane & o) ? add2(u, f) : add2(f, u);
-      }
+      const Float2Sum f = warp_sum(two_sum(sum[c], comp[c]));
       s = static_cast<double>(f.hi) + f.lo;
     } else {  // keeps infinities what they are
       s = warp_sum(static_cast<double>(sum[c]));

@@ -196,6 +196,8 @@ struct MlpArgs {
   const int32_t* idx;
   const float* w;
   float sigma, prior_scale, temperature;
+  float pf;             // 1 / (s^2 T) of the prior, 0 for a flat one
+  double prior_const;   // P (log s + 0.5 log 2 pi), 0 for a flat prior
   double* U;
   float* grad;
   float* lk;
@@ -217,6 +219,7 @@ struct MlpArgs {
   bf16 *sqa, *sqb;
   uint32_t* fmin;
   int *prefix1, *prefix2, *kblocks;
+  int tile_rows;   // rows of the row-ragged GEMMs' tiles: 128, or 256 (CTA pairs)
   // workspace views
   bf16 *wb, *xb, *z1, *z2g;
   float *yv, *outp, *pw3, *pb2, *pb1;
@@ -242,8 +245,9 @@ __global__ void mlp_ragged_kernel(const MlpArgs a) {
     const int v = __ldg(a.n_true + c);
     if (v < 1 || v > a.n) raise_status(a.status, GBSGMC_ERR_SHAPE);
     const int np = chain_rows_padded(a, c);
-    p1 += (np / 128) * (a.s.H1 / kBN);
-    p2 += (np / 128) * (a.s.H2 / kBN);
+    const int tm = (np + a.tile_rows - 1) / a.tile_rows;
+    p1 += tm * (a.s.H1 / kBN);
+    p2 += tm * (a.s.H2 / kBN);
     a.prefix1[c + 1] = p1;
     a.prefix2[c + 1] = p2;
     a.kblocks[c] = np / kGemmBK;
@@ -557,7 +561,7 @@ struct EpiGradCols {
 //    per-block column sums for dW3 (sum_i g_i Z2_ij) and db2 (sum_i G2_ij).
 // ---------------------------------------------------------------------------
 template <bool kFisher>
-__global__ void __launch_bounds__(256) mlp_out_kernel(const MlpArgs a) {
+__global__ void __launch_bounds__(256, kFisher ? 2 : 3) mlp_out_kernel(const MlpArgs a) {
   constexpr int kParts = kFisher ? 4 : 2;
   __shared__ float g_s[kTile];
   __shared__ double red[2][4];
@@ -621,7 +625,8 @@ __global__ void __launch_bounds__(256) mlp_out_kernel(const MlpArgs a) {
   // Every thread runs the same number of passes (the barriers below).
   for (int base = 0; base < cpr; base += CT) {
     const int ch = base + ct;
-    const bool active = ch < cpr;
+    // Threads past the last whole row group (CT not a divisor of 256) idle.
+    const bool active = ch < cpr && rg < RG;
     float w3[8], aw[8], ab[8], aw2[8], ab2[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -710,9 +715,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
   const int c = blockIdx.y, t = threadIdx.x;
   const float* w = a.w + static_cast<int64_t>(c) * s.P;
   const double s2 = static_cast<double>(a.prior_scale) * a.prior_scale;
-  const float pf = a.prior_scale > 0.f && !a.fused && !a.fisher
-                       ? static_cast<float>(1.0 / (s2 * a.temperature))
-                       : 0.f;
+  const float pf = a.fused || a.fisher ? 0.f : a.pf;
   const int nc = chain_rows(a, c), npad = chain_rows_padded(a, c);
   const int nb64 = npad / kTile, nb32 = npad / 32;
   if (a.want_grad) {
@@ -721,6 +724,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
     if (j < s.H1) {
       const float* p = a.pb1 + static_cast<int64_t>(c) * (a.n / 32) * s.H1 + j;
       float acc = 0.f;
+#pragma unroll 16
       for (int r = 0; r < nb32; ++r) acc += p[static_cast<int64_t>(r) * s.H1];
       g[s.ob1 + j] = fmaf(pf, __ldg(w + s.ob1 + j), acc);
       if (a.fisher) {
@@ -733,6 +737,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
     if (j < s.H2) {
       const int64_t base = static_cast<int64_t>(c) * (a.n / kTile) * s.H2 + j;
       float acc2 = 0.f, acc3 = 0.f;
+#pragma unroll 8
       for (int r = 0; r < nb64; ++r) {
         acc2 += a.pb2[base + static_cast<int64_t>(r) * s.H2];
         acc3 += a.pw3[base + static_cast<int64_t>(r) * s.H2];
@@ -751,21 +756,24 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
     }
   }
   if (blockIdx.x != 0) return;
-  double sq = 0.0, lm = 0.0, l1 = 0.0, l2 = 0.0, gs = 0.0;
-  for (int i = t; i < nprep; i += 256) sq += a.psq[static_cast<int64_t>(c) * nprep + i];
-  for (int i = t; i < nb64; i += 256) {
-    const double* p = a.plk + (static_cast<int64_t>(c) * (a.n / kTile) + i) * 4;
-    lm += p[0];
-    l1 += p[1];
-    l2 += p[2];
-    gs += p[3];
+  // Five FP64 sums, a warp each: as block-wide sums one after the other they
+  // held the launch (64 chains of 2,048 rows: 28.8 -> 13.8 us, with the
+  // column loads above in flight together).
+  const int warp = t >> 5, lane = t & 31;
+  if (warp < 5) {
+    double v = 0.0;
+    if (warp == 0) {
+      for (int i = lane; i < nprep; i += 32) v += a.psq[static_cast<int64_t>(c) * nprep + i];
+    } else {
+      const double* p = a.plk + static_cast<int64_t>(c) * (a.n / kTile) * 4 + (warp - 1);
+      for (int i = lane; i < nb64; i += 32) v += p[4 * i];
+    }
+    v = warp_sum(v);
+    if (lane == 0) red[warp] = v;
   }
-  sq = block_sum(sq, red);
-  lm = block_sum(lm, red);
-  l1 = block_sum(l1, red);
-  l2 = block_sum(l2, red);
-  gs = block_sum(gs, red);
+  __syncthreads();
   if (t != 0) return;
+  const double sq = red[0], lm = red[1], l1 = red[2], l2 = red[3], gs = red[4];
   if (a.fisher) {
     // b3: sum_i g_i and sum_i g_i^2; the correction's minimum starts at +inf.
     a.grad[static_cast<int64_t>(c) * s.P + s.ob3] = static_cast<float>(gs);
@@ -775,9 +783,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
   }
   double log_prior = 0.0;
   if (a.prior_scale > 0.f)
-    log_prior = -0.5 * sq / s2 -
-                static_cast<double>(s.P) * (log(static_cast<double>(a.prior_scale)) +
-                                            0.91893853320467274178);
+    log_prior = -0.5 * sq / s2 - a.prior_const;
   // -N * mean(lk) without a mask, -N/n * (lk . mask) with one (potential.py:183-185).
   const double lik = -static_cast<double>(a.n_obs) * (lm / nc);
   const double U = (lik - log_prior) / a.temperature;
@@ -915,15 +921,16 @@ T* view(void* ws, size_t off) {
   return reinterpret_cast<T*>(static_cast<unsigned char*>(ws) + off);
 }
 
-// A 256-wide GEMM of the network: on CTA pairs (tc_gemm2_kernel) for uniform
-// batches whose M is a multiple of 256, else on single CTAs.  tb_pair is the
-// B map for pairs (a K-major B is loaded in 128-row halves there).
+// A 256-wide GEMM of the network: on CTA pairs (tc_gemm2_kernel) where its M
+// is a multiple of 256, else on single CTAs.  tb_pair is the B map for pairs
+// (a K-major B is loaded in 128-row halves there).
 template <bool A_MN, bool B_MN, class Epi>
 int gemm256(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb_pair, int C,
-            int M, int N, int K, int* status, const Epi& e, cudaStream_t st,
-            const GemmRagged& rg, bool uniform) {
-  if (uniform && M % 256 == 0 && gemm_pair_enabled())
-    return launch_gemm2<kBN, A_MN, B_MN>(ta, tb_pair, C, M, N, K, status, e, st);
+            int M, int N, int K, int* status, const Epi& e, cudaStream_t st, GemmRagged rg,
+            bool pairs, bool reverse) {
+  rg.reverse = reverse;
+  if (pairs && M % 256 == 0 && gemm_pair_enabled())
+    return launch_gemm2<kBN, A_MN, B_MN>(ta, tb_pair, C, M, N, K, status, e, st, rg);
   return launch_gemm<kBN, A_MN, B_MN>(ta, tb, C, M, N, K, status, e, st, rg);
 }
 
@@ -948,12 +955,25 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
     a.pb1sq = view<float>(ws, L.pb1sq);
     a.fmin = view<uint32_t>(ws, L.fmin);
   }
+  a.pf = 0.f;
+  a.prior_const = 0.0;
+  if (a.prior_scale > 0.f) {
+    const double ps = a.prior_scale;
+    a.pf = static_cast<float>(1.0 / (ps * ps * a.temperature));
+    a.prior_const = static_cast<double>(s.P) * (std::log(ps) + 0.91893853320467274178);
+  }
   a.prefix1 = view<int>(ws, L.rag);
   a.prefix2 = a.prefix1 + (a.chains + 1);
   a.kblocks = a.prefix2 + (a.chains + 1);
   const int C = a.chains, n = a.n, D = s.D, H1 = s.H1, H2 = s.H2;
   // Ragged batches: GEMM tiles only over each chain's own rows.
+  // Pairs cover a ragged chain's rows in tiles of 256 instead of 128: with
+  // long minibatches what they save outweighs the extra half tile (32
+  // replicas of 64 to 4,096 rows: 3 % more rows, the four GEMMs of a gradient
+  // 479 -> 432 us).
   GemmRagged rows_h1, rows_h2, ksl;
+  const bool row_pairs = a.n_true == nullptr || (n % 256 == 0 && n >= 1024);
+  a.tile_rows = a.n_true != nullptr && row_pairs && gemm_pair_enabled() ? 256 : 128;
   if (a.n_true != nullptr) {
     mlp_ragged_kernel<<<1, 1, 0, st>>>(a);
     int rc0 = check_launch("mlp_ragged_kernel");
@@ -984,18 +1004,20 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
       (rc = make_tmap_bf16_3d(&m_z1, a.z1, H1, n, C, H1, s1, kGemmBK, kGemmBM)) ||
       (rc = make_tmap_bf16_3d(&m_w2, w2b, H2, H1, C, H2, pw, 64, 64)))
     return rc;
-  const bool uniform = a.n_true == nullptr;
+  // A GEMM walks the chains against the direction of the launch before it
+  // where that left a good part of its operands in L2 (64 chains of 2,048
+  // rows: dW1 62 -> 57 us, Z2 175 -> 170, dW2 222 -> 217).
   // 3: A1 = Xb W1 (W1 [D, H1] is the MN-major B operand).
   EpiHidden1 e1{a.w, s.P, s.ob1};
   if ((rc = make_tmap_rows(&e1.zmap, a.z1, false, H1, n, C, H1, s1))) return rc;
   if ((rc = gemm256<false, true>(m_xb, m_w1, m_w1, C, n, H1, D, a.status, e1, st, rows_h1,
-                                 uniform)))
+                                 row_pairs, false)))
     return rc;
   // 4: A2 = Z1 W2.
   EpiHidden2 e2{a.w, s.P, s.ob2, s.oW3, H2, n, a.outp};
   if ((rc = make_tmap_rows(&e2.zmap, a.z2g, false, H2, n, C, H2, s2))) return rc;
   if ((rc = gemm256<false, true>(m_z1, m_w2, m_w2, C, n, H2, H1, a.status, e2, st, rows_h2,
-                                 uniform)))
+                                 row_pairs, true)))
     return rc;
 
   if (a.fisher)
@@ -1013,17 +1035,15 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
         (rc = make_tmap_bf16_3d(&m_w2k_half, w2b, H2, H1, C, H2, pw, kGemmBK, kBN / 2)) ||
         (rc = make_tmap_bf16_3d(&m_xbmn, a.xb, D, n, C, D, sx, 64, 64)))
       return rc;
-    const double sc2 = static_cast<double>(a.prior_scale) * a.prior_scale;
-    const float pf = a.prior_scale > 0.f ? static_cast<float>(1.0 / (sc2 * a.temperature)) : 0.f;
     // 6: dW2 [H1, H2] = Z1^T G2 (both operands MN-major), before step 7
     //    overwrites Z1.
     // The prior's term pf w of W1 and W2 is added in the gradient GEMMs'
     // epilogues (not in the fused plans, whose update adds it, nor in the
     // Fisher model, which differentiates the likelihood alone).
-    const float pf_epi = a.fused || a.fisher ? 0.f : pf;
+    const float pf_epi = a.fused || a.fisher ? 0.f : a.pf;
     const EpiGradRows e6{a.grad, s.P, s.oW2, H2, a.w, pf_epi};
     if ((rc = gemm256<true, true>(m_z1mn, m_g2mn, m_g2mn, C, H1, H2, n, a.status, e6, st, ksl,
-                                  uniform)))
+                                  true, true)))
       return rc;
     if (a.fisher) {
       // 6b: sum_i d_i^2 of W2 = (Z1^2)^T (G2^2).
@@ -1037,18 +1057,19 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
         return rc;
       const EpiGradRows e6q{a.grad_sq, s.P, s.oW2, H2};
       if ((rc = gemm256<true, true>(m_qa, m_qb, m_qb, C, H1, H2, n, a.status, e6q, st, ksl,
-                                    uniform)))
+                                    true, false)))
         return rc;
     }
     // 7: G1 = (G2 W2^T) * (1 - Z1^2); W2 [H1, H2] is the K-major B operand.
     EpiAdjoint1 e7{a.z1, a.pb1, H1, n};
     if ((rc = make_tmap_rows(&e7.zmap, a.z1, false, H1, n, C, H1, s1))) return rc;
     if ((rc = gemm256<false, false>(m_g2, m_w2k, m_w2k_half, C, n, H1, H2, a.status, e7, st,
-                                    rows_h1, uniform)))
+                                    rows_h1, row_pairs, false)))
       return rc;
     // 8: dW1^T [H1, D] = G1^T Xb: GEMM row i (hidden unit), column f
     //    (feature) lands at dW1[f, i].
     const EpiGradCols e8{a.grad, s.P, s.oW1, H1, a.w, pf_epi};
+    ksl.reverse = true;
     if ((rc = launch_gemm<64, true, true>(m_z1mn, m_xbmn, C, H1, D, n, a.status, e8, st, ksl)))
       return rc;
     if (a.fisher) {

@@ -231,11 +231,13 @@ template <class Epi>
 int dispatch_pair(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb,
                   int batch, int M, int N, int K, int* status, const Epi& epi,
                   cudaStream_t st, uint64_t wait_ns) {
+  GemmRagged rg;
+  rg.wait_ns = wait_ns;
   if (a_mn)
-    return b_mn ? launch_gemm2<256, true, true>(ta, tb, batch, M, N, K, status, epi, st, wait_ns)
-                : launch_gemm2<256, true, false>(ta, tb, batch, M, N, K, status, epi, st, wait_ns);
-  return b_mn ? launch_gemm2<256, false, true>(ta, tb, batch, M, N, K, status, epi, st, wait_ns)
-              : launch_gemm2<256, false, false>(ta, tb, batch, M, N, K, status, epi, st, wait_ns);
+    return b_mn ? launch_gemm2<256, true, true>(ta, tb, batch, M, N, K, status, epi, st, rg)
+                : launch_gemm2<256, true, false>(ta, tb, batch, M, N, K, status, epi, st, rg);
+  return b_mn ? launch_gemm2<256, false, true>(ta, tb, batch, M, N, K, status, epi, st, rg)
+              : launch_gemm2<256, false, false>(ta, tb, batch, M, N, K, status, epi, st, rg);
 }
 
 template <int BN, class Epi>

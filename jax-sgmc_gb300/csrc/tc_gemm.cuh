@@ -228,6 +228,10 @@ struct GemmRagged {
   // stage or accumulator, a finished accumulator).  The waits of the clean-up
   // after a timeout (copies and MMAs already issued) keep kWaitLimitNs.
   uint64_t wait_ns = kWaitLimitNs;
+  // Tiles are taken last to first.  A GEMM that reads what the launch before
+  // it wrote first to last then starts with the part still in L2 (129 MB):
+  // callers alternate the direction along a chain of launches.
+  bool reverse = false;
 };
 
 __device__ __forceinline__ int ragged_batch(const GemmRagged& rg, int t, int per_batch,
@@ -300,6 +304,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   // (Virtual) batch of tile t, its index within the batch, its K slices and
   // the first of them.
   auto decode = [&](int t, int& b, int& r, int& KB, int& kb0) {
+    if (rg.reverse) t = tiles - 1 - t;
     b = ragged_batch(rg, t, per_batch, vbatch);
     r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
     KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK / rg.ksplit;
@@ -529,7 +534,7 @@ template <int BN, bool A_MN, bool B_MN, class Epi>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
     tc_gemm2_kernel(const __grid_constant__ CUtensorMap ta,
                     const __grid_constant__ CUtensorMap tb, int M, int N, int K, int batch,
-                    int* status, const __grid_constant__ Epi epi, uint64_t wait_ns) {
+                    int* status, const __grid_constant__ Epi epi, GemmRagged rg) {
   constexpr int BM = 2 * kGemmBM;  // rows of a pair tile, kGemmBM per CTA
   constexpr int BK = kGemmBK, STAGES = kGemm2Stages;
   constexpr int BNH = BN / 2;      // B rows held by each CTA
@@ -558,8 +563,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   const bool leader = rank == 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
-  const int tiles = per_batch * batch;
-  const int KB = K / BK;
+  const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
+                                              : per_batch * batch;
+  const uint64_t wait_ns = rg.wait_ns;
+  // Batch of tile t, its index within the batch and its K slices.
+  auto decode = [&](int t, int& b, int& r, int& KB) {
+    if (rg.reverse) t = tiles - 1 - t;
+    b = ragged_batch(rg, t, per_batch, batch);
+    r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
+    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK;
+  };
   const int first = static_cast<int>(tc::cluster_id());
   const int step = static_cast<int>(tc::cluster_count());
   const uint32_t peer_abort = tc::peer_addr(const_cast<int*>(abort_flag), rank ^ 1u);
@@ -597,7 +610,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       uint32_t it = 0;
       bool ok = true;
       for (int t = first; ok && t < tiles; t += step) {
-        const int b = t / per_batch, r = t % per_batch;
+        int b, r, KB;
+        decode(t, b, r, KB);
         const int m0 = (r / tiles_n) * BM + kGemmBM * static_cast<int>(rank);
         const int n0 = (r % tiles_n) * BN + BNH * static_cast<int>(rank);
         for (int kb = 0; kb < KB; ++kb, ++it) {
@@ -634,6 +648,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       uint32_t it = 0, acc = 0;
       bool ok = true;
       for (int t = first; ok && t < tiles; t += step, ++acc) {
+        int b, r, KB;
+        decode(t, b, r, KB);
         const uint32_t buf = acc & 1u, aph = (acc >> 1) & 1u;
         if (!tc::mbar_wait_cluster_bounded(&tempty[buf], aph ^ 1u, abort_flag, wait_ns)) {
           fail();
@@ -683,7 +699,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
         break;
       }
       tc::fence_after_sync();
-      const int b = t / per_batch, r = t % per_batch;
+      int b, r, KB;
+      decode(t, b, r, KB);
       const int row0 = (r / tiles_n) * BM + kGemmBM * static_cast<int>(rank) + q * 32;
       const uint32_t tbase =
           tmem + buf * BN + h * NC + (static_cast<uint32_t>(q * 32) << 16);
@@ -713,14 +730,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   }
 }
 
-// Launches the pair GEMM on `st` (uniform batches; M a multiple of 256, N of
-// BN, K of 64): one cluster per co-resident pair slot, at most one per pair
+// Launches the pair GEMM on `st` (M a multiple of 256, N of BN, K of 64; a
+// ragged batch's tile_prefix counts 256-row tiles): one cluster per co-resident pair slot, at most one per pair
 // tile.  Tensor maps as for launch_gemm except that a K-major B map has
 // boxes of 64 x BN/2.
 template <int BN, bool A_MN, bool B_MN, class Epi>
 int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, int batch, int M, int N, int K,
                  int* status, const Epi& epi, cudaStream_t st,
-                 uint64_t wait_ns = kWaitLimitNs) {
+                 GemmRagged rg = GemmRagged{}) {
   auto kern = tc_gemm2_kernel<BN, A_MN, B_MN, Epi>;
   const size_t smem = gemm2_smem_bytes(BN);
   static int max_clusters = 0;
@@ -747,7 +764,7 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, int batch, int M,
     return set_error(GBSGMC_ERR_SHAPE, "gemm (pairs): needs M %% 256, N %% %d, K %% 64", BN);
   const int64_t tiles = static_cast<int64_t>(M / (2 * kGemmBM)) * (N / BN) * batch;
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
-  kern<<<2 * clusters, kGemmThreads, smem, st>>>(ta, tb, M, N, K, batch, status, epi, wait_ns);
+  kern<<<2 * clusters, kGemmThreads, smem, st>>>(ta, tb, M, N, K, batch, status, epi, rg);
   return check_launch("tc_gemm2_kernel");
 }
 
