@@ -181,6 +181,8 @@ __device__ __forceinline__ float bf(bf16 v) { return __bfloat162float(v); }
 // groups >= 6 and outputs >= 32.  Grid (kPrepBlocks, chains).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) cnn_prep_kernel(const CnnArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double red[32];
   const int c = blockIdx.y;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
@@ -226,6 +228,8 @@ __host__ __device__ __forceinline__ void conv1_pixel(int r, int& h, int& w) {
 // Grid (n*1024/256, chains): one thread per pixel, one 16-byte store each.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) cnn_gather1_kernel(const CnnArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int p = blockIdx.x * 256 + threadIdx.x;
   if (p >= a.n * 1024) return;
@@ -265,6 +269,8 @@ __global__ void __launch_bounds__(256) cnn_gather1_kernel(const CnnArgs a) {
 // ---------------------------------------------------------------------------
 template <int H, int W, int C, int Kp>
 __global__ void __launch_bounds__(256) cnn_im2col_kernel(const bf16* Pin, bf16* Col, int n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int G = 9 * C / 8;  // 8-column groups per row
   const int c = blockIdx.y;
   const int groups = n * H * W * G;
@@ -300,6 +306,8 @@ constexpr size_t kDenseSmem =
     sizeof(float) * kFlat * kClasses + sizeof(bf16) * kDenseImgs * kFlat;
 
 __global__ void __launch_bounds__(kDenseImgs * 16) cnn_dense_kernel(const CnnArgs a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ float wd_s[];  // Wd [2048][10], then P3 rows [kDenseImgs][2048]
   bf16* x_s = reinterpret_cast<bf16*>(wd_s + kFlat * kClasses);
   __shared__ float g_s[kDenseImgs][kClasses];
@@ -388,6 +396,8 @@ __global__ void __launch_bounds__(kDenseImgs * 16) cnn_dense_kernel(const CnnArg
 // partial sums are added in group order.  dlogits are staged in shared
 // memory 512 images at a time.
 __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float gs[512 * kClasses];
   __shared__ float red[3][128 * kClasses];
   const int c = blockIdx.y, t = threadIdx.x, q = t >> 7;
@@ -464,6 +474,8 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
 template <int H, int W, int C, int ld, bool kConv1Rows = false>
 __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t* M,
                                                         const float* dp, int n, float* bpart) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[256 * 8];
   const int c = blockIdx.y;
   const int Ho = H / 2, Wo = W / 2;
@@ -526,6 +538,8 @@ constexpr int kBiasT = 1024;
 
 __global__ void __launch_bounds__(kBiasT) cnn_bias_sum_kernel(const float* bpart, int blocks,
                                                               int C, float* grad, int64_t off) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float acc[kBiasT];
   const int c = blockIdx.x, t = threadIdx.x, ch = t % C, g0 = t / C, step = kBiasT / C;
   const float* p = bpart + static_cast<int64_t>(c) * blocks * C + ch;
@@ -545,6 +559,8 @@ __global__ void __launch_bounds__(kBiasT) cnn_bias_sum_kernel(const float* bpart
 // over e < K * Cout (HWIO order).  Grid (ceil(K*Cout/256), chains).
 __global__ void __launch_bounds__(256) cnn_wsum_kernel(const float* part, int splits, int count,
                                                       float* grad, int64_t off) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
   if (e >= count) return;
   const float* p = part + static_cast<int64_t>(c) * splits * count + e;
@@ -556,6 +572,8 @@ __global__ void __launch_bounds__(256) cnn_wsum_kernel(const float* part, int sp
 // grad += w / (s^2 T) over every parameter; U and var(lk).  Grid
 // (ceil(P/256), chains); block 0 of a chain also writes U, var.
 __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a, float pf) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double red[32];
   const int c = blockIdx.y, t = threadIdx.x;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
@@ -954,7 +972,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   // gradient from the unpool blocks' partials.
   auto bias_sum = [&](int H, int Cr, int64_t off) {
     const int blocks = grid1(int64_t(n) * (H / 2) * (H / 2) * Cr / 8);
-    cnn_bias_sum_kernel<<<C, kBiasT, 0, st>>>(a.bpart, blocks, Cr, a.grad, off);
+    launch_pdl(cnn_bias_sum_kernel, C, kBiasT, 0, st, a.bpart, blocks, Cr, a.grad, off);
     return launched("cnn_bias_sum_kernel");
   };
   auto unpool_grid = [&](int H, int Cr) {
@@ -970,14 +988,14 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     int r = launch_gemm<64, true, true>(mdy, mcol, C, 128, Kp, static_cast<int>(rows), a.status,
                                         e, st, rg);
     if (r) return r;
-    cnn_wsum_kernel<<<dim3(grid1(int64_t(K) * Cout), C), 256, 0, st>>>(a.part, rg.ksplit,
+    launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(K) * Cout), C), 256, 0, st, a.part, rg.ksplit,
                                                                        K * Cout, a.grad, off);
     return launched("cnn_wsum_kernel");
   };
 
-  cnn_prep_kernel<<<dim3(kPrepBlocks, C), 256, 0, st>>>(a);
+  launch_pdl(cnn_prep_kernel, dim3(kPrepBlocks, C), 256, 0, st, a);
   if ((rc = launched("cnn_prep_kernel"))) return rc;
-  cnn_gather1_kernel<<<dim3(grid1(r1), C), 256, 0, st>>>(a);
+  launch_pdl(cnn_gather1_kernel, dim3(grid1(r1), C), 256, 0, st, a);
   if ((rc = launched("cnn_gather1_kernel"))) return rc;
 
   // Tensor maps (columns, rows, chains), and 4-D maps (channels, W, H,
@@ -1007,7 +1025,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   const Conv1Fwd<EpiConvPool<32, 32, 16, true>> e1{{a.w, ob1, kC1, a.p1, a.m1, n}, n};
   if ((rc = launch_gemm<64, false, false>(m_x8, m_w1i, C, r1, 64, kK1i, a.status, e1, st)))
     return rc;
-  cnn_im2col_kernel<16, 16, kC1, kK2p><<<dim3(grid1(r2 * kK2 / 8), C), 256, 0, st>>>(
+  launch_pdl(cnn_im2col_kernel<16, 16, kC1, kK2p>, dim3(grid1(r2 * kK2 / 8), C), 256, 0, st, 
       a.p1, a.col2, n);
   if ((rc = launched("cnn_im2col_kernel 2"))) return rc;
   const EpiConvPool<16, 16, 16, false> e2{a.w, ob2, kC2, a.p2, a.m2, n};
@@ -1022,17 +1040,16 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       cnn_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDenseSmem));
   if (dense_attr != cudaSuccess)
     return set_error(GBSGMC_ERR_CUDA, "cnn_dense_kernel: %s", cudaGetErrorString(dense_attr));
-  cnn_dense_kernel<<<dim3((n + kDenseImgs - 1) / kDenseImgs, C), kDenseImgs * 16, kDenseSmem,
-                     st>>>(a);
+  launch_pdl(cnn_dense_kernel, dim3((n + kDenseImgs - 1) / kDenseImgs, C), kDenseImgs * 16, kDenseSmem, st, a);
   if ((rc = launched("cnn_dense_kernel"))) return rc;
 
   if (a.want_grad) {
-    cnn_dense_grad_kernel<<<dim3(kFlat / 128 + 1, C), 512, 0, st>>>(a);
+    launch_pdl(cnn_dense_grad_kernel, dim3(kFlat / 128 + 1, C), 512, 0, st, a);
     if ((rc = launched("cnn_dense_grad_kernel"))) return rc;
     // Layer 3: dY3 (routing of dP3), db3, dW3 = dY3^T Col3 (implicit: B
     // blocks are P2's tap-shifted images), dP2 = the transposed convolution
     // of dY3 (implicit: A tiles are dY3's tap-shifted 2-image boxes).
-    cnn_unpool_kernel<8, 8, kC3, kC3><<<unpool_grid(8, kC3), 256, 0, st>>>(
+    launch_pdl(cnn_unpool_kernel<8, 8, kC3, kC3>, unpool_grid(8, kC3), 256, 0, st, 
         a.dy3, a.m3, a.dp3, n, a.bpart);
     if ((rc = launched("cnn_unpool_kernel 3")) || (rc = bias_sum(8, kC3, ob3))) return rc;
     CUtensorMap m_dy3t, m_p2b, m_dy3a, m_w3t;
@@ -1051,7 +1068,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       if ((rc = launch_gemm<64, true, true>(m_dy3t, m_p2b, C, 128, kK3, static_cast<int>(r3),
                                             a.status, e, st, rg)))
         return rc;
-      cnn_wsum_kernel<<<dim3(grid1(int64_t(kK3) * kC3), C), 256, 0, st>>>(a.part, rg.ksplit,
+      launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(kK3) * kC3), C), 256, 0, st, a.part, rg.ksplit,
                                                                           kK3 * kC3, a.grad, oW3);
       if ((rc = launched("cnn_wsum_kernel"))) return rc;
     }
@@ -1061,7 +1078,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       return rc;
     // Layer 2: dY2 (routing of dP2), db2, dW2 = dY2^T Col2, dP1 = the
     // transposed convolution of dY2 (implicit).
-    cnn_unpool_kernel<16, 16, kC2, kC2><<<unpool_grid(16, kC2), 256, 0, st>>>(
+    launch_pdl(cnn_unpool_kernel<16, 16, kC2, kC2>, unpool_grid(16, kC2), 256, 0, st, 
         a.dy2, a.m2, a.dp2, n, a.bpart);
     if ((rc = launched("cnn_unpool_kernel 2")) || (rc = bias_sum(16, kC2, ob2))) return rc;
     CUtensorMap m_dy2t, m_col2t, m_dy2a, m_w2t;
@@ -1079,7 +1096,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
                                             st)))
       return rc;
     // Layer 1.
-    cnn_unpool_kernel<32, 32, kC1, kA1ld, true><<<unpool_grid(32, kC1), 256, 0, st>>>(
+    launch_pdl(cnn_unpool_kernel<32, 32, kC1, kA1ld, true>, unpool_grid(32, kC1), 256, 0, st, 
         a.dy1, a.m1, a.dp1, n, a.bpart);
     if ((rc = launched("cnn_unpool_kernel 1")) || (rc = bias_sum(32, kC1, ob1))) return rc;
     // dW1 = dY1^T Col1, Col1 read by K group from X8 (N = 8 groups x 8 slots).
@@ -1093,7 +1110,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       if ((rc = launch_gemm<64, true, true>(m_dy1t, m_x8h, C, 128, kK1i, static_cast<int>(r1),
                                             a.status, e, st, rg)))
         return rc;
-      cnn_wsum_kernel<<<dim3(grid1(int64_t(kK1) * kC1), C), 256, 0, st>>>(a.part, rg.ksplit,
+      launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(kK1) * kC1), C), 256, 0, st, a.part, rg.ksplit,
                                                                           kK1 * kC1, a.grad, oW1);
       if ((rc = launched("cnn_wsum_kernel"))) return rc;
     }
@@ -1101,7 +1118,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
 
   const double s2 = static_cast<double>(a.prior_scale) * a.prior_scale;
   const float pf = a.prior_scale > 0.f ? static_cast<float>(1.0 / (s2 * a.temperature)) : 0.f;
-  cnn_finalize_kernel<<<dim3(a.want_grad ? grid1(kP) : 1, C), 256, 0, st>>>(a, pf);
+  launch_pdl(cnn_finalize_kernel, dim3(a.want_grad ? grid1(kP) : 1, C), 256, 0, st, a, pf);
   return launched("cnn_finalize_kernel");
 }
 

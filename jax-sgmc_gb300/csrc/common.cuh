@@ -23,6 +23,35 @@ __device__ __forceinline__ void raise_status(int* status, int code) {
   if (status != nullptr) atomicCAS(status, 0, code);
 }
 
+// Programmatic dependent launch: a kernel launched by launch_pdl may start
+// while the launch before it on the stream still runs.  pdl_wait returns
+// when that launch has completed (and with it, every one before), so it
+// comes before the first access to global memory; pdl_trigger lets the next
+// launch start once every block of this one has called it or ended.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// Launches `kern` (which calls pdl_wait) as a programmatic dependent of the
+// stream's previous launch: its launch latency and set-up overlap that
+// launch's end (some 2 us per launch of a chain of short kernels).
+template <class... P, class... A>
+inline void launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                       A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);   // its error is read by check_launch
+}
+
 // Nanosecond global timer, used to bound every spin-wait.
 __device__ __forceinline__ uint64_t global_ns() {
   uint64_t t;

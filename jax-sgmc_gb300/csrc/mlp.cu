@@ -238,6 +238,8 @@ __device__ __forceinline__ int chain_rows_padded(const MlpArgs& a, int c) {
 
 // Tile tables of a ragged batch for the GEMMs (one thread).
 __global__ void mlp_ragged_kernel(const MlpArgs a) {
+  pdl_trigger();
+  pdl_wait();
   int p1 = 0, p2 = 0;
   a.prefix1[0] = 0;
   a.prefix2[0] = 0;
@@ -260,6 +262,8 @@ __global__ void mlp_ragged_kernel(const MlpArgs a) {
 //    the vector leaves W3 | b1 | b2 | b3.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) mlp_prep_kernel(const MlpArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double red[32];
   const MlpShape& s = a.s;
   const int c = blockIdx.y, blk = blockIdx.x, t = threadIdx.x;
@@ -297,6 +301,8 @@ __global__ void __launch_bounds__(256) mlp_prep_kernel(const MlpArgs a) {
 //    Grid (n/64, D/64, chains).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) mlp_gather_kernel(const MlpArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int64_t rows[kTile];
   const MlpShape& s = a.s;
   const int i0 = blockIdx.x * kTile, f0 = blockIdx.y * kTile, c = blockIdx.z;
@@ -562,6 +568,8 @@ struct EpiGradCols {
 // ---------------------------------------------------------------------------
 template <bool kFisher>
 __global__ void __launch_bounds__(256, kFisher ? 2 : 3) mlp_out_kernel(const MlpArgs a) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int kParts = kFisher ? 4 : 2;
   __shared__ float g_s[kTile];
   __shared__ double red[2][4];
@@ -710,6 +718,8 @@ __global__ void __launch_bounds__(256, kFisher ? 2 : 3) mlp_out_kernel(const Mlp
 //    (ceil(max(H1,H2)/256), chains) with a gradient, (1, chains) without.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int nprep) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ double red[32];
   const MlpShape& s = a.s;
   const int c = blockIdx.y, t = threadIdx.x;
@@ -804,6 +814,8 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
 __global__ void __launch_bounds__(256) mlp_square_kernel(const bf16* __restrict__ src,
                                                          bf16* __restrict__ dst, int n, int H,
                                                          float* colsq) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float part[32][65];
   const int t = threadIdx.x, cc = t & 7, rg = t >> 3;
   const int64_t base = static_cast<int64_t>(blockIdx.z) * n * H;
@@ -846,6 +858,8 @@ __global__ void __launch_bounds__(256) mlp_fisher_corr_kernel(
     int64_t P, int n, float n_obs, float h, const float* __restrict__ grad,
     const float* __restrict__ fric, float friction, const float* __restrict__ s1, float* s2,
     uint32_t* fmin) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[8];
   const int c = blockIdx.y;
   const float scale_v = 1.0f / static_cast<float>(n - 1);
@@ -877,6 +891,8 @@ __global__ void __launch_bounds__(256) mlp_fisher_apply_kernel(int64_t P,
                                                                float friction,
                                                                const uint32_t* __restrict__ fmin,
                                                                float* cb, float* bs) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const float smallest = __uint_as_float(fmin[c]);
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; p < P;
@@ -975,7 +991,7 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
   const bool row_pairs = a.n_true == nullptr || (n % 256 == 0 && n >= 1024);
   a.tile_rows = a.n_true != nullptr && row_pairs && gemm_pair_enabled() ? 256 : 128;
   if (a.n_true != nullptr) {
-    mlp_ragged_kernel<<<1, 1, 0, st>>>(a);
+    launch_pdl(mlp_ragged_kernel, 1, 1, 0, st, a);
     int rc0 = check_launch("mlp_ragged_kernel");
     if (rc0 != GBSGMC_OK) return rc0;
     rows_h1.tile_prefix = a.prefix1;
@@ -989,10 +1005,10 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
   int rc;
 
   if (!a.fused) {
-    mlp_prep_kernel<<<dim3(nprep, C), 256, 0, st>>>(a);
+    launch_pdl(mlp_prep_kernel, dim3(nprep, C), 256, 0, st, a);
     if ((rc = check_launch("mlp_prep_kernel")) != GBSGMC_OK) return rc;
   }
-  mlp_gather_kernel<<<dim3(n / kTile, D / kTile, C), 256, 0, st>>>(a);
+  launch_pdl(mlp_gather_kernel, dim3(n / kTile, D / kTile, C), 256, 0, st, a);
   if ((rc = check_launch("mlp_gather_kernel")) != GBSGMC_OK) return rc;
 
   // Tensor maps (columns, rows, chains).  K-major operands use 64 x 128 (A)
@@ -1021,9 +1037,9 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
     return rc;
 
   if (a.fisher)
-    mlp_out_kernel<true><<<dim3(n / kTile, C), 256, 0, st>>>(a);
+    launch_pdl(mlp_out_kernel<true>, dim3(n / kTile, C), 256, 0, st, a);
   else
-    mlp_out_kernel<false><<<dim3(n / kTile, C), 256, 0, st>>>(a);
+    launch_pdl(mlp_out_kernel<false>, dim3(n / kTile, C), 256, 0, st, a);
   if ((rc = check_launch("mlp_out_kernel")) != GBSGMC_OK) return rc;
 
   if (a.want_grad) {
@@ -1047,9 +1063,9 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
       return rc;
     if (a.fisher) {
       // 6b: sum_i d_i^2 of W2 = (Z1^2)^T (G2^2).
-      mlp_square_kernel<<<dim3(n / kTile, H1 / 64, C), 256, 0, st>>>(a.z1, a.sqa, n, H1, nullptr);
+      launch_pdl(mlp_square_kernel, dim3(n / kTile, H1 / 64, C), 256, 0, st, a.z1, a.sqa, n, H1, nullptr);
       if ((rc = check_launch("mlp_square_kernel")) != GBSGMC_OK) return rc;
-      mlp_square_kernel<<<dim3(n / kTile, H2 / 64, C), 256, 0, st>>>(a.z2g, a.sqb, n, H2, nullptr);
+      launch_pdl(mlp_square_kernel, dim3(n / kTile, H2 / 64, C), 256, 0, st, a.z2g, a.sqb, n, H2, nullptr);
       if ((rc = check_launch("mlp_square_kernel")) != GBSGMC_OK) return rc;
       CUtensorMap m_qa, m_qb;
       if ((rc = make_tmap_bf16_3d(&m_qa, a.sqa, H1, n, C, H1, s1, 64, 64)) ||
@@ -1074,9 +1090,9 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
       return rc;
     if (a.fisher) {
       // 8b: sum_i d_i^2 of W1 = (G1^2)^T (Xb^2), and b1's sums of squares.
-      mlp_square_kernel<<<dim3(n / kTile, H1 / 64, C), 256, 0, st>>>(a.z1, a.sqa, n, H1, a.pb1sq);
+      launch_pdl(mlp_square_kernel, dim3(n / kTile, H1 / 64, C), 256, 0, st, a.z1, a.sqa, n, H1, a.pb1sq);
       if ((rc = check_launch("mlp_square_kernel")) != GBSGMC_OK) return rc;
-      mlp_square_kernel<<<dim3(n / kTile, D / 64, C), 256, 0, st>>>(a.xb, a.sqb, n, D, nullptr);
+      launch_pdl(mlp_square_kernel, dim3(n / kTile, D / 64, C), 256, 0, st, a.xb, a.sqb, n, D, nullptr);
       if ((rc = check_launch("mlp_square_kernel")) != GBSGMC_OK) return rc;
       CUtensorMap m_qa, m_qx;
       if ((rc = make_tmap_bf16_3d(&m_qa, a.sqa, H1, n, C, H1, s1, 64, 64)) ||
@@ -1088,7 +1104,7 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
     }
   }
   const int fx = a.want_grad ? ceil_div(H1 > H2 ? H1 : H2, 256) : 1;
-  mlp_finalize_kernel<<<dim3(fx, C), 256, 0, st>>>(a, nprep);
+  launch_pdl(mlp_finalize_kernel, dim3(fx, C), 256, 0, st, a, nprep);
   return check_launch("mlp_finalize_kernel");
 }
 
@@ -1289,11 +1305,11 @@ extern "C" int gbsgmc_mlp_fisher_noise(const gbsgmc_mlp* model, int chains, int 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if ((rc = run_mlp(a, L, workspace_dev, st)) != GBSGMC_OK) return rc;
   const int gx = static_cast<int>(std::min<int64_t>((s.P + 1023) / 1024, 1024));
-  mlp_fisher_corr_kernel<<<dim3(gx, chains), 256, 0, st>>>(
+  launch_pdl(mlp_fisher_corr_kernel, dim3(gx, chains), 256, 0, st, 
       s.P, n, static_cast<float>(model->n_obs), step_size, grad_dev, friction_dev, friction,
       b_sqrt_dev, cb_diff_sqrt_dev, a.fmin);
   if ((rc = check_launch("mlp_fisher_corr_kernel")) != GBSGMC_OK) return rc;
-  mlp_fisher_apply_kernel<<<dim3(gx, chains), 256, 0, st>>>(s.P, friction_dev, friction, a.fmin,
+  launch_pdl(mlp_fisher_apply_kernel, dim3(gx, chains), 256, 0, st, s.P, friction_dev, friction, a.fmin,
                                                             cb_diff_sqrt_dev, b_sqrt_dev);
   return check_launch("mlp_fisher_apply_kernel");
 }

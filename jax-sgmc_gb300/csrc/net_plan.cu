@@ -19,6 +19,8 @@ namespace gbsgmc {
 namespace {
 
 __global__ void mean_pair_kernel(int chains, double* a, const double* b) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < chains) a[c] = 0.5 * (a[c] + b[c]);
 }
@@ -287,7 +289,7 @@ int NetPlan::enqueue_obabo(int g, const UpdateFusion& moving, const UpdateFusion
   if ((rc = obabo_second_fused(chains, P, x, aux, grad2, integ.mass_dev, integ.friction,
                                ke_end, &sj, &noise, last, s)))
     return rc;
-  mean_pair_kernel<<<(chains + 127) / 128, 128, 0, s>>>(chains, U, U2);
+  launch_pdl(mean_pair_kernel, (chains + 127) / 128, 128, 0, s, chains, U, U2);
   return check_launch("plan: potential mean");
 }
 

@@ -297,20 +297,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
-  const int vbatch = batch * rg.ksplit;
-  const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
-                                              : per_batch * vbatch;
-  // (Virtual) batch of tile t, its index within the batch, its K slices and
-  // the first of them.
-  auto decode = [&](int t, int& b, int& r, int& KB, int& kb0) {
-    if (rg.reverse) t = tiles - 1 - t;
-    b = ragged_batch(rg, t, per_batch, vbatch);
-    r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
-    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK / rg.ksplit;
-    kb0 = (b % rg.ksplit) * KB;
-  };
-
   if (threadIdx.x == 0) {
     for (int i = 0; i < STAGES; ++i) {
       mbar_init(&full[i], 1);
@@ -332,6 +318,22 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  // The set-up above touched nothing that an earlier launch writes.
+  pdl_trigger();
+  pdl_wait();
+  const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
+  const int vbatch = batch * rg.ksplit;
+  const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
+                                              : per_batch * vbatch;
+  // (Virtual) batch of tile t, its index within the batch, its K slices and
+  // the first of them.
+  auto decode = [&](int t, int& b, int& r, int& KB, int& kb0) {
+    if (rg.reverse) t = tiles - 1 - t;
+    b = ragged_batch(rg, t, per_batch, vbatch);
+    r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
+    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK / rg.ksplit;
+    kb0 = (b % rg.ksplit) * KB;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -508,7 +510,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int batch, int M,
     return set_error(GBSGMC_ERR_CUDA, "gemm: cannot query the device");
   const int64_t tiles = static_cast<int64_t>(M / kGemmBM) * (N / BN) * batch * rg.ksplit;
   const int grid = static_cast<int>(tiles < int64_t(sms) * per_sm ? tiles : int64_t(sms) * per_sm);
-  kern<<<grid, kGemmThreads, smem, st>>>(ta, tb, M, N, K, batch, status, epi, rg);
+  launch_pdl(kern, grid, kGemmThreads, smem, st, ta, tb, M, N, K, batch, status, epi, rg);
   return check_launch("tc_gemm_kernel");
 }
 
@@ -562,17 +564,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   const uint32_t rank = tc::cluster_rank();
   const bool leader = rank == 0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
-  const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
-                                              : per_batch * batch;
-  const uint64_t wait_ns = rg.wait_ns;
-  // Batch of tile t, its index within the batch and its K slices.
-  auto decode = [&](int t, int& b, int& r, int& KB) {
-    if (rg.reverse) t = tiles - 1 - t;
-    b = ragged_batch(rg, t, per_batch, batch);
-    r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
-    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK;
-  };
   const int first = static_cast<int>(tc::cluster_id());
   const int step = static_cast<int>(tc::cluster_count());
   const uint32_t peer_abort = tc::peer_addr(const_cast<int*>(abort_flag), rank ^ 1u);
@@ -604,6 +595,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   tc::cluster_sync();  // both CTAs' barriers and flags are initialised
   tc::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
+  // The set-up above touched nothing that an earlier launch writes.
+  pdl_trigger();
+  pdl_wait();
+  const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
+  const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
+                                              : per_batch * batch;
+  const uint64_t wait_ns = rg.wait_ns;
+  // Batch of tile t, its index within the batch and its K slices.
+  auto decode = [&](int t, int& b, int& r, int& KB) {
+    if (rg.reverse) t = tiles - 1 - t;
+    b = ragged_batch(rg, t, per_batch, batch);
+    r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
+    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK;
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -764,7 +769,8 @@ int launch_gemm2(const CUtensorMap& ta, const CUtensorMap& tb, int batch, int M,
     return set_error(GBSGMC_ERR_SHAPE, "gemm (pairs): needs M %% 256, N %% %d, K %% 64", BN);
   const int64_t tiles = static_cast<int64_t>(M / (2 * kGemmBM)) * (N / BN) * batch;
   const int clusters = static_cast<int>(tiles < max_clusters ? tiles : max_clusters);
-  kern<<<2 * clusters, kGemmThreads, smem, st>>>(ta, tb, M, N, K, batch, status, epi, rg);
+  launch_pdl(kern, 2 * clusters, kGemmThreads, smem, st, ta, tb, M, N, K, batch, status, epi,
+             rg);
   return check_launch("tc_gemm2_kernel");
 }
 

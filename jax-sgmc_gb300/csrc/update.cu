@@ -106,6 +106,8 @@ __device__ __forceinline__ void store4(float* __restrict__ a, int64_t j0, int64_
 }
 
 __global__ void mirror_kernel(int64_t P, const float* x, Fuse f) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t groups = (P + 3) / 4;
   const int64_t off = static_cast<int64_t>(c) * P;
@@ -126,6 +128,8 @@ __global__ void mirror_kernel(int64_t P, const float* x, Fuse f) {
 __global__ void __launch_bounds__(kThreads, 4)
 sgld_update_kernel(int chains, int64_t P, float* x, const float* g, float* v, float alpha,
                    float lmbd, Sched sched, Noise noise, float* samples, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const float h = sched.step_size(k);
@@ -216,6 +220,8 @@ __device__ __forceinline__ void obabo_second_elem(const ObaboCoef& q, float mi, 
 __global__ void obabo_first_kernel(
     int chains, int64_t P, float* x, float* p, const float* g1, const float* mass,
     float friction, double* ke_start, Sched sched, Noise noise, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const ObaboCoef qc = obabo_coef(sched, k, c, friction);
@@ -251,6 +257,8 @@ __global__ void obabo_first_kernel(
 __global__ void obabo_second_kernel(
     int chains, int64_t P, const float* x, float* p, const float* g2, const float* mass,
     float friction, double* ke_end, Sched sched, Noise noise, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const ObaboCoef qc = obabo_coef(sched, k, c, friction);
@@ -288,6 +296,8 @@ __global__ void obabo_second_first_kernel(
     int chains, int64_t P, float* x, float* p, const float* g2, const float* g1,
     const float* mass, float friction, double* ke_end, double* ke_start, Sched sched,
     Noise noise, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const ObaboCoef q2 = obabo_coef(sched, k, c, friction);
@@ -330,6 +340,8 @@ __global__ void obabo_second_first_kernel(
 __global__ void sghmc_resample_kernel(int chains, int64_t P, float* p,
                                       const float* mass, Sched sched,
                                       Noise noise) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const int64_t groups = (P + 3) / 4;
@@ -351,6 +363,8 @@ __global__ void sghmc_position_kernel(int chains, int64_t P, float* x,
                                       float* p, const float* mass,
                                       const float* fric, float friction,
                                       Sched sched, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const float h = sched.step_size(k);
@@ -380,6 +394,8 @@ __global__ void sghmc_momentum_kernel(int chains, int64_t P, const float* x, flo
                                       const float* g, const float* fric,
                                       float friction, Sched sched,
                                       Noise noise, Fuse fz) {
+  pdl_trigger();
+  pdl_wait();
   const int c = blockIdx.y;
   const int64_t k = sched.step();
   const float h = sched.step_size(k);
@@ -508,6 +524,8 @@ __global__ void swap_rows_kernel(int pairs, int64_t width, float* a, float* b,
 // Stochastic-approximation update of the adjacent-pair variance estimates
 // (one block): k += 1, ssq[r] = (1 - 1/k) ssq[r] + (1/k) var[r].
 __global__ void resgld_sa_kernel(int replicas, const double* var, double* ssq, int64_t* kc) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t k = kc[0] + 1;
   __syncthreads();
   if (threadIdx.x == 0) kc[0] = k;
@@ -526,6 +544,8 @@ __global__ void resgld_decide_kernel(int replicas, Sched sched, int every, doubl
                                      double* var, const double* ssq, double F, uint64_t seed,
                                      const double* u_in, int32_t* flags, int32_t* counts,
                                      double* log_s_out) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t k = sched.step();
   const int64_t round = (k + 1) / every;
   const int parity = static_cast<int>(round & 1);
@@ -562,6 +582,8 @@ __global__ void resgld_decide_kernel(int replicas, Sched sched, int every, doubl
 }
 
 __global__ void swap_adjacent_rows_kernel(int64_t width, float* a, const int32_t* flags) {
+  pdl_trigger();
+  pdl_wait();
   const int r = blockIdx.y;
   if (flags[r] == 0) return;
   float* x = a + static_cast<int64_t>(r) * width;
@@ -708,7 +730,7 @@ extern "C" int gbsgmc_sgld_update(int chains, int64_t P, float* x_dev,
     return set_error(GBSGMC_ERR_ARG, "sgld_update: keep table without samples");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  sgld_update_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(sgld_update_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, x_dev, g_dev, v_dev, alpha, lmbd, to_sched(sched),
       to_noise(noise), samples_dev, to_fuse(nullptr));
   return check_launch("sgld_update");
@@ -727,7 +749,7 @@ extern "C" int gbsgmc_obabo_first(int chains, int64_t P, float* x_dev,
     return set_error(GBSGMC_ERR_ARG, "obabo_first: null pointer");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  obabo_first_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(obabo_first_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, x_dev, p_dev, g1_dev, mass_dev, friction, ke_start_dev,
       to_sched(sched), to_noise(noise), to_fuse(nullptr));
   return check_launch("obabo_first");
@@ -745,7 +767,7 @@ extern "C" int gbsgmc_obabo_second(int chains, int64_t P, float* p_dev,
     return set_error(GBSGMC_ERR_ARG, "obabo_second: null pointer");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  obabo_second_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(obabo_second_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, nullptr, p_dev, g2_dev, mass_dev, friction, ke_end_dev,
       to_sched(sched), to_noise(noise), to_fuse(nullptr));
   return check_launch("obabo_second");
@@ -762,7 +784,7 @@ extern "C" int gbsgmc_sghmc_resample(int chains, int64_t P, float* p_dev,
     return set_error(GBSGMC_ERR_ARG, "sghmc_resample: null pointer");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  sghmc_resample_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(sghmc_resample_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, p_dev, mass_dev, to_sched(sched), to_noise(noise));
   return check_launch("sghmc_resample");
 }
@@ -778,7 +800,7 @@ extern "C" int gbsgmc_sghmc_position(int chains, int64_t P, float* x_dev,
     return set_error(GBSGMC_ERR_ARG, "sghmc_position: null pointer");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  sghmc_position_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(sghmc_position_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, x_dev, p_dev, mass_dev, friction_dev, friction,
       to_sched(sched), to_fuse(nullptr));
   return check_launch("sghmc_position");
@@ -796,7 +818,7 @@ extern "C" int gbsgmc_sghmc_momentum(int chains, int64_t P, float* p_dev,
     return set_error(GBSGMC_ERR_ARG, "sghmc_momentum: null pointer");
   if (chains == 0 || P == 0) return GBSGMC_OK;
   const Grid4 g = grid4(chains, P);
-  sghmc_momentum_kernel<<<g.grid, kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+  launch_pdl(sghmc_momentum_kernel, g.grid, kThreads, 0, static_cast<cudaStream_t>(stream), 
       chains, P, nullptr, p_dev, g_dev, friction_dev, friction, to_sched(sched),
       to_noise(noise), to_fuse(nullptr));
   return check_launch("sghmc_momentum");
@@ -927,7 +949,7 @@ extern "C" int gbsgmc_resgld_sa_update(int replicas, const double* lk_var_dev, d
   if (replicas < 2 || replicas > 65536 || lk_var_dev == nullptr || ssq_dev == nullptr ||
       k_dev == nullptr)
     return set_error(GBSGMC_ERR_ARG, "resgld_sa_update: bad arguments");
-  resgld_sa_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(replicas, lk_var_dev,
+  launch_pdl(resgld_sa_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), replicas, lk_var_dev,
                                                                      ssq_dev, k_dev);
   return check_launch("resgld_sa_update");
 }
@@ -941,15 +963,15 @@ extern "C" int gbsgmc_resgld_exchange_adjacent(
       sched == nullptr || ssq_dev == nullptr || flags_dev == nullptr || every < 1 || !(F > 0))
     return set_error(GBSGMC_ERR_ARG, "resgld_exchange_adjacent: bad arguments");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  resgld_decide_kernel<<<1, 256, 0, st>>>(replicas, to_sched(sched), every, U_dev, lk_var_dev,
+  launch_pdl(resgld_decide_kernel, 1, 256, 0, st, replicas, to_sched(sched), every, U_dev, lk_var_dev,
                                          ssq_dev, F, seed, u_dev, flags_dev, counts_dev,
                                          log_s_dev);
   int rc = check_launch("resgld_exchange_adjacent: decide");
   if (rc != GBSGMC_OK || P == 0) return rc;
   const int chunks = static_cast<int>(std::min<int64_t>((P + 1023) / 1024, 64));
   dim3 grid(chunks, replicas - 1);
-  swap_adjacent_rows_kernel<<<grid, 256, 0, st>>>(P, x_dev, flags_dev);
-  if (v_dev != nullptr) swap_adjacent_rows_kernel<<<grid, 256, 0, st>>>(P, v_dev, flags_dev);
+  launch_pdl(swap_adjacent_rows_kernel, grid, 256, 0, st, P, x_dev, flags_dev);
+  if (v_dev != nullptr) launch_pdl(swap_adjacent_rows_kernel, grid, 256, 0, st, P, v_dev, flags_dev);
   return check_launch("resgld_exchange_adjacent: rows");
 }
 
@@ -962,6 +984,8 @@ int update_blocks(int chains, int64_t P) { return static_cast<int>(grid4(chains,
 __global__ void keep_row_kernel(int64_t P, const float* __restrict__ x,
                                 const double* __restrict__ U, Sched sched, float* samples,
                                 double* sample_lik) {
+  pdl_trigger();
+  pdl_wait();
   const int slot = sched.keep_slot(sched.step());
   if (slot < 0) return;
   for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < P;
@@ -974,7 +998,7 @@ __global__ void keep_row_kernel(int64_t P, const float* __restrict__ x,
 int keep_row(int64_t P, const float* x, const double* U, const gbsgmc_sched* sched,
              float* samples, double* sample_lik, cudaStream_t st) {
   const int blocks = static_cast<int>(std::min<int64_t>((P + 1023) / 1024, 1024));
-  keep_row_kernel<<<blocks, 256, 0, st>>>(P, x, U, to_sched(sched), samples, sample_lik);
+  launch_pdl(keep_row_kernel, blocks, 256, 0, st, P, x, U, to_sched(sched), samples, sample_lik);
   return check_launch("keep_row");
 }
 
@@ -982,7 +1006,7 @@ int sgld_update_fused(int chains, int64_t P, float* x, const float* g, float* v,
                       float alpha, float lmbd, const gbsgmc_sched* sched,
                       const gbsgmc_noise* noise, const UpdateFusion& f, cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  sgld_update_kernel<<<gr.grid, kThreads, 0, st>>>(chains, P, x, g, v, alpha, lmbd,
+  launch_pdl(sgld_update_kernel, gr.grid, kThreads, 0, st, chains, P, x, g, v, alpha, lmbd,
                                                    to_sched(sched), to_noise(noise), nullptr,
                                                    to_fuse(&f));
   return check_launch("sgld_update (fused)");
@@ -993,7 +1017,7 @@ int obabo_first_fused(int chains, int64_t P, float* x, float* p, const float* g1
                       const gbsgmc_sched* sched, const gbsgmc_noise* noise,
                       const UpdateFusion& f, cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  obabo_first_kernel<<<gr.grid, kThreads, 0, st>>>(chains, P, x, p, g1, mass, friction,
+  launch_pdl(obabo_first_kernel, gr.grid, kThreads, 0, st, chains, P, x, p, g1, mass, friction,
                                                    ke_start, to_sched(sched), to_noise(noise),
                                                    to_fuse(&f));
   return check_launch("obabo_first (fused)");
@@ -1004,7 +1028,7 @@ int obabo_second_fused(int chains, int64_t P, const float* x, float* p, const fl
                        const gbsgmc_sched* sched, const gbsgmc_noise* noise,
                        const UpdateFusion& f, cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  obabo_second_kernel<<<gr.grid, kThreads, 0, st>>>(chains, P, x, p, g2, mass, friction,
+  launch_pdl(obabo_second_kernel, gr.grid, kThreads, 0, st, chains, P, x, p, g2, mass, friction,
                                                     ke_end, to_sched(sched), to_noise(noise),
                                                     to_fuse(&f));
   return check_launch("obabo_second (fused)");
@@ -1016,7 +1040,7 @@ int obabo_second_first_fused(int chains, int64_t P, float* x, float* p, const fl
                              const gbsgmc_noise* noise, const UpdateFusion& f,
                              cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  obabo_second_first_kernel<<<gr.grid, kThreads, 0, st>>>(
+  launch_pdl(obabo_second_first_kernel, gr.grid, kThreads, 0, st, 
       chains, P, x, p, g2, g1, mass, friction, ke_end, ke_start, to_sched(sched),
       to_noise(noise), to_fuse(&f));
   return check_launch("obabo_second_first (fused)");
@@ -1026,7 +1050,7 @@ int sghmc_position_fused(int chains, int64_t P, float* x, float* p, const float*
                          float friction, const gbsgmc_sched* sched, const UpdateFusion& f,
                          cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  sghmc_position_kernel<<<gr.grid, kThreads, 0, st>>>(chains, P, x, p, mass, nullptr,
+  launch_pdl(sghmc_position_kernel, gr.grid, kThreads, 0, st, chains, P, x, p, mass, nullptr,
                                                       friction, to_sched(sched), to_fuse(&f));
   return check_launch("sghmc_position (fused)");
 }
@@ -1035,7 +1059,7 @@ int sghmc_momentum_fused(int chains, int64_t P, const float* x, float* p, const 
                          float friction, const gbsgmc_sched* sched, const gbsgmc_noise* noise,
                          const UpdateFusion& f, cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  sghmc_momentum_kernel<<<gr.grid, kThreads, 0, st>>>(chains, P, x, p, g, nullptr, friction,
+  launch_pdl(sghmc_momentum_kernel, gr.grid, kThreads, 0, st, chains, P, x, p, g, nullptr, friction,
                                                       to_sched(sched), to_noise(noise),
                                                       to_fuse(&f));
   return check_launch("sghmc_momentum (fused)");
@@ -1044,7 +1068,7 @@ int sghmc_momentum_fused(int chains, int64_t P, const float* x, float* p, const 
 int mirror_fused(int chains, int64_t P, const float* x, const UpdateFusion& f,
                  cudaStream_t st) {
   const Grid4 gr = grid4(chains, P);
-  mirror_kernel<<<gr.grid, kThreads, 0, st>>>(P, x, to_fuse(&f));
+  launch_pdl(mirror_kernel, gr.grid, kThreads, 0, st, P, x, to_fuse(&f));
   return check_launch("mirror (fused)");
 }
 
