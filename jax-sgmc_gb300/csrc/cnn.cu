@@ -87,7 +87,7 @@ struct CnnLayout {
   size_t labels;                      // int32
   size_t dp3, gl;                     // fp32 dP3 [n, 2048], dlogits [n, 10]
   size_t psq, plk;                    // fp64 partial sums
-  size_t part, bpart;                 // split-K weight partials, bias partials
+  size_t part[3], bpart[3];           // split-K weight partials, bias partials by layer
   size_t total;
 };
 
@@ -132,15 +132,12 @@ CnnLayout cnn_layout(int chains, int n) {
   L.gl = take(4 * N * kClasses);
   L.psq = take(8 * kPrepBlocks);
   L.plk = take(8 * 4 * N);
-  size_t part = 0;
-  part = std::max<size_t>(part, size_t(wsplit(1, n)) * kC1 * kK1);
-  part = std::max<size_t>(part, size_t(wsplit(2, n)) * kC2 * kK2);
-  part = std::max<size_t>(part, size_t(wsplit(3, n)) * kC3 * kK3);
-  L.part = take(4 * part);
+  const size_t wc[3] = {size_t(kC1) * kK1, size_t(kC2) * kK2, size_t(kC3) * kK3};
+  for (int l = 0; l < 3; ++l) L.part[l] = take(4 * wsplit(l + 1, n) * wc[l]);
   // Bias partials: one per unpool block and channel, 8 pooled elements per
   // thread and 256 threads per block: n*Ho*Wo*C / 2048 * C = 128 n floats
-  // for each of the three layers.
-  L.bpart = take(4 * 128 * N);
+  // for each of the three layers (at least one block).
+  for (int l = 0; l < 3; ++l) L.bpart[l] = take(4 * 128 * (N + 1));
   L.total = off;
   return L;
 }
@@ -168,7 +165,10 @@ struct CnnArgs {
   int32_t* lab;
   float *dp3, *gl;
   double *psq, *plk;
-  float *part, *bpart;
+  float *part[3], *bpart[3];
+  int split[3], bblocks[3];   // split-K partials, unpool blocks by layer
+  float pf;                   // 1 / (s^2 T) of the prior, 0 for a flat one
+  double prior_const;         // P (log s + 0.5 log 2 pi), 0 for a flat prior
 };
 
 __device__ __forceinline__ float bf(bf16 v) { return __bfloat162float(v); }
@@ -300,12 +300,17 @@ __global__ void __launch_bounds__(256) cnn_im2col_kernel(const bf16* Pin, bf16* 
 // half-warp then reads 16 Wd rows 40 bytes apart, 16 distinct banks (the
 // other half-warp the same words), and 16 consecutive P3 features.
 // ---------------------------------------------------------------------------
-constexpr int kDenseImgs = 16;
+// Few images leave most SMs without a block of 16, so blocks take 4 then (2 x
+// 50 images: 18.3 -> 9 us): the loads and the adjoint use all 256 threads
+// whatever the images.
+constexpr int kDenseThreads = 256;
 static_assert(oWd % 2 == 0 && kP % 2 == 0, "Wd is copied as float2");
-constexpr size_t kDenseSmem =
-    sizeof(float) * kFlat * kClasses + sizeof(bf16) * kDenseImgs * kFlat;
+constexpr size_t dense_smem(int imgs) {
+  return sizeof(float) * kFlat * kClasses + sizeof(bf16) * imgs * kFlat;
+}
 
-__global__ void __launch_bounds__(kDenseImgs * 16) cnn_dense_kernel(const CnnArgs a) {
+template <int kDenseImgs>
+__global__ void __launch_bounds__(kDenseThreads) cnn_dense_kernel(const CnnArgs a, float scale) {
   pdl_trigger();
   pdl_wait();
   extern __shared__ float wd_s[];  // Wd [2048][10], then P3 rows [kDenseImgs][2048]
@@ -314,79 +319,82 @@ __global__ void __launch_bounds__(kDenseImgs * 16) cnn_dense_kernel(const CnnArg
   const unsigned full = 0xffffffffu;
   const int c = blockIdx.y, t = threadIdx.x, j = t >> 4, sl = t & 15;
   const int i = blockIdx.x * kDenseImgs + j;
-  const bool live = i < a.n;
+  const bool live = j < kDenseImgs && i < a.n;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
   {
     // oWd and kP are even: the chain's Wd starts 8-byte aligned.
     const float2* src = reinterpret_cast<const float2*>(w + oWd);
     float2* dst = reinterpret_cast<float2*>(wd_s);
 #pragma unroll 8
-    for (int e = t; e < kFlat * kClasses / 2; e += kDenseImgs * 16) dst[e] = __ldg(src + e);
+    for (int e = t; e < kFlat * kClasses / 2; e += kDenseThreads) dst[e] = __ldg(src + e);
     // The block's images, 16 bytes per load (rows past n are not read).
     const int i0 = blockIdx.x * kDenseImgs;
     const int rows = min(kDenseImgs, a.n - i0);
     const uint4* xs = reinterpret_cast<const uint4*>(a.p3 + (static_cast<int64_t>(c) * a.n + i0) * kFlat);
     uint4* xd = reinterpret_cast<uint4*>(x_s);
 #pragma unroll 8
-    for (int e = t; e < kDenseImgs * kFlat / 8; e += kDenseImgs * 16)
+    for (int e = t; e < kDenseImgs * kFlat / 8; e += kDenseThreads)
       if (e < rows * (kFlat / 8)) xd[e] = __ldg(xs + e);
   }
   __syncthreads();
-  const bf16* x = x_s + j * kFlat;
-  float acc[kClasses];
+  if (j < kDenseImgs) {   // whole warps: an image is half of one
+    const bf16* x = x_s + j * kFlat;
+    float acc[kClasses];
 #pragma unroll
-  for (int k = 0; k < kClasses; ++k) acc[k] = 0.f;
+    for (int k = 0; k < kClasses; ++k) acc[k] = 0.f;
 #pragma unroll 4
-  for (int f = sl; f < kFlat; f += 16) {
-    const float xv = live ? bf(x[f]) : 0.f;
-    const float* wr = wd_s + f * kClasses;
+    for (int f = sl; f < kFlat; f += 16) {
+      const float xv = live ? bf(x[f]) : 0.f;
+      const float* wr = wd_s + f * kClasses;
 #pragma unroll
-    for (int k = 0; k < kClasses; ++k) acc[k] = fmaf(xv, wr[k], acc[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < kClasses; ++k)
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(full, acc[k], off);
-  if (sl == 0 && live) {
-    float logit[kClasses], mx = -INFINITY;
-    for (int k = 0; k < kClasses; ++k) {
-      logit[k] = acc[k] + __ldg(w + obd + k);
-      mx = fmaxf(mx, logit[k]);
+      for (int k = 0; k < kClasses; ++k) acc[k] = fmaf(xv, wr[k], acc[k]);
     }
-    float se = 0.f;
-    for (int k = 0; k < kClasses; ++k) se += expf(logit[k] - mx);
-    const float lse = mx + logf(se);
-    const int lab = a.lab[static_cast<int64_t>(c) * a.n + i];
-    const float lk = logit[lab] - lse;
-    const float m = a.mask != nullptr ? __ldg(a.mask + static_cast<int64_t>(c) * a.n + i) : 1.f;
-    const float scale = static_cast<float>(static_cast<double>(a.n_obs) / a.n / a.temperature);
-    for (int k = 0; k < kClasses; ++k) {
-      const float pk = expf(logit[k] - lse);
-      const float g = -scale * m * ((k == lab ? 1.f : 0.f) - pk);
-      g_s[j][k] = g;
-      a.gl[(static_cast<int64_t>(c) * a.n + i) * kClasses + k] = g;
+#pragma unroll
+    for (int k = 0; k < kClasses; ++k)
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(full, acc[k], off);
+    if (sl == 0 && live) {
+      float logit[kClasses], mx = -INFINITY;
+      for (int k = 0; k < kClasses; ++k) {
+        logit[k] = acc[k] + __ldg(w + obd + k);
+        mx = fmaxf(mx, logit[k]);
+      }
+      float se = 0.f;
+      for (int k = 0; k < kClasses; ++k) se += expf(logit[k] - mx);
+      const float lse = mx + logf(se);
+      const int lab = a.lab[static_cast<int64_t>(c) * a.n + i];
+      const float lk = logit[lab] - lse;
+      const float m = a.mask != nullptr ? __ldg(a.mask + static_cast<int64_t>(c) * a.n + i) : 1.f;
+      for (int k = 0; k < kClasses; ++k) {
+        const float pk = expf(logit[k] - lse);
+        const float g = -scale * m * ((k == lab ? 1.f : 0.f) - pk);
+        g_s[j][k] = g;
+        a.gl[(static_cast<int64_t>(c) * a.n + i) * kClasses + k] = g;
+      }
+      if (a.lk != nullptr) a.lk[static_cast<int64_t>(c) * a.n + i] = lk;
+      double* pl = a.plk + (static_cast<int64_t>(c) * a.n + i) * 4;
+      pl[0] = static_cast<double>(m) * lk;
+      pl[1] = lk;
+      pl[2] = static_cast<double>(lk) * lk;
+      pl[3] = 0.0;
     }
-    if (a.lk != nullptr) a.lk[static_cast<int64_t>(c) * a.n + i] = lk;
-    double* pl = a.plk + (static_cast<int64_t>(c) * a.n + i) * 4;
-    pl[0] = static_cast<double>(m) * lk;
-    pl[1] = lk;
-    pl[2] = static_cast<double>(lk) * lk;
-    pl[3] = 0.0;
   }
   if (!a.want_grad) return;
   __syncthreads();
-  if (!live) return;
-  float gk[kClasses];
+  // dP3 rows of the block's images: thread t takes the features t, t + 256, ...
+  const int rows = min(kDenseImgs, a.n - static_cast<int>(blockIdx.x) * kDenseImgs);
+  float* dx = a.dp3 + (static_cast<int64_t>(c) * a.n + blockIdx.x * kDenseImgs) * kFlat;
+#pragma unroll 2
+  for (int f = t; f < kFlat; f += kDenseThreads) {
+    float wr[kClasses];
 #pragma unroll
-  for (int k = 0; k < kClasses; ++k) gk[k] = g_s[j][k];
-  float* dx = a.dp3 + (static_cast<int64_t>(c) * a.n + i) * kFlat;
-#pragma unroll 4
-  for (int f = sl; f < kFlat; f += 16) {
-    const float* wr = wd_s + f * kClasses;
-    float sum = 0.f;
+    for (int k = 0; k < kClasses; ++k) wr[k] = wd_s[f * kClasses + k];
+    for (int r = 0; r < rows; ++r) {
+      float sum = 0.f;
 #pragma unroll
-    for (int k = 0; k < kClasses; ++k) sum = fmaf(gk[k], wr[k], sum);
-    dx[f] = sum;
+      for (int k = 0; k < kClasses; ++k) sum = fmaf(g_s[r][k], wr[k], sum);
+      dx[static_cast<int64_t>(r) * kFlat + f] = sum;
+    }
   }
 }
 
@@ -467,7 +475,7 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
 // The bias gradient is the column sum of dY, i.e. the sum over pooled
 // elements of the routed (BF16-rounded) values: each block adds its threads'
 // values per channel in a fixed order and writes
-// bpart[(chain * gridDim.x + block) * C + ch]; cnn_bias_sum_kernel adds the
+// bpart[(chain * gridDim.x + block) * C + ch]; cnn_finalize_kernel adds the
 // blocks.  2048 / C threads of a block share a channel group (256 * 8 is a
 // multiple of C, so the channel of thread t is 8 t mod C).
 // ---------------------------------------------------------------------------
@@ -528,82 +536,87 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
   }
 }
 
-// Bias gradient: grad[off + ch] = sum over the unpool blocks' partials in a
-// fixed order: thread t adds channel t % C of blocks t / C, t / C + kBiasT /
-// C, ... (coalesced along channels, eight loads in flight), then the
-// kBiasT / C partial sums of a channel are added in order.  Grid (chains),
-// kBiasT threads (enough loads in flight for the few blocks this grid has);
-// C divides kBiasT.
-constexpr int kBiasT = 1024;
+// What remains when the GEMMs are done, in one launch: the split-K partials of
+// the three weight gradients and the unpool blocks' bias partials summed in a
+// fixed order, the prior's w / (s^2 T) added to every parameter's gradient,
+// U and var(lk).  (As seven launches, most of them a few microseconds of
+// latency: 42 us of an 850 us gradient of 8 x 256 images, 26 us of 160 at 2 x
+// 50.)  Grid (weight blocks + kBiasBlocks + 1, chains), 256 threads: the
+// first ceil(P / 256) blocks take a parameter per thread, then a block per 8
+// bias channels (32 groups of partials each), the last block the values.
+constexpr int kBiasBlocks = (kC1 + kC2 + kC3) / 8;
 
-__global__ void __launch_bounds__(kBiasT) cnn_bias_sum_kernel(const float* bpart, int blocks,
-                                                              int C, float* grad, int64_t off) {
+__global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
+  __shared__ float acc[256];
+  __shared__ double red[4];
   pdl_trigger();
   pdl_wait();
-  __shared__ float acc[kBiasT];
-  const int c = blockIdx.x, t = threadIdx.x, ch = t % C, g0 = t / C, step = kBiasT / C;
-  const float* p = bpart + static_cast<int64_t>(c) * blocks * C + ch;
-  float s = 0.f;
-#pragma unroll 8
-  for (int q = g0; q < blocks; q += step) s += p[static_cast<int64_t>(q) * C];
-  acc[t] = s;
-  __syncthreads();
-  if (t < C) {
-    float tot = 0.f;
-    for (int u = 0; u < step; ++u) tot += acc[u * C + t];
-    grad[static_cast<int64_t>(c) * kP + off + t] = tot;
-  }
-}
-
-// Split-K reduction of a weight gradient: grad[off + e] = sum_s part[c, s, e]
-// over e < K * Cout (HWIO order).  Grid (ceil(K*Cout/256), chains).
-__global__ void __launch_bounds__(256) cnn_wsum_kernel(const float* part, int splits, int count,
-                                                      float* grad, int64_t off) {
-  pdl_trigger();
-  pdl_wait();
-  const int c = blockIdx.y, e = blockIdx.x * 256 + threadIdx.x;
-  if (e >= count) return;
-  const float* p = part + static_cast<int64_t>(c) * splits * count + e;
-  float s = 0.f;
-  for (int q = 0; q < splits; ++q) s += p[static_cast<int64_t>(q) * count];
-  grad[static_cast<int64_t>(c) * kP + off + e] = s;
-}
-
-// grad += w / (s^2 T) over every parameter; U and var(lk).  Grid
-// (ceil(P/256), chains); block 0 of a chain also writes U, var.
-__global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a, float pf) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ double red[32];
-  const int c = blockIdx.y, t = threadIdx.x;
+  const int c = blockIdx.y, t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
-  if (a.want_grad && pf != 0.f) {
+  const int weights = static_cast<int>(gridDim.x) - 1 - kBiasBlocks;
+  const int bx = static_cast<int>(blockIdx.x) - weights;
+  if (bx < 0) {
     const int64_t j = static_cast<int64_t>(blockIdx.x) * 256 + t;
-    if (j < kP) {
-      float* g = a.grad + static_cast<int64_t>(c) * kP + j;
-      *g = fmaf(pf, __ldg(w + j), *g);
+    if (!a.want_grad || j >= kP) return;
+    float* g = a.grad + static_cast<int64_t>(c) * kP + j;
+    float v;
+    if (j >= obd) {
+      v = *g;   // the dense layer's, already in place
+    } else {
+      const int l = j >= ob3 ? 2 : (j >= ob2 ? 1 : 0);
+      const int64_t off = l == 2 ? oW3 : (l == 1 ? oW2 : oW1);
+      if (j < off) return;   // a bias
+      const int64_t count = l == 2 ? kK3 * kC3 : (l == 1 ? kK2 * kC2 : kK1 * kC1);
+      const float* p = a.part[l] + static_cast<int64_t>(c) * a.split[l] * count + (j - off);
+      v = 0.f;
+#pragma unroll 8
+      for (int q = 0; q < a.split[l]; ++q) v += p[q * count];
     }
+    *g = a.pf != 0.f ? fmaf(a.pf, __ldg(w + j), v) : v;
+    return;
   }
-  if (blockIdx.x != 0) return;
-  double sq = 0.0, lm = 0.0, l1 = 0.0, l2 = 0.0;
-  for (int i = t; i < kPrepBlocks; i += 256) sq += a.psq[c * kPrepBlocks + i];
-  for (int i = t; i < a.n; i += 256) {
-    const double* p = a.plk + (static_cast<int64_t>(c) * a.n + i) * 4;
-    lm += p[0];
-    l1 += p[1];
-    l2 += p[2];
+  if (bx < kBiasBlocks) {
+    if (!a.want_grad) return;
+    int l = 0, ch0 = 8 * bx, C = kC1;
+    int64_t off = ob1;
+    if (ch0 >= kC1 + kC2) l = 2, ch0 -= kC1 + kC2, C = kC3, off = ob3;
+    else if (ch0 >= kC1) l = 1, ch0 -= kC1, C = kC2, off = ob2;
+    const int ch = ch0 + (t & 7), blocks = a.bblocks[l];
+    const float* p = a.bpart[l] + static_cast<int64_t>(c) * blocks * C + ch;
+    float v = 0.f;
+#pragma unroll 8
+    for (int q = t >> 3; q < blocks; q += 32) v += p[static_cast<int64_t>(q) * C];
+    acc[t] = v;
+    __syncthreads();
+    if (t < 8) {
+      float tot = 0.f;
+#pragma unroll
+      for (int u = 0; u < 32; ++u) tot += acc[8 * u + t];
+      const int64_t j = off + ch;
+      a.grad[static_cast<int64_t>(c) * kP + j] =
+          a.pf != 0.f ? fmaf(a.pf, __ldg(w + j), tot) : tot;
+    }
+    return;
   }
-  sq = block_sum(sq, red);
-  lm = block_sum(lm, red);
-  l1 = block_sum(l1, red);
-  l2 = block_sum(l2, red);
+  // The chain's values: four FP64 sums, a warp each.
+  if (warp < 4) {
+    double v = 0.0;
+    if (warp == 0) {
+      for (int i = lane; i < kPrepBlocks; i += 32) v += a.psq[c * kPrepBlocks + i];
+    } else {
+      const double* p = a.plk + static_cast<int64_t>(c) * a.n * 4 + (warp - 1);
+      for (int i = lane; i < a.n; i += 32) v += p[4 * static_cast<int64_t>(i)];
+    }
+    v = warp_sum(v);
+    if (lane == 0) red[warp] = v;
+  }
+  __syncthreads();
   if (t != 0) return;
+  const double sq = red[0], lm = red[1], l1 = red[2], l2 = red[3];
   double log_prior = 0.0;
   if (a.prior_scale > 0.f) {
     const double s2 = static_cast<double>(a.prior_scale) * a.prior_scale;
-    log_prior = -0.5 * sq / s2 -
-                static_cast<double>(kP) * (log(static_cast<double>(a.prior_scale)) +
-                                           0.91893853320467274178);
+    log_prior = -0.5 * sq / s2 - a.prior_const;
   }
   const double U = (-static_cast<double>(a.n_obs) * (lm / a.n) - log_prior) / a.temperature;
   a.U[c] = U;
@@ -961,38 +974,27 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   a.gl = view<float>(ws, L.gl);
   a.psq = view<double>(ws, L.psq);
   a.plk = view<double>(ws, L.plk);
-  a.part = view<float>(ws, L.part);
-  a.bpart = view<float>(ws, L.bpart);
   const int C = a.chains, n = a.n;
+  const int sizes[3] = {32, 16, 8}, couts[3] = {kC1, kC2, kC3};
+  for (int l = 0; l < 3; ++l) {
+    a.part[l] = view<float>(ws, L.part[l]);
+    a.bpart[l] = view<float>(ws, L.bpart[l]);
+    a.split[l] = wsplit(l + 1, n);
+    a.bblocks[l] = grid1(int64_t(n) * (sizes[l] / 2) * (sizes[l] / 2) * couts[l] / 8);
+  }
+  a.pf = 0.f;
+  a.prior_const = 0.0;
+  if (a.prior_scale > 0.f) {
+    const double ps = a.prior_scale;
+    a.pf = static_cast<float>(1.0 / (ps * ps * a.temperature));
+    a.prior_const = static_cast<double>(kP) * (std::log(ps) + 0.91893853320467274178);
+  }
   const int64_t r1 = int64_t(n) * 1024, r2 = int64_t(n) * 256, r3 = int64_t(n) * 64;
   int rc;
   auto launched = [&](const char* what) { return check_launch(what); };
-  // Bias gradient of a layer from its dY [rows, ld] (C real channels).
-  // Unpool of a layer (H x H before pooling, Cr channels) and its bias
-  // gradient from the unpool blocks' partials.
-  auto bias_sum = [&](int H, int Cr, int64_t off) {
-    const int blocks = grid1(int64_t(n) * (H / 2) * (H / 2) * Cr / 8);
-    launch_pdl(cnn_bias_sum_kernel, C, kBiasT, 0, st, a.bpart, blocks, Cr, a.grad, off);
-    return launched("cnn_bias_sum_kernel");
-  };
   auto unpool_grid = [&](int H, int Cr) {
     return dim3(grid1(int64_t(n) * (H / 2) * (H / 2) * Cr / 8), C);
   };
-  // Weight gradient of a layer: split-K GEMM into partials, then their sum.
-  auto weight_grad = [&](const CUtensorMap& mdy, const CUtensorMap& mcol, int layer, int Cout,
-                         int K, int Kp, int64_t rows, int64_t off) {
-    GemmRagged rg;
-    rg.ksplit = wsplit(layer, n);
-    if (Cout > 64) return set_error(GBSGMC_ERR_ARG, "cnn: weight gradient with %d outputs", Cout);
-    const HalfA<EpiConvGradW> e{{a.part, Cout, K}};
-    int r = launch_gemm<64, true, true>(mdy, mcol, C, 128, Kp, static_cast<int>(rows), a.status,
-                                        e, st, rg);
-    if (r) return r;
-    launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(K) * Cout), C), 256, 0, st, a.part, rg.ksplit,
-                                                                       K * Cout, a.grad, off);
-    return launched("cnn_wsum_kernel");
-  };
-
   launch_pdl(cnn_prep_kernel, dim3(kPrepBlocks, C), 256, 0, st, a);
   if ((rc = launched("cnn_prep_kernel"))) return rc;
   launch_pdl(cnn_gather1_kernel, dim3(grid1(r1), C), 256, 0, st, a);
@@ -1036,12 +1038,19 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
                                                    8, 8, kC2, 1, n};
   if ((rc = launch_gemm<128, false, true>(m_p2a, m_w3, C, r3, kC3, kK3, a.status, e3, st)))
     return rc;
-  static const cudaError_t dense_attr = cudaFuncSetAttribute(
-      cnn_dense_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kDenseSmem));
-  if (dense_attr != cudaSuccess)
-    return set_error(GBSGMC_ERR_CUDA, "cnn_dense_kernel: %s", cudaGetErrorString(dense_attr));
-  launch_pdl(cnn_dense_kernel, dim3((n + kDenseImgs - 1) / kDenseImgs, C), kDenseImgs * 16, kDenseSmem, st, a);
-  if ((rc = launched("cnn_dense_kernel"))) return rc;
+  const auto dense = [&](auto kern, int imgs) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(dense_smem(imgs)));
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_dense_kernel: %s", cudaGetErrorString(e));
+    const float scale = static_cast<float>(static_cast<double>(a.n_obs) / n / a.temperature);
+    launch_pdl(kern, dim3(ceil_div(n, imgs), C), kDenseThreads, dense_smem(imgs), st, a, scale);
+    return launched("cnn_dense_kernel");
+  };
+  // Sixteen images share a block's copy of Wd once that fills the SMs.
+  rc = int64_t(C) * n >= 16 * 148 / 2 ? dense(cnn_dense_kernel<16>, 16)
+                                      : dense(cnn_dense_kernel<4>, 4);
+  if (rc) return rc;
 
   if (a.want_grad) {
     launch_pdl(cnn_dense_grad_kernel, dim3(kFlat / 128 + 1, C), 512, 0, st, a);
@@ -1050,8 +1059,8 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     // blocks are P2's tap-shifted images), dP2 = the transposed convolution
     // of dY3 (implicit: A tiles are dY3's tap-shifted 2-image boxes).
     launch_pdl(cnn_unpool_kernel<8, 8, kC3, kC3>, unpool_grid(8, kC3), 256, 0, st, 
-        a.dy3, a.m3, a.dp3, n, a.bpart);
-    if ((rc = launched("cnn_unpool_kernel 3")) || (rc = bias_sum(8, kC3, ob3))) return rc;
+        a.dy3, a.m3, a.dp3, n, a.bpart[2]);
+    if ((rc = launched("cnn_unpool_kernel 3"))) return rc;
     CUtensorMap m_dy3t, m_p2b, m_dy3a, m_w3t;
     if ((rc = make_tmap_bf16_3d(&m_dy3t, a.dy3, kC3, r3, C, kC3, r3 * kC3, 64, 64)) ||
         (rc = make_tmap_bf16_4d(&m_p2b, a.p2, {kC2, 8, 8, imgs}, {kC2, 8 * kC2, 64 * kC2},
@@ -1063,14 +1072,11 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       return rc;
     {
       GemmRagged rg;
-      rg.ksplit = wsplit(3, n);
-      const ImplicitBmn<EpiConvGradW> e{{a.part, kC3, kK3}, 8, 8, kC2, n};
+      rg.ksplit = a.split[2];
+      const ImplicitBmn<EpiConvGradW> e{{a.part[2], kC3, kK3}, 8, 8, kC2, n};
       if ((rc = launch_gemm<64, true, true>(m_dy3t, m_p2b, C, 128, kK3, static_cast<int>(r3),
                                             a.status, e, st, rg)))
         return rc;
-      launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(kK3) * kC3), C), 256, 0, st, a.part, rg.ksplit,
-                                                                          kK3 * kC3, a.grad, oW3);
-      if ((rc = launched("cnn_wsum_kernel"))) return rc;
     }
     const TransposedB<ImplicitA<EpiStoreDX>> d3{{{a.dp2, kC2, r3}, 8, 8, kC3, -1, n}, kC3};
     if ((rc = launch_gemm<64, false, false>(m_dy3a, m_w3t, C, r3, kC2, 9 * kC3, a.status, d3,
@@ -1079,8 +1085,8 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     // Layer 2: dY2 (routing of dP2), db2, dW2 = dY2^T Col2, dP1 = the
     // transposed convolution of dY2 (implicit).
     launch_pdl(cnn_unpool_kernel<16, 16, kC2, kC2>, unpool_grid(16, kC2), 256, 0, st, 
-        a.dy2, a.m2, a.dp2, n, a.bpart);
-    if ((rc = launched("cnn_unpool_kernel 2")) || (rc = bias_sum(16, kC2, ob2))) return rc;
+        a.dy2, a.m2, a.dp2, n, a.bpart[1]);
+    if ((rc = launched("cnn_unpool_kernel 2"))) return rc;
     CUtensorMap m_dy2t, m_col2t, m_dy2a, m_w2t;
     if ((rc = make_tmap_bf16_3d(&m_dy2t, a.dy2, kC2, r2, C, kC2, r2 * kC2, 64, 64)) ||
         (rc = make_tmap_bf16_3d(&m_col2t, a.col2, kK2, r2, C, kK2p, r2 * kK2p, 64, 64)) ||
@@ -1089,7 +1095,14 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
         (rc = make_tmap_bf16_4d(&m_w2t, a.w2b, {kC2, kC1, 9, C}, {kC2, kC1 * kC2, kK2 * kC2},
                                 {64, kC1, 1, 1})))
       return rc;
-    if ((rc = weight_grad(m_dy2t, m_col2t, 2, kC2, kK2, kK2p, r2, oW2))) return rc;
+    {
+      GemmRagged rg;
+      rg.ksplit = a.split[1];
+      const HalfA<EpiConvGradW> e{{a.part[1], kC2, kK2}};
+      if ((rc = launch_gemm<64, true, true>(m_dy2t, m_col2t, C, 128, kK2p, static_cast<int>(r2),
+                                            a.status, e, st, rg)))
+        return rc;
+    }
     const TransposedBRows<ImplicitA<EpiStoreDX>, kC1> d2{
         {{{a.dp1, kC1, r2}, 16, 16, kC2, -1, n}, kC2}};
     if ((rc = launch_gemm<64, false, false>(m_dy2a, m_w2t, C, r2, 64, 9 * kC2, a.status, d2,
@@ -1097,28 +1110,24 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
       return rc;
     // Layer 1.
     launch_pdl(cnn_unpool_kernel<32, 32, kC1, kA1ld, true>, unpool_grid(32, kC1), 256, 0, st, 
-        a.dy1, a.m1, a.dp1, n, a.bpart);
-    if ((rc = launched("cnn_unpool_kernel 1")) || (rc = bias_sum(32, kC1, ob1))) return rc;
+        a.dy1, a.m1, a.dp1, n, a.bpart[0]);
+    if ((rc = launched("cnn_unpool_kernel 1"))) return rc;
     // dW1 = dY1^T Col1, Col1 read by K group from X8 (N = 8 groups x 8 slots).
     CUtensorMap m_dy1t;
     if ((rc = make_tmap_bf16_3d(&m_dy1t, a.dy1, kA1ld, r1, C, kA1ld, r1 * kA1ld, 64, 64)))
       return rc;
     {
       GemmRagged rg;
-      rg.ksplit = wsplit(1, n);
-      const Conv1Bmn<EpiConvGradW> e{{a.part, kC1, kK1, true}, n};
+      rg.ksplit = a.split[0];
+      const Conv1Bmn<EpiConvGradW> e{{a.part[0], kC1, kK1, true}, n};
       if ((rc = launch_gemm<64, true, true>(m_dy1t, m_x8h, C, 128, kK1i, static_cast<int>(r1),
                                             a.status, e, st, rg)))
         return rc;
-      launch_pdl(cnn_wsum_kernel, dim3(grid1(int64_t(kK1) * kC1), C), 256, 0, st, a.part, rg.ksplit,
-                                                                          kK1 * kC1, a.grad, oW1);
-      if ((rc = launched("cnn_wsum_kernel"))) return rc;
     }
   }
 
-  const double s2 = static_cast<double>(a.prior_scale) * a.prior_scale;
-  const float pf = a.prior_scale > 0.f ? static_cast<float>(1.0 / (s2 * a.temperature)) : 0.f;
-  launch_pdl(cnn_finalize_kernel, dim3(a.want_grad ? grid1(kP) : 1, C), 256, 0, st, a, pf);
+  launch_pdl(cnn_finalize_kernel, dim3((a.want_grad ? grid1(kP) : 0) + kBiasBlocks + 1, C), 256, 0,
+             st, a);
   return launched("cnn_finalize_kernel");
 }
 
