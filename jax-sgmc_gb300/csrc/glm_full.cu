@@ -7,7 +7,7 @@
 // glm_full_kernel is a tall matrix product (rows x chains over d) whose
 // outputs never leave the registers: thread t of a 128-thread CTA owns rows t
 // and t + 128 of a 256-row tile for CB chains, X passes through shared memory
-// in panels of 32 features (cp.async, double buffered, rows padded to an odd
+// in panels of 16 features (cp.async, double buffered, rows padded to an odd
 // number of 16-byte words so that a warp's 32 rows touch every bank), and the
 // chains' weights are broadcast reads.  Each x is read from memory once per
 // CB chains; evaluating the chains one by one through the minibatch kernel
@@ -29,17 +29,20 @@ namespace {
 
 constexpr int kFullThreads = 128;
 constexpr int kFullRows = 2 * kFullThreads;   // rows of a tile
-constexpr int kPanel = 8;                     // float4 columns of a panel
+constexpr int kPanel = 4;                     // float4 columns of a panel
 constexpr int kPanelStride = kPanel + 1;
 
 size_t full_smem(int dq, int cb) {
   return sizeof(float4) * (2ull * kFullRows * kPanelStride + static_cast<size_t>(cb) * dq);
 }
 
-// Row CTAs of a launch: depends on the data alone (see above).
+// Row CTAs of a launch, up to four per SM, whose warps fill the issue slots
+// that a thread's chain of links and sums leaves (100,000 rows of 64 features,
+// 16 chains: 25.8 us with one CTA per SM and panels of 32 features, 23.2 so).
+// Depends on the data alone (see above).
 int full_ctas(int64_t n_rows) {
   const int64_t tiles = (n_rows + kFullRows - 1) / kFullRows;
-  return static_cast<int>(std::min<int64_t>(tiles, glm_sm_count()));
+  return static_cast<int>(std::min<int64_t>(tiles, 4 * glm_sm_count()));
 }
 
 __device__ __forceinline__ void full_copy(const GlmArgs& a, float4* buf, int64_t row0, int q0,
@@ -488,7 +491,7 @@ extern "C" int gbsgmc_glm_mh_plan_create(
                                        p->stream), "glm_mh_plan_create: copy")))
       break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(chains, 1, n, model->d);
+    p->ctas = glm_loop_ctas(chains, 1, n);
     rc = plan_capture(p);
   } while (false);
   if (rc != GBSGMC_OK) {

@@ -9,8 +9,11 @@
 // cluster of S CTAs owns a chain for the whole block, and in each CTA
 //   * the copy warps run ahead: the minibatches of a block are known before it
 //     starts, so they gather the rows of the next chunks into a ring of shared
-//     memory buffers (cp.async, full / empty mbarriers), up to `depth` chunks
-//     before they are needed;
+//     memory buffers (full / empty mbarriers), up to `depth` chunks before
+//     they are needed: one bulk copy a row, each lane its own (a cp.async per
+//     16 bytes took a copy warp 110 cycles a row of 101 features, more than
+//     the rest of the step: 24 chains of 500 such rows 3.8 us a gradient
+//     against 3.0);
 //   * the row warps do what nothing else can do earlier: row tiles of the
 //     chunk exactly as glm_kernel takes them (same slices, warps, tiles and
 //     summation orders: the same bits), the reduction, the exchange and the
@@ -27,11 +30,13 @@
 // states; the rows are written to the slots they ended in when the block
 // ends.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 
 #include "glm.cuh"
 #include "internal.h"
+#include "tc.cuh"
 
 namespace gbsgmc {
 namespace {
@@ -43,10 +48,8 @@ constexpr int kCopyThreads = kCopyWarps * 32;
 constexpr int kClerkWarp = kRowWarps;
 constexpr int kNoiseWarp = kRowWarps + 1;
 constexpr int kLoopThreads = kRowThreads + 64 + kCopyThreads;  // 168 registers a thread
-constexpr int kMaxOwned = 4;                    // parameters of a row thread: d <= 1024
 constexpr int kMaxCtas = 8;                     // portable cluster size
 constexpr int kMaxDepth = 4;
-constexpr int kCopyBatch = 8;                   // rows a lane group copies at once
 
 struct LoopArgs {
   GlmArgs g;
@@ -60,7 +63,9 @@ struct LoopArgs {
   double* energy;  // leapfrog: energies [chains] to add to
   int ctas;        // CTAs per chain
   int chunk_rows, chunks, depth;
-  int row_shift;   // log2 of the lanes that copy one row
+  int row_quads;   // 16-byte words of a row in shared memory
+  int cp_y;        // y is copied by itself: rows are not aligned, or it is not in them
+  int cp_async;    // some copies are made by cp.async
   // pairs
   int pairs;
   double F;
@@ -76,7 +81,8 @@ struct LoopArgs {
 
 // What the clerk hands the row warps for one gradient.
 struct StepInfo {
-  float h, T, h_next;
+  float h, h_next;
+  float c[4];     // the integrator's coefficients (step_coefs)
   int want_next;  // want_u of the next gradient
   int slot;       // sample slot of this step, or -1
   int prev_slot;  // pairs: the previous step's slot if this chain is to store it
@@ -94,19 +100,21 @@ struct LoopBars {
   int stop;  // a wait ran out: the remaining ones give up at once
 };
 
-__device__ __forceinline__ void cp16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src)
-               : "memory");
-}
-// 4 bytes, or zeros when !ok.
+// 4 bytes global -> shared, or zeros when !ok.
 __device__ __forceinline__ void cp4(void* dst, const void* src, bool ok) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src),
                "r"(ok ? 4 : 0)
                : "memory");
 }
-// This thread's copies so far count as one arrival on `bar` when they land.
+// This thread's cp4 so far count as one arrival on `bar` when they land.
 __device__ __forceinline__ void cp_arrive(uint64_t* bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
+               : "memory");
+}
+// Bytes of bulk copies to come, counted on the barrier's current phase.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+               "r"(bytes)
                : "memory");
 }
 // Named barriers (ids below 16): sync waits, arrive does not.
@@ -161,33 +169,44 @@ __device__ __forceinline__ void cluster_wait() {
   asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The OBABO halves of one parameter, rounded as update.cu's kernels do.
-struct ObaboStep {
-  float h, keep, inject, half;
-  __device__ __forceinline__ ObaboStep(float step, float T, float friction) {
-    h = step;
+// What an update needs of the schedule alone: SGLD and SGHMC the noise scale
+// (c[0]); OBABO keep, inject and the half step; the leapfrog decay, 1 / (1 + h
+// f) and the noise scale.
+__device__ __forceinline__ void step_coefs(int kind, float h, float T, float friction,
+                                           float (&c)[4]) {
+  if (kind == kLoopObabo) {
     const float permanence = expf(-friction * h);
-    keep = sqrtf(permanence);
-    inject = sqrtf((1.0f - permanence) * T);
-    half = 0.5f * h;
+    c[0] = sqrtf(permanence);
+    c[1] = sqrtf((1.0f - permanence) * T);
+    c[2] = 0.5f * h;
+  } else if (kind == kLoopSghmc) {
+    c[0] = sqrtf(2.0f * h);
+  } else if (kind == kLoopLeapfrog) {
+    c[0] = 1.0f - h * friction;
+    c[1] = 1.0f / (1.0f + h * friction);
+    c[2] = sqrtf(4.0f * friction * h);
+  } else {
+    c[0] = sqrtf(2.0f * T * h);
   }
-  // Each returns the factors of the parameter's kinetic energy.
-  __device__ __forceinline__ float2 first(float mi, float ms, float g, float xi, float& p,
-                                          float& x) const {
-    float pj = __fmaf_rn(keep, p, __fmul_rn(inject, __fmul_rn(ms, xi)));
-    const float2 ke = make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
-    pj = __fmaf_rn(-half, g, pj);
-    p = pj;
-    x = __fmaf_rn(h, __fmul_rn(mi, pj), x);
-    return ke;
-  }
-  __device__ __forceinline__ float2 second(float mi, float ms, float g, float xi,
-                                           float& p) const {
-    const float pj = __fmaf_rn(-half, g, p);
-    p = __fmaf_rn(keep, pj, __fmul_rn(inject, __fmul_rn(ms, xi)));
-    return make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
-  }
-};
+}
+
+// The OBABO halves of one parameter, rounded as update.cu's kernels do; each
+// returns the factors of the parameter's kinetic energy.
+__device__ __forceinline__ float2 obabo_first(const StepInfo& q, float mi, float ms, float g,
+                                              float xi, float& p, float& x) {
+  float pj = __fmaf_rn(q.c[0], p, __fmul_rn(q.c[1], __fmul_rn(ms, xi)));
+  const float2 ke = make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
+  pj = __fmaf_rn(-q.c[2], g, pj);
+  p = pj;
+  x = __fmaf_rn(q.h, __fmul_rn(mi, pj), x);
+  return ke;
+}
+__device__ __forceinline__ float2 obabo_second(const StepInfo& q, float mi, float ms, float g,
+                                               float xi, float& p) {
+  const float pj = __fmaf_rn(-q.c[2], g, p);
+  p = __fmaf_rn(q.c[0], pj, __fmul_rn(q.c[1], __fmul_rn(ms, xi)));
+  return make_float2(__fmul_rn(0.5f, pj), __fmul_rn(mi, pj));
+}
 
 // A slice's sums, as one CTA publishes them: sum m lk, sum lk, sum lk^2, and
 // its chain's sum(w^2).
@@ -214,9 +233,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
   constexpr int LOG = Log2<RW>::v;
   constexpr int GROUP = 32 >> LOG;
   constexpr int kStride = kRowWarps * RW;
+  constexpr int kMaxOwned = QPL <= 2 ? 1 : QPL / 2;   // parameters of a row thread
   const GlmArgs& a = L.g;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int dq = a.dq, d = a.d, S = L.ctas, CH = L.chunk_rows, depth = L.depth;
+  const int dq = a.dq, d = a.d, rq = L.row_quads, S = L.ctas, CH = L.chunk_rows, depth = L.depth;
   const bool pairs = L.kind == kLoopPairs;
   const bool moves = L.kind == kLoopSgld || pairs;  // aux is the RMSprop state
 
@@ -248,7 +268,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
 
   if (tid == 0) {
     for (int i = 0; i < depth; ++i) {
-      mbar_init(bars->full + i, 2 * kCopyThreads);
+      mbar_init(bars->full + i, kCopyWarps + (L.cp_async ? kCopyThreads : 0));
       mbar_init(bars->empty + i, kRowWarps);
     }
     for (int i = 0; i < 2; ++i) {
@@ -272,11 +292,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
   if (warp > kNoiseWarp) {
     const int cw = warp - kNoiseWarp - 1;
     const int share = (CH + kCopyWarps - 1) / kCopyWarps;   // rows of a chunk per copy warp
-    const int sh = L.row_shift, per = 32 >> sh, sub = lane >> sh, ql = lane & ((1 << sh) - 1);
     const float* X = a.X;
     const float* yv = a.y;
     const int64_t ld = a.ld, n_rows = a.n_rows;
     const int vec4 = a.vec4, y_inline = a.y_inline, chunks = L.chunks;
+    const uint32_t row_bytes = static_cast<uint32_t>(rq) * 16;
     int buf = 0, use = 0;  // ring position, times round the ring
     for (int e = 0; e < events; ++e) {
       const int32_t* src = a.idx + (L.draws == 2 ? e >> 1 : e) * a.idx_step_stride +
@@ -287,60 +307,48 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
         const int r_end = min(cnt, (cw + 1) * share);
         int o = cw * share + lane < r_end ? __ldg(src + q * CH + cw * share + lane) : -1;
         if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
-        float4* dst = rows_s + buf * CH * dq;
+        float4* dst = rows_s + buf * CH * rq;
         for (int r0 = cw * share; r0 < r_end; r0 += 32) {
           const int r = r0 + lane;
           if (r0 > cw * share) o = r < r_end ? __ldg(src + q * CH + r) : -1;
           if (r < r_end) {
-            if (o < 0 || o >= n_rows) {
+            if (o < 0 || o >= n_rows) {   // left out: its row is zero
               raise_status(a.status, GBSGMC_ERR_INDEX);
               o = -1;
+              for (int v = 0; v < rq; ++v) dst[r * rq + v] = make_float4(0.f, 0.f, 0.f, 0.f);
+              tc::fence_async_shared();
             }
             idx_s[buf * CH + r] = o;
-            if (o >= 0) {
-              if (y_inline) cp4(y_s + buf * CH + r, X + o * ld + d, true);
-              else if (yv != nullptr) cp4(y_s + buf * CH + r, yv + o, true);
-            }
+            if (o >= 0 && L.cp_y) cp4(y_s + buf * CH + r, y_inline ? X + o * ld + d : yv + o, true);
           }
-          // Rows with an invalid index are never read (idx_s is -1).  Eight
-          // rows per lane group are addressed before any copy is issued: one
-          // by one each row took 330 cycles of dependent instructions.
-          const int m = min(32, r_end - r0);
-          for (int i0 = 0; i0 < m; i0 += kCopyBatch * per) {
-            const float* from[kCopyBatch];
-            bool live[kCopyBatch];
-#pragma unroll
-            for (int b = 0; b < kCopyBatch; ++b) {
-              const int i = i0 + b * per + sub;
-              const int oi = __shfl_sync(0xffffffffu, o, min(i, 31));
-              live[b] = i < m && oi >= 0;
-              from[b] = X + (live[b] ? oi * ld : 0);
-            }
-            float4* out = dst + (r0 + i0 + sub) * dq;
-            if (vec4) {
-              for (int v = ql; v < dq; v += 32) {
-#pragma unroll
-                for (int b = 0; b < kCopyBatch; ++b)
-                  if (live[b]) cp16(out + b * per * dq + v, from[b] + 4 * v);
-              }
-            } else {
-              for (int j = ql; j < 4 * dq; j += 1 << sh) {
-#pragma unroll
-                for (int b = 0; b < kCopyBatch; ++b)
-                  if (live[b])
-                    cp4(reinterpret_cast<float*>(out + b * per * dq) + j,
-                        from[b] + (j < d ? j : 0), j < d);
-              }
+          if (vec4) {   // one copy a row, its y with it
+            const unsigned live = __ballot_sync(0xffffffffu, o >= 0);
+            if (lane == 0) mbar_expect_tx(bars->full + buf, __popc(live) * row_bytes);
+            __syncwarp();
+            if (o >= 0) bulk_g2s(dst + r * rq, X + o * ld, row_bytes, bars->full + buf);
+          } else {
+            for (int i = 0; i < min(32, r_end - r0); ++i) {
+              const int oi = __shfl_sync(0xffffffffu, o, i);
+              if (oi < 0) continue;
+              float* out = reinterpret_cast<float*>(dst + (r0 + i) * rq);
+              for (int j = lane; j < 4 * dq; j += 32)
+                cp4(out + j, X + oi * ld + (j < d ? j : 0), j < d);
             }
           }
         }
-        cp_arrive(bars->full + buf);
-        mbar_arrive(bars->full + buf);
+        if (L.cp_async) cp_arrive(bars->full + buf);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bars->full + buf);
         if (++buf == depth) {
           buf = 0;
           ++use;
         }
       }
+    }
+    // No copy is in flight when the CTA ends, even if a wait has run out.
+    for (int i = 0; i < depth; ++i) {
+      const int last = use - (i < buf ? 0 : 1);
+      if (last >= 0) mbar_wait_bounded(bars->full + i, last & 1, nullptr);
     }
     return;
   }
@@ -418,7 +426,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
     auto hand_over = [&](int e) {
       const int64_t k = k0 + (L.draws == 2 ? e >> 1 : e);
       StepInfo out = in;
-      out.T = a.sched.temperature(k, pairs ? (role ? L.pairs + unit : unit) : unit);
+      step_coefs(L.kind, in.h,
+                 a.sched.temperature(k, pairs ? (role ? L.pairs + unit : unit) : unit),
+                 L.friction, out.c);
       out.prev_slot = -1;
       if (pairs) {
         out.prev_slot = role == 0 ? done_slot : -1;
@@ -626,6 +636,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
       if (i < owned) a.samples[at * d + tid + i * kRowThreads] = xs[i];
   };
 
+  // The cluster's shared-memory windows: address of `here` in each CTA.
+  const uint32_t here = smem_addr(smem);
+  uint32_t peer[kMaxCtas];
+#pragma unroll
+  for (int r = 0; r < kMaxCtas; ++r) peer[r] = r < S ? cluster_addr(smem, rank0 + r) : 0u;
+
+  const bool y_in_row = a.y_inline != 0;
   int want = pairs || (L.kind != kLoopLeapfrog &&
                        (a.steps == 1 || a.sched.keep_slot(k0) >= 0));
   int buf = 0, use = 0;
@@ -645,19 +662,21 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
     for (int q = 0; q < L.chunks; ++q) {
       wait_phase(bars, bars->full + buf, use, a.status);
       const int cnt = min(CH, R - q * CH);
-      const float4* rows = rows_s + buf * CH * dq;
+      const float4* rows = rows_s + buf * CH * rq;
       const int32_t* ix = idx_s + buf * CH;
       for (int r0 = warp * RW; r0 < cnt; r0 += kStride) {
         const int og = r0 + g < cnt ? ix[r0 + g] : -1;
-        const float yv = og >= 0 ? y_s[buf * CH + r0 + g] : 0.0f;
+        const float yv = og < 0     ? 0.0f
+                         : L.cp_y   ? y_s[buf * CH + r0 + g]
+                         : y_in_row ? reinterpret_cast<const float*>(rows + (r0 + g) * rq)[d]
+                                    : 0.0f;
         float4 xv[RW][QPL];
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
-          const bool ok = __shfl_sync(0xffffffffu, og, r * GROUP) >= 0;
 #pragma unroll
           for (int k = 0; k < QPL; ++k) {
             const int v = lane + 32 * k;
-            xv[r][k] = ok && v < dq ? rows[(r0 + r) * dq + v]
+            xv[r][k] = r0 + r < cnt && v < dq ? rows[(r0 + r) * rq + v]
                                     : make_float4(0.f, 0.f, 0.f, 0.f);
           }
         }
@@ -704,9 +723,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
 #pragma unroll
         for (int w = 1; w < kRowWarps; ++w) gl[i] += t[w];
         if (S > 1) {
-          const float* mine = partf + slice * 4 * dq + p;
-          for (int r = 0; r < S; ++r)
-            send4(cluster_addr(mine, rank0 + r), cluster_addr(bars->part + par, rank0 + r), gl[i]);
+          const uint32_t at = smem_addr(partf + slice * 4 * dq + p) - here;
+          const uint32_t bar = smem_addr(bars->part + par) - here;
+#pragma unroll
+          for (int r = 0; r < kMaxCtas; ++r)
+            if (r < S) send4(peer[r] + at, peer[r] + bar, gl[i]);
         }
       }
       if (S > 1) {
@@ -717,8 +738,13 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
         for (int i = 0; i < kMaxOwned; ++i) {
           if (i >= owned) continue;
           const float* all = partf + tid + i * kRowThreads;
-          gl[i] = all[0];
-          for (int r = 1; r < S; ++r) gl[i] += all[r * 4 * dq];
+          float t[kMaxCtas];
+#pragma unroll
+          for (int r = 0; r < kMaxCtas; ++r) t[r] = r < S ? all[r * 4 * dq] : 0.f;
+          gl[i] = t[0];
+#pragma unroll
+          for (int r = 1; r < kMaxCtas; ++r)
+            if (r < S) gl[i] += t[r];
         }
       }
 
@@ -733,7 +759,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
         const float gv = (-a.scale * gl[i] + xs[i] * a.inv_p2) * a.inv_temp;
         if (!isfinite(gv)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
         if (moves) {
-          const float noise_scale = sqrtf(2.0f * in.T * in.h);
+          const float noise_scale = in.c[0];
           const float x = xs[i];
           const float scaled_gradient = -in.h * gv;
           const float scaled_noise = noise_scale * xi;
@@ -747,11 +773,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
             xs[i] = x + (scaled_gradient + scaled_noise);
           }
         } else if (L.kind == kLoopObabo) {
-          const ObaboStep ob(in.h, in.T, L.friction);
-          if (par == 0) ke_s[p] = ob.first(mi[i], ms[i], gv, xi, as[i], xs[i]);
-          else ke_s[4 * dq + p] = ob.second(mi[i], ms[i], gv, xi, as[i]);
+          if (par == 0) ke_s[p] = obabo_first(in, mi[i], ms[i], gv, xi, as[i], xs[i]);
+          else ke_s[4 * dq + p] = obabo_second(in, mi[i], ms[i], gv, xi, as[i]);
         } else if (L.kind == kLoopSghmc) {
-          const float noise_scale = sqrtf(2.0f * in.h);
+          const float noise_scale = in.c[0];
           float pj = as[i] + (-in.h) * gv;
           pj = pj + L.friction * (noise_scale * xi);
           const bool more = j + 1 < a.steps;
@@ -767,9 +792,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
             as[i] = pj + (-h * L.friction) * sm;
           }
         } else {  // reversible leapfrog
-          const float decay = 1.0f - in.h * L.friction;
-          const float inv = 1.0f / (1.0f + in.h * L.friction);
-          const float ns = sqrtf(4.0f * L.friction * in.h);
+          const float decay = in.c[0], inv = in.c[1], ns = in.c[2];
           const float s = (j + 1 < a.steps ? 1.0f : 0.5f) * in.h;
           const float pj = as[i];
           const float noise_j = ns * (ms[i] * xi);
@@ -827,7 +850,7 @@ size_t loop_layout(LoopArgs& L, int rw, int ncta) {
   const size_t fixed = n_red + n_part + 6 * row + align16(n_ke) + align16(n_lane) +
                        align16(n_sums) + align16(n_step) + n_pair + align16(sizeof(LoopBars)) + 64;
   const auto ring = [&](int depth, int rows) {
-    return depth * static_cast<size_t>(rows) * (row + 8);
+    return depth * static_cast<size_t>(rows) * (16 * L.row_quads + 8);
   };
   if (fixed >= kLoopSmem) return 0;
   const size_t room = kLoopSmem - fixed;
@@ -849,7 +872,7 @@ size_t loop_layout(LoopArgs& L, int rw, int ncta) {
   L.depth = depth;
   L.chunk_rows = rows;
   L.chunks = std::max(1, ceil_div(R, rows));
-  size_t o = static_cast<size_t>(depth) * rows * row;
+  size_t o = static_cast<size_t>(depth) * rows * 16 * L.row_quads;
   const auto take = [&](size_t bytes) {
     const size_t at = o;
     o += align16(bytes);
@@ -911,11 +934,47 @@ struct LoopVariant {
 
 }  // namespace
 
-// CTAs per chain: as many as give every row warp a tile (n / (8 RW)) while
-// all CTAs of the launch still find an SM of their own, in powers of two up
-// to the portable cluster size.
-int glm_loop_ctas(int units, int chains_per_unit, int n, int d) {
-  const int rw = glm_rows_per_warp((d + 3) / 4);
+namespace {
+
+// Clusters of `ctas` loop CTAs (one per SM) that the device holds at once: its
+// GPCs are not whole multiples of 8 SMs, so fewer than SMs / ctas.  A CTA's
+// registers fill an SM in every variant.
+int clusters_at_once(int ctas) {
+  static std::atomic<int> known[4];
+  const int slot = ctas >= 8 ? 3 : ctas >= 4 ? 2 : ctas >= 2 ? 1 : 0;
+  int n = known[slot].load(std::memory_order_relaxed);
+  if (n > 0) return n;
+  n = glm_sm_count() / ctas;
+  if (ctas > 1 && LoopVariant<1, 4>::prepare() == GBSGMC_OK) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas));
+    cfg.blockDim = dim3(kLoopThreads);
+    cfg.dynamicSmemBytes = kLoopSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int held = 0;
+    if (cudaOccupancyMaxActiveClusters(&held, glm_loop_kernel<1, 4>, &cfg) == cudaSuccess &&
+        held > 0)
+      n = held;
+    else
+      cudaGetLastError();
+  }
+  known[slot].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+}  // namespace
+
+// CTAs per chain: in powers of two up to the portable cluster size, as long
+// as each keeps two rows a row warp and all clusters run at once.  16 chains
+// of 200 rows of 16 features, OBABO: 3,069, 1,969, 1,413 us with 1, 2, 4 CTAs,
+// and 1,898 with 8, where two clusters wait for the others; 8 chains: 1,361 us
+// with 4, 1,285 with 8.
+int glm_loop_ctas(int units, int chains_per_unit, int n) {
   const int most = kMaxCtas / chains_per_unit;
   const char* env = std::getenv("GBSGMC_GLM_SLICES");
   const int forced = env != nullptr ? std::atoi(env) : 0;
@@ -924,8 +983,8 @@ int glm_loop_ctas(int units, int chains_per_unit, int n, int d) {
     while (2 * s <= std::min(forced, most)) s *= 2;
     return s;
   }
-  while (2 * s <= most && n >= 2 * s * kRowWarps * rw &&
-         static_cast<int64_t>(units) * chains_per_unit * 2 * s <= glm_sm_count())
+  while (2 * s <= most && n >= 2 * s * kRowWarps * 2 &&
+         units <= clusters_at_once(2 * s * chains_per_unit))
     s *= 2;
   return s;
 }
@@ -1002,8 +1061,10 @@ int glm_loop(const GlmLoopCall& c, cudaStream_t st) {
   L.ke = c.kind == kLoopObabo ? c.ke : nullptr;
   L.energy = c.kind == kLoopLeapfrog ? c.energy : nullptr;
   L.ctas = c.ctas;
-  L.row_shift = 0;
-  while (L.row_shift < 5 && (1 << L.row_shift) < L.g.dq) ++L.row_shift;
+  const bool y_in_row = L.g.vec4 && L.g.y_inline;
+  L.row_quads = (L.g.d + (y_in_row ? 1 : 0) + 3) / 4;
+  L.cp_y = !y_in_row && (L.g.y_inline || L.g.y != nullptr) ? 1 : 0;
+  L.cp_async = !L.g.vec4 || L.cp_y ? 1 : 0;
   int units = c.chains, ncta = c.ctas;
   if (pairs) {
     units = L.pairs = c.chains / 2;

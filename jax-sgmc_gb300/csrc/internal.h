@@ -59,7 +59,7 @@ struct GlmLoopCall {
   int32_t* counts = nullptr;
   int* status = nullptr;
 };
-int glm_loop_ctas(int units, int chains_per_unit, int n, int d);
+int glm_loop_ctas(int units, int chains_per_unit, int n);
 int glm_loop_prepare();
 int glm_loop(const GlmLoopCall& c, cudaStream_t st);
 // glm.cu: the float4 columns per lane and default rows per warp of a row of

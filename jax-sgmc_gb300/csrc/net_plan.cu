@@ -850,7 +850,7 @@ extern "C" int gbsgmc_glm_plan_create_keep(
                           p->draws() * n;
     if ((rc = plan_alloc(p, &p->idx, ibytes, "glm_plan_create: index buffer"))) break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(chains, 1, n, model->d);
+    p->ctas = glm_loop_ctas(chains, 1, n);
     if ((rc = p->setup_external("glm_plan_create: index memset"))) break;
     rc = plan_capture(p);
   } while (false);

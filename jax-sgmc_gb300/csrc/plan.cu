@@ -440,9 +440,9 @@ int autotune(GlmPlan* p) {
   std::vector<GlmTune> cands;
   // With no more chains than half the SMs, blocks run as one glm_loop launch
   // with a cluster per chain: every other form leaves SMs idle or pays a
-  // launch per step (one chain, n = 128, d = 32: 10.9 us a step against 4.0;
-  // 24 chains, n = 500, d = 101: 18.8 us a gradient against 8.2).
-  const int ctas = glm_loop_ctas(C, 1, n, d);
+  // launch per step (one chain, n = 128, d = 32: 10.9 us a step against 1.5;
+  // 24 chains, n = 500, d = 101: 18.8 us a gradient against 3.0).
+  const int ctas = glm_loop_ctas(C, 1, n);
   const GlmTune loop{ctas, glm_rows_per_warp((d + 3) / 4), 8, 0, 0, 1, ctas};
   if (2 * C <= glm_sm_count()) {
     p->tune = loop;
@@ -817,7 +817,7 @@ extern "C" int gbsgmc_glm_resgld_plan_create(
                          "glm_resgld_plan_create: index buffer")))
       break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(pairs, 2, n, model->d);
+    p->ctas = glm_loop_ctas(pairs, 2, n);
     rc = plan_capture(p);
   } while (false);
   if (rc != GBSGMC_OK) {

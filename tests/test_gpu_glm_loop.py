@@ -133,6 +133,42 @@ def test_block_matches_oracle(lib, kind, C, n, d, family):
   assert torch.isfinite(plan.lk_var).all()
 
 
+@pytest.mark.parametrize("layout", ["inline", "unaligned", "unaligned inline"])
+@pytest.mark.parametrize("C,n,d", [(1, 65, 4), (2, 500, 33), (1, 200, 131)])
+def test_row_layouts_agree(lib, layout, C, n, d):
+  """However X and y lie in memory (y its own vector or column d; rows on
+  16-byte boundaries, copied whole, or not, copied in words), the same rows
+  are summed in the same order: bit-equal states."""
+  from gbsgmc import _lib, engine
+  X, y, ds, pot, x0, N = _setup(C, n, d, O.LOGISTIC)
+  h = (np.full(K, 0.02 / (N * max(1.0, 2.0 * d / n)))).astype(np.float32)
+  inline = "inline" in layout
+  ld = d + 1 if inline else d
+  ld = ld | 1 if "unaligned" in layout else (ld + 3) // 4 * 4
+  rows = np.zeros((N, ld), np.float32)
+  rows[:, :d] = X
+  if inline:
+    rows[:, d] = y
+  rows, yd = _cuda(rows), _cuda(y)
+  base, _ = pot.model(ds)
+  other = _lib.Glm(base.family, d, base.n_obs, ld, rows.data_ptr(),
+                   None if inline else yd.data_ptr(), base.sigma, base.prior_scale,
+                   base.temperature, int(inline), base.n_rows)
+  outs = []
+  for model in (None, other):
+    if model is not None:
+      object.__setattr__(pot, "model", lambda *a, **k: (other, (rows, yd)))
+    x = _cuda(x0)
+    plan = engine.NetPlan(pot, ds, x, None, n, "langevin", _cuda(h),
+                          _cuda(np.ones(K, np.float32)),
+                          engine.IndexSource(pcg=_cuda(_words(C))), 11, block_steps=3)
+    plan.run(0, K)
+    plan.check_status()
+    outs.append((x.cpu().numpy(), plan.U.cpu().numpy(), plan.lk_var.cpu().numpy()))
+  for a, b in zip(*outs):
+    np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("pairs,n,d", [(1, 33, 7), (2, 256, 64), (1, 900, 300), (90, 40, 12)])
 def test_pairs_match_the_per_pair_path(lib, pairs, n, d):
   """alias.re_sgld through the block launches against one chain at a time
