@@ -6,10 +6,10 @@
 //   interval"): x = next_uint32(); m = x * N; accept when (m mod 2^32) >=
 //   2^32 mod N, the index being m >> 32.  next_uint32 hands out the low half
 //   of a fresh PCG64 output and keeps the high half for the next call.  The
-//   accept test depends only on the 32-bit value, so a CTA expands 2048 PCG64
+//   accept test depends only on the 32-bit value, so a CTA expands 4096 PCG64
 //   outputs at once (each thread jumps ahead to its own 8 consecutive steps
 //   by LCG jump-ahead, Brown 1994, "Random number generation with arbitrary
-//   strides"), tests the 4096 halves, and compacts the accepted ones with a
+//   strides"), tests the 8192 halves, and compacts the accepted ones with a
 //   block scan.  The chain's stream state (128-bit LCG state,
 //   buffered half) is advanced exactly as numpy advances it.
 // * gbsgmc_index_draw_philox and gbsgmc_philox_normal use Philox4x32-10.
@@ -18,9 +18,56 @@
 namespace gbsgmc {
 namespace {
 
-constexpr int kDrawThreads = 256;
+constexpr int kDrawThreads = 512;
 constexpr int kDrawPerThread = 8;   // consecutive LCG outputs per thread per round
-constexpr int kDrawLog2Round = 11;  // log2(kDrawThreads * kDrawPerThread)
+
+// The LCG map s -> a s + inc applied k times is s -> a^k s + inc G_k with
+// G_k = 1 + a + ... + a^(k - 1) (Brown 1994): a^k and G_k do not depend on
+// the stream.  Tables of them, made at compile time, replace the 11 squarings
+// and up to 12 compositions that every thread did before its first draw: the
+// first steps of 16 neighbouring threads, the strides between such groups,
+// and a whole round.
+struct Jump {
+  unsigned long long a_hi, a_lo, g_hi, g_lo;
+};
+struct JumpTable {
+  Jump low[16];                    // t = 0 .. 15: t kDrawPerThread + 1 steps
+  Jump high[kDrawThreads / 16];    // u: 16 u kDrawPerThread steps
+  Jump round;                      // kDrawThreads kDrawPerThread steps
+};
+constexpr Jump jump_of(unsigned k) {
+  using u128 = unsigned __int128;
+  const u128 a = (static_cast<u128>(0x2360ED051FC65DA4ull) << 64) | 0x4385DF649FCCF645ull;
+  u128 A = 1, G = 0, p = a, s = 1;   // (p, s): the map of 2^i steps
+  while (k > 0) {
+    if (k & 1u) {
+      G = p * G + s;
+      A = p * A;
+    }
+    s = s * p + s;
+    p = p * p;
+    k >>= 1;
+  }
+  return Jump{static_cast<unsigned long long>(A >> 64), static_cast<unsigned long long>(A),
+              static_cast<unsigned long long>(G >> 64), static_cast<unsigned long long>(G)};
+}
+constexpr JumpTable make_jumps() {
+  JumpTable t{};
+  for (int i = 0; i < 16; ++i) t.low[i] = jump_of(i * kDrawPerThread + 1);
+  for (int i = 0; i < kDrawThreads / 16; ++i) t.high[i] = jump_of(16 * i * kDrawPerThread);
+  t.round = jump_of(kDrawThreads * kDrawPerThread);
+  return t;
+}
+__device__ const JumpTable g_jumps = make_jumps();
+
+__device__ __forceinline__ U128 load_hi_lo(const unsigned long long& hi,
+                                           const unsigned long long& lo) {
+  return U128{__ldg(&hi), __ldg(&lo)};
+}
+// The map of `j`'s steps on a stream of increment inc.
+__device__ __forceinline__ Affine jump_map(const Jump& j, U128 inc) {
+  return Affine{load_hi_lo(j.a_hi, j.a_lo), mul128(load_hi_lo(j.g_hi, j.g_lo), inc)};
+}
 
 // Block-wide exclusive scan of small non-negative ints; returns the exclusive
 // prefix and sets *total.  Contains __syncthreads.
@@ -51,9 +98,10 @@ __global__ void __launch_bounds__(kDrawThreads)
     pcg64_draw_kernel(gbsgmc_pcg64* states, int64_t n_obs, int64_t draws,
                       int per_step, int32_t* idx, int64_t chain_stride,
                       int64_t step_stride) {
-  // The LCG map applied 1, 2, 4, ..., 2^kDrawLog2Round times.
-  __shared__ Affine pow2[kDrawLog2Round + 1];
   __shared__ int warp_tot[kDrawThreads / 32];
+  // A round's values by rank, position p at p + p / 16: thread t's sixteen
+  // values start near 16 t, so that a warp's stores of value i hit 32 banks.
+  __shared__ int32_t vals[kDrawThreads * 2 * kDrawPerThread * 17 / 16 + 1];
 
   const int c = blockIdx.x;
   const int t = threadIdx.x;
@@ -76,23 +124,13 @@ __global__ void __launch_bounds__(kDrawThreads)
   const uint64_t N = static_cast<uint64_t>(n_obs);
   const uint32_t threshold = static_cast<uint32_t>((1ull << 32) % N);
 
-  if (t == 0) {
-    pow2[0].a = pcg_multiplier();
-    pow2[0].c = inc;
-    for (int i = 1; i <= kDrawLog2Round; ++i) pow2[i] = compose(pow2[i - 1], pow2[i - 1]);
-  }
-  __syncthreads();
   // A round is kDrawThreads * kDrawPerThread LCG steps; this thread's
   // outputs are steps t*K + 1 .. t*K + K of the round (K = kDrawPerThread),
   // so the thread order of the scan is the stream order.
-  Affine jump{U128{0, 1}, U128{0, 0}};
-  {
-    const int k = t * kDrawPerThread + 1;
-    for (int i = 0; i <= kDrawLog2Round; ++i)
-      if ((k >> i) & 1) jump = compose(jump, pow2[i]);
-  }
-  const Affine step1 = pow2[0];
-  const Affine round_jump = pow2[kDrawLog2Round];
+  const Affine jump =
+      compose(jump_map(g_jumps.high[t >> 4], inc), jump_map(g_jumps.low[t & 15], inc));
+  const Affine step1{pcg_multiplier(), inc};
+  const Affine round_jump = jump_map(g_jumps.round, inc);
 
   int64_t produced = 0;
   if (has) {  // the half buffered by the previous call comes first
@@ -127,25 +165,32 @@ __global__ void __launch_bounds__(kDrawThreads)
     }
     int total;
     const int excl = block_excl_scan(cnt, warp_tot, &total);
-    // Output position pos = q * per_step + r, advanced without divisions.
-    int64_t pos = produced + excl;
-    int64_t q = pos / per_step;
-    int r = static_cast<int>(pos - q * per_step);
-    int32_t* dst = out + q * step_stride;
+    // Through shared memory, so that the indices leave as whole segments
+    // (a thread's own sixteen stores each touched a sector of their own:
+    // 50,000 draws took 38 us against 27).
+    int rank0 = excl;
 #pragma unroll
     for (int i = 0; i < kDrawPerThread; ++i) {
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         if ((acc >> (2 * i + h)) & 1u) {
           const uint32_t v = h ? hi[i] : lo[i];
-          if (pos < draws) dst[r] = static_cast<int32_t>((v * N) >> 32);
-          ++pos;
-          if (++r == per_step) {
-            r = 0;
-            dst += step_stride;
-          }
+          vals[rank0 + (rank0 >> 4)] = static_cast<int32_t>((v * N) >> 32);
+          ++rank0;
         }
       }
+    }
+    __syncthreads();
+    const int64_t left = draws - produced;
+    const int out_n = left < total ? static_cast<int>(left) : total;
+    if (produced + out_n <= 0xffffffffll) {
+      const uint32_t base = static_cast<uint32_t>(produced), per = per_step;
+      for (int p = t; p < out_n; p += kDrawThreads) {
+        const uint32_t pos = base + p, q = pos / per;
+        out[q * step_stride + (pos - q * per)] = vals[p + (p >> 4)];
+      }
+    } else {
+      for (int p = t; p < out_n; p += kDrawThreads) put(produced + p, vals[p + (p >> 4)]);
     }
     if (produced + total >= draws) {
       // The thread holding the last value used stores the stream state after
