@@ -195,6 +195,21 @@ __device__ __forceinline__ uint64_t sdesc_none(const void* tile, uint32_t lbo, u
   return d;
 }
 
+// True in one lane of a converged warp.  A role of one thread is entered by
+// this rather than by `lane == 0`: under that test the compiler cannot tell
+// that one lane is active and issues each tcgen05 or TMA instruction through a
+// loop over lanes, 136 cycles an MMA of any shape against 39 (M = 64, N = 24)
+// to 63 (128 x 128), the rate of the tensor cores themselves.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(r));
+  return r != 0;
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T for one K=16 slice (single thread).
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc,
                                          uint64_t b_desc, uint32_t idesc,

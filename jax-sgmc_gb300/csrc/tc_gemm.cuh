@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN, A_MN, B_MN);
       uint32_t it = 0, acc = 0;
       bool ok = true;
@@ -611,7 +611,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc::elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int t = first; ok && t < tiles; t += step) {
@@ -648,7 +648,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       }
     }
   } else if (warp == 1) {
-    if (leader && lane == 0) {
+    if (leader && tc::elect_one()) {
       constexpr uint32_t idesc = tc::idesc_bf16_f32(BM, BN, A_MN, B_MN);
       uint32_t it = 0, acc = 0;
       bool ok = true;
