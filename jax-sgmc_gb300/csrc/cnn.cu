@@ -23,25 +23,18 @@
 //   inputs   dX = sum over taps of dY shifted back by the tap times the tap's
 //            W^T (the transposed convolution), A = dY (K-major), B = W
 //            (K-major), then the pooling's argmax routing and the ReLU mask.
-// conv1 reads its input by tap pairs from the images gathered as X8 [n, 32,
-// 32, 8]: pixel (h, w) holds the 3 channels of (h, w - 1), then its own 3,
-// then 2 zeros, so that one 16-byte core-matrix row of the unswizzled
-// layout serves the taps (kh, 0) and (kh, 1) together and another (kh, 2):
-// K = 3 kernel rows x 2 groups x 8 = 48 (padded to one 64-wide slice), each
-// group a shifted (16 W, 8 H) box; its weight gradient reads the same
-// boxes as an MN-major B.  Col is materialised for conv2 (32 input
+// conv1 and its weight gradient build their operands in shared memory from
+// the images (cnn_conv1_kernel).  Col is materialised for conv2 (32 input
 // channels).  Where
 // a tap's input channels fill a 128-byte row (64 BF16: conv3's input P2 and
 // the output gradients dY2, dY3 of the transposed convolutions) the GEMMs
 // are implicit: each 64-wide K slice of A (or 64-wide N block of dW's B) is
 // one tap's box of the NHWC map, shifted by the tap and read by TMA from a
-// 4-D tensor map, whose out-of-bounds zero fill is the SAME padding.  The forward GEMMs' epilogues apply bias and ReLU and
-// the 2x2 max-pool to the fp32 accumulators themselves (EpiConvPool): each
+// 4-D tensor map, whose out-of-bounds zero fill is the SAME padding.  The
+// forward GEMMs' epilogues apply bias and ReLU and the 2x2 max-pool to the
+// fp32 accumulators themselves (EpiConvPool for conv2 and conv3): each
 // epilogue warp holds whole pool windows in its 32 rows, so it writes the
-// pooled BF16 map and the argmax marks and no pre-pool activation is
-// stored.  For that the rows of conv1's GEMM (32 x 32 pixels) are ordered in
-// 16-pixel half rows, two image rows per 32 GEMM rows (conv1_row); conv2's
-// natural order (16 x 16) and conv3's (8 x 8) already have that property.
+// pooled BF16 map and the argmax marks and no pre-pool activation is stored.
 // Everything a GEMM reads is BF16.  Channel and K padding come from the tensor maps'
 // out-of-bounds zero fill; epilogues drop rows and columns past the real
 // extents.  The dense layer, softmax and their adjoints are small and run on
@@ -64,13 +57,9 @@ constexpr int kImg = 32, kInC = 3, kClasses = 10;
 constexpr int kC1 = 32, kC2 = 64, kC3 = 128;
 constexpr int kFlat = 4 * 4 * kC3;  // 2048
 constexpr int kK1 = 27;  // conv1's K (3 x 3 taps x 3 channels)
-constexpr int kX8 = 8;   // channels per gathered pixel: its left neighbour's 3, its own 3, 0, 0
-constexpr int kG1 = 8;   // conv1's K groups of 8 (6 real: kernel row kh, columns {0, 1} or {2})
-constexpr int kK1i = kG1 * kX8;  // conv1's GEMM K (one 64-wide slice)
-constexpr int kK2 = 9 * kC1, kK2p = 320;
+constexpr int kX8 = 8;   // slots of a pixel's word: its left neighbour's 3, its own 3, 0, 0
+constexpr int kK2 = 9 * kC1;
 constexpr int kK3 = 9 * kC2;  // conv3 reads P2 by tap: no padded im2col
-constexpr int kA1ld = kC1;  // conv1 output-gradient channels as stored (the dW1
-                            // GEMM's 64-wide box reads zeros past them)
 
 // Offsets of the leaves in a chain's flat parameter vector.
 constexpr int64_t ob1 = 0, oW1 = ob1 + kC1, ob2 = oW1 + kK1 * kC1, oW2 = ob2 + kC2,
@@ -79,9 +68,9 @@ constexpr int64_t ob1 = 0, oW1 = ob1 + kC1, ob2 = oW1 + kK1 * kC1, oW2 = ob2 + k
 static_assert(kP == 113738, "parameter count");
 
 struct CnnLayout {
-  size_t w1i, w2b, w3b;               // BF16 weights (conv1 unswizzled, others HWIO)
-  size_t x8, p1, col2, p2, p3;        // BF16 GEMM operands
-  size_t dy1, dy2, dy3;               // BF16 output gradients of the convs
+  size_t w2b, w3b;                    // BF16 weights (HWIO)
+  size_t p1, p2, p3;                  // BF16 GEMM operands
+  size_t dy2, dy3;                    // BF16 output gradients of conv2, conv3
   size_t m1, m2, m3;                  // uint8 argmax of each pool window
   size_t dp2, dp1;                    // fp32 input gradients of conv3, conv2
   size_t labels;                      // int32
@@ -93,11 +82,9 @@ struct CnnLayout {
 
 constexpr int kPrepBlocks = 64;  // Σw² partial sums per chain
 
-// Split-K factors of the weight-gradient GEMMs (K = pixels of n images:
-// 16n, 4n and n slices of 64 for the three layers; n is even; a factor
-// divides the slice count).  Layer 2 has 5 N tiles per chain: 16 splits
-// make 640 tiles for 8 chains (4.3 waves of 148 CTAs) where 8 made 320
-// (2.2 waves, the third one sixth full).
+// Split-K factors of the weight gradients (K = pixels of n images: 16n, 4n and
+// n slices of 64 for the three layers; n is even; a factor divides the slice
+// count).
 inline int wsplit(int layer, int n) {
   return layer == 1 ? 32 : layer == 2 ? (n % 4 == 0 ? 16 : 8) : (n % 4 == 0 ? 4 : 2);
 }
@@ -111,13 +98,9 @@ CnnLayout cnn_layout(int chains, int n) {
     return at;
   };
   const size_t N = n;
-  L.w1i = take(2 * kG1 * 64 * kX8);
   L.w2b = take(2 * kK2 * kC2);
   L.w3b = take(2 * kK3 * kC3);
-  L.x8 = take(2 * N * 1024 * kX8);
-  L.dy1 = take(2 * N * 1024 * kA1ld);
   L.p1 = take(2 * N * 256 * kC1);
-  L.col2 = take(2 * N * 256 * kK2p);
   L.dy2 = take(2 * N * 256 * kC2);
   L.p2 = take(2 * N * 64 * kC2);
   L.dy3 = take(2 * N * 64 * kC3);
@@ -136,7 +119,7 @@ CnnLayout cnn_layout(int chains, int n) {
   for (int l = 0; l < 3; ++l) L.part[l] = take(4 * wsplit(l + 1, n) * wc[l]);
   // Bias partials: one per unpool block and channel, 8 pooled elements per
   // thread and 256 threads per block: n*Ho*Wo*C / 2048 * C = 128 n floats
-  // for each of the three layers (at least one block).
+  // for layers 2 and 3 (at least one block), and layer 1's units as many.
   for (int l = 0; l < 3; ++l) L.bpart[l] = take(4 * 128 * (N + 1));
   L.total = off;
   return L;
@@ -158,9 +141,9 @@ struct CnnArgs {
   float* lk;
   double* lk_var;
   int* status;
-  bf16 *w1i, *w2b, *w3b, *x8, *p1, *col2, *p2, *p3;
+  bf16 *w2b, *w3b, *p1, *p2, *p3;
   float *dp2, *dp1;
-  bf16 *dy1, *dy2, *dy3;
+  bf16 *dy2, *dy3;
   uint8_t *m1, *m2, *m3;
   int32_t* lab;
   float *dp3, *gl;
@@ -174,119 +157,970 @@ struct CnnArgs {
 __device__ __forceinline__ float bf(bf16 v) { return __bfloat162float(v); }
 
 // ---------------------------------------------------------------------------
-// Weights to BF16 and partial sums of squares: conv2 and conv3 in HWIO
-// order, conv1 as the unswizzled K-major B of its GEMM, W1i [8 K groups][64
-// output channels][8 slots]: group g = 2 kh + p, slot s weighs input channel
-// s % 3 of tap (kh, p + s / 3); zero for s >= 6, for (p = 1, s < 3), for
-// groups >= 6 and outputs >= 32.  Grid (kPrepBlocks, chains).
+// conv1 straight from the images.
+//
+// conv1 has 27 inputs per output: as im2col boxes of 16 bytes a pixel its
+// GEMMs were bound by the rate at which TMA takes box rows (720 cycles per 64
+// pixels), and dY1, three quarters zeros, was the largest array of a
+// gradient.  Here a CTA takes a strip (8 pool windows of all 16 window rows of
+// an image) at a time and builds the operands in shared memory itself.
+//
+// X8: pixel (h, w) is one 16-byte word of BF16, the channels of (h, w - 1),
+// its own, two zeros.  Tap pair p = 0 of output pixel (h, w) and kernel row
+// kh is the word (h + kh - 1, w) (kw = 0, 1), p = 1 the word (.., w + 1) (its
+// slots 3-5 are kw = 2; slots 0-2 repeat kw = 1 and have zero weights), so a
+// K = 16 slice is a kernel row.  The words lie in planes by column parity (E:
+// w = 16 s + 2 j, O: w = 16 s + 2 j + 1; 34 image rows with the zero rows
+// above and below, 9 words a row): 8 neighbouring windows' words at one
+// position of the window are 128 contiguous bytes, a core matrix of the
+// unswizzled layout, and a descriptor's strides reach the other window rows,
+// the second tap pair and the other kernel rows.  Nothing is copied per tap.
+// Core matrices start on 16-byte boundaries, as that layout allows.
+// For 8 x 256 images the forward pass took 128 us as three launches (weights,
+// gather, GEMM) and takes 36; the output gradient with the weight GEMM took
+// 137 and takes 55 (32 splits of 8 chains leave a third of the SMs one CTA).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) cnn_prep_kernel(const CnnArgs a) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ double red[32];
-  const int c = blockIdx.y;
-  const float* w = a.w + static_cast<int64_t>(c) * kP;
-  for (int e = blockIdx.x * 256 + threadIdx.x; e < kG1 * 64 * kX8; e += kPrepBlocks * 256) {
-    const int g = e / (64 * kX8), co = (e / kX8) % 64, sl = e % kX8;
-    const int kh = g >> 1, pp = g & 1, kw = pp + sl / kInC, ci = sl % kInC;
-    const bool real = g < 6 && co < kC1 && sl < 2 * kInC && (pp == 0 || sl >= kInC);
-    const float v = real ? __ldg(w + oW1 + ((kh * 3 + kw) * kInC + ci) * kC1 + co) : 0.f;
-    a.w1i[static_cast<int64_t>(c) * kG1 * 64 * kX8 + e] = __float2bfloat16_rn(v);
-  }
-  float sq = 0.f;
-  for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < kP; i += kPrepBlocks * 256) {
-    const float v = __ldg(w + i);
-    sq = fmaf(v, v, sq);
-    if (i >= oW2 && i < ob3)
-      a.w2b[static_cast<int64_t>(c) * kK2 * kC2 + (i - oW2)] = __float2bfloat16_rn(v);
-    else if (i >= oW3 && i < obd)
-      a.w3b[static_cast<int64_t>(c) * kK3 * kC3 + (i - oW3)] = __float2bfloat16_rn(v);
-  }
-  const double tot = block_sum(static_cast<double>(sq), red);
-  if (threadIdx.x == 0) a.psq[c * kPrepBlocks + blockIdx.x] = tot;
+constexpr int kStripThreads = 128;
+constexpr int kPlaneRow = 9 * 16, kPlane = 34 * kPlaneRow;   // bytes
+constexpr int kStripItems = 32 * 9, kStripIters = (kStripItems + kStripThreads - 1) / kStripThreads;
+
+// Bounded wait that raises the CTA's abort flag and the status.
+__device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
+                                          int* status) {
+  if (mbar_wait_bounded(bar, parity, abort)) return true;
+  raise_status(status, GBSGMC_ERR_TIMEOUT);
+  *abort = 1;
+  return false;
 }
 
-// Row of pixel (h, w) of a 32 x 32 image in conv1's GEMM (and in its output
-// gradient dY1): a 128-row tile holds the 16 columns w0 .. w0 + 15 (w0 = 0
-// or 16) of image rows 8u .. 8u + 7, the (16 W, 8 H) box of one TMA load
-// in row-major order.  Every 32 rows hold image rows 2k (lanes 0-15) and
-// 2k + 1 (lanes 16-31), so that every 2 x 2 pool window lies in one warp's
-// rows, at lanes (l, l ^ 1, l ^ 16, l ^ 17).
-__host__ __device__ __forceinline__ int conv1_row(int h, int w) {
-  return ((h >> 3) << 8) | ((w >> 4) << 7) | ((h & 7) << 4) | (w & 15);
-}
-// Its inverse: the pixel of row r (0 <= r < 1024).
-__host__ __device__ __forceinline__ void conv1_pixel(int r, int& h, int& w) {
-  h = ((r >> 8) << 3) | ((r >> 4) & 7);
-  w = (((r >> 7) & 1) << 4) | (r & 15);
-}
-
-// ---------------------------------------------------------------------------
-// Gather of the minibatch images as BF16 X8 [n, 32, 32, 8] in natural pixel
-// order, pixel (h, w) holding channels 0-2 of (h, w - 1) (zero at w = 0),
-// channels 0-2 of (h, w) and two zeros, plus labels.
-// Grid (n*1024/256, chains): one thread per pixel, one 16-byte store each.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) cnn_gather1_kernel(const CnnArgs a) {
-  pdl_trigger();
-  pdl_wait();
-  const int c = blockIdx.y;
-  const int p = blockIdx.x * 256 + threadIdx.x;
-  if (p >= a.n * 1024) return;
-  const int i = p >> 10, hw = p & 1023;
-  int64_t o = a.idx[static_cast<int64_t>(c) * a.idx_stride + i];
-  if (o < 0 || o >= a.n_rows) {
-    raise_status(a.status, GBSGMC_ERR_INDEX);
-    o = 0;
-  }
-  if (hw == 0) {
-    const float lf = __ldg(a.labels + o * a.label_ld);
-    int lab = static_cast<int>(lf);
-    if (!(lf >= 0.f) || lab >= kClasses) {
-      raise_status(a.status, GBSGMC_ERR_INDEX);
-      lab = 0;
+// Pixels w - 1, w, w + 1 (w even) of an image row, px pointing at w; zeros
+// when !in, and at w - 1 when !left.  `pair`: rows are 8-byte aligned, so are
+// pixel pairs (6 floats).
+__device__ __forceinline__ void pair_load(const float* px, bool in, bool left, bool pair,
+                                          float (&v)[9]) {
+#pragma unroll
+  for (int e = 0; e < 9; ++e) v[e] = 0.f;
+  if (pair) {
+    if (in && left) {
+      v[0] = __ldg(px - 3);
+      const float2 q = __ldg(reinterpret_cast<const float2*>(px - 2));
+      v[1] = q.x;
+      v[2] = q.y;
     }
-    a.lab[static_cast<int64_t>(c) * a.n + i] = lab;
+    if (in) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const float2 q = __ldg(reinterpret_cast<const float2*>(px) + e);
+        v[3 + 2 * e] = q.x;
+        v[4 + 2 * e] = q.y;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 9; ++e)
+      if (in && (e >= 3 || left)) v[e] = __ldg(px - 3 + e);
   }
-  const float* px = a.X + o * a.ld + hw * kInC;
-  const bool left = (hw & 31) != 0;
-  const float l0 = left ? __ldg(px - 3) : 0.f, l1 = left ? __ldg(px - 2) : 0.f,
-              l2 = left ? __ldg(px - 1) : 0.f;
-  const __nv_bfloat162 q0 = __floats2bfloat162_rn(l0, l1);
-  const __nv_bfloat162 q1 = __floats2bfloat162_rn(l2, __ldg(px));
-  const __nv_bfloat162 q2 = __floats2bfloat162_rn(__ldg(px + 1), __ldg(px + 2));
-  reinterpret_cast<uint4*>(a.x8)[static_cast<int64_t>(c) * a.n * 1024 + p] =
-      make_uint4(*reinterpret_cast<const uint32_t*>(&q0), *reinterpret_cast<const uint32_t*>(&q1),
-                 *reinterpret_cast<const uint32_t*>(&q2), 0u);
+}
+
+// Their words: E of pixel w, O of pixel w + 1.
+__device__ __forceinline__ void pair_words(const float (&v)[9], uint4& e, uint4& o) {
+  uint32_t q[5];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    q[i] = *reinterpret_cast<const uint32_t*>(&p);
+  }
+  const __nv_bfloat162 last = __floats2bfloat162_rn(v[8], 0.f);
+  q[4] = *reinterpret_cast<const uint32_t*>(&last);
+  e = make_uint4(q[0], q[1], q[2], 0u);
+  o = make_uint4(__byte_perm(q[1], q[2], 0x5432), __byte_perm(q[2], q[3], 0x5432),
+                 __byte_perm(q[3], q[4], 0x5432), 0u);
+}
+__device__ __forceinline__ void store_word(uint8_t* at, const uint4& v) {
+  tc::sts128(at, v.x, v.y, v.z, v.w);
+}
+
+// Index of image `img` (of all chains'), as given.
+__device__ __forceinline__ int image_index(const CnnArgs& a, int64_t img) {
+  const int c = static_cast<int>(img / a.n), i = static_cast<int>(img - int64_t(c) * a.n);
+  return __ldg(a.idx + c * a.idx_stride + i);
+}
+// Its observation: the first one stands in for an invalid index (which the
+// forward pass reports).
+__device__ __forceinline__ int64_t valid_row(const CnnArgs& a, int o) {
+  return o >= 0 && o < a.n_rows ? o : 0;
+}
+
+// One thread's share of a strip, in registers: items (image row h, pair j),
+// item = 9 h + j: pixels w - 1, w, w + 1 with w = 16 s + 2 j.
+struct StripRegs {
+  float v[kStripIters][9];
+  float label;   // the last thread's
+};
+
+__device__ __forceinline__ void strip_load(const CnnArgs& a, int index, int s, bool pair,
+                                           StripRegs& x) {
+  const int64_t o = valid_row(a, index);
+  if (o != index) raise_status(a.status, GBSGMC_ERR_INDEX);
+  const float* row = a.X + o * a.ld;
+  if (threadIdx.x == kStripThreads - 1) x.label = __ldg(a.labels + o * a.label_ld);
+#pragma unroll
+  for (int k = 0; k < kStripIters; ++k) {
+    const int item = threadIdx.x + k * kStripThreads;
+    const int h = item / 9, w = 16 * s + 2 * (item % 9);
+    pair_load(row + (h * kImg + w) * kInC, item < kStripItems && w < kImg, w > 0, pair, x.v[k]);
+  }
+}
+
+// The strip's words into planes E, O and E again (so that the second tap pair
+// of an odd column lies a positive stride from the first).
+__device__ __forceinline__ void strip_store(const StripRegs& x, uint8_t* planes) {
+#pragma unroll
+  for (int k = 0; k < kStripIters; ++k) {
+    const int item = threadIdx.x + k * kStripThreads;
+    if (item >= kStripItems) break;
+    uint8_t* at = planes + kPlaneRow + 16 * item;
+    uint4 e, o;
+    pair_words(x.v[k], e, o);
+    store_word(at, e);
+    store_word(at + kPlane, o);
+    store_word(at + 2 * kPlane, e);
+  }
+}
+
+// Zero rows above and below the image in the planes.
+__device__ __forceinline__ void strip_borders(uint8_t* smem) {
+  for (int e = threadIdx.x; e < 3 * 18; e += kStripThreads) {
+    const int p = e / 18, r = e % 18;
+    tc::sts128(smem + p * kPlane + (r < 9 ? 16 * r : 33 * kPlaneRow + 16 * (r - 9)), 0u, 0u, 0u,
+               0u);
+  }
+}
+
+// BF16 weights of conv2 ([output octet][tap, input][8], so that outputs and
+// inputs both lie in core matrices) and conv3 (HWIO order) and part `b` of a chain's sum
+// of squares.
+__device__ __forceinline__ void cnn_prep(const CnnArgs& a, int c, int b, double* red) {
+  constexpr int kCols = 256, kEach = kCols / kStripThreads;
+  const float* w = a.w + static_cast<int64_t>(c) * kP;
+  float sq[kEach] = {};
+  for (int i = b * kCols + threadIdx.x; i < kP; i += kPrepBlocks * kCols) {
+#pragma unroll
+    for (int u = 0; u < kEach; ++u) {
+      const int j = i + u * kStripThreads;
+      if (j >= kP) break;
+      const float v = __ldg(w + j);
+      sq[u] = fmaf(v, v, sq[u]);
+      if (j >= oW2 && j < ob3)
+        a.w2b[static_cast<int64_t>(c) * kK2 * kC2 +
+              ((j - oW2) % kC2 / 8 * kK2 + (j - oW2) / kC2) * 8 + j % 8] = __float2bfloat16_rn(v);
+      else if (j >= oW3 && j < obd)
+        a.w3b[static_cast<int64_t>(c) * kK3 * kC3 + (j - oW3)] = __float2bfloat16_rn(v);
+    }
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int u = 0; u < kEach; ++u) {
+    const double part = warp_sum(static_cast<double>(sq[u]));
+    if (lane == 0) red[u * (kStripThreads / 32) + warp] = part;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double tot = 0.0;
+    for (int i = 0; i < kCols / 32; ++i) tot += red[i];
+    a.psq[c * kPrepBlocks + b] = tot;
+  }
+  __syncthreads();
+}
+
+// 16 columns of each of four accumulators 32 columns apart (one wait).
+__device__ __forceinline__ void tmem_ld16x4(uint32_t taddr, float (&v)[4][16]) {
+  uint32_t r[4][16];
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[p][0]), "=r"(r[p][1]), "=r"(r[p][2]), "=r"(r[p][3]), "=r"(r[p][4]),
+          "=r"(r[p][5]), "=r"(r[p][6]), "=r"(r[p][7]), "=r"(r[p][8]), "=r"(r[p][9]),
+          "=r"(r[p][10]), "=r"(r[p][11]), "=r"(r[p][12]), "=r"(r[p][13]), "=r"(r[p][14]),
+          "=r"(r[p][15])
+        : "r"(taddr + p * kC1));
+#pragma unroll
+  for (int p = 0; p < 4; ++p)   // the registers may be used after the wait only
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[p][0]), "+r"(r[p][1]), "+r"(r[p][2]), "+r"(r[p][3]), "+r"(r[p][4]),
+                   "+r"(r[p][5]), "+r"(r[p][6]), "+r"(r[p][7]), "+r"(r[p][8]), "+r"(r[p][9]),
+                   "+r"(r[p][10]), "+r"(r[p][11]), "+r"(r[p][12]), "+r"(r[p][13]),
+                   "+r"(r[p][14]), "+r"(r[p][15])
+                 :
+                 : "memory");
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[p][i] = __uint_as_float(r[p][i]);
+}
+
+// Forward: P1 and its marks, and beside it what needs no launch of its own:
+// the labels, the BF16 weights of the other layers and the sums of squares.
+// Four CTAs per SM (128 TMEM columns each), each a run of consecutive strips;
+// one CTA's loads and epilogue overlap the others' MMAs.  The four pixels of
+// a window are four accumulators (M = 128 windows, N = 32) of the same TMEM
+// lane, so the pooling needs no exchange between lanes.
+__global__ void __launch_bounds__(kStripThreads, 4) cnn_conv1_kernel(const CnnArgs a, int pair) {
+  __shared__ __align__(128) uint8_t planes[3 * kPlane];
+  __shared__ __align__(128) bf16 w_s[6 * kC1 * kX8];   // [tap pair 2 kh + p][output][slot]
+  __shared__ float b_s[kC1];
+  __shared__ double red[32];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_slot;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) {
+    mbar_init(&bar, 1);
+    mbar_fence_init();
+  }
+  if (warp == 0) {
+    tc::tmem_alloc(&tmem_slot, 128);
+    tc::tmem_relinquish();
+  }
+  strip_borders(planes);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+
+  const int64_t strips = 2 * static_cast<int64_t>(a.chains) * a.n;
+  const int64_t u0 = strips * blockIdx.x / gridDim.x, u1 = strips * (blockIdx.x + 1) / gridDim.x;
+  StripRegs x;
+  int next = 0;   // index of the strip after the loaded one
+  if (u0 < u1) {
+    strip_load(a, image_index(a, u0 >> 1), static_cast<int>(u0 & 1), pair, x);
+    if (u0 + 1 < u1) next = image_index(a, (u0 + 1) >> 1);
+  }
+  for (int e = blockIdx.x; e < a.chains * kPrepBlocks; e += gridDim.x)
+    cnn_prep(a, e / kPrepBlocks, e % kPrepBlocks, red);
+
+  constexpr uint32_t idesc = tc::idesc_bf16_f32(128, kC1);
+  int chain = -1;
+  uint32_t phase = 0;
+  bool ok = true;
+  for (int64_t u = u0; u < u1; ++u, phase ^= 1u) {
+    const int64_t img = u >> 1;
+    const int s = static_cast<int>(u & 1), c = static_cast<int>(img / a.n);
+    if (c != chain) {
+      chain = c;
+      const float* w = a.w + static_cast<int64_t>(c) * kP;
+      for (int e = t; e < 6 * kC1 * kX8; e += kStripThreads) {
+        const int g = e / (kC1 * kX8), co = (e / kX8) % kC1, sl = e % kX8;
+        const int kw = (g & 1) + sl / kInC, ci = sl % kInC;
+        const bool real = sl < 2 * kInC && ((g & 1) == 0 || sl >= kInC);
+        const float v = real ? __ldg(w + oW1 + (((g >> 1) * 3 + kw) * kInC + ci) * kC1 + co) : 0.f;
+        w_s[e] = __float2bfloat16_rn(v);
+      }
+      if (t < kC1) b_s[t] = __ldg(w + ob1 + t);
+    }
+    strip_store(x, planes);
+    tc::fence_async_shared();
+    if (t == kStripThreads - 1 && s == 0) {
+      int lab = static_cast<int>(x.label);
+      if (!(x.label >= 0.f) || lab >= kClasses) {
+        raise_status(a.status, GBSGMC_ERR_INDEX);
+        lab = 0;
+      }
+      a.lab[img] = lab;
+    }
+    // The next strip's loads are under way while this one is multiplied.
+    if (u + 1 < u1) {
+      strip_load(a, next, static_cast<int>((u + 1) & 1), pair, x);
+      if (u + 2 < u1) next = image_index(a, (u + 2) >> 1);
+    }
+    __syncthreads();
+    if (warp == 0 && tc::elect_one()) {
+      tc::fence_after_sync();
+      const uint64_t A0 = tc::sdesc_none(planes, kPlane, 2 * kPlaneRow);
+      const uint64_t A1 = tc::sdesc_none(planes + kPlane, kPlane + 16, 2 * kPlaneRow);
+      const uint64_t B = tc::sdesc_none(w_s, kC1 * 16, 128);
+#pragma unroll
+      for (int pos = 0; pos < 4; ++pos)
+#pragma unroll
+        for (int kh = 0; kh < 3; ++kh)
+          tc::mma_bf16(tmem + pos * kC1,
+                       ((pos & 1) ? A1 : A0) + ((pos >> 1) + kh) * (kPlaneRow / 16),
+                       B + kh * (2 * kC1 * kX8 * 2 / 16), idesc, kh != 0);
+      tc::mma_commit(&bar);
+    }
+    ok = mbar_wait_bounded(&bar, phase, nullptr);
+    tc::fence_after_sync();
+    if (ok) {
+      // Lane 8 i + j of warp q is the window (4 q + i, 8 s + j).
+      const int64_t pix = img * 256 + (4 * warp + (lane >> 3)) * 16 + 8 * s + (lane & 7);
+      bf16* p1 = a.p1 + ((img * 16 + 4 * warp + (lane >> 3)) * 64 + 8 * s + (lane & 7)) * 8;
+      const uint32_t acc = tmem + (static_cast<uint32_t>(warp * 32) << 16);
+#pragma unroll
+      for (int q = 0; q < kC1 / 16; ++q) {
+        float v[4][16];
+        tmem_ld16x4(acc + 16 * q, v);
+        uint32_t pk[8], mk[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mk[e] = 0u;
+        float best[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float b = b_s[16 * q + j];
+          const float y0 = v[0][j] + b, y1 = v[1][j] + b, y2 = v[2][j] + b, y3 = v[3][j] + b;
+          // The ReLU of the maximum, and the first position that has it (of no
+          // account where the ReLU is closed).
+          best[j] = fmaxf(fmaxf(fmaxf(y0, y1), fmaxf(y2, y3)), 0.f);
+          const uint32_t at = y0 == best[j] ? 4u : y1 == best[j] ? 5u : y2 == best[j] ? 6u : 7u;
+          mk[j >> 2] |= (best[j] > 0.f ? at : 0u) << (8 * (j & 3));
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(best[2 * e], best[2 * e + 1]);
+          pk[e] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        *reinterpret_cast<uint4*>(p1 + 256 * q) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+        *reinterpret_cast<uint4*>(p1 + 256 * q + 128) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        *reinterpret_cast<uint4*>(a.m1 + pix * kC1 + 16 * q) =
+            make_uint4(mk[0], mk[1], mk[2], mk[3]);
+      }
+    }
+    tc::fence_before_sync();
+    if (__syncthreads_or(!ok)) break;   // also: the planes and accumulators are free
+  }
+  if (!ok) {
+    raise_status(a.status, GBSGMC_ERR_TIMEOUT);
+    mbar_wait_bounded(&bar, phase, nullptr);   // MMAs still in flight
+  }
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 128);
+  }
+}
+
+// dW1 = dY1^T Col1 and db1, dY1 built from dP1 and the marks in units of 8
+// image rows.  A CTA adds its run of 64-pixel slices (4 rows of a 16-column
+// half; the order of slices: rows 0-3 and 4-7 of the left half, then of the
+// right) in one accumulator (M = 64 output channels, 32 real) and writes one
+// split-K partial; a K = 16 slice is the half's 16 pixels of an image row, its
+// even columns, then its odd ones.  Here a row's words lie in three runs of
+// 16, E, O and E one column on, and the N groups of an MMA are three rows' runs
+// (N = 72, the stride of a run): for the even columns E is tap pair 0 and O
+// pair 1, for the odd ones (one run further on) O and the shifted E, and the
+// third run of each row is dropped.  dY: [image row h][half][column parity]
+// [channel octet][8 windows] words of 8 channels; the rows past the octets
+// that the MMA reads belong to the next block of dY (or to the words) and end
+// in accumulator rows that nothing reads.  The operands are double buffered:
+// the MMAs of a unit (issued by a warp of its own) run while the next is
+// built.  db1 (another warp): the routed
+// (BF16-rounded) values of a unit's 64 windows are added in window order, a
+// partial per unit.  Grid (splits, chains).
+constexpr int kUnitBuilders = 256, kUnitThreads = kUnitBuilders + 64;
+constexpr int kUnitRow = 3 * 256;   // bytes of a row's E, O and shifted E
+constexpr int kUnitDy = 8 * 2 * 1024, kUnitWords = 11 * kUnitRow, kUnitBias = 64 * 36 * 4;
+constexpr int kUnitBuf = kUnitDy + kUnitWords + kUnitBias;
+static_assert(kUnitBuf % 128 == 0, "buffer alignment");
+constexpr int kUnitSmem = 2 * kUnitBuf;
+
+__global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const CnnArgs a,
+                                                                        int pair) {
+  extern __shared__ __align__(128) uint8_t unit_smem[];
+  __shared__ uint64_t full[2], free_[2];   // a buffer is built; its MMAs and sums are done
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_s;
+  volatile int* abort_flag = &abort_s;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  if (t == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(full + i, kUnitBuilders / 32);
+      mbar_init(free_ + i, 2);
+    }
+    abort_s = 0;
+    mbar_fence_init();
+  }
+  if (warp == 0) {
+    tc::tmem_alloc(&tmem_slot, 128);
+    tc::tmem_relinquish();
+  }
+  // The words' last row stands behind a unit's last for the dropped run.
+  for (int e = t; e < 2 * kUnitRow / 16; e += kUnitThreads)
+    store_word(unit_smem + (e & 1) * kUnitBuf + kUnitDy + 10 * kUnitRow + (e >> 1) * 16,
+               make_uint4(0u, 0u, 0u, 0u));
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+
+  const int c = blockIdx.y, S = gridDim.x;
+  const int each = 16 * a.n / S, q0 = each * blockIdx.x, q1 = q0 + each;   // slices
+  const int u0 = q0 >> 2, u1 = (q1 + 3) >> 2;                              // units
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    return conv_wait(bar, parity, abort_flag, a.status);
+  };
+  if (warp == kUnitBuilders / 32) {   // the MMAs
+    constexpr uint32_t idesc = tc::idesc_bf16_f32(64, 72, true, true);
+    if (tc::elect_one()) {
+      for (int u = u0; u < u1; ++u) {
+        const int it = u - u0, b = it & 1;
+        if (!wait(full + b, (it >> 1) & 1u)) break;
+        tc::fence_after_sync();
+        const uint8_t* dy = unit_smem + b * kUnitBuf;
+        const uint64_t A = tc::sdesc_none(dy, 512, 128);
+        const uint64_t B = tc::sdesc_none(dy + kUnitDy, 256, 256);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {   // the unit's slices: half q / 2, rows 4 (q % 2) ..
+          if (4 * u + q < q0 || 4 * u + q >= q1) continue;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const int h = 4 * (q & 1) + r, half = q >> 1;
+            tc::mma_bf16(tmem, A + (2 * h + half) * 64, B + (h * kUnitRow + half * 128) / 16,
+                         idesc, 4 * u + q > q0 || r > 0);
+          }
+        }
+        tc::mma_commit(free_ + b);
+      }
+    }
+    __syncwarp();
+  } else if (warp > kUnitBuilders / 32) {   // the bias
+    for (int u = u0; u < u1; ++u) {
+      const int it = u - u0, b = it & 1;
+      if (!__all_sync(0xffffffffu, wait(full + b, (it >> 1) & 1u))) break;
+      const float* bias =
+          reinterpret_cast<const float*>(unit_smem + b * kUnitBuf + kUnitDy + kUnitWords);
+      float sum = 0.f;
+#pragma unroll 16
+      for (int w = 0; w < 64; ++w) sum += bias[w * 36 + lane];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(free_ + b);
+      // A unit cut by a split boundary belongs to the split of its first slice.
+      if (4 * u >= q0) a.bpart[0][(int64_t(c) * 4 * a.n + u) * kC1 + lane] = sum;
+    }
+  } else {
+    // This thread's window (row wy of the unit's 4, column wx) and channels,
+    // and its pixel pair of X8 (rows -1 .. 8 of the unit, 17 pairs a row).
+    const int j = lane & 7, oct = lane >> 3, wx = 8 * (warp & 1) + j, wy = warp >> 1;
+    const int xr = t / 17, xj = t % 17;
+    struct Part {
+      float4 g[2];
+      uint2 mark;
+      float x[9];
+    };
+    auto row_of = [&](int u) { return image_index(a, int64_t(c) * a.n + (u >> 2)); };
+    auto load = [&](int u, int index, Part& p) {
+      const int64_t o = valid_row(a, index);
+      const int64_t img = int64_t(c) * a.n + (u >> 2);
+      const int hb = u & 3;
+      const float4* d = reinterpret_cast<const float4*>(
+          a.dp1 + ((img * 16 + 4 * hb + wy) * 64 + 16 * oct + wx) * 8);
+      p.g[0] = __ldg(d);
+      p.g[1] = __ldg(d + 1);
+      p.mark = __ldg(reinterpret_cast<const uint2*>(
+          a.m1 + (img * 256 + (4 * hb + wy) * 16 + wx) * kC1 + 8 * oct));
+      const int h = 8 * hb + xr - 1;
+      const bool in = xr < 10 && h >= 0 && h < kImg && xj < 16;
+      // The 17th pair holds the column past the image: zeros, as at w = -1.
+      pair_load(a.X + o * a.ld + (h * kImg + 2 * xj) * kInC, in, xj > 0, pair, p.x);
+    };
+    // Loads are two units ahead of their use, the observations' indices three.
+    Part part[2];
+    load(u0, row_of(u0), part[0]);
+    if (u0 + 1 < u1) load(u0 + 1, row_of(u0 + 1), part[1]);
+    int next = u0 + 2 < u1 ? row_of(u0 + 2) : 0;
+    auto unit = [&](int u, Part& p) -> bool {
+      const int it = u - u0, b = it & 1;
+      uint8_t* dy = unit_smem + b * kUnitBuf;
+      uint8_t* words = dy + kUnitDy;
+      float* bias = reinterpret_cast<float*>(words + kUnitWords);
+      if (it >= 2 && !__all_sync(0xffffffffu, wait(free_ + b, ((it >> 1) - 1) & 1u))) return false;
+      if (xr < 10) {
+        uint4 e, o;
+        pair_words(p.x, e, o);
+        uint8_t* at = words + xr * kUnitRow + 16 * xj;
+        if (xj < 16) {
+          store_word(at, e);
+          store_word(at + 256, o);
+        }
+        if (xj > 0) store_word(at + 512 - 16, e);
+      }
+      {
+        const float* gv = reinterpret_cast<const float*>(p.g);
+        const uint2 mark = p.mark;
+        uint32_t pk[4];
+        float4 bv[2];
+        float* bf8 = reinterpret_cast<float*>(bv);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          // BF16 pair, zero where the ReLU was closed (mark bit 2).
+          const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
+          const __nv_bfloat162 v = __floats2bfloat162_rn((m & 4u) ? gv[2 * e] : 0.f,
+                                                         (m & 0x400u) ? gv[2 * e + 1] : 0.f);
+          bf8[2 * e] = __low2float(v);
+          bf8[2 * e + 1] = __high2float(v);
+          pk[e] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+        float4* bd = reinterpret_cast<float4*>(bias + (16 * wy + wx) * 36 + 8 * oct);
+        bd[0] = bv[0];
+        bd[1] = bv[1];
+#pragma unroll
+        for (int pos = 0; pos < 4; ++pos) {
+          uint32_t o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
+            o[e] = pk[e] & (((m & 3u) == static_cast<uint32_t>(pos) ? 0xffffu : 0u) |
+                            (((m >> 8) & 3u) == static_cast<uint32_t>(pos) ? 0xffff0000u : 0u));
+          }
+          tc::sts128(dy + ((2 * wy + (pos >> 1)) * 2 + (warp & 1)) * 1024 + (pos & 1) * 512 +
+                         16 * lane,
+                     o[0], o[1], o[2], o[3]);
+        }
+      }
+      tc::fence_async_shared();
+      if (u + 2 < u1) {
+        load(u + 2, next, p);
+        if (u + 3 < u1) next = row_of(u + 3);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + b);
+      return true;
+    };
+    for (int u = u0; u < u1; u += 2) {
+      if (!unit(u, part[0])) break;
+      if (u + 1 < u1 && !unit(u + 1, part[1])) break;
+    }
+  }
+  // Every MMA has completed: the last two units' are waited for here.
+  const int done = u1 - u0;
+  for (int i = done > 1 ? done - 2 : 0; i < done; ++i)
+    if (!mbar_wait_bounded(free_ + (i & 1), (i >> 1) & 1u, abort_flag)) {
+      raise_status(a.status, GBSGMC_ERR_TIMEOUT);
+      *abort_flag = 1;
+    }
+  __syncthreads();
+  if (*abort_flag) {   // MMAs issued complete within microseconds
+    const uint64_t t0 = global_ns();
+    while (global_ns() - t0 < 2000000ull) {
+    }
+  }
+  tc::fence_after_sync();
+  if (warp < 2) {
+    // Accumulator row r of an M = 64 tile is TMEM lane 32 (r / 16) + r % 16.
+    float* dst = a.part[0] + (static_cast<int64_t>(c) * S + blockIdx.x) * kK1 * kC1 + 16 * warp +
+                 lane;
+#pragma unroll
+    for (int kh = 0; kh < 3; ++kh) {   // columns (kh, run, slot)
+      float v[32];
+      tc::tmem_ld32(tmem + 24 * kh + (static_cast<uint32_t>(warp * 32) << 16), v);
+      if (lane < 16) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+          for (int sl = p * kInC; sl < 2 * kInC; ++sl)
+            dst[((kh * 3 + p + sl / kInC) * kInC + sl % kInC) * kC1] = v[8 * p + sl];
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, 128);
+  }
+}
+
+// The 2 x 2 max-pool of 32 channels of a warp's 32 pixels (ReLU applied): the
+// window of lane l is lanes (base, base + 1, base + V, base + V + 1), base = l
+// & ~(V | 1), in window order.  Lane l ends with the maxima (BF16) and marks
+// of 8 channels, chunk `wp` (returned) of the 32.  The window maxima take two
+// exchange stages instead of four shuffles per channel: the two pixels of a
+// window row swap the halves of the channels they do not keep (16 shuffles)
+// and keep the pairwise maximum, then the two rows swap halves again (8
+// shuffles); comparisons are strict in window order (left before right, top
+// before bottom), which keeps the first maximum of the window as the
+// sequential scan does.
+template <int V>
+__device__ __forceinline__ int pool_windows(const float (&x)[32], uint4& p, uint2& mk) {
+  const unsigned full = 0xffffffffu;
+  const int lane = epi::lane_id();
+  const int wp = ((lane & V) ? 2 : 0) | (lane & 1);
+  // Stage 1, the window row's two pixels (lanes l, l ^ 1): keep the
+  // chunks {cbit, cbit + 2} of 8 channels (kept channel i: i < 8 in
+  // the first, i >= 8 in the second), send the other two.
+  const bool cbit = (lane & 1) != 0, rbit = (lane & V) != 0;
+  float m1[16];
+  uint32_t col_bits = 0;  // bit i: kept channel i's maximum is the right pixel
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int lo = q < 8 ? q : 8 + q, hi = lo + 8;
+    const float mine = cbit ? x[hi] : x[lo];
+    const float other = __shfl_xor_sync(full, cbit ? x[lo] : x[hi], 1);
+    const float left = cbit ? other : mine, right = cbit ? mine : other;
+    const bool rt = right > left;
+    m1[q] = rt ? right : left;
+    col_bits |= (rt ? 1u : 0u) << q;
+  }
+  // Stage 2, the window's two rows (lanes l, l ^ V): the top row keeps
+  // kept channels 0-7 (chunk cbit), the bottom row 8-15 (chunk
+  // cbit + 2): chunk wp of the 32 channels.
+  const uint32_t other_bits = __shfl_xor_sync(full, col_bits, V);
+  float best_mine[8];
+  uint32_t mark_mine[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int ki = rbit ? 8 + q : q;
+    const float mine = rbit ? m1[8 + q] : m1[q];
+    const float other = __shfl_xor_sync(full, rbit ? m1[q] : m1[8 + q], V);
+    const uint32_t my_col = (col_bits >> ki) & 1u, ot_col = (other_bits >> ki) & 1u;
+    const float top = rbit ? other : mine, bot = rbit ? mine : other;
+    const uint32_t top_col = rbit ? ot_col : my_col, bot_col = rbit ? my_col : ot_col;
+    const bool b2 = bot > top;
+    const float best = b2 ? bot : top;
+    best_mine[q] = best;
+    mark_mine[q] = (b2 ? 2u + bot_col : top_col) | (best > 0.f ? 4u : 0u);
+  }
+  uint32_t pk[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __nv_bfloat162 pr = __floats2bfloat162_rn(best_mine[2 * e], best_mine[2 * e + 1]);
+    pk[e] = *reinterpret_cast<const uint32_t*>(&pr);
+  }
+  p = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+  mk.x = mark_mine[0] | (mark_mine[1] << 8) | (mark_mine[2] << 16) | (mark_mine[3] << 24);
+  mk.y = mark_mine[4] | (mark_mine[5] << 8) | (mark_mine[6] << 16) | (mark_mine[7] << 24);
+  return wp;
 }
 
 // ---------------------------------------------------------------------------
-// im2col of a pooled map P [n, H, W, C] -> Col [n*H*W, Kp], K = (kh, kw, ci):
-// the 9C real columns of each row (row stride Kp); the columns 9C..Kp-1 are
-// never written (the tensor maps that read Col end at 9C, so their boxes
-// read zeros there).  One thread per 8 consecutive K entries (C is a
-// multiple of 8).  Grid (ceil(n*H*W*9C/8 / 256), chains).
+// conv2 (16 x 16 images), its input gradient and its weight gradient without
+// an im2col.
+//
+// The maps they read are stored in rows of channel octets, [image][h][octet]
+// [w][8]: one TMA box of a strip (8 columns of an image, all rows) with its
+// halo lands as [h][octet][10 columns] words of 16 bytes, zeros outside the
+// image (the SAME padding), and any 8 neighbouring pixels of an octet are a
+// core matrix of the unswizzled layout.  A tap is then only another start
+// address of the same box: conv2's box of 128 pixels is 72 rows of 160 bytes
+// for TMA instead of 9 boxes, or an im2col of 9 times the map, written and read
+// back.  2,048 images: 25 us against 147 with the im2col (335 MB), dP1 26
+// against 115 with a box per tap, dW2 25 against 95.  W2 lies in shared memory,
+// [output octet][tap, input][8], for a run of strips of one chain: MN-major B
+// of the forward GEMM, K-major B of the transposed one.
 // ---------------------------------------------------------------------------
-template <int H, int W, int C, int Kp>
-__global__ void __launch_bounds__(256) cnn_im2col_kernel(const bf16* Pin, bf16* Col, int n) {
+constexpr int kW2Bytes = kC2 * kK2 * 2, kW2Octet = kK2 * 16;
+constexpr int strip_box(int channels) { return 18 * (channels / 8) * 160; }
+
+// Forward (CK = 32 input channels, N = 64 outputs) or transposed (CK = 64, N
+// = 32): per strip D (128 pixels x N) = sum over taps and K = 16 slices of
+// the box's shifted words times W2, in the order (tap, channel).  Roles: warp
+// 0 (a lane) loads boxes into a ring and W2 when the chain changes, warp 1 (a
+// lane) issues the MMAs into two accumulators, eight warps run the epilogue
+//   epi.tile(image, chain, strip, lane quarter, first column, values)
+// on 32 lanes and 32 columns at a time: with N = 64 each accumulator's halves
+// go to four warps each, with N = 32 the two accumulators do.  Two CTAs per
+// SM, each a run of consecutive strips.
+constexpr int kConvStages = 3;   // 23 KB each for 64 channels
+constexpr int kConvThreads = 64 + 8 * 32;
+template <int CK>
+constexpr int conv_smem() {
+  return kW2Bytes + kConvStages * strip_box(CK) + 128 + 256;
+}
+
+template <int CK, int N, class Epi>
+__global__ void __launch_bounds__(kConvThreads, 2)
+    cnn_conv2_kernel(const __grid_constant__ CUtensorMap map, const bf16* wts, int chains, int n,
+                     int* status, const __grid_constant__ Epi epi) {
+  constexpr bool kFwd = N == kC2;
+  constexpr int kBox = strip_box(CK), kRow = (CK / 8) * 160;   // bytes of a box, an image row
+  constexpr uint32_t kCols = 2 * N;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* w_s = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
+  uint8_t* ring = w_s + kW2Bytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + kConvStages * kBox);
+  uint64_t* empty = full + kConvStages;
+  uint64_t* wfull = empty + kConvStages;
+  uint64_t* tfull = wfull + 1;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* drain = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kConvStages; ++i) {
+      mbar_init(full + i, 1);
+      mbar_init(empty + i, 1);
+    }
+    mbar_init(wfull, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(tfull + i, 1);
+      mbar_init(tempty + i, kFwd ? 8 : 4);
+    }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, kCols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
   pdl_trigger();
   pdl_wait();
-  constexpr int G = 9 * C / 8;  // 8-column groups per row
-  const int c = blockIdx.y;
-  const int groups = n * H * W * G;
-  const int e = blockIdx.x * 256 + threadIdx.x;
-  if (e >= groups) return;
-  const int k0 = (e % G) * 8;
-  const int pix = e / G;
-  const int x = pix % W, y = (pix / W) % H;
-  const int i = pix / (W * H);
-  uint4 v = make_uint4(0, 0, 0, 0);
-  const int tap = k0 / C, ci = k0 % C;
-  const int yy = y + tap / 3 - 1, xx = x + tap % 3 - 1;
-  if (yy >= 0 && yy < H && xx >= 0 && xx < W)
-    v = *reinterpret_cast<const uint4*>(Pin + static_cast<int64_t>(c) * n * H * W * C +
-                                        ((i * H + yy) * W + xx) * C + ci);
-  *reinterpret_cast<uint4*>(Col + (static_cast<int64_t>(c) * n * H * W + pix) * Kp + k0) = v;
+  const int64_t strips = 2 * static_cast<int64_t>(chains) * n;
+  const int64_t u0 = strips * blockIdx.x / gridDim.x, u1 = strips * (blockIdx.x + 1) / gridDim.x;
+
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      uint32_t it = 0, loads = 0;
+      int chain = -1;
+      for (int64_t u = u0; u < u1; ++u, ++it) {
+        const int64_t img = u >> 1;
+        const int c = static_cast<int>(img / n), s = it % kConvStages;
+        if (c != chain) {
+          // W2 is free once the last strip's MMAs are.
+          if (it > 0 && !conv_wait(empty + (it - 1) % kConvStages, ((it - 1) / kConvStages) & 1u,
+                                   abort_flag, status))
+            break;
+          chain = c;
+          mbar_arrive_expect_tx(wfull, kW2Bytes);
+          bulk_g2s(w_s, wts + static_cast<int64_t>(c) * kC2 * kK2, kW2Bytes, wfull);
+          ++loads;
+        }
+        if (!conv_wait(empty + s, ((it / kConvStages) & 1u) ^ 1u, abort_flag, status)) break;
+        mbar_arrive_expect_tx(full + s, kBox);
+        tc::tma_load_4d(ring + s * kBox, &map, 64 * static_cast<int>(u & 1) - 8, 0, -1,
+                        static_cast<int>(img), full + s);
+      }
+      if (*abort_flag) {   // copies in flight land before the CTA ends
+        for (uint32_t i = it > kConvStages ? it - kConvStages : 0; i < it; ++i)
+          mbar_wait_bounded(full + i % kConvStages, (i / kConvStages) & 1u, nullptr);
+        if (loads > 0) mbar_wait_bounded(wfull, (loads - 1) & 1u, nullptr);
+      }
+    }
+  } else if (warp == 1) {
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(128, N, false, kFwd);
+      const uint64_t B = kFwd ? tc::sdesc_none(w_s, 128, kW2Octet)
+                              : tc::sdesc_none(w_s, kW2Octet, 128);
+      uint32_t it = 0, loads = 0;
+      int chain = -1;
+      for (int64_t u = u0; u < u1; ++u, ++it) {
+        const int c = static_cast<int>((u >> 1) / n), s = it % kConvStages;
+        const uint32_t buf = it & 1u;
+        if (c != chain) {
+          chain = c;
+          if (!conv_wait(wfull, loads & 1u, abort_flag, status)) break;
+          ++loads;
+        }
+        if (!conv_wait(tempty + buf, ((it >> 1) & 1u) ^ 1u, abort_flag, status) ||
+            !conv_wait(full + s, (it / kConvStages) & 1u, abort_flag, status))
+          break;
+        tc::fence_after_sync();
+        const uint64_t A = tc::sdesc_none(ring + s * kBox, 160, kRow);
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap) {
+          const int kh = kFwd ? tap / 3 : 2 - tap / 3, kw = kFwd ? tap % 3 : 2 - tap % 3;
+#pragma unroll
+          for (int k = 0; k < CK / 16; ++k)
+            tc::mma_bf16(tmem + buf * N, A + (kh * kRow + kw * 16 + k * 320) / 16,
+                         B + (kFwd ? (tap * CK + 16 * k) : tap * N + k * (2 * kW2Octet / 16)),
+                         idesc, (tap | k) != 0);
+        }
+        tc::mma_commit(empty + s);
+        tc::mma_commit(tfull + buf);
+      }
+      tc::mma_commit(drain);   // every MMA of this CTA has completed once it flips
+      mbar_wait_bounded(drain, 0, nullptr);
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint32_t it = 0;
+    for (int64_t u = u0; u < u1; ++u, ++it) {
+      const uint32_t buf = it & 1u;
+      if (!kFwd && static_cast<int>(buf) != half) continue;
+      const bool ok = mbar_wait_bounded(tfull + buf, (it >> 1) & 1u, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0 && !*abort_flag) {
+          raise_status(status, GBSGMC_ERR_TIMEOUT);
+          *abort_flag = 1;
+        }
+        break;
+      }
+      tc::fence_after_sync();
+      const int col0 = kFwd ? 32 * half : 0;
+      const tc::TmemRows load{tmem + buf * N + col0 + (static_cast<uint32_t>(q * 32) << 16)};
+      float v[32];
+      load(0, v);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty + buf);   // the accumulator is in registers
+      epi.tile(u >> 1, static_cast<int>((u >> 1) / n), static_cast<int>(u & 1), q, col0, v);
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, kCols);
+  }
+}
+
+// conv2's pooling: lane 8 i + j of quarter q is the pixel (4 q + i, 8 s + j).
+struct EpiStripPool {
+  const float* w;
+  bf16* P;      // [images, 8, 8, 64]
+  uint8_t* M;
+  __device__ __forceinline__ void tile(int64_t img, int c, int s, int q, int col0,
+                                       float (&v)[32]) const {
+    const int lane = epi::lane_id();
+    const int base = lane & ~9;
+    const int64_t pix = img * 64 + (2 * q + (base >> 4)) * 8 + 4 * s + ((base & 7) >> 1);
+    const float bl = __ldg(w + static_cast<int64_t>(c) * kP + ob2 + col0 + lane);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j] + __shfl_sync(0xffffffffu, bl, j), 0.f);
+    uint4 p;
+    uint2 m;
+    const int wp = pool_windows<8>(v, p, m);
+    const int64_t at = pix * kC2 + col0 + 8 * wp;
+    *reinterpret_cast<uint4*>(P + at) = p;
+    *reinterpret_cast<uint2*>(M + at) = m;
+  }
+};
+
+// conv2's input gradient as fp32, [image][h][octet][w][8], a sector per store.
+struct EpiStripDX {
+  float* dx;
+  __device__ __forceinline__ void tile(int64_t img, int, int s, int q, int,
+                                       float (&v)[32]) const {
+    const int lane = epi::lane_id();
+    float* dst = dx + ((img * 16 + 4 * q + (lane >> 3)) * 64 + 8 * s + (lane & 7)) * 8;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      const float* e = v + 8 * o;
+      asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst + 128 * o),
+                   "f"(e[0]), "f"(e[1]), "f"(e[2]), "f"(e[3]), "f"(e[4]), "f"(e[5]), "f"(e[6]),
+                   "f"(e[7])
+                   : "memory");
+    }
+  }
+};
+
+// dW2 = dY2^T Col2: per 64-pixel slice (4 image rows) the boxes of dY2 and of
+// P1 with its halo, both MN-major with an image row's 16 pixels as K; a
+// column shift kw is one MMA of M = 64 outputs x N = 96 (three kernel rows x
+// 32 inputs: the box's [h][octet] words lie 288 bytes apart).  The sums of a
+// run of a chain's slices stay in TMEM and are written as one split-K partial
+// [tap, input][output].  Grid (splits, chains, Z): a CTA takes all three
+// column shifts (Z = 1) or one (Z = 3, when the splits alone leave SMs idle).
+constexpr int kDy2Box = 4 * (kC2 / 8) * 256, kP1Box = 6 * (kC1 / 8) * 288;
+constexpr int kDw2Stages = 7, kDw2Threads = 64 + 4 * 32;
+constexpr int kDw2Smem = kDw2Stages * (kDy2Box + kP1Box) + 128 + 256;
+constexpr int kDw2SmemAlone = 120 * 1024;   // Z = 1 takes all of the SM's TMEM
+
+__global__ void __launch_bounds__(kDw2Threads, 1)
+    cnn_conv2_dw_kernel(const __grid_constant__ CUtensorMap mdy,
+                        const __grid_constant__ CUtensorMap mp1, float* part, int n,
+                        int* status) {
+  constexpr int kStage = kDy2Box + kP1Box;
+  const uint32_t cols = gridDim.z == 1 ? 512 : 128;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + kDw2Stages * kStage);
+  uint64_t* empty = full + kDw2Stages;
+  uint64_t* done = empty + kDw2Stages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDw2Stages; ++i) {
+      mbar_init(full + i, 1);
+      mbar_init(empty + i, 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, cols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+  const int c = blockIdx.y, S = gridDim.x;
+  const int each = 4 * n / S, u0 = each * blockIdx.x, u1 = u0 + each;   // slices
+  const int kw0 = gridDim.z == 1 ? 0 : blockIdx.z, kw1 = gridDim.z == 1 ? 3 : kw0 + 1;
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      uint32_t it = 0;
+      for (int u = u0; u < u1; ++u, ++it) {
+        const int s = it % kDw2Stages, img = c * n + (u >> 2), h0 = 4 * (u & 3);
+        if (!conv_wait(empty + s, ((it / kDw2Stages) & 1u) ^ 1u, abort_flag, status)) break;
+        uint8_t* dst = ring + s * kStage;
+        mbar_arrive_expect_tx(full + s, kStage);
+        tc::tma_load_4d(dst, &mdy, 0, 0, h0, img, full + s);
+        tc::tma_load_4d(dst + kDy2Box, &mp1, -8, 0, h0 - 1, img, full + s);
+      }
+      if (*abort_flag)
+        for (uint32_t i = it > kDw2Stages ? it - kDw2Stages : 0; i < it; ++i)
+          mbar_wait_bounded(full + i % kDw2Stages, (i / kDw2Stages) & 1u, nullptr);
+    }
+  } else if (warp == 1) {
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(64, 96, true, true);
+      uint32_t it = 0;
+      for (int u = u0; u < u1; ++u, ++it) {
+        const int s = it % kDw2Stages;
+        if (!conv_wait(full + s, (it / kDw2Stages) & 1u, abort_flag, status)) break;
+        tc::fence_after_sync();
+        const uint64_t A = tc::sdesc_none(ring + s * kStage, 128, 256);
+        const uint64_t B = tc::sdesc_none(ring + s * kStage + kDy2Box, 128, 288);
+#pragma unroll
+        for (int h = 0; h < 4; ++h)
+          for (int kw = kw0; kw < kw1; ++kw)
+            tc::mma_bf16(tmem + 96 * (kw - kw0), A + h * (kC2 / 8) * 256 / 16,
+                         B + h * (kC1 / 8) * 288 / 16 + kw, idesc, it > 0 || h > 0);
+        tc::mma_commit(empty + s);
+      }
+      tc::mma_commit(done);
+      mbar_wait_bounded(done, 0, nullptr);
+    }
+  } else {
+    const bool ok = mbar_wait_bounded(done, 0, nullptr);
+    if (!__all_sync(0xffffffffu, ok) && lane == 0) raise_status(status, GBSGMC_ERR_TIMEOUT);
+    tc::fence_after_sync();
+    // Accumulator row r of an M = 64 tile is TMEM lane 32 (r / 16) + r % 16.
+    const int q = warp & 3;
+    float* dst = part + (static_cast<int64_t>(c) * S + blockIdx.x) * kK2 * kC2 + 16 * q + lane;
+#pragma unroll 1
+    for (int g = 0; g < 3 * (kw1 - kw0); ++g) {   // kw, kh
+      float v[32];
+      tc::tmem_ld32(tmem + 32 * g + (static_cast<uint32_t>(q * 32) << 16), v);
+      const int tap = 3 * (g % 3) + kw0 + g / 3;
+      if (lane < 16) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) dst[(tap * kC1 + j) * kC2] = v[j];
+      }
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, cols);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -464,13 +1298,12 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
 // ---------------------------------------------------------------------------
 // Pool-window routing + ReLU mask: for each pooled element (i, py, px, ch),
 // the gradient dP = dp[i, py, px, ch] (fp32: the dense layer's adjoint for
-// layer 3, the transposed convolution's output for layers 2 and 1) goes to
-// the window element its argmax chose if that element was positive (the
-// pool's mark byte, bits 0-1 and 2); the three others (and channels
-// C..ld-1) get 0:  dY [n, H, W, ld] BF16 (rows in conv1_row order for
-// layer 1, kConv1Rows).  One thread per pooled pixel and eight channels:
-// 128-bit loads of dp, 64-bit of the marks, 128-bit stores of dY; C and ld
-// are multiples of 8.  32-bit index arithmetic (per-chain counts < 2^31).
+// layer 3, the transposed convolution's output for layer 2) goes to the
+// window element its argmax chose if that element was positive (the pool's
+// mark byte, bits 0-1 and 2); the three others get 0:  dY [n, H, W, C] BF16.
+// One thread per pooled pixel and eight channels: 128-bit loads of dp, 64-bit
+// of the marks, 128-bit stores of dY; C is a multiple of 8.  32-bit index
+// arithmetic (per-chain counts < 2^31).
 // Grid (ceil(n*Ho*Wo*C/8 / 256), chains).
 // The bias gradient is the column sum of dY, i.e. the sum over pooled
 // elements of the routed (BF16-rounded) values: each block adds its threads'
@@ -479,7 +1312,7 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
 // blocks.  2048 / C threads of a block share a channel group (256 * 8 is a
 // multiple of C, so the channel of thread t is 8 t mod C).
 // ---------------------------------------------------------------------------
-template <int H, int W, int C, int ld, bool kConv1Rows = false>
+template <int H, int W, int C, bool kRows>
 __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t* M,
                                                         const float* dp, int n, float* bpart) {
   pdl_trigger();
@@ -492,23 +1325,27 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
   const bool active = e < pper;
   float bsum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (active) {
-  const int ch = e % C;
-  const int pix = e / C;
+  // kRows: neighbouring threads take a row's pooled pixels (Wo = 8) of an octet.
+  const int ch = kRows ? e / 64 % (C / 8) * 8 : e % C;
+  const int pix = kRows ? e / (8 * C) * 8 + e / 8 % 8 : e / C;
   const int px = pix % Wo, py = (pix / Wo) % Ho, i = pix / (Wo * Ho);
+  const int64_t at = static_cast<int64_t>(c) * pper + int64_t(pix) * C + ch;
   float g[8];
   {
-    const float4* d4 = reinterpret_cast<const float4*>(dp + static_cast<int64_t>(c) * pper + e);
+    const float4* d4 = reinterpret_cast<const float4*>(dp + at);
     const float4 u = d4[0], v = d4[1];
     g[0] = u.x; g[1] = u.y; g[2] = u.z; g[3] = u.w;
     g[4] = v.x; g[5] = v.y; g[6] = v.z; g[7] = v.w;
   }
-  const uint2 mk = *reinterpret_cast<const uint2*>(M + static_cast<int64_t>(c) * pper + e);
+  const uint2 mk = *reinterpret_cast<const uint2*>(M + at);
   const uint32_t marks[2] = {mk.x, mk.y};
-  const int64_t base = static_cast<int64_t>(c) * n * H * W * ld;
+  const int64_t base = static_cast<int64_t>(c) * n * H * W * C;
+  __nv_bfloat162 prev[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const int y = 2 * py + (q >> 1), x = 2 * px + (q & 1);
-    const int off = (kConv1Rows ? i * H * W + conv1_row(y, x) : (i * H + y) * W + x) * ld;
+    const int off = kRows ? ((i * H + y) * (C / 8) + ch / 8) * W * 8 + x * 8
+                          : ((i * H + y) * W + x) * C + ch;
     __nv_bfloat162 o[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -520,9 +1357,20 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
       bsum[2 * k] += __low2float(o[k]);
       bsum[2 * k + 1] += __high2float(o[k]);
     }
-    *reinterpret_cast<uint4*>(dY + base + off + ch) = *reinterpret_cast<const uint4*>(o);
-    for (int extra = C + ch; extra < ld; extra += C)
-      *reinterpret_cast<uint4*>(dY + base + off + extra) = make_uint4(0u, 0u, 0u, 0u);
+    if (!kRows) {
+      *reinterpret_cast<uint4*>(dY + base + off) = *reinterpret_cast<const uint4*>(o);
+    } else if ((q & 1) == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) prev[k] = o[k];
+    } else {   // both columns: a whole sector
+      const uint32_t* l = reinterpret_cast<const uint32_t*>(prev);
+      const uint32_t* r = reinterpret_cast<const uint32_t*>(o);
+      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dY + base +
+                                                                                  off - 8),
+                   "r"(l[0]), "r"(l[1]), "r"(l[2]), "r"(l[3]), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+                   "r"(r[3])
+                   : "memory");
+    }
   }
   }  // active
 #pragma unroll
@@ -531,7 +1379,8 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
   if (static_cast<int>(threadIdx.x) < C) {
     const int t = threadIdx.x, group = t / 8, k = t % 8, groups = C / 8;
     float s = 0.f;
-    for (int u = group; u < 256; u += groups) s += red[u * 8 + k];
+    for (int u = 0; u < 256 / groups; ++u)
+      s += red[(kRows ? u / 8 * 8 * groups + group * 8 + u % 8 : u * groups + group) * 8 + k];
     bpart[(static_cast<int64_t>(c) * gridDim.x + blockIdx.x) * C + t] = s;
   }
 }
@@ -542,9 +1391,10 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
 // U and var(lk).  (As seven launches, most of them a few microseconds of
 // latency: 42 us of an 850 us gradient of 8 x 256 images, 26 us of 160 at 2 x
 // 50.)  Grid (weight blocks + kBiasBlocks + 1, chains), 256 threads: the
-// first ceil(P / 256) blocks take a parameter per thread, then a block per 8
-// bias channels (32 groups of partials each), the last block the values.
-constexpr int kBiasBlocks = (kC1 + kC2 + kC3) / 8;
+// first ceil(P / 256) blocks take a parameter per thread, then four blocks a
+// layer's bias (C / 4 channels each, 1024 / C groups of partials), the last
+// block the values.
+constexpr int kBiasBlocks = 12;
 
 __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
   __shared__ float acc[256];
@@ -577,21 +1427,19 @@ __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
   }
   if (bx < kBiasBlocks) {
     if (!a.want_grad) return;
-    int l = 0, ch0 = 8 * bx, C = kC1;
-    int64_t off = ob1;
-    if (ch0 >= kC1 + kC2) l = 2, ch0 -= kC1 + kC2, C = kC3, off = ob3;
-    else if (ch0 >= kC1) l = 1, ch0 -= kC1, C = kC2, off = ob2;
-    const int ch = ch0 + (t & 7), blocks = a.bblocks[l];
+    const int l = bx >> 2, C = l == 2 ? kC3 : (l == 1 ? kC2 : kC1);
+    const int64_t off = l == 2 ? ob3 : (l == 1 ? ob2 : ob1);
+    const int own = C / 4, groups = 256 / own, blocks = a.bblocks[l];
+    const int ch = (bx & 3) * own + t % own;
     const float* p = a.bpart[l] + static_cast<int64_t>(c) * blocks * C + ch;
     float v = 0.f;
 #pragma unroll 8
-    for (int q = t >> 3; q < blocks; q += 32) v += p[static_cast<int64_t>(q) * C];
+    for (int q = t / own; q < blocks; q += groups) v += p[static_cast<int64_t>(q) * C];
     acc[t] = v;
     __syncthreads();
-    if (t < 8) {
+    if (t < own) {
       float tot = 0.f;
-#pragma unroll
-      for (int u = 0; u < 32; ++u) tot += acc[8 * u + t];
+      for (int u = 0; u < groups; ++u) tot += acc[u * own + t];
       const int64_t j = off + ch;
       a.grad[static_cast<int64_t>(c) * kP + j] =
           a.pf != 0.f ? fmaf(a.pf, __ldg(w + j), tot) : tot;
@@ -634,14 +1482,14 @@ __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
 // Forward: ReLU(acc + b) in fp32 and the 2 x 2 max-pool of it, straight from
 // the accumulator.  A warp's 32 rows hold whole pool windows: the window of
 // lane l is lanes (base, base + 1, base + V, base + V + 1), base = l & ~(V | 1),
-// in row-major window order, with V = 16 for conv1 (conv1_row order) and
-// conv2 (16 pixels per image row) and V = 8 for conv3 (8 per row).  Per
+// in row-major window order, with V = 16 for conv2 (16 pixels per
+// image row) and V = 8 for conv3 (8 per row).  Per
 // output the maximum (first one in window order, as jax's max-pool argmax
 // routes the gradient) goes to P [n, Ho, Wo, C] as BF16 and the mark byte
 // to M: bits 0-1 the argmax, bit 2 (maximum > 0), the ReLU mask of the
 // element the backward pass routes the gradient to.  The four lanes of a
 // window each write 8 of every 32 channels (16-byte P stores, 8-byte mark
-// stores).  Columns >= C (conv1's padding to N = 64) are skipped.  The
+// stores).  The
 // window maxima of a 32-channel chunk take two exchange stages instead of
 // four shuffles per channel: the two pixels of a window row swap the
 // halves of the channels they do not keep (16 shuffles) and keep the
@@ -649,7 +1497,7 @@ __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
 // that each lane ends with the maxima of its 8 channels; comparisons are
 // strict in window order (left before right, top before bottom), which
 // keeps the first maximum of the window as the sequential scan does.
-template <int H, int W, int V, bool kConv1Rows>
+template <int H, int W, int V>
 struct EpiConvPool {
   const float* w;
   int64_t boff;
@@ -660,24 +1508,13 @@ struct EpiConvPool {
   template <int NC, class Load>
   __device__ __forceinline__ void tile(int b, int row0, int col0, const Load& load,
                                        uint32_t*) const {
-    if (col0 >= C) return;  // padding columns (warp-uniform)
     const unsigned full = 0xffffffffu;
     const int lane = epi::lane_id();
     const int base = lane & ~(V | 1);
-    const int wp = ((lane & V) ? 2 : 0) | (lane & 1);
     // The window's pooled pixel, from the row of its first lane.
     const int r = row0 + base;
     const int i = r / (H * W), rr = r % (H * W);
-    int yp, xp;
-    if (kConv1Rows) {
-      int h, x;
-      conv1_pixel(rr, h, x);
-      yp = h >> 1;
-      xp = x >> 1;
-    } else {
-      yp = (rr / W) >> 1;
-      xp = (rr % W) >> 1;
-    }
+    const int yp = (rr / W) >> 1, xp = (rr % W) >> 1;
     const int64_t pix = (static_cast<int64_t>(b) * n + i) * (H / 2) * (W / 2) +
                         yp * (W / 2) + xp;
     const float* bias = w + b * kP + boff;
@@ -690,52 +1527,11 @@ struct EpiConvPool {
       float x[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) x[j] = fmaxf(v[j] + __shfl_sync(full, bl, j), 0.f);
-      // Stage 1, the window row's two pixels (lanes l, l ^ 1): keep the
-      // chunks {cbit, cbit + 2} of 8 channels (kept channel i: i < 8 in
-      // the first, i >= 8 in the second), send the other two.
-      const bool cbit = (lane & 1) != 0, rbit = (lane & V) != 0;
-      float m1[16];
-      uint32_t col_bits = 0;  // bit i: kept channel i's maximum is the right pixel
-#pragma unroll
-      for (int q = 0; q < 16; ++q) {
-        const int lo = q < 8 ? q : 8 + q, hi = lo + 8;
-        const float mine = cbit ? x[hi] : x[lo];
-        const float other = __shfl_xor_sync(full, cbit ? x[lo] : x[hi], 1);
-        const float left = cbit ? other : mine, right = cbit ? mine : other;
-        const bool rt = right > left;
-        m1[q] = rt ? right : left;
-        col_bits |= (rt ? 1u : 0u) << q;
-      }
-      // Stage 2, the window's two rows (lanes l, l ^ V): the top row keeps
-      // kept channels 0-7 (chunk cbit), the bottom row 8-15 (chunk
-      // cbit + 2): chunk wp of the 32 channels.
-      const uint32_t other_bits = __shfl_xor_sync(full, col_bits, V);
-      float best_mine[8];
-      uint32_t mark_mine[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int ki = rbit ? 8 + q : q;
-        const float mine = rbit ? m1[8 + q] : m1[q];
-        const float other = __shfl_xor_sync(full, rbit ? m1[q] : m1[8 + q], V);
-        const uint32_t my_col = (col_bits >> ki) & 1u, ot_col = (other_bits >> ki) & 1u;
-        const float top = rbit ? other : mine, bot = rbit ? mine : other;
-        const uint32_t top_col = rbit ? ot_col : my_col, bot_col = rbit ? my_col : ot_col;
-        const bool b2 = bot > top;
-        const float best = b2 ? bot : top;
-        best_mine[q] = best;
-        mark_mine[q] = (b2 ? 2u + bot_col : top_col) | (best > 0.f ? 4u : 0u);
-      }
-      uint32_t pk[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const __nv_bfloat162 pr = __floats2bfloat162_rn(best_mine[2 * e], best_mine[2 * e + 1]);
-        pk[e] = *reinterpret_cast<const uint32_t*>(&pr);
-      }
-      const int64_t at = pix * C + k0 + 8 * wp;
-      *reinterpret_cast<uint4*>(P + at) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+      uint4 p;
       uint2 mk;
-      mk.x = mark_mine[0] | (mark_mine[1] << 8) | (mark_mine[2] << 16) | (mark_mine[3] << 24);
-      mk.y = mark_mine[4] | (mark_mine[5] << 8) | (mark_mine[6] << 16) | (mark_mine[7] << 24);
+      const int wp = pool_windows<V>(x, p, mk);
+      const int64_t at = pix * C + k0 + 8 * wp;
+      *reinterpret_cast<uint4*>(P + at) = p;
       *reinterpret_cast<uint2*>(M + at) = mk;
     }
   }
@@ -743,14 +1539,10 @@ struct EpiConvPool {
 
 // Weights: element (row = output channel co, col = im2col column k) of the
 // split-K partial product of (virtual) batch bv = chain * splits + split
-// lands at part[bv][k][co] (HWIO order), rows < Cout, cols < K.  With x8 the
-// columns are conv1's K groups x 8 slots: column 8 g + s (g = 2 kh + p) is
-// input channel s % 3 of tap (kh, p + s / 3), for g < 6, s < 6, and p = 0
-// or s >= 3.
+// lands at part[bv][k][co] (HWIO order), rows < Cout, cols < K.
 struct EpiConvGradW {
   float* part;
   int Cout, K;
-  bool x8 = false;
   template <int NC, class Load>
   __device__ __forceinline__ void tile(int bv, int row0, int col0, const Load& load,
                                        uint32_t*) const {
@@ -764,14 +1556,7 @@ struct EpiConvGradW {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const int k = col0 + 32 * cb + j;
-          if (x8) {
-            const int g = k >> 3, sl = k & 7;
-            const int kw = (g & 1) + sl / kInC;
-            if (g < 6 && sl < 2 * kInC && ((g & 1) == 0 || sl >= kInC))
-              dst[static_cast<int64_t>(((g >> 1) * 3 + kw) * kInC + sl % kInC) * Cout] = v[j];
-          } else if (k < K) {
-            dst[static_cast<int64_t>(k) * Cout] = v[j];
-          }
+          if (k < K) dst[static_cast<int64_t>(k) * Cout] = v[j];
         }
       }
     }
@@ -858,93 +1643,6 @@ struct TransposedB : Inner {
   }
 };
 
-// conv1's operands, read by K group from the gathered images X8 and from its
-// weights W1i, unswizzled: a pixel's 8 slots (16 bytes) are one core-matrix
-// row.  X8 is mapped as image rows of 256 elements (32 pixels x 8 slots):
-// 4-D map (256, 32, chains * n, 1) with boxes (128, R, 1, 1), 16 pixels of
-// R rows (8 for the forward GEMM, 4 for the weight gradient), whose shift by
-// a group's column offset is 8 elements (16 bytes) per pixel; a box is R
-// rows of 256 bytes for TMA.  K group g = 2 kh + p of output pixel (h, w)
-// is the pixel (h + kh - 1, w + p) of X8 (zeros outside the image).
-// Groups 6 and 7 read a box wholly below the image (zeros).  W1i is mapped
-// as (256, 2, 8, chains), a group's 64 x 8 weights as two rows of 256, box
-// (256, 2, 8, 1).  Forward: the 128-row tile at m0 (columns w0 .. w0 + 15 of
-// image rows 8u .. 8u + 7, conv1_row order) is, per group, one box 2 KB
-// apart; B is the weights' box.
-template <class Inner>
-struct Conv1Fwd : Inner {
-  int n;
-  static constexpr bool kLoadA = true, kLoadB = true, kInterleaveA = true,
-                        kInterleaveB = true;
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* map, int, int m0, int b,
-                                         uint64_t* bar) const {
-    const int img = b * n + m0 / 1024, t = (m0 % 1024) / 128;
-    const int u = t >> 1, w0 = (t & 1) * 16;
-    uint8_t* d = static_cast<uint8_t*>(dst);
-#pragma unroll
-    for (int g = 0; g < kG1; ++g) {
-      const int kh = g >> 1, dx = g & 1;
-      const int y = g < 6 ? 8 * u + kh - 1 : 64;
-      tc::tma_load_4d(d + g * 2048, map, (w0 + dx) * kX8, y, img, 0, bar);
-    }
-  }
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* map, int nn, int, int b,
-                                         uint64_t* bar) const {
-    tc::tma_load_4d(dst, map, 0, nn / 32, 0, b, bar);
-  }
-};
-
-// conv1's weight gradient dW1 = dY1^T Col1 with Col1 read from X8: the
-// 64-pixel K slice k0 (the upper or lower 4 rows of a conv1 tile, conv1_row
-// order) of the MN-major B is, per real K group (0-5), that slice's (16 W,
-// 4 H) box shifted by the group, 1 KB apart.  Only the parts of the stage
-// whose products are stored are loaded: A's first 64 rows (output channels;
-// 32 real) and B's first 48 columns; the MMAs' other rows and columns read
-// whatever the stage held and the epilogue drops them.
-template <class Inner>
-struct Conv1Bmn : Inner {
-  int n;
-  static constexpr bool kLoadA = true, kLoadB = true, kInterleaveB = true;
-  static constexpr uint32_t kStageBytes = 64 * kGemmBK * 2 + 6 * 1024;
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* map, int k0, int m0,
-                                         int b, uint64_t* bar) const {
-    tc::tma_load_3d(dst, map, m0, k0, b, bar);
-  }
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* map, int, int k0, int b,
-                                         uint64_t* bar) const {
-    const int img = b * n + k0 / 1024, rr = k0 % 1024, t = rr >> 7;
-    const int h0 = 8 * (t >> 1) + 4 * ((rr >> 6) & 1), w0 = (t & 1) * 16;
-    uint8_t* d = static_cast<uint8_t*>(dst);
-#pragma unroll
-    for (int g = 0; g < 6; ++g) {
-      const int kh = g >> 1, dx = g & 1;
-      tc::tma_load_4d(d + g * 1024, map, (w0 + dx) * kX8, h0 + kh - 1, img, 0, bar);
-    }
-  }
-};
-
-// A weight gradient whose output channels fill only the first 64 of the
-// GEMM's 128 rows: A's first 64 rows are loaded (one MN-major box), the
-// MMAs' other rows read whatever the stage held and the epilogue drops them.
-template <class Inner>
-struct HalfA : Inner {
-  static constexpr bool kLoadA = true;
-  static constexpr uint32_t kStageBytes = 2 * 64 * kGemmBK * 2;
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* map, int k0, int m0,
-                                         int b, uint64_t* bar) const {
-    tc::tma_load_3d(dst, map, m0, k0, b, bar);
-  }
-};
-
-// A transposed convolution whose output channels fill only kRows of the
-// GEMM's N = 64 columns: B's box holds those kRows rows (the map's box is
-// 64 x kRows), the MMAs' other columns read whatever the stage held and the
-// epilogue drops them; the stage expects A's bytes and kRows rows of B.
-template <class Inner, int kRows>
-struct TransposedBRows : TransposedB<Inner> {
-  static constexpr uint32_t kStageBytes = (kGemmBM + kRows) * kGemmBK * 2;
-};
-
 template <class T>
 T* view(void* ws, size_t off) {
   return reinterpret_cast<T*>(static_cast<unsigned char*>(ws) + off);
@@ -953,13 +1651,9 @@ T* view(void* ws, size_t off) {
 int grid1(int64_t work) { return static_cast<int>((work + 255) / 256); }
 
 int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
-  a.w1i = view<bf16>(ws, L.w1i);
   a.w2b = view<bf16>(ws, L.w2b);
   a.w3b = view<bf16>(ws, L.w3b);
-  a.x8 = view<bf16>(ws, L.x8);
-  a.dy1 = view<bf16>(ws, L.dy1);
   a.p1 = view<bf16>(ws, L.p1);
-  a.col2 = view<bf16>(ws, L.col2);
   a.dy2 = view<bf16>(ws, L.dy2);
   a.p2 = view<bf16>(ws, L.p2);
   a.dy3 = view<bf16>(ws, L.dy3);
@@ -989,52 +1683,50 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     a.pf = static_cast<float>(1.0 / (ps * ps * a.temperature));
     a.prior_const = static_cast<double>(kP) * (std::log(ps) + 0.91893853320467274178);
   }
-  const int64_t r1 = int64_t(n) * 1024, r2 = int64_t(n) * 256, r3 = int64_t(n) * 64;
+  const int64_t r3 = int64_t(n) * 64;
   int rc;
   auto launched = [&](const char* what) { return check_launch(what); };
   auto unpool_grid = [&](int H, int Cr) {
     return dim3(grid1(int64_t(n) * (H / 2) * (H / 2) * Cr / 8), C);
   };
-  launch_pdl(cnn_prep_kernel, dim3(kPrepBlocks, C), 256, 0, st, a);
-  if ((rc = launched("cnn_prep_kernel"))) return rc;
-  launch_pdl(cnn_gather1_kernel, dim3(grid1(r1), C), 256, 0, st, a);
-  if ((rc = launched("cnn_gather1_kernel"))) return rc;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return set_error(GBSGMC_ERR_CUDA, "cnn: cannot query the device");
+  const int pair = reinterpret_cast<uintptr_t>(a.X) % 8 == 0 && a.ld % 2 == 0;
+  launch_pdl(cnn_conv1_kernel,
+             static_cast<int>(std::min<int64_t>(
+                 4 * sms, std::max<int64_t>(2 * int64_t(C) * n, int64_t(C) * kPrepBlocks))),
+             kStripThreads, 0, st, a, pair);
+  if ((rc = launched("cnn_conv1_kernel"))) return rc;
 
   // Tensor maps (columns, rows, chains), and 4-D maps (channels, W, H,
   // images) of the NHWC maps the implicit GEMMs read by tap.
   const int64_t imgs = int64_t(C) * n;
-  CUtensorMap m_x8, m_x8h, m_w1i, m_col2, m_w2, m_w3, m_p2a;
-  if ((rc = make_tmap_bf16_4d_plain(&m_x8, a.x8, {32 * kX8, 32, imgs, 1},
-                                    {32 * kX8, 1024 * kX8, imgs * 1024 * kX8},
-                                    {16 * kX8, 8, 1, 1})) ||
-      (rc = make_tmap_bf16_4d_plain(&m_x8h, a.x8, {32 * kX8, 32, imgs, 1},
-                                    {32 * kX8, 1024 * kX8, imgs * 1024 * kX8},
-                                    {16 * kX8, 4, 1, 1})) ||
-      (rc = make_tmap_bf16_4d_plain(&m_w1i, a.w1i, {32 * kX8, 2, kG1, C},
-                                    {32 * kX8, 64 * kX8, kG1 * 64 * kX8},
-                                    {32 * kX8, 2, kG1, 1})) ||
-      (rc = make_tmap_bf16_3d(&m_col2, a.col2, kK2, r2, C, kK2p, r2 * kK2p, kGemmBK, kGemmBM)) ||
-      (rc = make_tmap_bf16_3d(&m_w2, a.w2b, kC2, kK2, C, kC2, kK2 * kC2, 64, 64)) ||
+  CUtensorMap m_p1, m_w3, m_p2a;
+  if ((rc = make_tmap_bf16_4d_plain(&m_p1, a.p1, {128, kC1 / 8, 16, imgs},
+                                    {128, 16 * kC1, 256 * kC1}, {80, kC1 / 8, 18, 1})) ||
       (rc = make_tmap_bf16_3d(&m_w3, a.w3b, kC3, kK3, C, kC3, kK3 * kC3, 64, 64)) ||
       (rc = make_tmap_bf16_4d(&m_p2a, a.p2, {kC2, 8, 8, imgs}, {kC2, 8 * kC2, 64 * kC2},
                               {64, 8, 8, 2})))
     return rc;
 
-  // conv1+pool1 (implicit) -> im2col2 -> conv2+pool2 -> conv3+pool3
-  // (implicit): each conv GEMM's epilogue writes the pooled BF16 map and the
-  // marks.  conv1 runs as N = 64 (W1i's zero output channels past 32) and
-  // K = 8 groups x 8 slots; its epilogue skips the padding columns.
-  const Conv1Fwd<EpiConvPool<32, 32, 16, true>> e1{{a.w, ob1, kC1, a.p1, a.m1, n}, n};
-  if ((rc = launch_gemm<64, false, false>(m_x8, m_w1i, C, r1, 64, kK1i, a.status, e1, st)))
-    return rc;
-  launch_pdl(cnn_im2col_kernel<16, 16, kC1, kK2p>, dim3(grid1(r2 * kK2 / 8), C), 256, 0, st, 
-      a.p1, a.col2, n);
-  if ((rc = launched("cnn_im2col_kernel 2"))) return rc;
-  const EpiConvPool<16, 16, 16, false> e2{a.w, ob2, kC2, a.p2, a.m2, n};
-  if ((rc = launch_gemm<64, false, true>(m_col2, m_w2, C, r2, kC2, kK2p, a.status, e2, st)))
+  // conv1+pool1 -> conv2+pool2 -> conv3+pool3: each epilogue writes the pooled
+  // BF16 map and the marks.
+  const auto conv2 = [&](auto kern, int bytes, const CUtensorMap& map, const auto& epi) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_conv2_kernel: %s", cudaGetErrorString(e));
+    launch_pdl(kern, static_cast<int>(std::min<int64_t>(2 * sms, 2 * imgs)), kConvThreads, bytes,
+               st, map, static_cast<const bf16*>(a.w2b), C, n, a.status, epi);
+    return launched("cnn_conv2_kernel");
+  };
+  if ((rc = conv2(cnn_conv2_kernel<kC1, kC2, EpiStripPool>, conv_smem<kC1>(), m_p1,
+                  EpiStripPool{a.w, a.p2, a.m2})))
     return rc;
   // conv3, implicit: A tiles are P2's tap-shifted 2-image boxes.
-  const ImplicitA<EpiConvPool<8, 8, 8, false>> e3{{a.w, ob3, kC3, a.p3, a.m3, n},
+  const ImplicitA<EpiConvPool<8, 8, 8>> e3{{a.w, ob3, kC3, a.p3, a.m3, n},
                                                    8, 8, kC2, 1, n};
   if ((rc = launch_gemm<128, false, true>(m_p2a, m_w3, C, r3, kC3, kK3, a.status, e3, st)))
     return rc;
@@ -1058,7 +1750,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     // Layer 3: dY3 (routing of dP3), db3, dW3 = dY3^T Col3 (implicit: B
     // blocks are P2's tap-shifted images), dP2 = the transposed convolution
     // of dY3 (implicit: A tiles are dY3's tap-shifted 2-image boxes).
-    launch_pdl(cnn_unpool_kernel<8, 8, kC3, kC3>, unpool_grid(8, kC3), 256, 0, st, 
+    launch_pdl(cnn_unpool_kernel<8, 8, kC3, false>, unpool_grid(8, kC3), 256, 0, st, 
         a.dy3, a.m3, a.dp3, n, a.bpart[2]);
     if ((rc = launched("cnn_unpool_kernel 3"))) return rc;
     CUtensorMap m_dy3t, m_p2b, m_dy3a, m_w3t;
@@ -1082,48 +1774,38 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     if ((rc = launch_gemm<64, false, false>(m_dy3a, m_w3t, C, r3, kC2, 9 * kC3, a.status, d3,
                                             st)))
       return rc;
-    // Layer 2: dY2 (routing of dP2), db2, dW2 = dY2^T Col2, dP1 = the
-    // transposed convolution of dY2 (implicit).
-    launch_pdl(cnn_unpool_kernel<16, 16, kC2, kC2>, unpool_grid(16, kC2), 256, 0, st, 
+    // Layer 2: dY2 (routing of dP2), db2, dW2, and dP1, the transposed
+    // convolution of dY2.
+    launch_pdl(cnn_unpool_kernel<16, 16, kC2, true>, unpool_grid(16, kC2), 256, 0, st, 
         a.dy2, a.m2, a.dp2, n, a.bpart[1]);
     if ((rc = launched("cnn_unpool_kernel 2"))) return rc;
-    CUtensorMap m_dy2t, m_col2t, m_dy2a, m_w2t;
-    if ((rc = make_tmap_bf16_3d(&m_dy2t, a.dy2, kC2, r2, C, kC2, r2 * kC2, 64, 64)) ||
-        (rc = make_tmap_bf16_3d(&m_col2t, a.col2, kK2, r2, C, kK2p, r2 * kK2p, 64, 64)) ||
-        (rc = make_tmap_bf16_4d(&m_dy2a, a.dy2, {kC2, 16, 16, imgs},
-                                {kC2, 16 * kC2, 256 * kC2}, {64, 16, 8, 1})) ||
-        (rc = make_tmap_bf16_4d(&m_w2t, a.w2b, {kC2, kC1, 9, C}, {kC2, kC1 * kC2, kK2 * kC2},
-                                {64, kC1, 1, 1})))
+    CUtensorMap m_dy2, m_dy2h, m_p1w;
+    if ((rc = make_tmap_bf16_4d_plain(&m_dy2, a.dy2, {128, kC2 / 8, 16, imgs},
+                                      {128, 16 * kC2, 256 * kC2}, {128, kC2 / 8, 4, 1})) ||
+        (rc = make_tmap_bf16_4d_plain(&m_p1w, a.p1, {128, kC1 / 8, 16, imgs},
+                                      {128, 16 * kC1, 256 * kC1}, {144, kC1 / 8, 6, 1})) ||
+        (rc = make_tmap_bf16_4d_plain(&m_dy2h, a.dy2, {128, kC2 / 8, 16, imgs},
+                                      {128, 16 * kC2, 256 * kC2}, {80, kC2 / 8, 18, 1})))
       return rc;
-    {
-      GemmRagged rg;
-      rg.ksplit = a.split[1];
-      const HalfA<EpiConvGradW> e{{a.part[1], kC2, kK2}};
-      if ((rc = launch_gemm<64, true, true>(m_dy2t, m_col2t, C, 128, kK2p, static_cast<int>(r2),
-                                            a.status, e, st, rg)))
-        return rc;
-    }
-    const TransposedBRows<ImplicitA<EpiStoreDX>, kC1> d2{
-        {{{a.dp1, kC1, r2}, 16, 16, kC2, -1, n}, kC2}};
-    if ((rc = launch_gemm<64, false, false>(m_dy2a, m_w2t, C, r2, 64, 9 * kC2, a.status, d2,
-                                            st)))
+    cudaError_t e = cudaFuncSetAttribute(
+        cnn_conv2_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDw2SmemAlone);
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_conv2_dw_kernel: %s", cudaGetErrorString(e));
+    const bool apart = 3 * a.split[1] * C <= 2 * sms;
+    launch_pdl(cnn_conv2_dw_kernel, dim3(a.split[1], C, apart ? 3 : 1), kDw2Threads,
+               apart ? kDw2Smem : kDw2SmemAlone, st, m_dy2, m_p1w, a.part[1], n, a.status);
+    if ((rc = launched("cnn_conv2_dw_kernel"))) return rc;
+    if ((rc = conv2(cnn_conv2_kernel<kC2, kC1, EpiStripDX>, conv_smem<kC2>(), m_dy2h,
+                    EpiStripDX{a.dp1})))
       return rc;
-    // Layer 1.
-    launch_pdl(cnn_unpool_kernel<32, 32, kC1, kA1ld, true>, unpool_grid(32, kC1), 256, 0, st, 
-        a.dy1, a.m1, a.dp1, n, a.bpart[0]);
-    if ((rc = launched("cnn_unpool_kernel 1"))) return rc;
-    // dW1 = dY1^T Col1, Col1 read by K group from X8 (N = 8 groups x 8 slots).
-    CUtensorMap m_dy1t;
-    if ((rc = make_tmap_bf16_3d(&m_dy1t, a.dy1, kA1ld, r1, C, kA1ld, r1 * kA1ld, 64, 64)))
-      return rc;
-    {
-      GemmRagged rg;
-      rg.ksplit = a.split[0];
-      const Conv1Bmn<EpiConvGradW> e{{a.part[0], kC1, kK1, true}, n};
-      if ((rc = launch_gemm<64, true, true>(m_dy1t, m_x8h, C, 128, kK1i, static_cast<int>(r1),
-                                            a.status, e, st, rg)))
-        return rc;
-    }
+    // Layer 1: routing of dP1, db1 and dW1 in one launch.
+    e = cudaFuncSetAttribute(
+        cnn_conv1_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kUnitSmem);
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_conv1_grad_kernel: %s", cudaGetErrorString(e));
+    launch_pdl(cnn_conv1_grad_kernel, dim3(a.split[0], C), kUnitThreads, kUnitSmem, st, a,
+               pair);
+    if ((rc = launched("cnn_conv1_grad_kernel"))) return rc;
   }
 
   launch_pdl(cnn_finalize_kernel, dim3((a.want_grad ? grid1(kP) : 0) + kBiasBlocks + 1, C), 256, 0,
