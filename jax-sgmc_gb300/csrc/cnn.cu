@@ -15,30 +15,22 @@
 //   | bd 10 | Wd [2048,10],   P = 113,738.
 //
 // Each convolution is a GEMM over the im2col matrix Col [pixels, K] with K
-// ordered (kh, kw, ci) and zero-padded to a multiple of 64:
-//   forward  Y = ReLU(Col W + b)          A = Col (K-major), B = W (HWIO rows
-//                                         = K, MN-major)
-//   weights  dW = dY^T Col                 both MN-major; written into the
-//                                         HWIO gradient directly
+// ordered (kh, kw, ci), which is never formed:
+//   forward  Y = ReLU(Col W + b)          A = Col (K-major), B = W
+//   weights  dW = dY^T Col                 both MN-major
 //   inputs   dX = sum over taps of dY shifted back by the tap times the tap's
 //            W^T (the transposed convolution), A = dY (K-major), B = W
 //            (K-major), then the pooling's argmax routing and the ReLU mask.
 // conv1 and its weight gradient build their operands in shared memory from
-// the images (cnn_conv1_kernel).  Col is materialised for conv2 (32 input
-// channels).  Where
-// a tap's input channels fill a 128-byte row (64 BF16: conv3's input P2 and
-// the output gradients dY2, dY3 of the transposed convolutions) the GEMMs
-// are implicit: each 64-wide K slice of A (or 64-wide N block of dW's B) is
-// one tap's box of the NHWC map, shifted by the tap and read by TMA from a
-// 4-D tensor map, whose out-of-bounds zero fill is the SAME padding.  The
-// forward GEMMs' epilogues apply bias and ReLU and the 2x2 max-pool to the
-// fp32 accumulators themselves (EpiConvPool for conv2 and conv3): each
-// epilogue warp holds whole pool windows in its 32 rows, so it writes the
-// pooled BF16 map and the argmax marks and no pre-pool activation is stored.
-// Everything a GEMM reads is BF16.  Channel and K padding come from the tensor maps'
-// out-of-bounds zero fill; epilogues drop rows and columns past the real
-// extents.  The dense layer, softmax and their adjoints are small and run on
-// the CUDA cores in fp32.
+// the images; the others' maps are stored in rows of channel octets, so that a
+// box of a strip or an image pair with its halo serves all taps (see the
+// kernels).  The epilogues apply bias and ReLU and the 2x2 max-pool to the
+// fp32 accumulators themselves and write the pooled BF16 map and the argmax
+// marks; no pre-pool activation is stored.  A mark byte holds the argmax (bits
+// 0-1) and whether the maximum is positive (bit 2), the ReLU mask of the
+// element that the backward pass routes the gradient to.
+// Everything a GEMM reads is BF16.  The dense layer, softmax and their
+// adjoints are small and run on the CUDA cores in fp32.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -59,7 +51,7 @@ constexpr int kFlat = 4 * 4 * kC3;  // 2048
 constexpr int kK1 = 27;  // conv1's K (3 x 3 taps x 3 channels)
 constexpr int kX8 = 8;   // slots of a pixel's word: its left neighbour's 3, its own 3, 0, 0
 constexpr int kK2 = 9 * kC1;
-constexpr int kK3 = 9 * kC2;  // conv3 reads P2 by tap: no padded im2col
+constexpr int kK3 = 9 * kC2;
 
 // Offsets of the leaves in a chain's flat parameter vector.
 constexpr int64_t ob1 = 0, oW1 = ob1 + kC1, ob2 = oW1 + kK1 * kC1, oW2 = ob2 + kC2,
@@ -68,11 +60,11 @@ constexpr int64_t ob1 = 0, oW1 = ob1 + kC1, ob2 = oW1 + kK1 * kC1, oW2 = ob2 + k
 static_assert(kP == 113738, "parameter count");
 
 struct CnnLayout {
-  size_t w2b, w3b;                    // BF16 weights (HWIO)
+  size_t w2b, w3b;                    // BF16 weights (cnn_prep)
   size_t p1, p2, p3;                  // BF16 GEMM operands
   size_t dy2, dy3;                    // BF16 output gradients of conv2, conv3
   size_t m1, m2, m3;                  // uint8 argmax of each pool window
-  size_t dp2, dp1;                    // fp32 input gradients of conv3, conv2
+  size_t dp1;                         // fp32 input gradient of conv2
   size_t labels;                      // int32
   size_t dp3, gl;                     // fp32 dP3 [n, 2048], dlogits [n, 10]
   size_t psq, plk;                    // fp64 partial sums
@@ -108,7 +100,6 @@ CnnLayout cnn_layout(int chains, int n) {
   L.m1 = take(N * 256 * kC1);
   L.m2 = take(N * 64 * kC2);
   L.m3 = take(N * 16 * kC3);
-  L.dp2 = take(4 * N * 64 * kC2);
   L.dp1 = take(4 * N * 256 * kC1);
   L.labels = take(4 * N);
   L.dp3 = take(4 * N * kFlat);
@@ -142,7 +133,7 @@ struct CnnArgs {
   double* lk_var;
   int* status;
   bf16 *w2b, *w3b, *p1, *p2, *p3;
-  float *dp2, *dp1;
+  float* dp1;
   bf16 *dy2, *dy3;
   uint8_t *m1, *m2, *m3;
   int32_t* lab;
@@ -191,6 +182,34 @@ __device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volati
   raise_status(status, GBSGMC_ERR_TIMEOUT);
   *abort = 1;
   return false;
+}
+
+// Routing of a pooled map's gradient by the marks: o[pos] = the BF16 pairs of
+// 8 channels at window position pos (zero where the ReLU was closed), val the
+// routed (rounded) values.
+__device__ __forceinline__ void route_octet(const float (&g)[8], uint2 mark, uint32_t (&o)[4][4],
+                                            float (&val)[8]) {
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
+    const __nv_bfloat162 p = __floats2bfloat162_rn((m & 4u) ? g[2 * e] : 0.f,
+                                                   (m & 0x400u) ? g[2 * e + 1] : 0.f);
+    val[2 * e] = __low2float(p);
+    val[2 * e + 1] = __high2float(p);
+    const uint32_t pk = *reinterpret_cast<const uint32_t*>(&p);
+#pragma unroll
+    for (int pos = 0; pos < 4; ++pos)
+      o[pos][e] = pk & (((m & 3u) == static_cast<uint32_t>(pos) ? 0xffffu : 0u) |
+                        (((m >> 8) & 3u) == static_cast<uint32_t>(pos) ? 0xffff0000u : 0u));
+  }
+}
+
+// 8 words (a 32-byte sector).
+__device__ __forceinline__ void store_sector(void* at, const uint32_t (&l)[4],
+                                             const uint32_t (&r)[4]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(l[0]),
+               "r"(l[1]), "r"(l[2]), "r"(l[3]), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3])
+               : "memory");
 }
 
 // Pixels w - 1, w, w + 1 (w even) of an image row, px pointing at w; zeros
@@ -298,7 +317,8 @@ __device__ __forceinline__ void strip_borders(uint8_t* smem) {
 }
 
 // BF16 weights of conv2 ([output octet][tap, input][8], so that outputs and
-// inputs both lie in core matrices) and conv3 (HWIO order) and part `b` of a chain's sum
+// inputs both lie in core matrices) and conv3 ([tap][output octet][input][8])
+// and part `b` of a chain's sum
 // of squares.
 __device__ __forceinline__ void cnn_prep(const CnnArgs& a, int c, int b, double* red) {
   constexpr int kCols = 256, kEach = kCols / kStripThreads;
@@ -315,7 +335,9 @@ __device__ __forceinline__ void cnn_prep(const CnnArgs& a, int c, int b, double*
         a.w2b[static_cast<int64_t>(c) * kK2 * kC2 +
               ((j - oW2) % kC2 / 8 * kK2 + (j - oW2) / kC2) * 8 + j % 8] = __float2bfloat16_rn(v);
       else if (j >= oW3 && j < obd)
-        a.w3b[static_cast<int64_t>(c) * kK3 * kC3 + (j - oW3)] = __float2bfloat16_rn(v);
+        a.w3b[static_cast<int64_t>(c) * kK3 * kC3 +
+              (((j - oW3) / kC3 / kC2 * (kC3 / 8) + (j - oW3) % kC3 / 8) * kC2 +
+               (j - oW3) / kC3 % kC2) * 8 + (j - oW3) % 8] = __float2bfloat16_rn(v);
     }
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -648,37 +670,19 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
         if (xj > 0) store_word(at + 512 - 16, e);
       }
       {
-        const float* gv = reinterpret_cast<const float*>(p.g);
-        const uint2 mark = p.mark;
-        uint32_t pk[4];
-        float4 bv[2];
-        float* bf8 = reinterpret_cast<float*>(bv);
+        const float4 &g0 = p.g[0], &g1 = p.g[1];
+      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+      uint32_t o[4][4];
+      float val[8];
+      route_octet(g, p.mark, o, val);
+      float4* bd = reinterpret_cast<float4*>(bias + (16 * wy + wx) * 36 + 8 * oct);
+      bd[0] = make_float4(val[0], val[1], val[2], val[3]);
+      bd[1] = make_float4(val[4], val[5], val[6], val[7]);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          // BF16 pair, zero where the ReLU was closed (mark bit 2).
-          const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
-          const __nv_bfloat162 v = __floats2bfloat162_rn((m & 4u) ? gv[2 * e] : 0.f,
-                                                         (m & 0x400u) ? gv[2 * e + 1] : 0.f);
-          bf8[2 * e] = __low2float(v);
-          bf8[2 * e + 1] = __high2float(v);
-          pk[e] = *reinterpret_cast<const uint32_t*>(&v);
-        }
-        float4* bd = reinterpret_cast<float4*>(bias + (16 * wy + wx) * 36 + 8 * oct);
-        bd[0] = bv[0];
-        bd[1] = bv[1];
-#pragma unroll
-        for (int pos = 0; pos < 4; ++pos) {
-          uint32_t o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
-            o[e] = pk[e] & (((m & 3u) == static_cast<uint32_t>(pos) ? 0xffffu : 0u) |
-                            (((m >> 8) & 3u) == static_cast<uint32_t>(pos) ? 0xffff0000u : 0u));
-          }
-          tc::sts128(dy + ((2 * wy + (pos >> 1)) * 2 + (warp & 1)) * 1024 + (pos & 1) * 512 +
-                         16 * lane,
-                     o[0], o[1], o[2], o[3]);
-        }
+      for (int pos = 0; pos < 4; ++pos)
+        tc::sts128(dy + ((2 * wy + (pos >> 1)) * 2 + (warp & 1)) * 1024 + (pos & 1) * 512 +
+                       16 * lane,
+                   o[pos][0], o[pos][1], o[pos][2], o[pos][3]);
       }
       tc::fence_async_shared();
       if (u + 2 < u1) {
@@ -976,22 +980,22 @@ __global__ void __launch_bounds__(kConvThreads, 2)
 // conv2's pooling: lane 8 i + j of quarter q is the pixel (4 q + i, 8 s + j).
 struct EpiStripPool {
   const float* w;
-  bf16* P;      // [images, 8, 8, 64]
+  bf16* P;      // [pair][h][image of the pair][octet][w][8]
   uint8_t* M;
   __device__ __forceinline__ void tile(int64_t img, int c, int s, int q, int col0,
                                        float (&v)[32]) const {
     const int lane = epi::lane_id();
     const int base = lane & ~9;
-    const int64_t pix = img * 64 + (2 * q + (base >> 4)) * 8 + 4 * s + ((base & 7) >> 1);
+    const int h = 2 * q + (base >> 4), x = 4 * s + ((base & 7) >> 1);
     const float bl = __ldg(w + static_cast<int64_t>(c) * kP + ob2 + col0 + lane);
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j] + __shfl_sync(0xffffffffu, bl, j), 0.f);
     uint4 p;
     uint2 m;
     const int wp = pool_windows<8>(v, p, m);
-    const int64_t at = pix * kC2 + col0 + 8 * wp;
-    *reinterpret_cast<uint4*>(P + at) = p;
-    *reinterpret_cast<uint2*>(M + at) = m;
+    *reinterpret_cast<uint4*>(
+        P + ((((img >> 1) * 8 + h) * 2 + (img & 1)) * 8 + col0 / 8 + wp) * 64 + x * 8) = p;
+    *reinterpret_cast<uint2*>(M + (img * 64 + h * 8 + x) * kC2 + col0 + 8 * wp) = m;
   }
 };
 
@@ -1124,94 +1128,469 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Dense layer, softmax likelihood and its adjoint for kDenseImgs images of a
-// chain per block.  Writes lk, dlogits g = dU/dlogits (fp32), dP3 = g Wd^T
-// and the per-image likelihood terms.  Grid (ceil(n / kDenseImgs), chains),
-// 16 threads per image: thread (image j = t / 16, slice s = t % 16) handles
-// the features f = s, s + 16, ...; an image's 16 threads are one half-warp
-// and reduce by shuffles.  The block first copies Wd (80 KB) and its images'
-// P3 rows (4 KB each) into shared memory with all loads in flight: a
-// half-warp then reads 16 Wd rows 40 bytes apart, 16 distinct banks (the
-// other half-warp the same words), and 16 consecutive P3 features.
+// conv3 (8 x 8 images) and its gradients: as conv2, on pairs of images.
+//
+// P2 and dY3 are stored as [pair][h][image of the pair][octet][w][8], so that
+// a pair's box with its halo ([h][image][octet][10 columns] words) has 16 rows
+// of 8 pixels a uniform stride apart: a tile of M = 128.  W3 ([tap][output
+// octet][input][8], MN-major B of the forward GEMM and K-major B of the
+// transposed one) streams through a ring, 16 KB a tap: resident it would leave
+// no room for two boxes of dY3.  2,048 images: conv3 18 us against 27 with a
+// swizzled box per tap, dP2 26 with its routing against 41 + 21.
+//
+// Forward (CK = 64, N = 128) or transposed (CK = 128, N = 64).  Roles: warp 0
+// loads boxes, warp 1 issues the MMAs into two accumulators, warp 2 loads
+// weights, warps 4-11 run the epilogue
+//   epi.tile(pair, chain, lane quarter, half, accumulator)
+// on 32 lanes and the columns [half N / 2, (half + 1) N / 2).  One CTA per SM,
+// pairs blockIdx.x, + gridDim.x, ...
 // ---------------------------------------------------------------------------
-// Few images leave most SMs without a block of 16, so blocks take 4 then (2 x
-// 50 images: 18.3 -> 9 us): the loads and the adjoint use all 256 threads
-// whatever the images.
-constexpr int kDenseThreads = 256;
+constexpr int kW3Tap = kC2 * kC3 * 2, kW3Stages = 5;
+constexpr int kConv3Threads = 128 + 8 * 32;
+constexpr int pair_box(int channels) { return 10 * 2 * (channels / 8) * 160; }
+template <int CK>
+constexpr int conv3_stages() { return CK == kC2 ? 3 : 2; }
+template <int CK, class Epi>
+constexpr int conv3_smem() {
+  return kW3Stages * kW3Tap + conv3_stages<CK>() * pair_box(CK) + Epi::kStage + 128 + 256;
+}
+
+// Whether `ok` holds for all eight epilogue warps; a barrier among them.
+__device__ __forceinline__ bool epilogue_vote(bool ok) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.pred q, 1, 256, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(static_cast<uint32_t>(ok))
+      : "memory");
+  return r != 0;
+}
+
+template <int CK, int N, class Epi>
+__global__ void __launch_bounds__(kConv3Threads, 1)
+    cnn_conv3_kernel(const __grid_constant__ CUtensorMap map, const bf16* wts, int chains, int n,
+                     int* status, const __grid_constant__ Epi epi) {
+  constexpr bool kFwd = N == kC3;
+  constexpr int kBox = pair_box(CK), kRow = (CK / 8) * 160, kStages = conv3_stages<CK>();
+  constexpr uint32_t kCols = 2 * N;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* w_s = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
+  uint8_t* ring = w_s + kW3Stages * kW3Tap;
+  uint8_t* stage = ring + kStages * kBox;
+  uint64_t* full = reinterpret_cast<uint64_t*>(stage + Epi::kStage);
+  uint64_t* empty = full + kStages;
+  uint64_t* wfull = empty + kStages;
+  uint64_t* wempty = wfull + kW3Stages;
+  uint64_t* tfull = wempty + kW3Stages;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* drain = tempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(full + i, 1);
+      mbar_init(empty + i, 1);
+    }
+    for (int i = 0; i < kW3Stages; ++i) {
+      mbar_init(wfull + i, 1);
+      mbar_init(wempty + i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(tfull + i, 1);
+      mbar_init(tempty + i, 8);
+    }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, kCols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+  const int pairs = chains * (n / 2), per = n / 2;
+
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      uint32_t it = 0;
+      for (int p = blockIdx.x; p < pairs; p += gridDim.x, ++it) {
+        const int s = it % kStages;
+        if (!conv_wait(empty + s, ((it / kStages) & 1u) ^ 1u, abort_flag, status)) break;
+        mbar_arrive_expect_tx(full + s, kBox);
+        tc::tma_load_4d(ring + s * kBox, &map, -8, 0, -1, p, full + s);
+      }
+      if (*abort_flag)   // copies in flight land before the CTA ends
+        for (uint32_t i = it > kStages ? it - kStages : 0; i < it; ++i)
+          mbar_wait_bounded(full + i % kStages, (i / kStages) & 1u, nullptr);
+    }
+  } else if (warp == 2) {
+    if (tc::elect_one()) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int p = blockIdx.x; ok && p < pairs; p += gridDim.x) {
+        const bf16* src = wts + static_cast<int64_t>(p / per) * kK3 * kC3;
+        for (int tap = 0; tap < 9; ++tap, ++it) {
+          const int s = it % kW3Stages;
+          ok = conv_wait(wempty + s, ((it / kW3Stages) & 1u) ^ 1u, abort_flag, status);
+          if (!ok) break;
+          mbar_arrive_expect_tx(wfull + s, kW3Tap);
+          bulk_g2s(w_s + s * kW3Tap, src + tap * kC2 * kC3, kW3Tap, wfull + s);
+        }
+      }
+      if (*abort_flag)
+        for (uint32_t i = it > kW3Stages ? it - kW3Stages : 0; i < it; ++i)
+          mbar_wait_bounded(wfull + i % kW3Stages, (i / kW3Stages) & 1u, nullptr);
+    }
+  } else if (warp == 1) {
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc = tc::idesc_bf16_f32(128, N, false, kFwd);
+      uint32_t it = 0, wt = 0;
+      bool ok = true;
+      for (int p = blockIdx.x; ok && p < pairs; p += gridDim.x, ++it) {
+        const int s = it % kStages;
+        const uint32_t buf = it & 1u;
+        if (!conv_wait(tempty + buf, ((it >> 1) & 1u) ^ 1u, abort_flag, status) ||
+            !conv_wait(full + s, (it / kStages) & 1u, abort_flag, status))
+          break;
+        const uint64_t A = tc::sdesc_none(ring + s * kBox, 160, kRow);
+#pragma unroll
+        for (int tap = 0; tap < 9; ++tap, ++wt) {
+          const int ws = wt % kW3Stages;
+          ok = ok && conv_wait(wfull + ws, (wt / kW3Stages) & 1u, abort_flag, status);
+          if (!ok) break;
+          tc::fence_after_sync();
+          const uint64_t B = kFwd ? tc::sdesc_none(w_s + ws * kW3Tap, 128, 1024)
+                                  : tc::sdesc_none(w_s + ws * kW3Tap, 1024, 128);
+          const int kh = kFwd ? tap / 3 : 2 - tap / 3, kw = kFwd ? tap % 3 : 2 - tap % 3;
+#pragma unroll
+          for (int k = 0; k < CK / 16; ++k)
+            tc::mma_bf16(tmem + buf * N, A + (2 * kh * kRow + kw * 16 + k * 320) / 16,
+                         B + k * (kFwd ? 16 : 128), idesc, (tap | k) != 0);
+          tc::mma_commit(wempty + ws);
+        }
+        tc::mma_commit(empty + s);
+        if (ok) tc::mma_commit(tfull + buf);
+      }
+      tc::mma_commit(drain);   // every MMA of this CTA has completed once it flips
+      mbar_wait_bounded(drain, 0, nullptr);
+    }
+  } else if (warp >= 4) {
+    const int q = warp & 3, half = (warp - 4) >> 2;
+    uint32_t it = 0;
+    for (int p = blockIdx.x; p < pairs; p += gridDim.x, ++it) {
+      const uint32_t buf = it & 1u;
+      // The eight warps leave together: the epilogue synchronises them.
+      if (!epilogue_vote(conv_wait(tfull + buf, (it >> 1) & 1u, abort_flag, status))) break;
+      tc::fence_after_sync();
+      const tc::TmemRows load{tmem + buf * N + half * (N / 2) +
+                              (static_cast<uint32_t>(q * 32) << 16)};
+      epi.tile(p, p / per, q, half, load, stage);
+      tc::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty + buf);
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, kCols);
+  }
+}
+
+// conv3's pooling: lane 16 i + 8 m + x of quarter q is the pixel (2 q + i, x)
+// of the pair's image m.
+struct EpiPairPool {
+  static constexpr int kStage = 0;
+  const float* w;
+  bf16* P;      // [images, 4, 4, 128]
+  uint8_t* M;
+  template <class Load>
+  __device__ __forceinline__ void tile(int pair, int c, int q, int half, const Load& load,
+                                       uint8_t*) const {
+    const int lane = epi::lane_id();
+    const int64_t pix = (2 * static_cast<int64_t>(pair) + ((lane >> 3) & 1)) * 16 + 4 * q +
+                        ((lane & 7) >> 1);
+#pragma unroll 1
+    for (int cb = 0; cb < 2; ++cb) {
+      const int col0 = 64 * half + 32 * cb;
+      const float bl = __ldg(w + static_cast<int64_t>(c) * kP + ob3 + col0 + lane);
+      float v[32];
+      load(cb, v);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j] + __shfl_sync(0xffffffffu, bl, j), 0.f);
+      uint4 p;
+      uint2 m;
+      const int wp = pool_windows<16>(v, p, m);
+      const int64_t at = pix * kC3 + col0 + 8 * wp;
+      *reinterpret_cast<uint4*>(P + at) = p;
+      *reinterpret_cast<uint2*>(M + at) = m;
+    }
+  }
+};
+
+// dP2 never leaves the chip: a lane routes its pooled pixel's 32 channels into
+// dY2 [image][h][octet][w][8], and db2's partials add the routed values of 32
+// pooled pixels (half an image) in order.
+struct EpiPairRoute {
+  static constexpr int kLd = kC2 + 1, kStage = 128 * kLd * 4;
+  const uint8_t* M;
+  bf16* dy;
+  float* bpart;   // [chain, blocks, 64], block 2 (image of the chain) + half
+  template <class Load>
+  __device__ __forceinline__ void tile(int pair, int, int q, int half, const Load& load,
+                                       uint8_t* stage) const {
+    float* st = reinterpret_cast<float*>(stage);
+    const int lane = epi::lane_id(), x = lane & 7, im = (lane >> 3) & 1, h = 2 * q + (lane >> 4);
+    const int64_t img = 2 * static_cast<int64_t>(pair) + im;
+    const uint2* mk = reinterpret_cast<const uint2*>(M + (img * 64 + h * 8 + x) * kC2) + 4 * half;
+    uint2 mark[4];
+#pragma unroll
+    for (int o = 0; o < 4; ++o) mark[o] = __ldg(mk + o);
+    float v[32];
+    load(0, v);
+    float* mine = st + (64 * im + 8 * h + x) * kLd + 32 * half;
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      float g[8], val[8];
+      uint32_t w[4][4];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) g[e] = v[8 * o + e];
+      route_octet(g, mark[o], w, val);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mine[8 * o + e] = val[e];
+      bf16* at = dy + ((img * 16 + 2 * h) * 8 + 4 * half + o) * 128 + 16 * x;
+      store_sector(at, w[0], w[1]);
+      store_sector(at + 8 * 128, w[2], w[3]);
+    }
+    epilogue_vote(true);
+    const int t = threadIdx.x - 128, col = t & 63, blk = t >> 6;
+    float sum = 0.f;
+#pragma unroll 8
+    for (int u = 0; u < 32; ++u) sum += st[(32 * blk + u) * kLd + col];
+    bpart[(4 * static_cast<int64_t>(pair) + blk) * kC2 + col] = sum;
+  }   // the next tile's vote comes before anything is written here again
+};
+
+// dW3 = dY3^T Col3: per image the boxes of dY3 and of P2 with its halo, two
+// image rows (16 pixels) as K; M = 128 outputs.  Z = 3: a CTA takes a column
+// shift, N = 192 (three kernel rows x 64 inputs, words 160 bytes apart); Z =
+// 9, when the splits leave SMs idle: one tap, N = 64.  Grid (splits, chains,
+// Z), one split-K partial [tap, input][output] of a run of a chain's images
+// each.
+constexpr int kDy3Box = 8 * (kC3 / 8) * 128, kP2Box = 10 * (kC2 / 8) * 160;
+constexpr int kDw3Stages = 7, kDw3Threads = 64 + 4 * 32;
+constexpr int kDw3Smem = kDw3Stages * (kDy3Box + kP2Box) + 128 + 256;
+
+__global__ void __launch_bounds__(kDw3Threads, 1)
+    cnn_conv3_dw_kernel(const __grid_constant__ CUtensorMap mdy,
+                        const __grid_constant__ CUtensorMap mp2, float* part, int n,
+                        int* status) {
+  constexpr int kStage = kDy3Box + kP2Box, kRow = (kC2 / 8) * 160;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
+  uint64_t* full = reinterpret_cast<uint64_t*>(ring + kDw3Stages * kStage);
+  uint64_t* empty = full + kDw3Stages;
+  uint64_t* done = empty + kDw3Stages;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool single = gridDim.z == 9;
+  const uint32_t cols = single ? 64 : 256;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kDw3Stages; ++i) {
+      mbar_init(full + i, 1);
+      mbar_init(empty + i, 1);
+    }
+    mbar_init(done, 1);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, cols);
+    tc::tmem_relinquish();
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
+  const int c = blockIdx.y, S = gridDim.x;
+  const int each = n / S, u0 = c * n + each * blockIdx.x, u1 = u0 + each;   // images
+  const int kw = blockIdx.z % 3, kh0 = single ? blockIdx.z / 3 : 0;
+  if (warp == 0) {
+    if (tc::elect_one()) {
+      uint32_t it = 0;
+      for (int u = u0; u < u1; ++u, ++it) {
+        const int s = it % kDw3Stages;
+        if (!conv_wait(empty + s, ((it / kDw3Stages) & 1u) ^ 1u, abort_flag, status)) break;
+        uint8_t* dst = ring + s * kStage;
+        mbar_arrive_expect_tx(full + s, kStage);
+        tc::tma_load_4d(dst, &mdy, 0, (u & 1) * (kC3 / 8), 0, u >> 1, full + s);
+        tc::tma_load_4d(dst + kDy3Box, &mp2, -8, (u & 1) * (kC2 / 8), -1, u >> 1, full + s);
+      }
+      if (*abort_flag)
+        for (uint32_t i = it > kDw3Stages ? it - kDw3Stages : 0; i < it; ++i)
+          mbar_wait_bounded(full + i % kDw3Stages, (i / kDw3Stages) & 1u, nullptr);
+    }
+  } else if (warp == 1) {
+    if (tc::elect_one()) {
+      const uint32_t idesc = single ? tc::idesc_bf16_f32(128, 64, true, true)
+                                    : tc::idesc_bf16_f32(128, 192, true, true);
+      uint32_t it = 0;
+      for (int u = u0; u < u1; ++u, ++it) {
+        const int s = it % kDw3Stages;
+        if (!conv_wait(full + s, (it / kDw3Stages) & 1u, abort_flag, status)) break;
+        tc::fence_after_sync();
+        const uint64_t A = tc::sdesc_none(ring + s * kStage, (kC3 / 8) * 128, 128);
+        const uint64_t B = tc::sdesc_none(ring + s * kStage + kDy3Box, kRow, 160) +
+                           (kh0 * kRow + kw * 16) / 16;
+#pragma unroll
+        for (int h = 0; h < 8; h += 2)
+          tc::mma_bf16(tmem, A + h * (kC3 / 8) * 128 / 16, B + h * kRow / 16, idesc,
+                       it > 0 || h > 0);
+        tc::mma_commit(empty + s);
+      }
+      tc::mma_commit(done);
+      mbar_wait_bounded(done, 0, nullptr);
+    }
+  } else {
+    const bool ok = mbar_wait_bounded(done, 0, nullptr);
+    if (!__all_sync(0xffffffffu, ok) && lane == 0) raise_status(status, GBSGMC_ERR_TIMEOUT);
+    tc::fence_after_sync();
+    const int q = warp & 3;
+    float* dst = part + (static_cast<int64_t>(c) * S + blockIdx.x) * kK3 * kC3 + 32 * q + lane;
+#pragma unroll 1
+    for (int g = 0; g < (single ? 2 : 6); ++g) {   // kh, input half
+      float v[32];
+      tc::tmem_ld32(tmem + 32 * g + (static_cast<uint32_t>(q * 32) << 16), v);
+      const int k0 = (3 * (kh0 + (g >> 1)) + kw) * kC2 + 32 * (g & 1);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) dst[(k0 + j) * kC3] = v[j];
+    }
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    tc::fence_after_sync();
+    tc::tmem_dealloc(tmem, cols);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Dense layer, softmax likelihood and its adjoint for kImgs images of a chain
+// per block.  Writes lk, dlogits g = dU/dlogits (fp32), dP3 = g Wd^T and the
+// per-image likelihood terms.  Grid (ceil(n / kImgs), chains), kParts x 16
+// threads per image: thread (class part p, image j, slice s) handles the
+// features f = s, s + 16, ... of 10 / kParts classes; the 16 threads of a part
+// are one half-warp and reduce by shuffles.  The block first copies Wd (80 KB)
+// and its images' P3 rows (4 KB each) into shared memory with all loads in
+// flight: a half-warp then reads 16 Wd rows 40 bytes apart, 16 distinct banks
+// (the other half-warp the same words), and 16 consecutive P3 features.
+// Few images leave most SMs without a block of 16, so blocks take 4 then, and
+// more parts: what a block takes is the latency of its loads and of 128
+// dependent steps a thread.
+// ---------------------------------------------------------------------------
 static_assert(oWd % 2 == 0 && kP % 2 == 0, "Wd is copied as float2");
 constexpr size_t dense_smem(int imgs) {
   return sizeof(float) * kFlat * kClasses + sizeof(bf16) * imgs * kFlat;
 }
 
-template <int kDenseImgs>
-__global__ void __launch_bounds__(kDenseThreads) cnn_dense_kernel(const CnnArgs a, float scale) {
+template <int kDenseImgs, int kParts>
+__global__ void __launch_bounds__(kDenseImgs * kParts * 16)
+    cnn_dense_kernel(const CnnArgs a, float scale) {
   pdl_trigger();
   pdl_wait();
+  constexpr int kDenseThreads = kDenseImgs * kParts * 16, kEach = kClasses / kParts;
+  static_assert(kEach * kParts == kClasses, "whole classes");
   extern __shared__ float wd_s[];  // Wd [2048][10], then P3 rows [kDenseImgs][2048]
   bf16* x_s = reinterpret_cast<bf16*>(wd_s + kFlat * kClasses);
-  __shared__ float g_s[kDenseImgs][kClasses];
+  __shared__ float g_s[kDenseImgs][kClasses];   // logits, then their adjoints
   const unsigned full = 0xffffffffu;
-  const int c = blockIdx.y, t = threadIdx.x, j = t >> 4, sl = t & 15;
+  const int c = blockIdx.y, t = threadIdx.x;
+  const int part = t / (kDenseImgs * 16), j = (t >> 4) % kDenseImgs, sl = t & 15;
   const int i = blockIdx.x * kDenseImgs + j;
-  const bool live = j < kDenseImgs && i < a.n;
+  const bool live = i < a.n;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
   {
     // oWd and kP are even: the chain's Wd starts 8-byte aligned.
     const float2* src = reinterpret_cast<const float2*>(w + oWd);
     float2* dst = reinterpret_cast<float2*>(wd_s);
-#pragma unroll 8
-    for (int e = t; e < kFlat * kClasses / 2; e += kDenseThreads) dst[e] = __ldg(src + e);
     // The block's images, 16 bytes per load (rows past n are not read).
     const int i0 = blockIdx.x * kDenseImgs;
     const int rows = min(kDenseImgs, a.n - i0);
-    const uint4* xs = reinterpret_cast<const uint4*>(a.p3 + (static_cast<int64_t>(c) * a.n + i0) * kFlat);
+    const uint4* xs =
+        reinterpret_cast<const uint4*>(a.p3 + (static_cast<int64_t>(c) * a.n + i0) * kFlat);
     uint4* xd = reinterpret_cast<uint4*>(x_s);
-#pragma unroll 8
+#pragma unroll 16
+    for (int e = t; e < kFlat * kClasses / 2; e += kDenseThreads) dst[e] = __ldg(src + e);
+#pragma unroll 4
     for (int e = t; e < kDenseImgs * kFlat / 8; e += kDenseThreads)
       if (e < rows * (kFlat / 8)) xd[e] = __ldg(xs + e);
   }
   __syncthreads();
-  if (j < kDenseImgs) {   // whole warps: an image is half of one
+  {
     const bf16* x = x_s + j * kFlat;
-    float acc[kClasses];
+    float acc[kEach];
 #pragma unroll
-    for (int k = 0; k < kClasses; ++k) acc[k] = 0.f;
-#pragma unroll 4
+    for (int k = 0; k < kEach; ++k) acc[k] = 0.f;
+#pragma unroll 8
     for (int f = sl; f < kFlat; f += 16) {
       const float xv = live ? bf(x[f]) : 0.f;
-      const float* wr = wd_s + f * kClasses;
+      const float* wr = wd_s + f * kClasses + part * kEach;
 #pragma unroll
-      for (int k = 0; k < kClasses; ++k) acc[k] = fmaf(xv, wr[k], acc[k]);
+      for (int k = 0; k < kEach; ++k) acc[k] = fmaf(xv, wr[k], acc[k]);
     }
 #pragma unroll
-    for (int k = 0; k < kClasses; ++k)
+    for (int k = 0; k < kEach; ++k)
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(full, acc[k], off);
-    if (sl == 0 && live) {
-      float logit[kClasses], mx = -INFINITY;
-      for (int k = 0; k < kClasses; ++k) {
-        logit[k] = acc[k] + __ldg(w + obd + k);
-        mx = fmaxf(mx, logit[k]);
-      }
-      float se = 0.f;
-      for (int k = 0; k < kClasses; ++k) se += expf(logit[k] - mx);
-      const float lse = mx + logf(se);
-      const int lab = a.lab[static_cast<int64_t>(c) * a.n + i];
-      const float lk = logit[lab] - lse;
-      const float m = a.mask != nullptr ? __ldg(a.mask + static_cast<int64_t>(c) * a.n + i) : 1.f;
-      for (int k = 0; k < kClasses; ++k) {
-        const float pk = expf(logit[k] - lse);
-        const float g = -scale * m * ((k == lab ? 1.f : 0.f) - pk);
-        g_s[j][k] = g;
-        a.gl[(static_cast<int64_t>(c) * a.n + i) * kClasses + k] = g;
-      }
-      if (a.lk != nullptr) a.lk[static_cast<int64_t>(c) * a.n + i] = lk;
-      double* pl = a.plk + (static_cast<int64_t>(c) * a.n + i) * 4;
-      pl[0] = static_cast<double>(m) * lk;
-      pl[1] = lk;
-      pl[2] = static_cast<double>(lk) * lk;
-      pl[3] = 0.0;
+    if (sl == 0) {
+#pragma unroll
+      for (int k = 0; k < kEach; ++k)
+        g_s[j][part * kEach + k] = acc[k] + __ldg(w + obd + part * kEach + k);
     }
+  }
+  __syncthreads();
+  if (part == 0 && sl == 0 && live) {
+    float logit[kClasses], mx = -INFINITY;
+#pragma unroll
+    for (int k = 0; k < kClasses; ++k) {
+      logit[k] = g_s[j][k];
+      mx = fmaxf(mx, logit[k]);
+    }
+    float se = 0.f;
+#pragma unroll
+    for (int k = 0; k < kClasses; ++k) se += expf(logit[k] - mx);
+    const float lse = mx + logf(se);
+    const int lab = a.lab[static_cast<int64_t>(c) * a.n + i];
+    const float lk = g_s[j][lab] - lse;
+    const float m = a.mask != nullptr ? __ldg(a.mask + static_cast<int64_t>(c) * a.n + i) : 1.f;
+#pragma unroll
+    for (int k = 0; k < kClasses; ++k) {
+      const float pk = expf(logit[k] - lse);
+      const float g = -scale * m * ((k == lab ? 1.f : 0.f) - pk);
+      g_s[j][k] = g;
+      a.gl[(static_cast<int64_t>(c) * a.n + i) * kClasses + k] = g;
+    }
+    if (a.lk != nullptr) a.lk[static_cast<int64_t>(c) * a.n + i] = lk;
+    double* pl = a.plk + (static_cast<int64_t>(c) * a.n + i) * 4;
+    pl[0] = static_cast<double>(m) * lk;
+    pl[1] = lk;
+    pl[2] = static_cast<double>(lk) * lk;
+    pl[3] = 0.0;
   }
   if (!a.want_grad) return;
   __syncthreads();
@@ -1232,17 +1611,51 @@ __global__ void __launch_bounds__(kDenseThreads) cnn_dense_kernel(const CnnArgs 
   }
 }
 
-// dWd [2048, 10] = sum_i P3_i (x) g_i and dbd = sum_i g_i (likelihood part).
-// Grid (kFlat / 128 + 1, chains), 512 threads: feature f = 128 x + t % 128,
-// image group q = t / 128 adds the images i = q (mod 4) in order; the four
-// partial sums are added in group order.  dlogits are staged in shared
-// memory 512 images at a time.
+// What depends on the dense layer's adjoint alone, in one launch.  Blocks
+// 0 .. kFlat / 128: dWd [2048, 10] = sum_i P3_i (x) g_i and dbd = sum_i g_i
+// (likelihood part); feature f = 128 x + t % 128, image group q = t / 128 adds
+// the images i = q (mod 4) in order; the four partial sums are added in group
+// order; dlogits are staged in shared memory 512 images at a time.  The other
+// blocks: the routing of dP3 into dY3 [pair][h][image of the pair][octet][w]
+// [8], a thread per pooled pixel and octet, 256 threads (16 pooled pixels, an
+// image) of a block for each partial of db3: the routed (BF16-rounded) values
+// of a channel, added in order.  Grid (kFlat / 128 + 1 + n / 2, chains).
+constexpr int kDenseGradBlocks = kFlat / 128 + 1;
+
 __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
   pdl_trigger();
   pdl_wait();
-  __shared__ float gs[512 * kClasses];
-  __shared__ float red[3][128 * kClasses];
-  const int c = blockIdx.y, t = threadIdx.x, q = t >> 7;
+  __shared__ float smem[512 * kClasses + 3 * 128 * kClasses];
+  const int c = blockIdx.y, t = threadIdx.x;
+  if (blockIdx.x >= kDenseGradBlocks) {
+    float* red = smem + (t >> 8) * 2048;
+    const int i = 2 * (blockIdx.x - kDenseGradBlocks) + (t >> 8), tt = t & 255;
+    const int px = tt & 3, oct = (tt >> 2) & 15, py = tt >> 6;
+    const int in = (4 * py + px) * kC3 + 8 * oct;
+    const int64_t img = static_cast<int64_t>(c) * a.n + i, at = img * kFlat + in;
+    const float4* d = reinterpret_cast<const float4*>(a.dp3 + at);
+    const float4 u = __ldg(d), v = __ldg(d + 1);
+    const float g[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+    uint32_t o[4][4];
+    float val[8];
+    route_octet(g, __ldg(reinterpret_cast<const uint2*>(a.m3 + at)), o, val);
+    bf16* dst = a.dy3 + ((((img >> 1) * 8 + 2 * py) * 2 + (img & 1)) * 16 + oct) * 64 + 16 * px;
+    store_sector(dst, o[0], o[1]);
+    store_sector(dst + 2 * 16 * 64, o[2], o[3]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) red[in + e] = val[e];
+    __syncthreads();
+    if (tt < kC3) {
+      float s = 0.f;
+#pragma unroll
+      for (int w = 0; w < 16; ++w) s += red[w * kC3 + tt];
+      a.bpart[2][img * kC3 + tt] = s;
+    }
+    return;
+  }
+  float* gs = smem;
+  float(*red)[128 * kClasses] = reinterpret_cast<float(*)[128 * kClasses]>(smem + 512 * kClasses);
+  const int q = t >> 7;
   float* g = a.grad + static_cast<int64_t>(c) * kP;
   const float* gl = a.gl + static_cast<int64_t>(c) * a.n * kClasses;
   if (blockIdx.x == kFlat / 128) {
@@ -1295,96 +1708,6 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
   }
 }
 
-// ---------------------------------------------------------------------------
-// Pool-window routing + ReLU mask: for each pooled element (i, py, px, ch),
-// the gradient dP = dp[i, py, px, ch] (fp32: the dense layer's adjoint for
-// layer 3, the transposed convolution's output for layer 2) goes to the
-// window element its argmax chose if that element was positive (the pool's
-// mark byte, bits 0-1 and 2); the three others get 0:  dY [n, H, W, C] BF16.
-// One thread per pooled pixel and eight channels: 128-bit loads of dp, 64-bit
-// of the marks, 128-bit stores of dY; C is a multiple of 8.  32-bit index
-// arithmetic (per-chain counts < 2^31).
-// Grid (ceil(n*Ho*Wo*C/8 / 256), chains).
-// The bias gradient is the column sum of dY, i.e. the sum over pooled
-// elements of the routed (BF16-rounded) values: each block adds its threads'
-// values per channel in a fixed order and writes
-// bpart[(chain * gridDim.x + block) * C + ch]; cnn_finalize_kernel adds the
-// blocks.  2048 / C threads of a block share a channel group (256 * 8 is a
-// multiple of C, so the channel of thread t is 8 t mod C).
-// ---------------------------------------------------------------------------
-template <int H, int W, int C, bool kRows>
-__global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t* M,
-                                                        const float* dp, int n, float* bpart) {
-  pdl_trigger();
-  pdl_wait();
-  __shared__ float red[256 * 8];
-  const int c = blockIdx.y;
-  const int Ho = H / 2, Wo = W / 2;
-  const int pper = n * Ho * Wo * C;
-  const int e = (blockIdx.x * 256 + threadIdx.x) * 8;
-  const bool active = e < pper;
-  float bsum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (active) {
-  // kRows: neighbouring threads take a row's pooled pixels (Wo = 8) of an octet.
-  const int ch = kRows ? e / 64 % (C / 8) * 8 : e % C;
-  const int pix = kRows ? e / (8 * C) * 8 + e / 8 % 8 : e / C;
-  const int px = pix % Wo, py = (pix / Wo) % Ho, i = pix / (Wo * Ho);
-  const int64_t at = static_cast<int64_t>(c) * pper + int64_t(pix) * C + ch;
-  float g[8];
-  {
-    const float4* d4 = reinterpret_cast<const float4*>(dp + at);
-    const float4 u = d4[0], v = d4[1];
-    g[0] = u.x; g[1] = u.y; g[2] = u.z; g[3] = u.w;
-    g[4] = v.x; g[5] = v.y; g[6] = v.z; g[7] = v.w;
-  }
-  const uint2 mk = *reinterpret_cast<const uint2*>(M + at);
-  const uint32_t marks[2] = {mk.x, mk.y};
-  const int64_t base = static_cast<int64_t>(c) * n * H * W * C;
-  __nv_bfloat162 prev[4];
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const int y = 2 * py + (q >> 1), x = 2 * px + (q & 1);
-    const int off = kRows ? ((i * H + y) * (C / 8) + ch / 8) * W * 8 + x * 8
-                          : ((i * H + y) * W + x) * C + ch;
-    __nv_bfloat162 o[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const uint32_t m0 = (marks[k >> 1] >> (16 * (k & 1))) & 0xffu;
-      const uint32_t m1 = (marks[k >> 1] >> (16 * (k & 1) + 8)) & 0xffu;
-      const float v0 = ((m0 & 3u) == static_cast<uint32_t>(q) && (m0 & 4u)) ? g[2 * k] : 0.f;
-      const float v1 = ((m1 & 3u) == static_cast<uint32_t>(q) && (m1 & 4u)) ? g[2 * k + 1] : 0.f;
-      o[k] = __floats2bfloat162_rn(v0, v1);
-      bsum[2 * k] += __low2float(o[k]);
-      bsum[2 * k + 1] += __high2float(o[k]);
-    }
-    if (!kRows) {
-      *reinterpret_cast<uint4*>(dY + base + off) = *reinterpret_cast<const uint4*>(o);
-    } else if ((q & 1) == 0) {
-#pragma unroll
-      for (int k = 0; k < 4; ++k) prev[k] = o[k];
-    } else {   // both columns: a whole sector
-      const uint32_t* l = reinterpret_cast<const uint32_t*>(prev);
-      const uint32_t* r = reinterpret_cast<const uint32_t*>(o);
-      asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dY + base +
-                                                                                  off - 8),
-                   "r"(l[0]), "r"(l[1]), "r"(l[2]), "r"(l[3]), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-                   "r"(r[3])
-                   : "memory");
-    }
-  }
-  }  // active
-#pragma unroll
-  for (int k = 0; k < 8; ++k) red[threadIdx.x * 8 + k] = bsum[k];
-  __syncthreads();
-  if (static_cast<int>(threadIdx.x) < C) {
-    const int t = threadIdx.x, group = t / 8, k = t % 8, groups = C / 8;
-    float s = 0.f;
-    for (int u = 0; u < 256 / groups; ++u)
-      s += red[(kRows ? u / 8 * 8 * groups + group * 8 + u % 8 : u * groups + group) * 8 + k];
-    bpart[(static_cast<int64_t>(c) * gridDim.x + blockIdx.x) * C + t] = s;
-  }
-}
-
 // What remains when the GEMMs are done, in one launch: the split-K partials of
 // the three weight gradients and the unpool blocks' bias partials summed in a
 // fixed order, the prior's w / (s^2 T) added to every parameter's gradient,
@@ -1395,6 +1718,17 @@ __global__ void __launch_bounds__(256) cnn_unpool_kernel(bf16* dY, const uint8_t
 // layer's bias (C / 4 channels each, 1024 / C groups of partials), the last
 // block the values.
 constexpr int kBiasBlocks = 12;
+
+// Partials added in order, all loads in flight at once.
+template <int S>
+__device__ __forceinline__ float sum_splits(const float* p, int64_t count) {
+  float x[S], v = 0.f;
+#pragma unroll
+  for (int q = 0; q < S; ++q) x[q] = __ldg(p + q * count);
+#pragma unroll
+  for (int q = 0; q < S; ++q) v += x[q];
+  return v;
+}
 
 __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
   __shared__ float acc[256];
@@ -1418,9 +1752,12 @@ __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
       if (j < off) return;   // a bias
       const int64_t count = l == 2 ? kK3 * kC3 : (l == 1 ? kK2 * kC2 : kK1 * kC1);
       const float* p = a.part[l] + static_cast<int64_t>(c) * a.split[l] * count + (j - off);
-      v = 0.f;
-#pragma unroll 8
-      for (int q = 0; q < a.split[l]; ++q) v += p[q * count];
+      const int splits = a.split[l];
+      v = splits == 32   ? sum_splits<32>(p, count)
+          : splits == 16 ? sum_splits<16>(p, count)
+          : splits == 8  ? sum_splits<8>(p, count)
+          : splits == 4  ? sum_splits<4>(p, count)
+                         : sum_splits<2>(p, count);
     }
     *g = a.pf != 0.f ? fmaf(a.pf, __ldg(w + j), v) : v;
     return;
@@ -1475,174 +1812,6 @@ __global__ void __launch_bounds__(256) cnn_finalize_kernel(const CnnArgs a) {
   if (!isfinite(U)) raise_status(a.status, GBSGMC_ERR_NONFINITE);
 }
 
-// ---------------------------------------------------------------------------
-// GEMM epilogues.
-// ---------------------------------------------------------------------------
-
-// Forward: ReLU(acc + b) in fp32 and the 2 x 2 max-pool of it, straight from
-// the accumulator.  A warp's 32 rows hold whole pool windows: the window of
-// lane l is lanes (base, base + 1, base + V, base + V + 1), base = l & ~(V | 1),
-// in row-major window order, with V = 16 for conv2 (16 pixels per
-// image row) and V = 8 for conv3 (8 per row).  Per
-// output the maximum (first one in window order, as jax's max-pool argmax
-// routes the gradient) goes to P [n, Ho, Wo, C] as BF16 and the mark byte
-// to M: bits 0-1 the argmax, bit 2 (maximum > 0), the ReLU mask of the
-// element the backward pass routes the gradient to.  The four lanes of a
-// window each write 8 of every 32 channels (16-byte P stores, 8-byte mark
-// stores).  The
-// window maxima of a 32-channel chunk take two exchange stages instead of
-// four shuffles per channel: the two pixels of a window row swap the
-// halves of the channels they do not keep (16 shuffles) and keep the
-// pairwise maximum, then the two rows swap halves again (8 shuffles), so
-// that each lane ends with the maxima of its 8 channels; comparisons are
-// strict in window order (left before right, top before bottom), which
-// keeps the first maximum of the window as the sequential scan does.
-template <int H, int W, int V>
-struct EpiConvPool {
-  const float* w;
-  int64_t boff;
-  int C;
-  bf16* P;
-  uint8_t* M;
-  int n;
-  template <int NC, class Load>
-  __device__ __forceinline__ void tile(int b, int row0, int col0, const Load& load,
-                                       uint32_t*) const {
-    const unsigned full = 0xffffffffu;
-    const int lane = epi::lane_id();
-    const int base = lane & ~(V | 1);
-    // The window's pooled pixel, from the row of its first lane.
-    const int r = row0 + base;
-    const int i = r / (H * W), rr = r % (H * W);
-    const int yp = (rr / W) >> 1, xp = (rr % W) >> 1;
-    const int64_t pix = (static_cast<int64_t>(b) * n + i) * (H / 2) * (W / 2) +
-                        yp * (W / 2) + xp;
-    const float* bias = w + b * kP + boff;
-#pragma unroll 1
-    for (int cb = 0; cb < NC / 32; ++cb) {
-      const int k0 = col0 + 32 * cb;
-      const float bl = __ldg(bias + k0 + lane);
-      float v[32];
-      load(cb, v);
-      float x[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = fmaxf(v[j] + __shfl_sync(full, bl, j), 0.f);
-      uint4 p;
-      uint2 mk;
-      const int wp = pool_windows<V>(x, p, mk);
-      const int64_t at = pix * C + k0 + 8 * wp;
-      *reinterpret_cast<uint4*>(P + at) = p;
-      *reinterpret_cast<uint2*>(M + at) = mk;
-    }
-  }
-};
-
-// Weights: element (row = output channel co, col = im2col column k) of the
-// split-K partial product of (virtual) batch bv = chain * splits + split
-// lands at part[bv][k][co] (HWIO order), rows < Cout, cols < K.
-struct EpiConvGradW {
-  float* part;
-  int Cout, K;
-  template <int NC, class Load>
-  __device__ __forceinline__ void tile(int bv, int row0, int col0, const Load& load,
-                                       uint32_t*) const {
-    const int co = row0 + epi::lane_id();
-    float* dst = part + static_cast<int64_t>(bv) * K * Cout + co;
-#pragma unroll 1
-    for (int cb = 0; cb < NC / 32; ++cb) {
-      float v[32];
-      load(cb, v);
-      if (co < Cout) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int k = col0 + 32 * cb + j;
-          if (k < K) dst[static_cast<int64_t>(k) * Cout] = v[j];
-        }
-      }
-    }
-  }
-};
-
-// The transposed convolution's output dX as fp32 [rows, C] (columns >= C of
-// the N = 64 tile are skipped), one 128-byte row segment per store.
-struct EpiStoreDX {
-  float* dx;
-  int C;
-  int64_t rows;  // rows per chain
-  template <int NC, class Load>
-  __device__ __forceinline__ void tile(int b, int row0, int col0, const Load& load,
-                                       uint32_t* st) const {
-    if (col0 >= C) return;  // padding columns (warp-uniform)
-    float* dst = dx + (b * rows + row0) * C + col0 + epi::lane_id();
-#pragma unroll 1
-    for (int cb = 0; cb < NC / 32; ++cb) {
-      if (col0 + 32 * cb >= C) break;
-      float v[32];
-      uint32_t u[32];
-      load(cb, v);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) u[j] = __float_as_uint(v[j]);
-      epi::put_rows(st, u);
-#pragma unroll 4
-      for (int r = 0; r < 32; ++r) dst[r * C + 32 * cb] = __uint_as_float(epi::get(st, r));
-    }
-  }
-};
-
-// Implicit A operand: the K slice k0 of a GEMM over pixels (rows) and taps x
-// channels (K) is tap t = k0 / Ck, channels [k0 % Ck, + 64), of the NHWC map
-// shifted by the tap: the box (64 channels, W, rows / W, images) of a 4-D map
-// (Ck, W, H, chains * n) at (k0 % Ck, s (kw - 1), h0 + s (kh - 1), image),
-// s = +1 for a convolution and -1 for its transpose (the box reads zeros
-// outside the image: SAME padding).  A tile of 128 rows covers whole image
-// rows (W | 128) of one image, or whole images (H W | 128).
-template <class Inner>
-struct ImplicitA : Inner {
-  int H, W, Ck, sign, n;
-  static constexpr bool kLoadA = true;
-  __device__ __forceinline__ void load_a(void* dst, const CUtensorMap* map, int k0, int m0,
-                                         int b, uint64_t* bar) const {
-    const int tap = k0 / Ck, c0 = k0 - tap * Ck;
-    const int kh = tap / 3, kw = tap - 3 * kh;
-    const int img = m0 / (H * W), h0 = (m0 - img * H * W) / W;
-    tc::tma_load_4d(dst, map, c0, sign * (kw - 1), h0 + sign * (kh - 1), b * n + img, bar);
-  }
-};
-
-// Implicit MN-major B operand of a weight gradient dW = dY^T Col: the
-// 64-wide N block starting at column nn is tap t = nn / Ck, input channels
-// [nn % Ck, + 64), and the K slice k0 is 64 pixels (whole rows of one
-// image): the box (64 channels, W, 64 / W, 1) of the 4-D map of the
-// layer's input, shifted by the tap.
-template <class Inner>
-struct ImplicitBmn : Inner {
-  int H, W, Ck, n;
-  static constexpr bool kLoadB = true;
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* map, int nn, int k0,
-                                         int b, uint64_t* bar) const {
-    const int tap = nn / Ck, c0 = nn - tap * Ck;
-    const int kh = tap / 3, kw = tap - 3 * kh;
-    const int img = k0 / (H * W), h0 = (k0 - img * H * W) / W;
-    tc::tma_load_4d(dst, map, c0, kw - 1, h0 + kh - 1, b * n + img, bar);
-  }
-};
-
-// K-major B operand of a transposed convolution: for the K slice k0 (tap
-// t = k0 / Ckb, output channels [k0 % Ckb, + 64)) the rows n.. of W^T, i.e.
-// the box (64 output channels, 64 input channels, 1, 1) of the HWIO weights
-// as a 4-D map (Cout, Cin, 9, chains) at (k0 % Ckb, n, t, chain); input
-// channels past Cin read zeros.
-template <class Inner>
-struct TransposedB : Inner {
-  int Ckb;
-  static constexpr bool kLoadB = true;
-  __device__ __forceinline__ void load_b(void* dst, const CUtensorMap* map, int nn, int k0,
-                                         int b, uint64_t* bar) const {
-    const int tap = k0 / Ckb, c0 = k0 - tap * Ckb;
-    tc::tma_load_4d(dst, map, c0, nn, tap, b, bar);
-  }
-};
-
 template <class T>
 T* view(void* ws, size_t off) {
   return reinterpret_cast<T*>(static_cast<unsigned char*>(ws) + off);
@@ -1661,7 +1830,6 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   a.m1 = view<uint8_t>(ws, L.m1);
   a.m2 = view<uint8_t>(ws, L.m2);
   a.m3 = view<uint8_t>(ws, L.m3);
-  a.dp2 = view<float>(ws, L.dp2);
   a.dp1 = view<float>(ws, L.dp1);
   a.lab = view<int32_t>(ws, L.labels);
   a.dp3 = view<float>(ws, L.dp3);
@@ -1683,12 +1851,8 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     a.pf = static_cast<float>(1.0 / (ps * ps * a.temperature));
     a.prior_const = static_cast<double>(kP) * (std::log(ps) + 0.91893853320467274178);
   }
-  const int64_t r3 = int64_t(n) * 64;
   int rc;
   auto launched = [&](const char* what) { return check_launch(what); };
-  auto unpool_grid = [&](int H, int Cr) {
-    return dim3(grid1(int64_t(n) * (H / 2) * (H / 2) * Cr / 8), C);
-  };
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -1700,15 +1864,13 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
              kStripThreads, 0, st, a, pair);
   if ((rc = launched("cnn_conv1_kernel"))) return rc;
 
-  // Tensor maps (columns, rows, chains), and 4-D maps (channels, W, H,
-  // images) of the NHWC maps the implicit GEMMs read by tap.
-  const int64_t imgs = int64_t(C) * n;
-  CUtensorMap m_p1, m_w3, m_p2a;
+  // 4-D maps of the octet layouts, with the boxes that the kernels take.
+  const int64_t imgs = int64_t(C) * n, pairs = imgs / 2;
+  CUtensorMap m_p1, m_p2;
   if ((rc = make_tmap_bf16_4d_plain(&m_p1, a.p1, {128, kC1 / 8, 16, imgs},
                                     {128, 16 * kC1, 256 * kC1}, {80, kC1 / 8, 18, 1})) ||
-      (rc = make_tmap_bf16_3d(&m_w3, a.w3b, kC3, kK3, C, kC3, kK3 * kC3, 64, 64)) ||
-      (rc = make_tmap_bf16_4d(&m_p2a, a.p2, {kC2, 8, 8, imgs}, {kC2, 8 * kC2, 64 * kC2},
-                              {64, 8, 8, 2})))
+      (rc = make_tmap_bf16_4d_plain(&m_p2, a.p2, {64, kC2 / 4, 8, pairs},
+                                    {64, 16 * kC2, 128 * kC2}, {80, kC2 / 4, 10, 1})))
     return rc;
 
   // conv1+pool1 -> conv2+pool2 -> conv3+pool3: each epilogue writes the pooled
@@ -1725,60 +1887,56 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   if ((rc = conv2(cnn_conv2_kernel<kC1, kC2, EpiStripPool>, conv_smem<kC1>(), m_p1,
                   EpiStripPool{a.w, a.p2, a.m2})))
     return rc;
-  // conv3, implicit: A tiles are P2's tap-shifted 2-image boxes.
-  const ImplicitA<EpiConvPool<8, 8, 8>> e3{{a.w, ob3, kC3, a.p3, a.m3, n},
-                                                   8, 8, kC2, 1, n};
-  if ((rc = launch_gemm<128, false, true>(m_p2a, m_w3, C, r3, kC3, kK3, a.status, e3, st)))
+  const auto conv3 = [&](auto kern, int bytes, const CUtensorMap& map, const auto& epi) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_conv3_kernel: %s", cudaGetErrorString(e));
+    launch_pdl(kern, static_cast<int>(std::min<int64_t>(sms, pairs)), kConv3Threads, bytes, st,
+               map, static_cast<const bf16*>(a.w3b), C, n, a.status, epi);
+    return launched("cnn_conv3_kernel");
+  };
+  if ((rc = conv3(cnn_conv3_kernel<kC2, kC3, EpiPairPool>, conv3_smem<kC2, EpiPairPool>(), m_p2,
+                  EpiPairPool{a.w, a.p3, a.m3})))
     return rc;
-  const auto dense = [&](auto kern, int imgs) {
+  const auto dense = [&](auto kern, int imgs, int parts) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(dense_smem(imgs)));
     if (e != cudaSuccess)
       return set_error(GBSGMC_ERR_CUDA, "cnn_dense_kernel: %s", cudaGetErrorString(e));
     const float scale = static_cast<float>(static_cast<double>(a.n_obs) / n / a.temperature);
-    launch_pdl(kern, dim3(ceil_div(n, imgs), C), kDenseThreads, dense_smem(imgs), st, a, scale);
+    launch_pdl(kern, dim3(ceil_div(n, imgs), C), 16 * imgs * parts, dense_smem(imgs), st, a, scale);
     return launched("cnn_dense_kernel");
   };
   // Sixteen images share a block's copy of Wd once that fills the SMs.
-  rc = int64_t(C) * n >= 16 * 148 / 2 ? dense(cnn_dense_kernel<16>, 16)
-                                      : dense(cnn_dense_kernel<4>, 4);
+  rc = int64_t(C) * n >= 16 * 152 / 2 ? dense(cnn_dense_kernel<16, 2>, 16, 2)
+                                      : dense(cnn_dense_kernel<4, 5>, 4, 5);
   if (rc) return rc;
 
   if (a.want_grad) {
-    launch_pdl(cnn_dense_grad_kernel, dim3(kFlat / 128 + 1, C), 512, 0, st, a);
+    // dWd, dbd; layer 3: dY3 (routing of dP3) and db3.
+    launch_pdl(cnn_dense_grad_kernel, dim3(kDenseGradBlocks + n / 2, C), 512, 0, st, a);
     if ((rc = launched("cnn_dense_grad_kernel"))) return rc;
-    // Layer 3: dY3 (routing of dP3), db3, dW3 = dY3^T Col3 (implicit: B
-    // blocks are P2's tap-shifted images), dP2 = the transposed convolution
-    // of dY3 (implicit: A tiles are dY3's tap-shifted 2-image boxes).
-    launch_pdl(cnn_unpool_kernel<8, 8, kC3, false>, unpool_grid(8, kC3), 256, 0, st, 
-        a.dy3, a.m3, a.dp3, n, a.bpart[2]);
-    if ((rc = launched("cnn_unpool_kernel 3"))) return rc;
-    CUtensorMap m_dy3t, m_p2b, m_dy3a, m_w3t;
-    if ((rc = make_tmap_bf16_3d(&m_dy3t, a.dy3, kC3, r3, C, kC3, r3 * kC3, 64, 64)) ||
-        (rc = make_tmap_bf16_4d(&m_p2b, a.p2, {kC2, 8, 8, imgs}, {kC2, 8 * kC2, 64 * kC2},
-                                {64, 8, 8, 1})) ||
-        (rc = make_tmap_bf16_4d(&m_dy3a, a.dy3, {kC3, 8, 8, imgs}, {kC3, 8 * kC3, 64 * kC3},
-                                {64, 8, 8, 2})) ||
-        (rc = make_tmap_bf16_4d(&m_w3t, a.w3b, {kC3, kC2, 9, C}, {kC3, kC2 * kC3, kK3 * kC3},
-                                {64, 64, 1, 1})))
+    // dW3; dP2, the transposed convolution of dY3, routed into dY2, and db2.
+    CUtensorMap m_dy3, m_dy3h, m_p2w;
+    if ((rc = make_tmap_bf16_4d_plain(&m_dy3, a.dy3, {64, kC3 / 4, 8, pairs},
+                                      {64, 16 * kC3, 128 * kC3}, {64, kC3 / 8, 8, 1})) ||
+        (rc = make_tmap_bf16_4d_plain(&m_p2w, a.p2, {64, kC2 / 4, 8, pairs},
+                                      {64, 16 * kC2, 128 * kC2}, {80, kC2 / 8, 10, 1})) ||
+        (rc = make_tmap_bf16_4d_plain(&m_dy3h, a.dy3, {64, kC3 / 4, 8, pairs},
+                                      {64, 16 * kC3, 128 * kC3}, {80, kC3 / 4, 10, 1})))
       return rc;
-    {
-      GemmRagged rg;
-      rg.ksplit = a.split[2];
-      const ImplicitBmn<EpiConvGradW> e{{a.part[2], kC3, kK3}, 8, 8, kC2, n};
-      if ((rc = launch_gemm<64, true, true>(m_dy3t, m_p2b, C, 128, kK3, static_cast<int>(r3),
-                                            a.status, e, st, rg)))
-        return rc;
-    }
-    const TransposedB<ImplicitA<EpiStoreDX>> d3{{{a.dp2, kC2, r3}, 8, 8, kC3, -1, n}, kC3};
-    if ((rc = launch_gemm<64, false, false>(m_dy3a, m_w3t, C, r3, kC2, 9 * kC3, a.status, d3,
-                                            st)))
+    cudaError_t e = cudaFuncSetAttribute(
+        cnn_conv3_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDw3Smem);
+    if (e != cudaSuccess)
+      return set_error(GBSGMC_ERR_CUDA, "cnn_conv3_dw_kernel: %s", cudaGetErrorString(e));
+    launch_pdl(cnn_conv3_dw_kernel, dim3(a.split[2], C, 9 * a.split[2] * C <= sms ? 9 : 3),
+               kDw3Threads, kDw3Smem, st, m_dy3, m_p2w, a.part[2], n, a.status);
+    if ((rc = launched("cnn_conv3_dw_kernel"))) return rc;
+    if ((rc = conv3(cnn_conv3_kernel<kC3, kC2, EpiPairRoute>, conv3_smem<kC3, EpiPairRoute>(),
+                    m_dy3h, EpiPairRoute{a.m2, a.dy2, a.bpart[1]})))
       return rc;
-    // Layer 2: dY2 (routing of dP2), db2, dW2, and dP1, the transposed
-    // convolution of dY2.
-    launch_pdl(cnn_unpool_kernel<16, 16, kC2, true>, unpool_grid(16, kC2), 256, 0, st, 
-        a.dy2, a.m2, a.dp2, n, a.bpart[1]);
-    if ((rc = launched("cnn_unpool_kernel 2"))) return rc;
+    // Layer 2: dW2, and dP1, the transposed convolution of dY2.
     CUtensorMap m_dy2, m_dy2h, m_p1w;
     if ((rc = make_tmap_bf16_4d_plain(&m_dy2, a.dy2, {128, kC2 / 8, 16, imgs},
                                       {128, 16 * kC2, 256 * kC2}, {128, kC2 / 8, 4, 1})) ||
@@ -1787,7 +1945,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
         (rc = make_tmap_bf16_4d_plain(&m_dy2h, a.dy2, {128, kC2 / 8, 16, imgs},
                                       {128, 16 * kC2, 256 * kC2}, {80, kC2 / 8, 18, 1})))
       return rc;
-    cudaError_t e = cudaFuncSetAttribute(
+    e = cudaFuncSetAttribute(
         cnn_conv2_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDw2SmemAlone);
     if (e != cudaSuccess)
       return set_error(GBSGMC_ERR_CUDA, "cnn_conv2_dw_kernel: %s", cudaGetErrorString(e));

@@ -139,11 +139,6 @@ int make_tmap_bf16_3d(CUtensorMap* map, const void* base, int64_t cols,
                       int64_t rows, int64_t batch, int64_t row_stride,
                       int64_t batch_stride, int box_cols, int box_rows);
 
-// 4-D BF16 tensor map (dims[0] innermost, strides of dims 1..3 in elements)
-// with a 128-byte swizzled box; dims[0] x 2 bytes of a box row must be 128.
-int make_tmap_bf16_4d(CUtensorMap* map, const void* base, const int64_t (&dims)[4],
-                      const int64_t (&strides)[3], const int (&box)[4]);
-
 // 4-D BF16 tensor map without swizzle (dims[0] innermost, strides of dims
 // 1..3 in elements), for the unswizzled operand layouts: a box row of
 // box[0] BF16 (a multiple of 8) lands as box[0] * 2 contiguous bytes.
@@ -157,25 +152,6 @@ int make_tmap_rows(CUtensorMap* map, const void* base, bool f32, int64_t cols, i
                    int64_t batch, int64_t row_stride, int64_t batch_stride);
 
 size_t gemm_smem_bytes(int bn);
-
-// Operand loaders.  An epilogue type may replace the tiled 3-D loads of the
-// single-CTA GEMM's operands: with `static constexpr bool kLoadA = true` and
-//   load_a(dst, map, k0, m0, b, bar)  (a K-major 128 x 64 A tile)
-// and with `kLoadB = true` and
-//   load_b(dst, map, n, k0, b, bar)   (a B tile: for an MN-major B one
-//                                      64 x 64 block starting at column n,
-//                                      for a K-major B the BN x 64 tile)
-// the producer calls these instead, e.g. to read shifted boxes of an NHWC
-// map for an implicit convolution.  They must load the bytes the default
-// loads would.
-template <class E, class = void>
-struct LoadsA : std::false_type {};
-template <class E>
-struct LoadsA<E, std::void_t<decltype(E::kLoadA)>> : std::bool_constant<E::kLoadA> {};
-template <class E, class = void>
-struct LoadsB : std::false_type {};
-template <class E>
-struct LoadsB<E, std::void_t<decltype(E::kLoadB)>> : std::bool_constant<E::kLoadB> {};
 
 // CTA-pair GEMM (tc_gemm2_kernel): shared-memory ring depth, bytes, and
 // whether it is used where it applies (the GBSGMC_GEMM_PAIR environment
@@ -191,10 +167,6 @@ bool gemm_pair_enabled();
 struct GemmRagged {
   const int* tile_prefix = nullptr;  // [batch + 1], tile_prefix[0] = 0
   const int* kblocks = nullptr;      // [batch]
-  // Split-K (uniform batches only): each output tile is computed as ksplit
-  // partial products over consecutive K ranges by different CTAs; the
-  // epilogue sees batch index b * ksplit + s for split s.
-  int ksplit = 1;
   // Bound of each wait for pipeline progress (a stage's operands, a free
   // stage or accumulator, a finished accumulator).  The waits of the clean-up
   // after a timeout (copies and MMAs already issued) keep kWaitLimitNs.
@@ -293,17 +265,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   pdl_trigger();
   pdl_wait();
   const int tiles_n = N / BN, per_batch = (M / BM) * tiles_n;
-  const int vbatch = batch * rg.ksplit;
   const int tiles = rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + batch)
-                                              : per_batch * vbatch;
-  // (Virtual) batch of tile t, its index within the batch, its K slices and
-  // the first of them.
-  auto decode = [&](int t, int& b, int& r, int& KB, int& kb0) {
+                                              : per_batch * batch;
+  // Batch of tile t, its index within the batch and its K slices.
+  auto decode = [&](int t, int& b, int& r, int& KB) {
     if (rg.reverse) t = tiles - 1 - t;
-    b = ragged_batch(rg, t, per_batch, vbatch);
+    b = ragged_batch(rg, t, per_batch, batch);
     r = t - (rg.tile_prefix != nullptr ? __ldg(rg.tile_prefix + b) : b * per_batch);
-    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK / rg.ksplit;
-    kb0 = (b % rg.ksplit) * KB;
+    KB = rg.kblocks != nullptr ? __ldg(rg.kblocks + b) : K / BK;
   };
 
   if (warp == 0) {
@@ -311,9 +280,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-        int bv, r, KB, kb0;
-        decode(t, bv, r, KB, kb0);
-        const int b = bv / rg.ksplit;
+        int b, r, KB;
+        decode(t, b, r, KB);
         const int m0 = (r / tiles_n) * BM, n0 = (r % tiles_n) * BN;
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % STAGES;
@@ -325,29 +293,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             break;
           }
           mbar_arrive_expect_tx(&full[s], A_BYTES + B_BYTES);
-          const int k0 = (kb0 + kb) * BK;
+          const int k0 = kb * BK;
           if constexpr (A_MN) {
 #pragma unroll
             for (int j = 0; j < BM / 64; ++j)
               tc::tma_load_3d(sa + s * A_BYTES + j * BLOCK_BYTES, &ta, m0 + 64 * j, k0, b,
                               &full[s]);
-          } else if constexpr (LoadsA<Epi>::value) {
-            epi.load_a(sa + s * A_BYTES, &ta, k0, m0, b, &full[s]);
           } else {
             tc::tma_load_3d(sa + s * A_BYTES, &ta, k0, m0, b, &full[s]);
           }
           if constexpr (B_MN) {
 #pragma unroll
-            for (int j = 0; j < BN / 64; ++j) {
-              if constexpr (LoadsB<Epi>::value)
-                epi.load_b(sb + s * B_BYTES + j * BLOCK_BYTES, &tb, n0 + 64 * j, k0, b,
-                           &full[s]);
-              else
-                tc::tma_load_3d(sb + s * B_BYTES + j * BLOCK_BYTES, &tb, n0 + 64 * j, k0, b,
-                                &full[s]);
-            }
-          } else if constexpr (LoadsB<Epi>::value) {
-            epi.load_b(sb + s * B_BYTES, &tb, n0, k0, b, &full[s]);
+            for (int j = 0; j < BN / 64; ++j)
+              tc::tma_load_3d(sb + s * B_BYTES + j * BLOCK_BYTES, &tb, n0 + 64 * j, k0, b,
+                              &full[s]);
           } else {
             tc::tma_load_3d(sb + s * B_BYTES, &tb, k0, n0, b, &full[s]);
           }
@@ -365,8 +324,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       uint32_t it = 0, acc = 0;
       bool ok = true;
       for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x, ++acc) {
-        int b, r, KB, kb0;
-        decode(t, b, r, KB, kb0);
+        int b, r, KB;
+        decode(t, b, r, KB);
         const uint32_t buf = acc & 1u, aph = (acc >> 1) & 1u;
         if (!mbar_wait_bounded(&tempty[buf], aph ^ 1u, abort_flag, rg.wait_ns)) {
           raise_status(status, GBSGMC_ERR_TIMEOUT);
@@ -424,8 +383,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         break;
       }
       tc::fence_after_sync();
-      int b, r, KB, kb0;
-      decode(t, b, r, KB, kb0);
+      int b, r, KB;
+      decode(t, b, r, KB);
       const int row0 = (r / tiles_n) * BM + q * 32;
       const uint32_t tbase =
           tmem + buf * BN + h * NC + (static_cast<uint32_t>(q * 32) << 16);
@@ -469,7 +428,7 @@ int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, int batch, int M,
   if (cudaGetDevice(&dev) != cudaSuccess ||
       cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     return set_error(GBSGMC_ERR_CUDA, "gemm: cannot query the device");
-  const int64_t tiles = static_cast<int64_t>(M / kGemmBM) * (N / BN) * batch * rg.ksplit;
+  const int64_t tiles = static_cast<int64_t>(M / kGemmBM) * (N / BN) * batch;
   const int grid = static_cast<int>(tiles < int64_t(sms) * per_sm ? tiles : int64_t(sms) * per_sm);
   launch_pdl(kern, grid, kGemmThreads, smem, st, ta, tb, M, N, K, batch, status, epi, rg);
   return check_launch("tc_gemm_kernel");
@@ -505,8 +464,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
   constexpr uint32_t BLOCK_BYTES = 64 * BK * 2;  // one 64 x 64 MN-major box
   constexpr uint32_t TMEM_COLS = 2 * BN;
   static_assert(BN == 256, "pair tiles are 256 x 256");
-  static_assert(!LoadsA<Epi>::value && !LoadsB<Epi>::value,
-                "pair tiles take no operand loaders");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
