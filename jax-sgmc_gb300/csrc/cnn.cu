@@ -190,17 +190,31 @@ __device__ __forceinline__ bool conv_wait(uint64_t* bar, uint32_t parity, volati
 __device__ __forceinline__ void route_octet(const float (&g)[8], uint2 mark, uint32_t (&o)[4][4],
                                             float (&val)[8]) {
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const uint32_t m = (e < 2 ? mark.x : mark.y) >> (16 * (e & 1));
-    const __nv_bfloat162 p = __floats2bfloat162_rn((m & 4u) ? g[2 * e] : 0.f,
-                                                   (m & 0x400u) ? g[2 * e + 1] : 0.f);
-    val[2 * e] = __low2float(p);
-    val[2 * e + 1] = __high2float(p);
-    const uint32_t pk = *reinterpret_cast<const uint32_t*>(&p);
+  for (int half = 0; half < 2; ++half) {   // four channels, a word of marks
+    uint32_t pk[2];
 #pragma unroll
-    for (int pos = 0; pos < 4; ++pos)
-      o[pos][e] = pk & (((m & 3u) == static_cast<uint32_t>(pos) ? 0xffffu : 0u) |
-                        (((m >> 8) & 3u) == static_cast<uint32_t>(pos) ? 0xffff0000u : 0u));
+    for (int e = 0; e < 2; ++e) {
+      const __nv_bfloat162 p = __floats2bfloat162_rn(g[4 * half + 2 * e], g[4 * half + 2 * e + 1]);
+      pk[e] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    const uint32_t m = (half ? mark.y : mark.x) & 0x07070707u;
+#pragma unroll
+    for (int pos = 0; pos < 4; ++pos) {
+      // Bit 7 of a byte: its mark is not 4 + pos; spread over the channel's 16
+      // bits by prmt's sign mode.
+      const uint32_t off = (m ^ (0x01010101u * (4 + pos))) + 0x7f7f7f7fu;
+      uint32_t lo, hi;
+      asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(lo) : "r"(off));
+      asm("prmt.b32 %0, %1, 0, 0xbbaa;" : "=r"(hi) : "r"(off));
+      o[pos][2 * half] = pk[0] & ~lo;
+      o[pos][2 * half + 1] = pk[1] & ~hi;
+    }
+#pragma unroll
+    for (int e = 2 * half; e < 2 * half + 2; ++e) {
+      const uint32_t v = o[0][e] | o[1][e] | o[2][e] | o[3][e];
+      val[2 * e] = __uint_as_float(v << 16);
+      val[2 * e + 1] = __uint_as_float(v & 0xffff0000u);
+    }
   }
 }
 
@@ -540,7 +554,7 @@ __global__ void __launch_bounds__(kStripThreads, 4) cnn_conv1_kernel(const CnnAr
 // built.  db1 (another warp): the routed
 // (BF16-rounded) values of a unit's 64 windows are added in window order, a
 // partial per unit.  Grid (splits, chains).
-constexpr int kUnitBuilders = 256, kUnitThreads = kUnitBuilders + 64;
+constexpr int kDyWarps = 8, kWordWarps = 6, kUnitThreads = 32 * (kDyWarps + kWordWarps + 2);
 constexpr int kUnitRow = 3 * 256;   // bytes of a row's E, O and shifted E
 constexpr int kUnitDy = 8 * 2 * 1024, kUnitWords = 11 * kUnitRow, kUnitBias = 64 * 36 * 4;
 constexpr int kUnitBuf = kUnitDy + kUnitWords + kUnitBias;
@@ -557,7 +571,7 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   if (t == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(full + i, kUnitBuilders / 32);
+      mbar_init(full + i, kDyWarps + kWordWarps);
       mbar_init(free_ + i, 2);
     }
     abort_s = 0;
@@ -584,7 +598,7 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
   auto wait = [&](uint64_t* bar, uint32_t parity) {
     return conv_wait(bar, parity, abort_flag, a.status);
   };
-  if (warp == kUnitBuilders / 32) {   // the MMAs
+  if (warp == kDyWarps + kWordWarps) {   // the MMAs
     constexpr uint32_t idesc = tc::idesc_bf16_f32(64, 72, true, true);
     if (tc::elect_one()) {
       for (int u = u0; u < u1; ++u) {
@@ -608,7 +622,7 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
       }
     }
     __syncwarp();
-  } else if (warp > kUnitBuilders / 32) {   // the bias
+  } else if (warp > kDyWarps + kWordWarps) {   // the bias
     for (int u = u0; u < u1; ++u) {
       const int it = u - u0, b = it & 1;
       if (!__all_sync(0xffffffffu, wait(full + b, (it >> 1) & 1u))) break;
@@ -622,75 +636,89 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
       // A unit cut by a split boundary belongs to the split of its first slice.
       if (4 * u >= q0) a.bpart[0][(int64_t(c) * 4 * a.n + u) * kC1 + lane] = sum;
     }
-  } else {
-    // This thread's window (row wy of the unit's 4, column wx) and channels,
-    // and its pixel pair of X8 (rows -1 .. 8 of the unit, 17 pairs a row).
+  } else if (warp < kDyWarps) {
+    // dY: this thread's window (row wy of the unit's 4, column wx) and octet.
     const int j = lane & 7, oct = lane >> 3, wx = 8 * (warp & 1) + j, wy = warp >> 1;
-    const int xr = t / 17, xj = t % 17;
     struct Part {
       float4 g[2];
       uint2 mark;
-      float x[9];
     };
-    auto row_of = [&](int u) { return image_index(a, int64_t(c) * a.n + (u >> 2)); };
-    auto load = [&](int u, int index, Part& p) {
-      const int64_t o = valid_row(a, index);
-      const int64_t img = int64_t(c) * a.n + (u >> 2);
-      const int hb = u & 3;
-      const float4* d = reinterpret_cast<const float4*>(
-          a.dp1 + ((img * 16 + 4 * hb + wy) * 64 + 16 * oct + wx) * 8);
+    auto load = [&](int u, Part& p) {
+      const int64_t row = (int64_t(c) * a.n + (u >> 2)) * 16 + 4 * (u & 3) + wy;
+      const float4* d = reinterpret_cast<const float4*>(a.dp1 + (row * 64 + 16 * oct + wx) * 8);
       p.g[0] = __ldg(d);
       p.g[1] = __ldg(d + 1);
-      p.mark = __ldg(reinterpret_cast<const uint2*>(
-          a.m1 + (img * 256 + (4 * hb + wy) * 16 + wx) * kC1 + 8 * oct));
-      const int h = 8 * hb + xr - 1;
-      const bool in = xr < 10 && h >= 0 && h < kImg && xj < 16;
-      // The 17th pair holds the column past the image: zeros, as at w = -1.
-      pair_load(a.X + o * a.ld + (h * kImg + 2 * xj) * kInC, in, xj > 0, pair, p.x);
+      p.mark = __ldg(reinterpret_cast<const uint2*>(a.m1 + (row * 16 + wx) * kC1 + 8 * oct));
     };
-    // Loads are two units ahead of their use, the observations' indices three.
-    Part part[2];
-    load(u0, row_of(u0), part[0]);
-    if (u0 + 1 < u1) load(u0 + 1, row_of(u0 + 1), part[1]);
-    int next = u0 + 2 < u1 ? row_of(u0 + 2) : 0;
     auto unit = [&](int u, Part& p) -> bool {
       const int it = u - u0, b = it & 1;
       uint8_t* dy = unit_smem + b * kUnitBuf;
-      uint8_t* words = dy + kUnitDy;
-      float* bias = reinterpret_cast<float*>(words + kUnitWords);
+      float* bias = reinterpret_cast<float*>(dy + kUnitDy + kUnitWords);
       if (it >= 2 && !__all_sync(0xffffffffu, wait(free_ + b, ((it >> 1) - 1) & 1u))) return false;
-      if (xr < 10) {
-        uint4 e, o;
-        pair_words(p.x, e, o);
-        uint8_t* at = words + xr * kUnitRow + 16 * xj;
-        if (xj < 16) {
-          store_word(at, e);
-          store_word(at + 256, o);
-        }
-        if (xj > 0) store_word(at + 512 - 16, e);
-      }
-      {
-        const float4 &g0 = p.g[0], &g1 = p.g[1];
+      const float4 &g0 = p.g[0], &g1 = p.g[1];
       const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
       uint32_t o[4][4];
       float val[8];
       route_octet(g, p.mark, o, val);
-      float4* bd = reinterpret_cast<float4*>(bias + (16 * wy + wx) * 36 + 8 * oct);
-      bd[0] = make_float4(val[0], val[1], val[2], val[3]);
-      bd[1] = make_float4(val[4], val[5], val[6], val[7]);
 #pragma unroll
       for (int pos = 0; pos < 4; ++pos)
         tc::sts128(dy + ((2 * wy + (pos >> 1)) * 2 + (warp & 1)) * 1024 + (pos & 1) * 512 +
                        16 * lane,
                    o[pos][0], o[pos][1], o[pos][2], o[pos][3]);
+      float4* bd = reinterpret_cast<float4*>(bias + (16 * wy + wx) * 36 + 8 * oct);
+      bd[0] = make_float4(val[0], val[1], val[2], val[3]);
+      bd[1] = make_float4(val[4], val[5], val[6], val[7]);
+      tc::fence_async_shared();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + b);
+      if (u + 2 < u1) load(u + 2, p);
+      return true;
+    };
+    Part part[2];   // loads are two units ahead of their use
+    load(u0, part[0]);
+    if (u0 + 1 < u1) load(u0 + 1, part[1]);
+    for (int u = u0; u < u1; u += 2) {
+      if (!unit(u, part[0])) break;
+      if (u + 1 < u1 && !unit(u + 1, part[1])) break;
+    }
+  } else {
+    // X8: this thread's pixel pair (rows -1 .. 8 of the unit, 17 pairs a row;
+    // the last holds the column past the image: zeros, as at w = -1).
+    const int e = t - 32 * kDyWarps, xr = e / 17, xj = e % 17;
+    struct Pair {
+      float x[9];
+    };
+    auto row_of = [&](int u) { return image_index(a, int64_t(c) * a.n + (u >> 2)); };
+    auto load = [&](int u, int index, Pair& p) {
+      const int h = 8 * (u & 3) + xr - 1;
+      const bool in = xr < 10 && h >= 0 && h < kImg && xj < 16;
+      pair_load(a.X + valid_row(a, index) * a.ld + (h * kImg + 2 * xj) * kInC, in, xj > 0, pair,
+                p.x);
+    };
+    Pair part[2];
+    load(u0, row_of(u0), part[0]);
+    if (u0 + 1 < u1) load(u0 + 1, row_of(u0 + 1), part[1]);
+    int next = u0 + 2 < u1 ? row_of(u0 + 2) : 0;   // indices a unit further ahead
+    auto unit = [&](int u, Pair& p) -> bool {
+      const int it = u - u0, b = it & 1;
+      uint8_t* at = unit_smem + b * kUnitBuf + kUnitDy + xr * kUnitRow + 16 * xj;
+      if (it >= 2 && !__all_sync(0xffffffffu, wait(free_ + b, ((it >> 1) - 1) & 1u))) return false;
+      if (xr < 10) {
+        uint4 even, odd;
+        pair_words(p.x, even, odd);
+        if (xj < 16) {
+          store_word(at, even);
+          store_word(at + 256, odd);
+        }
+        if (xj > 0) store_word(at + 512 - 16, even);
       }
       tc::fence_async_shared();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + b);
       if (u + 2 < u1) {
         load(u + 2, next, p);
         if (u + 3 < u1) next = row_of(u + 3);
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(full + b);
       return true;
     };
     for (int u = u0; u < u1; u += 2) {
@@ -1659,11 +1687,18 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
   float* g = a.grad + static_cast<int64_t>(c) * kP;
   const float* gl = a.gl + static_cast<int64_t>(c) * a.n * kClasses;
   if (blockIdx.x == kFlat / 128) {
-    if (t < kClasses) {
-      float s = 0.f;
-      for (int i = 0; i < a.n; ++i) s += gl[i * kClasses + t];
-      g[obd + t] = s;
+    float s = 0.f;
+    for (int i0 = 0; i0 < a.n; i0 += 512) {
+      const int cnt = min(512, a.n - i0);
+      __syncthreads();
+      for (int e = t; e < cnt * kClasses; e += 512) gs[e] = gl[i0 * kClasses + e];
+      __syncthreads();
+      if (t < kClasses) {
+#pragma unroll 16
+        for (int i = 0; i < cnt; ++i) s += gs[i * kClasses + t];
+      }
     }
+    if (t < kClasses) g[obd + t] = s;
     return;
   }
   const int f = blockIdx.x * 128 + (t & 127);
@@ -1677,12 +1712,12 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
     for (int e = t; e < cnt * kClasses; e += 512) gs[e] = gl[i0 * kClasses + e];
     __syncthreads();
     int i = q;
-    for (; i + 12 < cnt; i += 16) {
-      float xv[4];
+    for (; i + 28 < cnt; i += 32) {
+      float xv[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) xv[u] = bf(x[static_cast<int64_t>(i0 + i + 4 * u) * kFlat]);
+      for (int u = 0; u < 8; ++u) xv[u] = bf(x[static_cast<int64_t>(i0 + i + 4 * u) * kFlat]);
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < 8; ++u)
 #pragma unroll
         for (int k = 0; k < kClasses; ++k)
           acc[k] = fmaf(xv[u], gs[(i + 4 * u) * kClasses + k], acc[k]);
