@@ -335,25 +335,32 @@ __device__ __forceinline__ void strip_borders(uint8_t* smem) {
 // and part `b` of a chain's sum
 // of squares.
 __device__ __forceinline__ void cnn_prep(const CnnArgs& a, int c, int b, double* red) {
-  constexpr int kCols = 256, kEach = kCols / kStripThreads;
+  constexpr int kCols = 256, kEach = kCols / kStripThreads, kStride = kPrepBlocks * kCols;
+  constexpr int kRounds = static_cast<int>((kP + kStride - 1) / kStride);
   const float* w = a.w + static_cast<int64_t>(c) * kP;
-  float sq[kEach] = {};
-  for (int i = b * kCols + threadIdx.x; i < kP; i += kPrepBlocks * kCols) {
+  float sq[kEach] = {}, v[kRounds][kEach];
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
 #pragma unroll
     for (int u = 0; u < kEach; ++u) {
-      const int j = i + u * kStripThreads;
-      if (j >= kP) break;
-      const float v = __ldg(w + j);
-      sq[u] = fmaf(v, v, sq[u]);
+      const int j = b * kCols + threadIdx.x + r * kStride + u * kStripThreads;
+      v[r][u] = j < kP ? __ldg(w + j) : 0.f;
+    }
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+    for (int u = 0; u < kEach; ++u) {
+      const int j = b * kCols + threadIdx.x + r * kStride + u * kStripThreads;
+      const float x = v[r][u];
+      if (j < kP) sq[u] = fmaf(x, x, sq[u]);
       if (j >= oW2 && j < ob3)
         a.w2b[static_cast<int64_t>(c) * kK2 * kC2 +
-              ((j - oW2) % kC2 / 8 * kK2 + (j - oW2) / kC2) * 8 + j % 8] = __float2bfloat16_rn(v);
+              ((j - oW2) % kC2 / 8 * kK2 + (j - oW2) / kC2) * 8 + j % 8] = __float2bfloat16_rn(x);
       else if (j >= oW3 && j < obd)
         a.w3b[static_cast<int64_t>(c) * kK3 * kC3 +
               (((j - oW3) / kC3 / kC2 * (kC3 / 8) + (j - oW3) % kC3 / 8) * kC2 +
-               (j - oW3) / kC3 % kC2) * 8 + (j - oW3) % 8] = __float2bfloat16_rn(v);
+               (j - oW3) / kC3 % kC2) * 8 + (j - oW3) % 8] = __float2bfloat16_rn(x);
     }
-  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int u = 0; u < kEach; ++u) {
@@ -427,15 +434,19 @@ __global__ void __launch_bounds__(kStripThreads, 4) cnn_conv1_kernel(const CnnAr
   pdl_trigger();
   pdl_wait();
 
+  // CTAs past the strips' prepare weights alone; without such, all do.
   const int64_t strips = 2 * static_cast<int64_t>(a.chains) * a.n;
-  const int64_t u0 = strips * blockIdx.x / gridDim.x, u1 = strips * (blockIdx.x + 1) / gridDim.x;
+  const int own = strips < gridDim.x ? static_cast<int>(strips) : gridDim.x;
+  const int b = blockIdx.x;
+  const int64_t u0 = b < own ? strips * b / own : 0, u1 = b < own ? strips * (b + 1) / own : 0;
+  const int preps = gridDim.x > own ? gridDim.x - own : own;
   StripRegs x;
   int next = 0;   // index of the strip after the loaded one
   if (u0 < u1) {
     strip_load(a, image_index(a, u0 >> 1), static_cast<int>(u0 & 1), pair, x);
     if (u0 + 1 < u1) next = image_index(a, (u0 + 1) >> 1);
   }
-  for (int e = blockIdx.x; e < a.chains * kPrepBlocks; e += gridDim.x)
+  for (int e = preps == own ? b : b - own; e >= 0 && e < a.chains * kPrepBlocks; e += preps)
     cnn_prep(a, e / kPrepBlocks, e % kPrepBlocks, red);
 
   constexpr uint32_t idesc = tc::idesc_bf16_f32(128, kC1);
@@ -1520,37 +1531,34 @@ __global__ void __launch_bounds__(kDw3Threads, 1)
 // ---------------------------------------------------------------------------
 // Dense layer, softmax likelihood and its adjoint for kImgs images of a chain
 // per block.  Writes lk, dlogits g = dU/dlogits (fp32), dP3 = g Wd^T and the
-// per-image likelihood terms.  Grid (ceil(n / kImgs), chains), kParts x 16
-// threads per image: thread (class part p, image j, slice s) handles the
-// features f = s, s + 16, ... of 10 / kParts classes; the 16 threads of a part
-// are one half-warp and reduce by shuffles.  The block first copies Wd (80 KB)
-// and its images' P3 rows (4 KB each) into shared memory with all loads in
-// flight: a half-warp then reads 16 Wd rows 40 bytes apart, 16 distinct banks
-// (the other half-warp the same words), and 16 consecutive P3 features.
-// Few images leave most SMs without a block of 16, so blocks take 4 then, and
-// more parts: what a block takes is the latency of its loads and of 128
-// dependent steps a thread.
+// per-image likelihood terms.  Grid (ceil(n / kImgs), chains), 80 threads per
+// kPer images: thread (class pair p, images j, slice s) handles the features
+// f = s, s + 16, ... of two classes; the 16 threads of a pair are one
+// half-warp and reduce by shuffles.  The block first copies Wd (80 KB) and its
+// images' P3 rows (4 KB each) into shared memory with all loads in flight: a
+// half-warp then reads 8 bytes of 16 Wd rows 40 bytes apart, 32 distinct banks,
+// and 16 consecutive P3 features of each image.  Shared memory's words are the
+// limit: kPer images share what is read of Wd.
+// Few images leave most SMs without a block of 16, so blocks take 4 then, one
+// a thread: what a block takes is the latency of its loads and of 128 steps.
 // ---------------------------------------------------------------------------
 static_assert(oWd % 2 == 0 && kP % 2 == 0, "Wd is copied as float2");
 constexpr size_t dense_smem(int imgs) {
   return sizeof(float) * kFlat * kClasses + sizeof(bf16) * imgs * kFlat;
 }
 
-template <int kDenseImgs, int kParts>
-__global__ void __launch_bounds__(kDenseImgs * kParts * 16)
+template <int kDenseImgs, int kPer>
+__global__ void __launch_bounds__(kDenseImgs / kPer * 80)
     cnn_dense_kernel(const CnnArgs a, float scale) {
   pdl_trigger();
   pdl_wait();
-  constexpr int kDenseThreads = kDenseImgs * kParts * 16, kEach = kClasses / kParts;
-  static_assert(kEach * kParts == kClasses, "whole classes");
-  extern __shared__ float wd_s[];  // Wd [2048][10], then P3 rows [kDenseImgs][2048]
+  constexpr int kSets = kDenseImgs / kPer, kDenseThreads = kSets * 80;
+  extern __shared__ __align__(16) float wd_s[];  // Wd [2048][10], then P3 rows [kDenseImgs][2048]
   bf16* x_s = reinterpret_cast<bf16*>(wd_s + kFlat * kClasses);
-  __shared__ float g_s[kDenseImgs][kClasses];   // logits, then their adjoints
+  __shared__ __align__(8) float g_s[kDenseImgs][kClasses];   // logits, then their adjoints
   const unsigned full = 0xffffffffu;
   const int c = blockIdx.y, t = threadIdx.x;
-  const int part = t / (kDenseImgs * 16), j = (t >> 4) % kDenseImgs, sl = t & 15;
-  const int i = blockIdx.x * kDenseImgs + j;
-  const bool live = i < a.n;
+  const int part = t / (kSets * 16), set = (t >> 4) % kSets, sl = t & 15;
   const float* w = a.w + static_cast<int64_t>(c) * kP;
   {
     // oWd and kP are even: the chain's Wd starts 8-byte aligned.
@@ -1570,29 +1578,32 @@ __global__ void __launch_bounds__(kDenseImgs * kParts * 16)
   }
   __syncthreads();
   {
-    const bf16* x = x_s + j * kFlat;
-    float acc[kEach];
-#pragma unroll
-    for (int k = 0; k < kEach; ++k) acc[k] = 0.f;
+    const bf16* x = x_s + set * kPer * kFlat;
+    float acc[kPer][2] = {};
 #pragma unroll 8
     for (int f = sl; f < kFlat; f += 16) {
-      const float xv = live ? bf(x[f]) : 0.f;
-      const float* wr = wd_s + f * kClasses + part * kEach;
+      const float2 wr = *reinterpret_cast<const float2*>(wd_s + f * kClasses + 2 * part);
 #pragma unroll
-      for (int k = 0; k < kEach; ++k) acc[k] = fmaf(xv, wr[k], acc[k]);
+      for (int r = 0; r < kPer; ++r) {   // rows past n are not set: their sums go nowhere
+        const float xv = bf(x[r * kFlat + f]);
+        acc[r][0] = fmaf(xv, wr.x, acc[r][0]);
+        acc[r][1] = fmaf(xv, wr.y, acc[r][1]);
+      }
     }
 #pragma unroll
-    for (int k = 0; k < kEach; ++k)
+    for (int r = 0; r < kPer; ++r)
 #pragma unroll
-      for (int off = 8; off > 0; off >>= 1) acc[k] += __shfl_xor_sync(full, acc[k], off);
-    if (sl == 0) {
+      for (int k = 0; k < 2; ++k) {
 #pragma unroll
-      for (int k = 0; k < kEach; ++k)
-        g_s[j][part * kEach + k] = acc[k] + __ldg(w + obd + part * kEach + k);
-    }
+        for (int off = 8; off > 0; off >>= 1)
+          acc[r][k] += __shfl_xor_sync(full, acc[r][k], off);
+        if (sl == 0)
+          g_s[set * kPer + r][2 * part + k] = acc[r][k] + __ldg(w + obd + 2 * part + k);
+      }
   }
   __syncthreads();
-  if (part == 0 && sl == 0 && live) {
+  const int j = t, i = blockIdx.x * kDenseImgs + j;
+  if (j < kDenseImgs && i < a.n) {
     float logit[kClasses], mx = -INFINITY;
 #pragma unroll
     for (int k = 0; k < kClasses; ++k) {
@@ -1622,19 +1633,32 @@ __global__ void __launch_bounds__(kDenseImgs * kParts * 16)
   }
   if (!a.want_grad) return;
   __syncthreads();
-  // dP3 rows of the block's images: thread t takes the features t, t + 256, ...
+  // dP3 rows of the block's images, two features of a thread at a time.
   const int rows = min(kDenseImgs, a.n - static_cast<int>(blockIdx.x) * kDenseImgs);
   float* dx = a.dp3 + (static_cast<int64_t>(c) * a.n + blockIdx.x * kDenseImgs) * kFlat;
+  for (int f0 = t; f0 < kFlat; f0 += 2 * kDenseThreads) {
+    const int f1 = f0 + kDenseThreads < kFlat ? f0 + kDenseThreads : f0;
+    float2 wr[2][kClasses / 2];
+#pragma unroll
+    for (int k = 0; k < kClasses / 2; ++k) {
+      wr[0][k] = reinterpret_cast<const float2*>(wd_s + f0 * kClasses)[k];
+      wr[1][k] = reinterpret_cast<const float2*>(wd_s + f1 * kClasses)[k];
+    }
 #pragma unroll 2
-  for (int f = t; f < kFlat; f += kDenseThreads) {
-    float wr[kClasses];
-#pragma unroll
-    for (int k = 0; k < kClasses; ++k) wr[k] = wd_s[f * kClasses + k];
     for (int r = 0; r < rows; ++r) {
-      float sum = 0.f;
+      const float2* g = reinterpret_cast<const float2*>(g_s[r]);
+      float sum[2] = {0.f, 0.f};
 #pragma unroll
-      for (int k = 0; k < kClasses; ++k) sum = fmaf(g_s[r][k], wr[k], sum);
-      dx[static_cast<int64_t>(r) * kFlat + f] = sum;
+      for (int k = 0; k < kClasses / 2; ++k) {
+        const float2 gv = g[k];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          sum[u] = fmaf(gv.x, wr[u][k].x, sum[u]);
+          sum[u] = fmaf(gv.y, wr[u][k].y, sum[u]);
+        }
+      }
+      dx[static_cast<int64_t>(r) * kFlat + f0] = sum[0];
+      dx[static_cast<int64_t>(r) * kFlat + f1] = sum[1];
     }
   }
 }
@@ -1653,7 +1677,7 @@ constexpr int kDenseGradBlocks = kFlat / 128 + 1;
 __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
   pdl_trigger();
   pdl_wait();
-  __shared__ float smem[512 * kClasses + 3 * 128 * kClasses];
+  __shared__ __align__(16) float smem[512 * kClasses + 3 * 128 * kClasses];
   const int c = blockIdx.y, t = threadIdx.x;
   if (blockIdx.x >= kDenseGradBlocks) {
     float* red = smem + (t >> 8) * 2048;
@@ -1719,8 +1743,11 @@ __global__ void __launch_bounds__(512) cnn_dense_grad_kernel(const CnnArgs a) {
 #pragma unroll
       for (int u = 0; u < 8; ++u)
 #pragma unroll
-        for (int k = 0; k < kClasses; ++k)
-          acc[k] = fmaf(xv[u], gs[(i + 4 * u) * kClasses + k], acc[k]);
+        for (int k = 0; k < kClasses; k += 2) {   // rows of 40 bytes
+          const float2 gv = *reinterpret_cast<const float2*>(gs + (i + 4 * u) * kClasses + k);
+          acc[k] = fmaf(xv[u], gv.x, acc[k]);
+          acc[k + 1] = fmaf(xv[u], gv.y, acc[k + 1]);
+        }
     }
     for (; i < cnt; i += 4) {
       const float xv = bf(x[static_cast<int64_t>(i0 + i) * kFlat]);
@@ -1895,7 +1922,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   const int pair = reinterpret_cast<uintptr_t>(a.X) % 8 == 0 && a.ld % 2 == 0;
   launch_pdl(cnn_conv1_kernel,
              static_cast<int>(std::min<int64_t>(
-                 4 * sms, std::max<int64_t>(2 * int64_t(C) * n, int64_t(C) * kPrepBlocks))),
+                 4 * sms, 2 * int64_t(C) * n + int64_t(C) * kPrepBlocks)),
              kStripThreads, 0, st, a, pair);
   if ((rc = launched("cnn_conv1_kernel"))) return rc;
 
@@ -1934,18 +1961,18 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
   if ((rc = conv3(cnn_conv3_kernel<kC2, kC3, EpiPairPool>, conv3_smem<kC2, EpiPairPool>(), m_p2,
                   EpiPairPool{a.w, a.p3, a.m3})))
     return rc;
-  const auto dense = [&](auto kern, int imgs, int parts) {
+  const auto dense = [&](auto kern, int imgs, int per) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(dense_smem(imgs)));
     if (e != cudaSuccess)
       return set_error(GBSGMC_ERR_CUDA, "cnn_dense_kernel: %s", cudaGetErrorString(e));
     const float scale = static_cast<float>(static_cast<double>(a.n_obs) / n / a.temperature);
-    launch_pdl(kern, dim3(ceil_div(n, imgs), C), 16 * imgs * parts, dense_smem(imgs), st, a, scale);
+    launch_pdl(kern, dim3(ceil_div(n, imgs), C), imgs / per * 80, dense_smem(imgs), st, a, scale);
     return launched("cnn_dense_kernel");
   };
   // Sixteen images share a block's copy of Wd once that fills the SMs.
   rc = int64_t(C) * n >= 16 * 152 / 2 ? dense(cnn_dense_kernel<16, 2>, 16, 2)
-                                      : dense(cnn_dense_kernel<4, 5>, 4, 5);
+                                      : dense(cnn_dense_kernel<4, 1>, 4, 1);
   if (rc) return rc;
 
   if (a.want_grad) {
