@@ -90,7 +90,8 @@ int glm_sgld_step(const gbsgmc_glm* model, int chains, int n,
 // step's samples.  Pair p's uniform is Philox(counter (0, k + 1), key
 // (seed << 32) | pair_chain[p]).
 // The MLP's value and gradient (gbsgmc_mlp_value_and_grad) where row c of
-// the batch reads its minibatch from row ident_dev[c] of idx.
+// the batch reads its minibatch from row ident_dev[c] of idx; the prior's
+// gradient is left to the update.
 int mlp_value_and_grad_ident(const gbsgmc_mlp* model, int chains, int n, const int32_t* idx,
                              int64_t idx_stride, const int32_t* ident_dev, const float* w,
                              double* U, float* grad, double* lk_var, void* ws, size_t ws_bytes,
@@ -154,9 +155,11 @@ int mirror_fused(int chains, int64_t P, const float* x, const UpdateFusion& f,
 // gradient left to the update.
 int mlp_mirror_region(const gbsgmc_mlp* model, int chains, int n, void* ws,
                       void** mirror, int64_t* count, int64_t* stride);
+// Without sq_parts the call sums the squares (and converts the weights) itself;
+// n_dev: a ragged batch's rows, or null.
 int mlp_value_and_grad_fused(const gbsgmc_mlp* model, int chains, int n,
-                             const int32_t* idx, int64_t idx_stride, const float* w,
-                             double* U, float* grad, double* lk_var, void* ws,
+                             const int32_t* n_dev, const int32_t* idx, int64_t idx_stride,
+                             const float* w, double* U, float* grad, double* lk_var, void* ws,
                              size_t ws_bytes, int* status, cudaStream_t st,
                              const double* sq_parts, int sq_count);
 

@@ -207,9 +207,9 @@ struct MlpArgs {
   const int32_t* n_true;
   // Row c of the batch reads its minibatch from row ident[c] of idx (null: c).
   const int32_t* ident;
-  // Fused with the integrator: the BF16 weights and the sums of squares
-  // (sq_count per chain in psq) are supplied, the prior's gradient is the
-  // update's.
+  // Fused with the integrator: the prior's gradient is the update's, and with
+  // sq_count > 0 the BF16 weights and the sums of squares (sq_count per chain
+  // in psq) are supplied.
   int fused, sq_count;
   // Fisher noise model: the adjoint is the likelihood's (grad receives
   // sum_i d_i), grad_sq receives sum_i d_i^2.
@@ -714,9 +714,43 @@ __global__ void __launch_bounds__(256, kFisher ? 2 : 3) mlp_out_kernel(const Mlp
 }
 
 // ---------------------------------------------------------------------------
-// 9. Bias and output-layer gradients, U and var(lk).  Grid
-//    (ceil(max(H1,H2)/256), chains) with a gradient, (1, chains) without.
+// 9. Bias and output-layer gradients, U and var(lk).  Grid (ceil(H1/256) +
+//    ceil(H2/256) + 1, chains) with a gradient, (1, chains) without: blocks of
+//    the first layer's columns, of the second's, and one of the values, whose
+//    loads would otherwise follow one another (64 chains of 2,048 rows: 22 ->
+//    11 us behind the last GEMM).
 // ---------------------------------------------------------------------------
+// Adds rows r .. of a column of partials (ld apart) in order, K loads in
+// flight, while K are left before n.
+template <int K>
+__device__ __forceinline__ void add_rows(float& acc, const float* p, int& r, int n, int64_t ld) {
+  for (; r + K <= n; r += K) {
+    float v[K];
+#pragma unroll
+    for (int u = 0; u < K; ++u) v[u] = p[(r + u) * ld];
+#pragma unroll
+    for (int u = 0; u < K; ++u) acc += v[u];
+  }
+}
+// Of two columns.
+template <int K>
+__device__ __forceinline__ void add_rows(float& acc, float& acc2, const float* p, const float* p2,
+                                         int& r, int n, int64_t ld) {
+  for (; r + K <= n; r += K) {
+    float v[K], v2[K];
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      v[u] = p[(r + u) * ld];
+      v2[u] = p2[(r + u) * ld];
+    }
+#pragma unroll
+    for (int u = 0; u < K; ++u) {
+      acc += v[u];
+      acc2 += v2[u];
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int nprep) {
   pdl_trigger();
   pdl_wait();
@@ -730,12 +764,15 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
   const int nb64 = npad / kTile, nb32 = npad / 32;
   if (a.want_grad) {
     float* g = a.grad + static_cast<int64_t>(c) * s.P;
-    const int j = blockIdx.x * 256 + t;
-    if (j < s.H1) {
+    const int blocks1 = (s.H1 + 255) / 256, bx = blockIdx.x;
+    const int j = (bx < blocks1 ? bx : bx - blocks1) * 256 + t;
+    if (bx < blocks1 && j < s.H1) {
       const float* p = a.pb1 + static_cast<int64_t>(c) * (a.n / 32) * s.H1 + j;
       float acc = 0.f;
-#pragma unroll 16
-      for (int r = 0; r < nb32; ++r) acc += p[static_cast<int64_t>(r) * s.H1];
+      int r = 0;
+      add_rows<32>(acc, p, r, nb32, s.H1);
+      add_rows<8>(acc, p, r, nb32, s.H1);
+      add_rows<1>(acc, p, r, nb32, s.H1);
       g[s.ob1 + j] = fmaf(pf, __ldg(w + s.ob1 + j), acc);
       if (a.fisher) {
         const float* q = a.pb1sq + static_cast<int64_t>(c) * (a.n / kTile) * s.H1 + j;
@@ -744,14 +781,13 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
         a.grad_sq[static_cast<int64_t>(c) * s.P + s.ob1 + j] = sq;
       }
     }
-    if (j < s.H2) {
+    if (bx >= blocks1 && bx + 1 < static_cast<int>(gridDim.x) && j < s.H2) {
       const int64_t base = static_cast<int64_t>(c) * (a.n / kTile) * s.H2 + j;
       float acc2 = 0.f, acc3 = 0.f;
-#pragma unroll 8
-      for (int r = 0; r < nb64; ++r) {
-        acc2 += a.pb2[base + static_cast<int64_t>(r) * s.H2];
-        acc3 += a.pw3[base + static_cast<int64_t>(r) * s.H2];
-      }
+      int r = 0;
+      add_rows<16>(acc2, acc3, a.pb2 + base, a.pw3 + base, r, nb64, s.H2);
+      add_rows<4>(acc2, acc3, a.pb2 + base, a.pw3 + base, r, nb64, s.H2);
+      add_rows<1>(acc2, acc3, a.pb2 + base, a.pw3 + base, r, nb64, s.H2);
       g[s.ob2 + j] = fmaf(pf, __ldg(w + s.ob2 + j), acc2);
       g[s.oW3 + j] = fmaf(pf, __ldg(w + s.oW3 + j), acc3);
       if (a.fisher) {
@@ -765,7 +801,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
       }
     }
   }
-  if (blockIdx.x != 0) return;
+  if (blockIdx.x + 1 != gridDim.x) return;
   // Five FP64 sums, a warp each: as block-wide sums one after the other they
   // held the launch (64 chains of 2,048 rows: 28.8 -> 13.8 us, with the
   // column loads above in flight together).
@@ -773,6 +809,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
   if (warp < 5) {
     double v = 0.0;
     if (warp == 0) {
+#pragma unroll 8
       for (int i = lane; i < nprep; i += 32) v += a.psq[static_cast<int64_t>(c) * nprep + i];
     } else {
       const double* p = a.plk + static_cast<int64_t>(c) * (a.n / kTile) * 4 + (warp - 1);
@@ -961,7 +998,7 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
   a.pw3 = view<float>(ws, L.pw3);
   a.pb2 = view<float>(ws, L.pb2);
   a.pb1 = view<float>(ws, L.pb1);
-  if (!a.fused) a.psq = view<double>(ws, L.psq);
+  if (a.sq_count == 0) a.psq = view<double>(ws, L.psq);
   a.plk = view<double>(ws, L.plk);
   if (a.fisher) {
     a.sqa = view<bf16>(ws, L.sqa);
@@ -999,12 +1036,12 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
     ksl.kblocks = a.kblocks;
   }
   const int64_t pw = matrix_params(s);
-  const int nprep = a.fused ? a.sq_count : prep_blocks(s);
+  const int nprep = a.sq_count > 0 ? a.sq_count : prep_blocks(s);
   const bf16* w1b = a.wb;
   const bf16* w2b = a.wb + s.oW2;
   int rc;
 
-  if (!a.fused) {
+  if (a.sq_count == 0) {
     launch_pdl(mlp_prep_kernel, dim3(nprep, C), 256, 0, st, a);
     if ((rc = check_launch("mlp_prep_kernel")) != GBSGMC_OK) return rc;
   }
@@ -1103,7 +1140,7 @@ int run_mlp(MlpArgs& a, const MlpLayout& L, void* ws, cudaStream_t st) {
         return rc;
     }
   }
-  const int fx = a.want_grad ? ceil_div(H1 > H2 ? H1 : H2, 256) : 1;
+  const int fx = a.want_grad ? ceil_div(H1, 256) + ceil_div(H2, 256) + 1 : 1;
   launch_pdl(mlp_finalize_kernel, dim3(fx, C), 256, 0, st, a, nprep);
   return check_launch("mlp_finalize_kernel");
 }
@@ -1132,7 +1169,7 @@ int mlp_call(const gbsgmc_mlp* model, int chains, int n, const int32_t* n_dev,
              const float* w_dev, double* U_dev, float* grad_dev, float* lk_dev,
              double* lk_var_dev, void* workspace_dev, size_t workspace_bytes,
              int* status_dev, gbsgmc_stream_t stream, const double* sq_parts = nullptr,
-             int sq_count = 0, const int32_t* ident_dev = nullptr) {
+             int sq_count = 0, const int32_t* ident_dev = nullptr, bool prior_apart = false) {
   int rc = check_model(model, "mlp_value_and_grad");
   if (rc != GBSGMC_OK) return rc;
   if (chains < 0 || n < 0)
@@ -1180,7 +1217,7 @@ int mlp_call(const gbsgmc_mlp* model, int chains, int n, const int32_t* n_dev,
   a.status = status_dev;
   a.n_true = n_dev;
   a.ident = ident_dev;
-  a.fused = sq_parts != nullptr ? 1 : 0;
+  a.fused = prior_apart || sq_parts != nullptr ? 1 : 0;
   a.sq_count = sq_count;
   a.psq = const_cast<double*>(sq_parts);
   return run_mlp(a, L, workspace_dev, static_cast<cudaStream_t>(stream));
@@ -1206,17 +1243,18 @@ int mlp_value_and_grad_ident(const gbsgmc_mlp* model, int chains, int n, const i
                              int* status, cudaStream_t st) {
   if (ident_dev == nullptr) return set_error(GBSGMC_ERR_ARG, "mlp (identities): null map");
   return mlp_call(model, chains, n, nullptr, idx, idx_stride, nullptr, w, U, grad, nullptr,
-                  lk_var, ws, ws_bytes, status, st, nullptr, 0, ident_dev);
+                  lk_var, ws, ws_bytes, status, st, nullptr, 0, ident_dev, true);
 }
 
-int mlp_value_and_grad_fused(const gbsgmc_mlp* model, int chains, int n, const int32_t* idx,
-                             int64_t idx_stride, const float* w, double* U, float* grad,
-                             double* lk_var, void* ws, size_t ws_bytes, int* status,
-                             cudaStream_t st, const double* sq_parts, int sq_count) {
-  if (sq_parts == nullptr || sq_count < 1)
+int mlp_value_and_grad_fused(const gbsgmc_mlp* model, int chains, int n,
+                             const int32_t* n_dev, const int32_t* idx, int64_t idx_stride,
+                             const float* w, double* U, float* grad, double* lk_var, void* ws,
+                             size_t ws_bytes, int* status, cudaStream_t st,
+                             const double* sq_parts, int sq_count) {
+  if (sq_parts != nullptr && sq_count < 1)
     return set_error(GBSGMC_ERR_ARG, "mlp (fused): missing sums of squares");
-  return mlp_call(model, chains, n, nullptr, idx, idx_stride, nullptr, w, U, grad, nullptr,
-                  lk_var, ws, ws_bytes, status, st, sq_parts, sq_count);
+  return mlp_call(model, chains, n, n_dev, idx, idx_stride, nullptr, w, U, grad, nullptr,
+                  lk_var, ws, ws_bytes, status, st, sq_parts, sq_count, nullptr, true);
 }
 
 }  // namespace gbsgmc

@@ -293,6 +293,13 @@ int NetPlan::enqueue_obabo(int g, const UpdateFusion& moving, const UpdateFusion
   return check_launch("plan: potential mean");
 }
 
+// 1 / (s^2 T) of the prior, 0 for a flat one, as the gradient's kernels take it.
+float prior_factor(const gbsgmc_mlp& m) {
+  if (!(m.prior_scale > 0.f)) return 0.f;
+  return static_cast<float>(1.0 /
+                            (static_cast<double>(m.prior_scale) * m.prior_scale * m.temperature));
+}
+
 // reSGLD over R replicas with ragged minibatches and adjacent exchanges.
 struct ResgldPlan final : gbsgmc_plan {
   GradFn grad_fn;
@@ -315,6 +322,8 @@ struct ResgldPlan final : gbsgmc_plan {
   int32_t* idx = nullptr;  // owned [G, R, n_max]
   void* ws = nullptr;      // owned
   size_t ws_size = 0;
+  float pf = 0.f;          // the prior's 1 / (s^2 T), added by the update: the
+                           // gradient's epilogues then read no weights
 
   ~ResgldPlan() override {
     if (stream != nullptr) cudaStreamSynchronize(stream);
@@ -349,8 +358,10 @@ struct ResgldPlan final : gbsgmc_plan {
       gbsgmc_sched step_sched = sj;
       step_sched.keep_slot_dev = nullptr;  // kept samples are taken after the exchange
       if ((rc = grad_fn(idx + j * cn, n_max, U, lk_var, grad, s))) return rc;
-      if ((rc = gbsgmc_sgld_update(replicas, P, x, grad, v, alpha, lmbd, &step_sched, &noise,
-                                   nullptr, s)))
+      UpdateFusion with_prior;
+      with_prior.prior_pf = pf;
+      if ((rc = sgld_update_fused(replicas, P, x, grad, v, alpha, lmbd, &step_sched, &noise,
+                                  with_prior, s)))
         return rc;
       if ((rc = gbsgmc_resgld_sa_update(replicas, lk_var, temp.ssq_dev, temp.k_dev, s)))
         return rc;
@@ -415,6 +426,7 @@ struct MlpPairsPlan final : gbsgmc_plan {
     if (rc != GBSGMC_OK) return rc;
     UpdateFusion by_identity;
     by_identity.ident = ident;
+    by_identity.prior_pf = prior_factor(model);
     for (int j = 0; j < g; ++j) {
       gbsgmc_sched sj = sched;
       sj.base_dev = base;
@@ -517,15 +529,13 @@ extern "C" int gbsgmc_mlp_plan_create(gbsgmc_plan** out, const gbsgmc_mlp* model
       mlp_mirror_region(&m, chains, n, wsp, &p->fz.mirror, &p->fz.mirror_count,
                         &p->fz.mirror_stride);
       p->fz.sq_parts = p->sq;
-      if (m.prior_scale > 0.f)
-        p->pf = static_cast<float>(1.0 / (static_cast<double>(m.prior_scale) *
-                                          m.prior_scale * m.temperature));
+      p->pf = prior_factor(m);
       const double* sqp = p->sq;
       p->grad_fn = [m, chains, n, x, wsp, ws, status_dev, sqp, nb](
                        const int32_t* idx, int64_t stride, double* U, double* var, float* grad,
                        cudaStream_t s) {
-        return mlp_value_and_grad_fused(&m, chains, n, idx, stride, x, U, grad, var, wsp, ws,
-                                        status_dev, s, sqp, nb);
+        return mlp_value_and_grad_fused(&m, chains, n, nullptr, idx, stride, x, U, grad, var, wsp,
+                                        ws, status_dev, s, sqp, nb);
       };
     } else {
       p->grad_fn = [m, chains, n, x, wsp, ws, status_dev](
@@ -688,12 +698,12 @@ extern "C" int gbsgmc_mlp_resgld_plan_create_keep(
     const gbsgmc_mlp m = *model;
     void* wsp = p->ws;
     const float* x = x_dev;
+    p->pf = prior_factor(m);
     p->grad_fn = [m, replicas, n_max, n_dev, x, wsp, ws, status_dev](
                      const int32_t* idx, int64_t stride, double* U, double* var, float* grad,
                      cudaStream_t s) {
-      return gbsgmc_mlp_value_and_grad_ragged(&m, replicas, n_max, n_dev, idx, stride, nullptr,
-                                              x, U, grad, nullptr, var, wsp, ws, status_dev,
-                                              s);
+      return mlp_value_and_grad_fused(&m, replicas, n_max, n_dev, idx, stride, x, U, grad, var,
+                                      wsp, ws, status_dev, s, nullptr, 0);
     };
     rc = plan_capture(p);
   } while (false);

@@ -41,9 +41,10 @@ namespace epi {
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 
 // Waits until the warp's last TMA store (store_box) has read the staging
-// tile; warp-collective.
+// tile; warp-collective.  elect_one names the same lane each time: the one
+// that stores.
 __device__ __forceinline__ void reclaim() {
-  if (lane_id() == 0) tc::bulk_wait_read();
+  if (tc::elect_one()) tc::bulk_wait_read();
   __syncwarp();
 }
 
@@ -90,7 +91,7 @@ __device__ __forceinline__ void store_box(uint32_t* st, const uint32_t (&w)[32],
     tc::sts128(row + ((q ^ (l & 7)) << 4), w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
   tc::fence_async_shared();
   __syncwarp();
-  if (l == 0) {
+  if (tc::elect_one()) {
     tc::tma_store_3d(map, st, x, y, z);
     tc::bulk_commit();
   }
@@ -394,7 +395,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[buf]);
     }
-    if (lane == 0) tc::bulk_wait();  // the epilogue's TMA stores
+    if (tc::elect_one()) tc::bulk_wait();  // the epilogue's TMA stores
   }
   tc::fence_before_sync();
   __syncthreads();
@@ -634,7 +635,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
       // else has to be ordered before the leader may overwrite them.
       if (lane == 0) tc::mbar_arrive_cluster_relaxed(buf ? drained1 : drained0);
     }
-    if (lane == 0) tc::bulk_wait();  // the epilogue's TMA stores
+    if (tc::elect_one()) tc::bulk_wait();  // the epilogue's TMA stores
   }
   tc::fence_before_sync();
   __syncthreads();
