@@ -137,7 +137,8 @@ __device__ __forceinline__ U32x4 philox4x32_10(U32x4 c, uint32_t k0,
 // Uniform in (0,1): the top 23 bits plus one half, (2m+1)/2^24, which fp32
 // represents exactly over the whole interval.
 __device__ __forceinline__ float u32_to_open01(uint32_t v) {
-  return (static_cast<float>(v >> 9) + 0.5f) * (1.0f / 8388608.0f);
+  // 1 + m 2^-23 by its bits, minus 1 - 2^-24: exact, and no conversion.
+  return __uint_as_float(0x3f800000u | (v >> 9)) - 0.999999940395355224609375f;
 }
 
 // Box-Muller: (a, b) uniform words -> two standard normals.
