@@ -272,7 +272,7 @@ def langevin_diffusion(potential_fn, batch_fn, adaption: AdaptionStrategy = None
     return LangevinChains(W, V, alpha, lmbd, pipelines, key_to_seed(key),
                           init_model_state, tdef)
 
-  init_fn.many = init_many
+  init_chains = util.with_many(init_fn, init_many)
 
   def get_fn(state: LangevinState):
     return {"variables": state.latent_variables,
@@ -300,7 +300,7 @@ def langevin_diffusion(potential_fn, batch_fn, adaption: AdaptionStrategy = None
                           data_state=data_state, potential=r.U[0],
                           variance=r.lk_var[0], step=state.step + 1)
 
-  return IntegratorTriplet(init_fn, update_fn, get_fn, kind="langevin",
+  return IntegratorTriplet(init_chains, update_fn, get_fn, kind="langevin",
                            potential=potential_fn, batch_fn=batch_fn,
                            adaption=adaption, noise_source=noise_source)
 
@@ -395,7 +395,7 @@ def obabo(potential_fn, batch_fn, steps=10, friction=1.0, const_mass=None,
                       lambda: torch.zeros(W.shape, dtype=torch.float32, device="cuda"),
                       make)
 
-  init_fn.many = init_many
+  init_chains = util.with_many(init_fn, init_many)
 
   def integrate(state: ObaboState, parameters, mass=None):
     x, p = state.positions, state.momentum
@@ -444,7 +444,7 @@ def obabo(potential_fn, batch_fn, steps=10, friction=1.0, const_mass=None,
     return {"variables": state.positions, "energy": state.potential,
             "model_state": state.model_state}
 
-  return IntegratorTriplet(init_fn, integrate, get_fn, kind="obabo",
+  return IntegratorTriplet(init_chains, integrate, get_fn, kind="obabo",
                            potential=potential_fn, batch_fn=batch_fn,
                            steps=steps, friction=friction,
                            const_mass=const_mass, noise_source=noise_source)
@@ -493,7 +493,7 @@ def friction_leapfrog(potential_fn, batch_fn, steps=10, friction=0.25,
 
     return ChainBatch(W, pipelines, seed, init_model_state, tdef, W.cuda, make)
 
-  init_fn.many = init_many
+  init_chains = util.with_many(init_fn, init_many)
 
   def integrate(state: LeapfrogState, parameters, mass=None):
     x, p = state.positions, state.momentum
@@ -537,7 +537,7 @@ def friction_leapfrog(potential_fn, batch_fn, steps=10, friction=0.25,
     return {"variables": state.positions, "energy": state.potential,
             "model_state": state.model_state}
 
-  return IntegratorTriplet(init_fn, integrate, get_fn, kind="sghmc",
+  return IntegratorTriplet(init_chains, integrate, get_fn, kind="sghmc",
                            potential=potential_fn, batch_fn=batch_fn,
                            steps=steps, friction=friction,
                            const_mass=const_mass, noise_source=noise_source,
@@ -623,7 +623,7 @@ def reversible_leapfrog(potential_fn, batch_fn, steps: int = 10,
 
     return ChainBatch(W, pipelines, seed, init_model_state, tdef, momenta, make)
 
-  init_fn.many = init_many
+  init_chains = util.with_many(init_fn, init_many)
 
   def integrate(state: LeapfrogState, parameters, mass=None):
     import torch
@@ -673,7 +673,7 @@ def reversible_leapfrog(potential_fn, batch_fn, steps: int = 10,
     return {"variables": state.positions, "energy": state.potential,
             "model_state": state.model_state}
 
-  return IntegratorTriplet(init_fn, integrate, get_fn, kind="reversible_leapfrog",
+  return IntegratorTriplet(init_chains, integrate, get_fn, kind="reversible_leapfrog",
                            potential=potential_fn, batch_fn=batch_fn,
                            steps=steps, friction=friction,
                            const_mass=const_mass, noise_source=noise_source)

@@ -16,7 +16,7 @@ from typing import Any, NamedTuple
 
 import numpy as np
 
-from . import _lib, engine, io, scheduler as sched_mod
+from . import _lib, engine, io, scheduler as sched_mod, util
 
 
 class SolverTriplet(tuple):
@@ -273,8 +273,8 @@ def _mh_solver(kind, integrator, full_potential_fn, full_data_map,
       return [state(c, U[i:i + 1].clone()) for i, c in enumerate(chains)]
     return MHChains(chains, U, seed, lambda i: state(chains[i], U[i:i + 1].clone()))
 
-  if getattr(init_integrator, "many", None) is not None:
-    init.many = init_many
+  chains_init = init if getattr(init_integrator, "many", None) is None else \
+      util.with_many(init, init_many)
 
   def update(state: MHState, schedule):
     import torch
@@ -337,7 +337,7 @@ def _mh_solver(kind, integrator, full_potential_fn, full_data_map,
       out["potential"] = state.potential
     return out
 
-  return init, update, get
+  return chains_init, update, get
 
 
 def amagold(integrator_fn, full_potential_fn, full_data_map,

@@ -8,6 +8,7 @@ Leaves may be numpy arrays, torch tensors or Python scalars.
 
 from __future__ import annotations
 
+import functools
 from typing import Any, List, NamedTuple, Tuple
 
 import numpy as np
@@ -162,3 +163,15 @@ def unravel(tdef: TreeDef, flat) -> PyTree:
     leaves.append(flat[..., o:o + n].reshape(lead + tuple(shape)))
     o += n
   return tree_unflatten(tdef, leaves)
+
+
+def with_many(init, many):
+  """``init`` with the bulk form ``many`` as its attribute.  The attribute is
+  set on a wrapper: ``many`` falls back on ``init``, and set on ``init`` itself
+  the two would keep each other, the dataset and its device memory alive until
+  a garbage collection."""
+  @functools.wraps(init)
+  def init_or_many(*args, **kwargs):
+    return init(*args, **kwargs)
+  init_or_many.many = many
+  return init_or_many
