@@ -62,19 +62,6 @@ __device__ __forceinline__ uint32_t get(const uint32_t* st, int r) {
   return st[r * 32 + (lane_id() ^ r)];
 }
 
-// The reverse: word `lane` of row r was written by the whole warp (set,
-// after reclaim), and lane l collects its own row.
-__device__ __forceinline__ void set(uint32_t* st, int r, uint32_t v) {
-  st[r * 32 + (lane_id() ^ r)] = v;
-}
-__device__ __forceinline__ void get_row(const uint32_t* st, uint32_t (&w)[32]) {
-  const int l = lane_id();
-  __syncwarp();
-#pragma unroll
-  for (int j = 0; j < 32; ++j) w[j] = st[l * 32 + (j ^ l)];
-  __syncwarp();
-}
-
 // Stores the warp's 32 rows of 128 bytes (lane l's words w = row l) as one
 // box of a tensor map with a 128-byte swizzle and a box of 128 bytes x 32
 // rows, at coordinates (x, y, z): the rows are written to the staging tile
