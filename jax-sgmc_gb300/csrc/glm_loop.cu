@@ -10,10 +10,13 @@
 //   * the copy warps run ahead: the minibatches of a block are known before it
 //     starts, so they gather the rows of the next chunks into a ring of shared
 //     memory buffers (full / empty mbarriers), up to `depth` chunks before
-//     they are needed: one bulk copy a row, each lane its own (a cp.async per
-//     16 bytes took a copy warp 110 cycles a row of 101 features, more than
-//     the rest of the step: 24 chains of 500 such rows 3.8 us a gradient
-//     against 3.0);
+//     they are needed.  Issuing the copies is what bounds a step of more than
+//     about 16 rows a CTA: a cp.async per 16 bytes took a copy warp 110 cycles
+//     a row of 101 features, a bulk copy per row (each lane its own) is better
+//     (24 chains of 500 such rows: 3.8 to 3.0 us a gradient) and a gather of
+//     four rows per instruction takes the copies off the critical path (1.9
+//     us; 64 chains of 512 rows of 32 features 299 to 136 us a 50 steps, 64
+//     of 128 features 307 to 153; never slower);
 //   * the row warps do what nothing else can do earlier: row tiles of the
 //     chunk exactly as glm_kernel takes them (same slices, warps, tiles and
 //     summation orders: the same bits), the reduction, the exchange and the
@@ -37,6 +40,7 @@
 #include "glm.cuh"
 #include "internal.h"
 #include "tc.cuh"
+#include "tc_gemm.cuh"
 
 namespace gbsgmc {
 namespace {
@@ -66,6 +70,8 @@ struct LoopArgs {
   int row_quads;   // 16-byte words of a row in shared memory
   int cp_y;        // y is copied by itself: rows are not aligned, or it is not in them
   int cp_async;    // some copies are made by cp.async
+  int gather;      // rows are copied four at a time
+  int row_cols;    // floats of a row that are read (16-byte words)
   // pairs
   int pairs;
   double F;
@@ -228,7 +234,8 @@ __device__ __forceinline__ double slice_total(const SliceSums* s, int ctas, int 
 }
 
 template <int QPL, int RW>
-__global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArgs L) {
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    glm_loop_kernel(const __grid_constant__ LoopArgs L, const __grid_constant__ CUtensorMap map) {
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int LOG = Log2<RW>::v;
   constexpr int GROUP = 32 >> LOG;
@@ -305,34 +312,76 @@ __global__ void __launch_bounds__(kLoopThreads, 1) glm_loop_kernel(const LoopArg
       for (int q = 0; q < chunks; ++q) {
         const int cnt = min(CH, R - q * CH);
         const int r_end = min(cnt, (cw + 1) * share);
-        int o = cw * share + lane < r_end ? __ldg(src + q * CH + cw * share + lane) : -1;
-        if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
         float4* dst = rows_s + buf * CH * rq;
-        for (int r0 = cw * share; r0 < r_end; r0 += 32) {
-          const int r = r0 + lane;
-          if (r0 > cw * share) o = r < r_end ? __ldg(src + q * CH + r) : -1;
-          if (r < r_end) {
-            if (o < 0 || o >= n_rows) {   // left out: its row is zero
-              raise_status(a.status, GBSGMC_ERR_INDEX);
-              o = -1;
-              for (int v = 0; v < rq; ++v) dst[r * rq + v] = make_float4(0.f, 0.f, 0.f, 0.f);
-              tc::fence_async_shared();
-            }
-            idx_s[buf * CH + r] = o;
-            if (o >= 0 && L.cp_y) cp4(y_s + buf * CH + r, y_inline ? X + o * ld + d : yv + o, true);
-          }
-          if (vec4) {   // one copy a row, its y with it
-            const unsigned live = __ballot_sync(0xffffffffu, o >= 0);
-            if (lane == 0) mbar_expect_tx(bars->full + buf, __popc(live) * row_bytes);
+        const int32_t* at = src + q * CH;
+        int* idx_b = idx_s + buf * CH;
+        float* y_b = y_s + buf * CH;
+        if (L.gather) {
+          // Lane l takes rows 4 l .. 4 l + 3 of each 128.  An index out of
+          // range, or past the chunk, is sent to the row after the last one,
+          // which the copy reads as zeros.
+          int o[4];
+          const auto fetch = [&](int r) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) o[j] = r + j < r_end ? __ldg(at + r + j) : -1;
+          };
+          fetch(cw * share + 4 * lane);
+          if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
+          for (int r0 = cw * share; r0 < r_end; r0 += 128) {
+            const int r = r0 + 4 * lane;
+            if (r0 > cw * share) fetch(r);
+            if (lane == 0)
+              mbar_expect_tx(bars->full + buf, min(32, (r_end - r0 + 3) / 4) * 4 * row_bytes);
             __syncwarp();
-            if (o >= 0) bulk_g2s(dst + r * rq, X + o * ld, row_bytes, bars->full + buf);
-          } else {
-            for (int i = 0; i < min(32, r_end - r0); ++i) {
-              const int oi = __shfl_sync(0xffffffffu, o, i);
-              if (oi < 0) continue;
-              float* out = reinterpret_cast<float*>(dst + (r0 + i) * rq);
-              for (int j = lane; j < 4 * dq; j += 32)
-                cp4(out + j, X + oi * ld + (j < d ? j : 0), j < d);
+            if (r < r_end) {
+              int at_row[4];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (r + j < r_end && (o[j] < 0 || o[j] >= n_rows)) {
+                  raise_status(a.status, GBSGMC_ERR_INDEX);
+                  o[j] = -1;
+                }
+                at_row[j] = o[j] < 0 ? static_cast<int>(n_rows) : o[j];
+              }
+              tc::tma_gather4(dst + r * rq, &map, 0, at_row[0], at_row[1], at_row[2], at_row[3],
+                              bars->full + buf);
+              *reinterpret_cast<int4*>(idx_b + r) = make_int4(o[0], o[1], o[2], o[3]);
+              if (L.cp_y) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  if (o[j] >= 0) cp4(y_b + r + j, yv + o[j], true);
+              }
+            }
+          }
+        } else {
+          int o = cw * share + lane < r_end ? __ldg(at + cw * share + lane) : -1;
+          if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
+          for (int r0 = cw * share; r0 < r_end; r0 += 32) {
+            const int r = r0 + lane;
+            if (r0 > cw * share) o = r < r_end ? __ldg(at + r) : -1;
+            if (r < r_end) {
+              if (o < 0 || o >= n_rows) {   // left out: its row is zero
+                raise_status(a.status, GBSGMC_ERR_INDEX);
+                o = -1;
+                for (int v = 0; v < rq; ++v) dst[r * rq + v] = make_float4(0.f, 0.f, 0.f, 0.f);
+                tc::fence_async_shared();
+              }
+              idx_b[r] = o;
+              if (o >= 0 && L.cp_y) cp4(y_b + r, y_inline ? X + o * ld + d : yv + o, true);
+            }
+            if (vec4) {   // one copy a row, its y with it
+              const unsigned live = __ballot_sync(0xffffffffu, o >= 0);
+              if (lane == 0) mbar_expect_tx(bars->full + buf, __popc(live) * row_bytes);
+              __syncwarp();
+              if (o >= 0) bulk_g2s(dst + r * rq, X + o * ld, row_bytes, bars->full + buf);
+            } else {
+              for (int i = 0; i < min(32, r_end - r0); ++i) {
+                const int oi = __shfl_sync(0xffffffffu, o, i);
+                if (oi < 0) continue;
+                float* out = reinterpret_cast<float*>(dst + (r0 + i) * rq);
+                for (int j = lane; j < 4 * dq; j += 32)
+                  cp4(out + j, X + oi * ld + (j < d ? j : 0), j < d);
+              }
             }
           }
         }
@@ -925,7 +974,12 @@ struct LoopVariant {
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, glm_loop_kernel<QPL, RW>, L);
+    CUtensorMap map = {};
+    if (L.gather &&
+        (rc = make_tmap_f32_gather(&map, L.g.X, L.row_cols, L.g.n_rows, L.g.ld, 4 * L.row_quads)) !=
+            GBSGMC_OK)
+      return rc;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, glm_loop_kernel<QPL, RW>, L, map);
     if (e != cudaSuccess)
       return set_error(GBSGMC_ERR_CUDA, "glm_loop: %s", cudaGetErrorString(e));
     return check_launch("glm_loop");
@@ -1065,6 +1119,15 @@ int glm_loop(const GlmLoopCall& c, cudaStream_t st) {
   L.row_quads = (L.g.d + (y_in_row ? 1 : 0) + 3) / 4;
   L.cp_y = !y_in_row && (L.g.y_inline || L.g.y != nullptr) ? 1 : 0;
   L.cp_async = !L.g.vec4 || L.cp_y ? 1 : 0;
+  // Rows on 16-byte boundaries are copied four at a time where a box holds a
+  // row (256 columns); in shared memory they then start on multiples of 32
+  // bytes, so that four rows, the target of one copy, start on 128.  The row
+  // after the last one has to be an int32 coordinate.  Wider rows are copied
+  // one by one; from about 200 columns the bytes bound a step, not the copies
+  // (24 chains of 250 rows of 200 features: 209 us for 40 gradients by either).
+  L.row_cols = 4 * L.row_quads;
+  L.gather = L.g.vec4 && L.row_quads <= 64 && L.g.n_rows < (1ll << 31) - 1 ? 1 : 0;
+  if (L.gather) L.row_quads += L.row_quads & 1;
   int units = c.chains, ncta = c.ctas;
   if (pairs) {
     units = L.pairs = c.chains / 2;

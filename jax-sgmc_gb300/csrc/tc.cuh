@@ -231,6 +231,18 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// Four rows of a 2-D map (boxes of one row) from column x, one after the other
+// in shared memory (128-byte aligned); rows past the extent read zeros.
+__device__ __forceinline__ void tma_gather4(void* dst, const CUtensorMap* map, int x, int r0,
+                                            int r1, int r2, int r3, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3),
+      "r"(smem_addr(bar))
+      : "memory");
+}
+
 // 3-D tiled load (x = innermost, K elements; y = rows; z = batch), completing
 // on `bar`.  x must be a multiple of 8 for BF16 (16 bytes).
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map,

@@ -149,6 +149,28 @@ int make_tmap_bf16_4d_plain(CUtensorMap* map, const void* base, const int64_t (&
   return GBSGMC_OK;
 }
 
+int make_tmap_f32_gather(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
+                         int64_t ld, int box_cols) {
+  auto fn = encode_fn();
+  if (fn == nullptr)
+    return set_error(GBSGMC_ERR_CUDA, "tensor map: cuTensorMapEncodeTiled unavailable");
+  if (reinterpret_cast<uintptr_t>(base) % 16 != 0 || ld % 4 != 0 || box_cols % 4 != 0 ||
+      box_cols > 256)
+    return set_error(GBSGMC_ERR_ARG,
+                     "tensor map (gather): base and rows 16-byte aligned, at most 256 columns");
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 4};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), 1}, es[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims,
+                        strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                        CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return set_error(GBSGMC_ERR_CUDA, "cuTensorMapEncodeTiled (gather) failed (%d)",
+                     static_cast<int>(r));
+  return GBSGMC_OK;
+}
+
 int make_tmap_rows(CUtensorMap* map, const void* base, bool f32, int64_t cols, int64_t rows,
                    int64_t batch, int64_t row_stride, int64_t batch_stride) {
   auto fn = encode_fn();

@@ -133,6 +133,11 @@ int make_tmap_bf16_3d(CUtensorMap* map, const void* base, int64_t cols,
 int make_tmap_bf16_4d_plain(CUtensorMap* map, const void* base, const int64_t (&dims)[4],
                             const int64_t (&strides)[3], const int (&box)[4]);
 
+// 2-D fp32 tensor map (cols innermost, rows `ld` elements apart) without
+// swizzle whose boxes are one row of box_cols, for tile::gather4 loads.
+int make_tmap_f32_gather(CUtensorMap* map, const void* base, int64_t cols, int64_t rows,
+                         int64_t ld, int box_cols);
+
 // 3-D tensor map (cols innermost, rows, batch) of an epilogue's output for
 // epi::store_box: 128-byte swizzle, boxes of 128 bytes x 32 rows (64 BF16 or
 // 32 fp32 columns); strides in elements.

@@ -169,6 +169,58 @@ def test_row_layouts_agree(lib, layout, C, n, d):
     np.testing.assert_array_equal(a, b)
 
 
+class _Given:
+  """An index feed that deals out the rows of a [K, C, n] array."""
+
+  def __init__(self, idx):
+    self.idx, self.at = idx, 0
+
+  def next(self, g, out):
+    out[:g] = self.idx[self.at:self.at + g]
+    self.at += g
+
+
+@pytest.mark.parametrize("bad", [False, True])
+@pytest.mark.parametrize("C,n,d", [(1, 2, 2), (2, 131, 3), (1, 258, 31), (70, 67, 32),
+                                   (1, 258, 251), (1, 129, 255), (1, 130, 256)])
+def test_gathered_rows_agree(lib, C, n, d, bad):
+  """Rows copied four at a time (up to 256 columns with y) or one by one
+  against rows copied in words: numbers of rows that leave remainders of 1 to
+  3, widths around whole 32 bytes and the widest box, and indices beyond the
+  last row, which both leave out and report: bit-equal states."""
+  from gbsgmc import _lib, engine
+  X, y, ds, pot, x0, N = _setup(C, n, d, O.LOGISTIC)
+  h = (np.full(K, 0.02 / (N * max(1.0, 2.0 * d / n)))).astype(np.float32)
+  idx = np.random.default_rng(n).integers(0, N, (K, C, n)).astype(np.int32)
+  idx[:, :, -1] = N - 1
+  if bad:
+    idx[::2, :, n // 2] = [[N]]
+    idx[1::2, :, 0] = [[-1]]
+  base, _ = pot.model(ds)
+  outs = []
+  for ld in ((d + 4) // 4 * 4, (d + 1) | 1):
+    rows = np.zeros((N, ld), np.float32)
+    rows[:, :d], rows[:, d] = X, y
+    rows = _cuda(rows)
+    model = _lib.Glm(base.family, d, base.n_obs, ld, rows.data_ptr(), None, base.sigma,
+                     base.prior_scale, base.temperature, 1, N)
+    object.__setattr__(pot, "model", lambda *a, **k: (model, (rows,)))
+    x = _cuda(x0)
+    plan = engine.NetPlan(pot, ds, x, None, n, "langevin", _cuda(h),
+                          _cuda(np.ones(K, np.float32)), engine.IndexSource(external=True), 11,
+                          block_steps=3, feed=_Given(idx))
+    plan.run(0, K)
+    if bad:
+      with pytest.raises(_lib.GbsgmcError) as e:
+        plan.check_status()
+      assert e.value.code == _lib.ERR_INDEX
+    else:
+      plan.check_status()
+    outs.append((x.cpu().numpy(), plan.U.cpu().numpy(), plan.lk_var.cpu().numpy()))
+  for a, b in zip(*outs):
+    np.testing.assert_array_equal(a, b)
+
+
 @pytest.mark.parametrize("pairs,n,d", [(1, 33, 7), (2, 256, 64), (1, 900, 300), (90, 40, 12)])
 def test_pairs_match_the_per_pair_path(lib, pairs, n, d):
   """alias.re_sgld through the block launches against one chain at a time
