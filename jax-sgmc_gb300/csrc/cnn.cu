@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(kStripThreads, 4) cnn_conv1_kernel(const CnnAr
 // the MMAs of a unit (issued by a warp of its own) run while the next is
 // built.  db1 (another warp): the routed
 // (BF16-rounded) values of a unit's 64 windows are added in window order, a
-// partial per unit.  Grid (splits, chains).
+// partial per unit.
 constexpr int kDyWarps = 8, kWordWarps = 6, kUnitThreads = 32 * (kDyWarps + kWordWarps + 2);
 constexpr int kUnitRow = 3 * 256;   // bytes of a row's E, O and shifted E
 constexpr int kUnitDy = 8 * 2 * 1024, kUnitWords = 11 * kUnitRow, kUnitBias = 64 * 36 * 4;
@@ -572,9 +572,8 @@ constexpr int kUnitBuf = kUnitDy + kUnitWords + kUnitBias;
 static_assert(kUnitBuf % 128 == 0, "buffer alignment");
 constexpr int kUnitSmem = 2 * kUnitBuf;
 
-__global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const CnnArgs a,
-                                                                        int pair) {
-  extern __shared__ __align__(128) uint8_t unit_smem[];
+__device__ __forceinline__ void conv1_grad(const CnnArgs& a, int pair, uint8_t* unit_smem, int c,
+                                           int split, int S) {
   __shared__ uint64_t full[2], free_[2];   // a buffer is built; its MMAs and sums are done
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_s;
@@ -603,8 +602,7 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
   pdl_trigger();
   pdl_wait();
 
-  const int c = blockIdx.y, S = gridDim.x;
-  const int each = 16 * a.n / S, q0 = each * blockIdx.x, q1 = q0 + each;   // slices
+  const int each = 16 * a.n / S, q0 = each * split, q1 = q0 + each;   // slices
   const int u0 = q0 >> 2, u1 = (q1 + 3) >> 2;                              // units
   auto wait = [&](uint64_t* bar, uint32_t parity) {
     return conv_wait(bar, parity, abort_flag, a.status);
@@ -753,7 +751,7 @@ __global__ void __launch_bounds__(kUnitThreads, 2) cnn_conv1_grad_kernel(const C
   tc::fence_after_sync();
   if (warp < 2) {
     // Accumulator row r of an M = 64 tile is TMEM lane 32 (r / 16) + r % 16.
-    float* dst = a.part[0] + (static_cast<int64_t>(c) * S + blockIdx.x) * kK1 * kC1 + 16 * warp +
+    float* dst = a.part[0] + (static_cast<int64_t>(c) * S + split) * kK1 * kC1 + 16 * warp +
                  lane;
 #pragma unroll
     for (int kh = 0; kh < 3; ++kh) {   // columns (kh, run, slot)
@@ -1061,20 +1059,15 @@ struct EpiStripDX {
 // column shift kw is one MMA of M = 64 outputs x N = 96 (three kernel rows x
 // 32 inputs: the box's [h][octet] words lie 288 bytes apart).  The sums of a
 // run of a chain's slices stay in TMEM and are written as one split-K partial
-// [tap, input][output].  Grid (splits, chains, Z): a CTA takes all three
-// column shifts (Z = 1) or one (Z = 3, when the splits alone leave SMs idle).
+// [tap, input][output].  A CTA takes a split and a column shift.
 constexpr int kDy2Box = 4 * (kC2 / 8) * 256, kP1Box = 6 * (kC1 / 8) * 288;
 constexpr int kDw2Stages = 7, kDw2Threads = 64 + 4 * 32;
 constexpr int kDw2Smem = kDw2Stages * (kDy2Box + kP1Box) + 128 + 256;
-constexpr int kDw2SmemAlone = 120 * 1024;   // Z = 1 takes all of the SM's TMEM
 
-__global__ void __launch_bounds__(kDw2Threads, 1)
-    cnn_conv2_dw_kernel(const __grid_constant__ CUtensorMap mdy,
-                        const __grid_constant__ CUtensorMap mp1, float* part, int n,
-                        int* status) {
+__device__ __forceinline__ void conv2_dw(const CUtensorMap& mdy, const CUtensorMap& mp1,
+                                         float* part, int n, int* status, uint8_t* smem_raw, int c,
+                                         int split, int S, int kw) {
   constexpr int kStage = kDy2Box + kP1Box;
-  const uint32_t cols = gridDim.z == 1 ? 512 : 128;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + kDw2Stages * kStage);
@@ -1093,7 +1086,7 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
     mbar_fence_init();
   }
   if (warp == 1) {
-    tc::tmem_alloc(tmem_slot, cols);
+    tc::tmem_alloc(tmem_slot, 128);
     tc::tmem_relinquish();
   }
   tc::fence_before_sync();
@@ -1102,9 +1095,7 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
   const uint32_t tmem = *tmem_slot;
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.y, S = gridDim.x;
-  const int each = 4 * n / S, u0 = each * blockIdx.x, u1 = u0 + each;   // slices
-  const int kw0 = gridDim.z == 1 ? 0 : blockIdx.z, kw1 = gridDim.z == 1 ? 3 : kw0 + 1;
+  const int each = 4 * n / S, u0 = each * split, u1 = u0 + each;   // slices
   if (warp == 0) {
     if (tc::elect_one()) {
       uint32_t it = 0;
@@ -1132,26 +1123,25 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
         const uint64_t B = tc::sdesc_none(ring + s * kStage + kDy2Box, 128, 288);
 #pragma unroll
         for (int h = 0; h < 4; ++h)
-          for (int kw = kw0; kw < kw1; ++kw)
-            tc::mma_bf16(tmem + 96 * (kw - kw0), A + h * (kC2 / 8) * 256 / 16,
-                         B + h * (kC1 / 8) * 288 / 16 + kw, idesc, it > 0 || h > 0);
+          tc::mma_bf16(tmem, A + h * (kC2 / 8) * 256 / 16, B + h * (kC1 / 8) * 288 / 16 + kw, idesc,
+                       it > 0 || h > 0);
         tc::mma_commit(empty + s);
       }
       tc::mma_commit(done);
       mbar_wait_bounded(done, 0, nullptr);
     }
-  } else {
+  } else if (warp < kDw2Threads / 32) {
     const bool ok = mbar_wait_bounded(done, 0, nullptr);
     if (!__all_sync(0xffffffffu, ok) && lane == 0) raise_status(status, GBSGMC_ERR_TIMEOUT);
     tc::fence_after_sync();
     // Accumulator row r of an M = 64 tile is TMEM lane 32 (r / 16) + r % 16.
     const int q = warp & 3;
-    float* dst = part + (static_cast<int64_t>(c) * S + blockIdx.x) * kK2 * kC2 + 16 * q + lane;
+    float* dst = part + (static_cast<int64_t>(c) * S + split) * kK2 * kC2 + 16 * q + lane;
 #pragma unroll 1
-    for (int g = 0; g < 3 * (kw1 - kw0); ++g) {   // kw, kh
+    for (int kh = 0; kh < 3; ++kh) {
       float v[32];
-      tc::tmem_ld32(tmem + 32 * g + (static_cast<uint32_t>(q * 32) << 16), v);
-      const int tap = 3 * (g % 3) + kw0 + g / 3;
+      tc::tmem_ld32(tmem + 32 * kh + (static_cast<uint32_t>(q * 32) << 16), v);
+      const int tap = 3 * kh + kw;
       if (lane < 16) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) dst[(tap * kC1 + j) * kC2] = v[j];
@@ -1162,7 +1152,7 @@ __global__ void __launch_bounds__(kDw2Threads, 1)
   __syncthreads();
   if (warp == 1) {
     tc::fence_after_sync();
-    tc::tmem_dealloc(tmem, cols);
+    tc::tmem_dealloc(tmem, 128);
   }
 }
 
@@ -1422,21 +1412,18 @@ struct EpiPairRoute {
 };
 
 // dW3 = dY3^T Col3: per image the boxes of dY3 and of P2 with its halo, two
-// image rows (16 pixels) as K; M = 128 outputs.  Z = 3: a CTA takes a column
-// shift, N = 192 (three kernel rows x 64 inputs, words 160 bytes apart); Z =
-// 9, when the splits leave SMs idle: one tap, N = 64.  Grid (splits, chains,
-// Z), one split-K partial [tap, input][output] of a run of a chain's images
-// each.
+// image rows (16 pixels) as K; M = 128 outputs.  A CTA takes a split and one of
+// Z = 3 column shifts, N = 192 (three kernel rows x 64 inputs, words 160 bytes
+// apart), or of Z = 9 taps, N = 64; it writes a split-K partial [tap,
+// input][output] of a run of a chain's images.
 constexpr int kDy3Box = 8 * (kC3 / 8) * 128, kP2Box = 10 * (kC2 / 8) * 160;
-constexpr int kDw3Stages = 7, kDw3Threads = 64 + 4 * 32;
+constexpr int kDw3Stages = 3, kDw3Threads = 64 + 4 * 32;   // two CTAs an SM
 constexpr int kDw3Smem = kDw3Stages * (kDy3Box + kP2Box) + 128 + 256;
 
-__global__ void __launch_bounds__(kDw3Threads, 1)
-    cnn_conv3_dw_kernel(const __grid_constant__ CUtensorMap mdy,
-                        const __grid_constant__ CUtensorMap mp2, float* part, int n,
-                        int* status) {
+__device__ __forceinline__ void conv3_dw(const CUtensorMap& mdy, const CUtensorMap& mp2,
+                                         float* part, int n, int* status, uint8_t* smem_raw, int c,
+                                         int split, int S, int z, int Z) {
   constexpr int kStage = kDy3Box + kP2Box, kRow = (kC2 / 8) * 160;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* ring = reinterpret_cast<uint8_t*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   uint64_t* full = reinterpret_cast<uint64_t*>(ring + kDw3Stages * kStage);
@@ -1445,7 +1432,7 @@ __global__ void __launch_bounds__(kDw3Threads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool single = gridDim.z == 9;
+  const bool single = Z == 9;
   const uint32_t cols = single ? 64 : 256;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kDw3Stages; ++i) {
@@ -1466,9 +1453,8 @@ __global__ void __launch_bounds__(kDw3Threads, 1)
   const uint32_t tmem = *tmem_slot;
   pdl_trigger();
   pdl_wait();
-  const int c = blockIdx.y, S = gridDim.x;
-  const int each = n / S, u0 = c * n + each * blockIdx.x, u1 = u0 + each;   // images
-  const int kw = blockIdx.z % 3, kh0 = single ? blockIdx.z / 3 : 0;
+  const int each = n / S, u0 = c * n + each * split, u1 = u0 + each;   // images
+  const int kw = z % 3, kh0 = single ? z / 3 : 0;
   if (warp == 0) {
     if (tc::elect_one()) {
       uint32_t it = 0;
@@ -1505,12 +1491,12 @@ __global__ void __launch_bounds__(kDw3Threads, 1)
       tc::mma_commit(done);
       mbar_wait_bounded(done, 0, nullptr);
     }
-  } else {
+  } else if (warp < kDw3Threads / 32) {
     const bool ok = mbar_wait_bounded(done, 0, nullptr);
     if (!__all_sync(0xffffffffu, ok) && lane == 0) raise_status(status, GBSGMC_ERR_TIMEOUT);
     tc::fence_after_sync();
     const int q = warp & 3;
-    float* dst = part + (static_cast<int64_t>(c) * S + blockIdx.x) * kK3 * kC3 + 32 * q + lane;
+    float* dst = part + (static_cast<int64_t>(c) * S + split) * kK3 * kC3 + 32 * q + lane;
 #pragma unroll 1
     for (int g = 0; g < (single ? 2 : 6); ++g) {   // kh, input half
       float v[32];
@@ -1526,6 +1512,39 @@ __global__ void __launch_bounds__(kDw3Threads, 1)
     tc::fence_after_sync();
     tc::tmem_dealloc(tmem, cols);
   }
+}
+
+// The three weight gradients in one launch, two CTAs an SM: none depends on
+// another, and their launches one after the other, each with a tail that
+// leaves SMs idle and MMAs of small N that wait on the issue, took 279 us of a
+// gradient of 8 x 256 images where the one launch leaves 266; with few images,
+// where each is mostly latency, 4 chains of 50: 83 to 69, 2 of 256: 152 to 118,
+// 2 of 2,048: 966 to 726.  Grid (parts, chains): a chain's splits of dW1 (the
+// longest), then of dW2 by column shift, then of dW3 in z3 parts.
+constexpr int kGradsSmem = std::max({kUnitSmem, kDw2Smem, kDw3Smem});
+
+__global__ void __launch_bounds__(kUnitThreads, 2)
+    cnn_weight_grads_kernel(const __grid_constant__ CnnArgs a, int pair,
+                            const __grid_constant__ CUtensorMap mdy2,
+                            const __grid_constant__ CUtensorMap mp1,
+                            const __grid_constant__ CUtensorMap mdy3,
+                            const __grid_constant__ CUtensorMap mp2, int z3) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const int c = blockIdx.y, S1 = a.split[0], S2 = a.split[1], S3 = a.split[2];
+  int b = blockIdx.x;
+  if (b < S1) return conv1_grad(a, pair, smem_raw, c, b, S1);
+  b -= S1;
+  if (b < 3 * S2)
+    return conv2_dw(mdy2, mp1, a.part[1], a.n, a.status, smem_raw, c, b % S2, S2, b / S2);
+  b -= 3 * S2;
+  conv3_dw(mdy3, mp2, a.part[2], a.n, a.status, smem_raw, c, b % S3, S3, b / S3, z3);
+}
+
+// Parts of a split of dW3: a tap each while all CTAs of the launch run at once
+// (4 chains of 50 images 71 to 69 us), else a column shift each, which reads
+// dY3 a third as often (8 of 256: 281 and 266 us).
+int dw3_parts(const CnnArgs& a, int sms) {
+  return a.chains * (a.split[0] + 3 * a.split[1] + 9 * a.split[2]) <= 2 * sms ? 9 : 3;
 }
 
 // ---------------------------------------------------------------------------
@@ -1979,7 +1998,7 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     // dWd, dbd; layer 3: dY3 (routing of dP3) and db3.
     launch_pdl(cnn_dense_grad_kernel, dim3(kDenseGradBlocks + n / 2, C), 512, 0, st, a);
     if ((rc = launched("cnn_dense_grad_kernel"))) return rc;
-    // dW3; dP2, the transposed convolution of dY3, routed into dY2, and db2.
+    // Layer 3: dP2, the transposed convolution of dY3, routed into dY2, and db2.
     CUtensorMap m_dy3, m_dy3h, m_p2w;
     if ((rc = make_tmap_bf16_4d_plain(&m_dy3, a.dy3, {64, kC3 / 4, 8, pairs},
                                       {64, 16 * kC3, 128 * kC3}, {64, kC3 / 8, 8, 1})) ||
@@ -1988,17 +2007,10 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
         (rc = make_tmap_bf16_4d_plain(&m_dy3h, a.dy3, {64, kC3 / 4, 8, pairs},
                                       {64, 16 * kC3, 128 * kC3}, {80, kC3 / 4, 10, 1})))
       return rc;
-    cudaError_t e = cudaFuncSetAttribute(
-        cnn_conv3_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDw3Smem);
-    if (e != cudaSuccess)
-      return set_error(GBSGMC_ERR_CUDA, "cnn_conv3_dw_kernel: %s", cudaGetErrorString(e));
-    launch_pdl(cnn_conv3_dw_kernel, dim3(a.split[2], C, 9 * a.split[2] * C <= sms ? 9 : 3),
-               kDw3Threads, kDw3Smem, st, m_dy3, m_p2w, a.part[2], n, a.status);
-    if ((rc = launched("cnn_conv3_dw_kernel"))) return rc;
     if ((rc = conv3(cnn_conv3_kernel<kC3, kC2, EpiPairRoute>, conv3_smem<kC3, EpiPairRoute>(),
                     m_dy3h, EpiPairRoute{a.m2, a.dy2, a.bpart[1]})))
       return rc;
-    // Layer 2: dW2, and dP1, the transposed convolution of dY2.
+    // Layer 2: dP1, the transposed convolution of dY2.
     CUtensorMap m_dy2, m_dy2h, m_p1w;
     if ((rc = make_tmap_bf16_4d_plain(&m_dy2, a.dy2, {128, kC2 / 8, 16, imgs},
                                       {128, 16 * kC2, 256 * kC2}, {128, kC2 / 8, 4, 1})) ||
@@ -2007,25 +2019,18 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
         (rc = make_tmap_bf16_4d_plain(&m_dy2h, a.dy2, {128, kC2 / 8, 16, imgs},
                                       {128, 16 * kC2, 256 * kC2}, {80, kC2 / 8, 18, 1})))
       return rc;
-    e = cudaFuncSetAttribute(
-        cnn_conv2_dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDw2SmemAlone);
-    if (e != cudaSuccess)
-      return set_error(GBSGMC_ERR_CUDA, "cnn_conv2_dw_kernel: %s", cudaGetErrorString(e));
-    const bool apart = 3 * a.split[1] * C <= 2 * sms;
-    launch_pdl(cnn_conv2_dw_kernel, dim3(a.split[1], C, apart ? 3 : 1), kDw2Threads,
-               apart ? kDw2Smem : kDw2SmemAlone, st, m_dy2, m_p1w, a.part[1], n, a.status);
-    if ((rc = launched("cnn_conv2_dw_kernel"))) return rc;
     if ((rc = conv2(cnn_conv2_kernel<kC2, kC1, EpiStripDX>, conv_smem<kC2>(), m_dy2h,
                     EpiStripDX{a.dp1})))
       return rc;
-    // Layer 1: routing of dP1, db1 and dW1 in one launch.
-    e = cudaFuncSetAttribute(
-        cnn_conv1_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kUnitSmem);
+    // Routing of dP1 and db1; all dW.
+    const cudaError_t e = cudaFuncSetAttribute(
+        cnn_weight_grads_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradsSmem);
     if (e != cudaSuccess)
-      return set_error(GBSGMC_ERR_CUDA, "cnn_conv1_grad_kernel: %s", cudaGetErrorString(e));
-    launch_pdl(cnn_conv1_grad_kernel, dim3(a.split[0], C), kUnitThreads, kUnitSmem, st, a,
-               pair);
-    if ((rc = launched("cnn_conv1_grad_kernel"))) return rc;
+      return set_error(GBSGMC_ERR_CUDA, "cnn_weight_grads_kernel: %s", cudaGetErrorString(e));
+    const int z3 = dw3_parts(a, sms);
+    launch_pdl(cnn_weight_grads_kernel, dim3(a.split[0] + 3 * a.split[1] + z3 * a.split[2], C),
+               kUnitThreads, kGradsSmem, st, a, pair, m_dy2, m_p1w, m_dy3, m_p2w, z3);
+    if ((rc = launched("cnn_weight_grads_kernel"))) return rc;
   }
 
   launch_pdl(cnn_finalize_kernel, dim3((a.want_grad ? grid1(kP) : 0) + kBiasBlocks + 1, C), 256, 0,

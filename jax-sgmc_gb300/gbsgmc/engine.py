@@ -285,7 +285,7 @@ class NetPlan:
                                  float(alpha), float(lmbd), 0, _lib.ptr(mass))
     handle = _lib.C.c_void_p()
     # Kernel launches of one value-and-gradient call.
-    self.launches_per_gradient = 11 if potential.is_cnn else \
+    self.launches_per_gradient = 9 if potential.is_cnn else \
         9 if potential.is_mlp else 0
     create = "gbsgmc_cnn_plan_create" if potential.is_cnn else \
         "gbsgmc_mlp_plan_create" if potential.is_mlp else \

@@ -57,3 +57,17 @@ def test_unaligned_images(lib):
   b = pot.evaluate(Wd, idxd, ds, grad=True, lk=True, observation_count=N)
   pot.check_status()
   assert torch.equal(a.U, b.U) and torch.equal(a.lk, b.lk) and torch.equal(a.grad, b.grad)
+
+
+@pytest.mark.parametrize("C,n", [(5, 64), (6, 50), (9, 2)])
+def test_weight_gradients_do_not_depend_on_the_batch(lib, C, n):
+  """Many chains (dW3 by column shift) and one (by tap): the same sums in the
+  same order, so the same bits."""
+  import torch
+  N = 200
+  lik, images, labels, W, idx, ds, pot, Wd, idxd = base.setup(N, C, n, seed=n)
+  many = pot.evaluate(Wd, idxd, ds, grad=True, lk=True, observation_count=N)
+  for c in range(C):
+    one = pot.evaluate(Wd[c:c + 1], idxd[c:c + 1], ds, grad=True, lk=True, observation_count=N)
+    assert torch.equal(many.grad[c], one.grad[0]) and torch.equal(many.U[c], one.U[0])
+  pot.check_status()
