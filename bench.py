@@ -987,8 +987,8 @@ def run_cnn(args):
         "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak,
                      "unit": "TFLOP/s", "frac": achieved / peak, "traffic": None,
                      "peak_kind": "measured bf16_tflops_sustained",
-                     "kernel": "batched value-and-gradient (8 tcgen05 GEMMs + im2col, "
-                               "pooling, dense kernels), 8 chains",
+                     "kernel": "batched value-and-gradient (convolutions on tcgen05 with "
+                               "their pooling, dense kernels), 8 chains",
                      "kernel_ms": grad_ms, "algorithmic_flop_per_launch": flops},
         "cpu_baseline": cpu,
         "e2e": {"value": e2e_value, "unit": "chain-steps/s",
