@@ -102,6 +102,8 @@ struct GlmPlan final : gbsgmc_plan {
   int enqueue(int g, cudaStream_t s) override;
   int run_blocks(int64_t full, int rem) override;
   int draw(int g, int32_t* buf, cudaStream_t s);
+  gbsgmc::GlmLoopCall loop_call(int g, int ctas, const int32_t* buf, float* x, float* rms,
+                                const gbsgmc_sched* sc) const;
   int steps_launch(int g, int32_t* buf, cudaStream_t s);
   int pipelined_block(int parity, bool prefetch, cudaStream_t s);
   int setup_pipeline();
@@ -278,6 +280,30 @@ int GlmPlan::draw(int g, int32_t* buf, cudaStream_t s) {
                              g, n, rows, buf, n, cn, s);
 }
 
+// g steps of all chains in one glm_loop launch on positions `x` and RMSprop
+// state `rms`, without samples or a status word.
+gbsgmc::GlmLoopCall GlmPlan::loop_call(int g, int ctas, const int32_t* buf, float* x, float* rms,
+                                       const gbsgmc_sched* sc) const {
+  gbsgmc::GlmLoopCall c;
+  c.model = &model;
+  c.chains = chains;
+  c.n = n;
+  c.steps = g;
+  c.ctas = ctas;
+  c.idx = buf;
+  c.idx_stride = n;
+  c.idx_step_stride = static_cast<int64_t>(chains) * n;
+  c.x = x;
+  c.aux = rms;
+  c.alpha = alpha;
+  c.lmbd = lmbd;
+  c.sched = sc;
+  c.noise = &noise;
+  c.U = U;
+  c.lk_var = lk_var;
+  return c;
+}
+
 // One launch running g steps from the index sets in buf, then the counter
 // advance.
 int GlmPlan::steps_launch(int g, int32_t* buf, cudaStream_t s) {
@@ -287,23 +313,7 @@ int GlmPlan::steps_launch(int g, int32_t* buf, cudaStream_t s) {
   s0.base_dev = base;
   s0.offset = 0;
   if (tune.loop > 0) {
-    GlmLoopCall c;
-    c.model = &model;
-    c.chains = chains;
-    c.n = n;
-    c.steps = g;
-    c.ctas = tune.loop;
-    c.idx = buf;
-    c.idx_stride = n;
-    c.idx_step_stride = cn;
-    c.x = w;
-    c.aux = v;
-    c.alpha = alpha;
-    c.lmbd = lmbd;
-    c.sched = &s0;
-    c.noise = &noise;
-    c.U = U;
-    c.lk_var = lk_var;
+    GlmLoopCall c = loop_call(g, tune.loop, buf, w, v, &s0);
     c.samples = samples;
     c.sample_lik = sample_lik;
     c.status = status;
@@ -522,23 +532,14 @@ int autotune(GlmPlan* p) {
     const bool verbose = vb != nullptr && vb[0] == '1';
     for (const GlmTune& t : cands) {
       if (t.loop > 0) {
-        // A warm-up block, then six steps in one launch.
-        const GlmTune keep = p->tune;
-        p->tune = t;
-        float* const w0 = p->w;
-        float* const v0 = p->v;
-        const gbsgmc_sched s0 = p->sched;
-        p->w = w;
-        p->v = v0 != nullptr ? v : nullptr;
-        p->sched.keep_slot_dev = nullptr;
-        rc = p->steps_launch(6, p->idx, p->stream);
+        // A warm-up launch, then a timed one, of the same six steps: like the
+        // other trials they read the first entries of the schedule alone (a
+        // run may have no more than six) and report to the scratch status.
+        GlmLoopCall c = p->loop_call(6, t.loop, p->idx, w, p->v != nullptr ? v : nullptr, &sch);
+        c.status = status;
+        rc = glm_loop(c, p->stream);
         cudaEventRecord(e0, p->stream);
-        if (rc == GBSGMC_OK) rc = p->steps_launch(6, p->idx, p->stream);
-        p->tune = keep;
-        p->w = w0;
-        p->v = v0;
-        p->sched = s0;
-        if (rc == GBSGMC_OK) rc = plan_advance(p, -12, p->stream);
+        if (rc == GBSGMC_OK) rc = glm_loop(c, p->stream);
       } else if (t.multistep) {
         // Two warm-up steps, then six steps in one launch.
         for (int rep = 0; rep < 2 && rc == GBSGMC_OK; ++rep)

@@ -1,0 +1,58 @@
+"""The SGLD plan's choice of a launch form and what it may leave behind: its
+trials run on scratch copies, read no more of the schedule than the run has,
+and report to a scratch status word.
+"""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _cuda(a):
+  import torch
+  return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _words(C):
+  from gbsgmc.data.numpy_loader import pcg64_words
+  return np.array([pcg64_words(c) for c in range(C)], np.uint64).view(np.int64)
+
+
+def _setup(C, d, N=5003):
+  from gbsgmc import data, likelihoods as L, potential
+  rng = np.random.default_rng(d)
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (rng.random(N) < 0.5).astype(np.float32)
+  lik = L.Logistic()
+  pot = potential.minibatch_potential(L.GaussianPrior(3.0), lik)
+  x0 = (0.1 * rng.normal(size=(C, d))).astype(np.float32)
+  ds = data.NumpyDataLoader(x=X, y=y).device_dataset()
+  return lik, ds, pot, x0, N
+
+
+@pytest.mark.parametrize("C,n,d,K", [(96, 93, 21, 6), (160, 71, 21, 8), (600, 35, 9, 11)])
+def test_trials_stay_within_a_short_schedule(lib, monkeypatch, C, n, d, K):
+  """Runs of 6 to 11 steps with more chains than half the SMs.  The first plan
+  of a shape makes the trials; its tables end where the run does, and what
+  follows them in the same buffer (finite, absurd) reaches neither the status
+  nor the chains: the second plan, which takes over the first one's choice,
+  gives the same bits with zeros there."""
+  from gbsgmc import engine
+  monkeypatch.delenv("GBSGMC_AUTOTUNE", raising=False)
+  _, ds, pot, x0, N = _setup(C, d)
+  h = (0.02 / (0.25 * N) * 0.9 ** np.arange(K)).astype(np.float32)
+  outs = []
+  for rest in (1e30, 0.0):
+    h_buf, t_buf = np.full(64, rest, np.float32), np.full(64, rest, np.float32)
+    h_buf[:K], t_buf[:K] = h, 1.0
+    x, v = _cuda(x0), _cuda(np.zeros_like(x0))
+    plan = engine.SgldGlmPlan(pot, ds, x, v, 0.9, 1e-5, n, _cuda(h_buf), _cuda(t_buf),
+                              _cuda(np.full(K, -1, np.int32)), 0,
+                              engine.IndexSource(pcg=_cuda(_words(C))), 11, 0, K)
+    plan.run(0, K)
+    plan.check_status()
+    outs.append([plan.launch_shape()] + [a.cpu().numpy() for a in (x, v, plan.U, plan.lk_var)])
+  for a, b in zip(*outs):
+    np.testing.assert_array_equal(a, b)
+  assert np.isfinite(outs[0][1]).all() and (outs[0][1] != x0).all()
