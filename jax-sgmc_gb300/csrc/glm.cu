@@ -1069,12 +1069,6 @@ void glm_tune_store(int chains, int n, int d, int64_t ld, GlmTune t) {
 }
 
 int glm_qpl(int dq) { return qpl_for(dq); }
-int glm_rows_per_warp(int dq) {
-  const int qpl = qpl_for(dq);
-  const int forced = rows_override();
-  return qpl <= 2 && (forced == 2 || forced == 4 || forced == 8) ? forced
-                                                                 : default_rows_per_warp(qpl);
-}
 
 // Shared with the plan implementation.
 size_t glm_ws_bytes(int chains, int n, int d) { return ws_bytes(chains, n, d); }

@@ -22,6 +22,7 @@ struct GlmTune {
   int dynamic = 0;        // 1: warps claim items of `slices` per chain
   int multistep = 0;      // 1: plans run a block of steps in one launch
   int loop = 0;           // > 0: that launch is glm_loop with `loop` CTAs per chain
+                          // (the other fields: glm_kernel's shape)
 };
 
 // glm_loop.cu: a block of integrator steps of all chains in one launch.
@@ -62,10 +63,9 @@ struct GlmLoopCall {
 int glm_loop_ctas(int units, int chains_per_unit, int n);
 int glm_loop_prepare();
 int glm_loop(const GlmLoopCall& c, cudaStream_t st);
-// glm.cu: the float4 columns per lane and default rows per warp of a row of
-// dq float4, and the device's SM count.
+// glm.cu: the float4 columns per lane of a row of dq float4, and the device's
+// SM count.
 int glm_qpl(int dq);
-int glm_rows_per_warp(int dq);
 int glm_sm_count();
 
 size_t glm_ws_bytes(int chains, int n, int d);

@@ -434,7 +434,10 @@ namespace {
 // Autotuner: times candidate launch shapes of the fused step (CTAs per chain
 // and rows per warp) on scratch copies of the chain state and keeps the
 // fastest.  The choice is cached per problem shape for the process, and
-// direct step launches of that shape use it too.
+// direct step launches and evaluations of that shape use glm_kernel's shape in
+// it too: the fastest of those, whether or not the plan runs glm_loop.  A
+// choice of glm_loop that was not timed is not cached, so that it changes
+// nothing but its plan.
 int autotune(GlmPlan* p) {
   const char* env = std::getenv("GBSGMC_AUTOTUNE");
   if (env != nullptr && env[0] == '0') return GBSGMC_OK;
@@ -452,11 +455,11 @@ int autotune(GlmPlan* p) {
   // with a cluster per chain: every other form leaves SMs idle or pays a
   // launch per step (one chain, n = 128, d = 32: 10.9 us a step against 1.5;
   // 24 chains, n = 500, d = 101: 18.8 us a gradient against 3.0).
-  const int ctas = glm_loop_ctas(C, 1, n);
-  const GlmTune loop{ctas, glm_rows_per_warp((d + 3) / 4), 8, 0, 0, 1, ctas};
+  GlmTune loop;
+  loop.loop = glm_loop_ctas(C, 1, n);
+  loop.multistep = 1;
   if (2 * C <= glm_sm_count()) {
     p->tune = loop;
-    glm_tune_store(C, n, d, p->model.ld, loop);
     return GBSGMC_OK;
   }
   {
@@ -526,8 +529,8 @@ int autotune(GlmPlan* p) {
     sch.base_dev = nullptr;
     sch.keep_slot_dev = nullptr;
     sch.offset = 0;
-    float best_ms = 1e30f;
-    GlmTune best = cands[0];
+    float best_ms = 1e30f, kernel_ms = 1e30f;
+    GlmTune best = cands[0], kernel = cands[0];   // of all, of glm_kernel's
     const char* vb = std::getenv("GBSGMC_AUTOTUNE_VERBOSE");
     const bool verbose = vb != nullptr && vb[0] == '1';
     for (const GlmTune& t : cands) {
@@ -573,15 +576,24 @@ int autotune(GlmPlan* p) {
       if (verbose)
         std::fprintf(stderr,
                      "gbsgmc autotune: slices %d rows/warp %d warps %d prefetch %d "
-                     "dynamic %d multistep %d: %.4f ms\n",
+                     "dynamic %d multistep %d loop %d: %.4f ms\n",
                      t.slices, t.rows_per_warp, t.warps, t.prefetch, t.dynamic,
-                     t.multistep, ms / 6.0f);
+                     t.multistep, t.loop, ms / 6.0f);
       if (ms < best_ms) {
         best_ms = ms;
         best = t;
       }
+      if (t.loop == 0 && ms < kernel_ms) {
+        kernel_ms = ms;
+        kernel = t;
+      }
     }
     if (rc != GBSGMC_OK) break;
+    if (best.loop > 0) {
+      kernel.loop = best.loop;
+      kernel.multistep = 1;
+      best = kernel;
+    }
     p->tune = best;
     glm_tune_store(p->chains, p->n, p->model.d, p->model.ld, best);
   } while (false);
@@ -879,7 +891,7 @@ extern "C" int gbsgmc_plan_launch_shape(const gbsgmc_plan* p, int* slices,
   *slices = *rows_per_warp = *warps = *prefetch = *dynamic = 0;
   *steps_per_launch = 1;
   if (const GlmPlan* g = dynamic_cast<const GlmPlan*>(p)) {
-    *slices = g->tune.slices;
+    *slices = g->tune.loop > 0 ? g->tune.loop : g->tune.slices;
     *rows_per_warp = g->tune.rows_per_warp;
     *warps = g->tune.warps;
     *prefetch = g->tune.prefetch;

@@ -56,3 +56,29 @@ def test_trials_stay_within_a_short_schedule(lib, monkeypatch, C, n, d, K):
   for a, b in zip(*outs):
     np.testing.assert_array_equal(a, b)
   assert np.isfinite(outs[0][1]).all() and (outs[0][1] != x0).all()
+
+
+@pytest.mark.parametrize("C,n,d", [(1, 1024, 40), (3, 1500, 24)])
+def test_a_sampler_leaves_gradient_calls_as_they_were(lib, monkeypatch, C, n, d):
+  """One evaluation before and after an SGLD plan of its shape whose form was
+  chosen without a trial: the same bits."""
+  import torch
+  from gbsgmc import engine
+  monkeypatch.delenv("GBSGMC_AUTOTUNE", raising=False)
+  _, ds, pot, x0, N = _setup(C, d)
+  idx = torch.from_numpy(np.random.default_rng(n).integers(0, N, (C, n)).astype(np.int32)).cuda()
+  K = 12
+
+  def evaluate():
+    r = pot.evaluate(_cuda(x0), idx, ds)
+    return [a.cpu().numpy() for a in (r.U, r.grad, r.lk_var)]
+
+  before = evaluate()
+  plan = engine.SgldGlmPlan(pot, ds, _cuda(x0), None, 0.9, 1e-5, n,
+                            _cuda(np.full(K, 1e-6, np.float32)), _cuda(np.ones(K, np.float32)),
+                            _cuda(np.full(K, -1, np.int32)), 0,
+                            engine.IndexSource(pcg=_cuda(_words(C))), 11, 0, K)
+  plan.run(0, K)
+  plan.check_status()
+  for a, b in zip(before, evaluate()):
+    np.testing.assert_array_equal(a, b)
