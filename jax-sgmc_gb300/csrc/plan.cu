@@ -671,7 +671,10 @@ extern "C" int gbsgmc_sgld_glm_plan_create(
     if (const char* ms = std::getenv("GBSGMC_GLM_MULTISTEP"))
       if (ms[0] == '0' || ms[0] == '1') {
         p->tune.multistep = ms[0] == '1';
-        p->tune.loop = 0;
+        if (p->tune.loop > 0) {   // one launch takes one CTA per chain of glm_kernel
+          p->tune.loop = 0;
+          if (p->tune.multistep) p->tune.slices = 1, p->tune.dynamic = 0;
+        }
       }
     if ((rc = plan_capture(p))) break;
     // GBSGMC_PLAN_PIPELINE=1 overlaps the next block's index draws with this

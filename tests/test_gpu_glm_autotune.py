@@ -82,3 +82,23 @@ def test_a_sampler_leaves_gradient_calls_as_they_were(lib, monkeypatch, C, n, d)
   plan.check_status()
   for a, b in zip(before, evaluate()):
     np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("multi,steps", [("1", 12), ("0", 1)])
+def test_forced_launch_form(lib, monkeypatch, multi, steps):
+  """GBSGMC_GLM_MULTISTEP where the plan would choose a cluster per chain: one
+  launch a block (index draw, block, counter) or one a step, as it promises."""
+  from gbsgmc import engine
+  monkeypatch.delenv("GBSGMC_AUTOTUNE", raising=False)
+  monkeypatch.setenv("GBSGMC_GLM_MULTISTEP", multi)
+  C, n, d, K = 2, 600, 17, 12
+  _, ds, pot, x0, N = _setup(C, d)
+  plan = engine.SgldGlmPlan(pot, ds, _cuda(x0), None, 0.9, 1e-5, n,
+                            _cuda(np.full(K, 1e-6, np.float32)), _cuda(np.ones(K, np.float32)),
+                            _cuda(np.full(K, -1, np.int32)), 0,
+                            engine.IndexSource(pcg=_cuda(_words(C))), 11, 0, K)
+  plan.run(0, K)
+  plan.check_status()
+  shape = plan.launch_shape()
+  assert shape[5] == steps
+  assert multi == "0" or shape[0] == 1
