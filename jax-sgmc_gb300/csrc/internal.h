@@ -113,10 +113,11 @@ struct UpdateFusion {
                                    //   c draws as chain ident[c]); null: c
 };
 int update_blocks(int chains, int64_t P);
-// At the schedule's kept steps: row 0 of x to samples[slot], -U[0] to
+// At the schedule's kept steps: the first `rows` (at most 65,535) rows of x to
+// samples[slot], sign U (with U2: sign times the mean of the two) to
 // sample_lik[slot] (may be null).
-int keep_row(int64_t P, const float* x, const double* U, const gbsgmc_sched* sched,
-             float* samples, double* sample_lik, cudaStream_t st);
+int keep_rows(int rows, int64_t P, const float* x, const double* U, const double* U2, double sign,
+              const gbsgmc_sched* sched, float* samples, double* sample_lik, cudaStream_t st);
 int sgld_update_fused(int chains, int64_t P, float* x, const float* g, float* v,
                       float alpha, float lmbd, const gbsgmc_sched* sched,
                       const gbsgmc_noise* noise, const UpdateFusion& f,

@@ -57,7 +57,8 @@ struct NetPlan final : gbsgmc_plan {
   UpdateFusion fz;          // the mirror and squares of the new positions
   float pf = 0.f;           // 1 / (s^2 T) of the prior, 0 for a flat prior
   double* sq = nullptr;     // owned [chains, update_blocks]
-  // GLM families: a block's steps in one launch (glm_loop).
+  // GLM families: a block's steps in one launch (glm_loop), or a launch per
+  // gradient and update as for the networks.
   bool loop = false;
   gbsgmc_glm glm{};
   int ctas = 1;
@@ -65,6 +66,11 @@ struct NetPlan final : gbsgmc_plan {
   double* sample_lik = nullptr;
 
   int draws() const { return integ.kind == GBSGMC_INTEGRATOR_OBABO ? 2 : 1; }
+  // Kept samples of the steps with launches of their own.
+  int keep(const double* U_second, double sign, const gbsgmc_sched& sj, cudaStream_t s) const {
+    if (sched.keep_slot_dev == nullptr) return GBSGMC_OK;
+    return keep_rows(chains, P, x, U, U_second, sign, &sj, samples, sample_lik, s);
+  }
 
   ~NetPlan() override {
     if (stream != nullptr) cudaStreamSynchronize(stream);
@@ -110,11 +116,12 @@ struct NetPlan final : gbsgmc_plan {
     // fused, the mirror.
     const int64_t fixed = (fused ? 3 : 2) - (isrc.external ? 1 : 0);
     if (loop) return fixed + 1;
+    const int64_t kept = sched.keep_slot_dev != nullptr ? g : 0;
     switch (integ.kind) {
-      case GBSGMC_INTEGRATOR_OBABO: return fixed + 2 + static_cast<int64_t>(g);
+      case GBSGMC_INTEGRATOR_OBABO: return fixed + kept + 2 + static_cast<int64_t>(g);
       case GBSGMC_INTEGRATOR_SGHMC:
-        return fixed + 2 * static_cast<int64_t>(g) + g / integ.leapfrog_steps;
-      default: return fixed + static_cast<int64_t>(g);
+        return fixed + kept + 2 * static_cast<int64_t>(g) + g / integ.leapfrog_steps;
+      default: return fixed + kept + static_cast<int64_t>(g);
     }
   }
 
@@ -176,22 +183,28 @@ struct NetPlan final : gbsgmc_plan {
       sj.base_dev = base;
       sj.offset = j;
       const int32_t* ij = idx + j * cn;
+      gbsgmc_sched su = sj;
+      su.keep_slot_dev = nullptr;   // the updates keep nothing themselves
       switch (integ.kind) {
         case GBSGMC_INTEGRATOR_SGLD:
           if ((rc = grad_fn(ij, per, U, lk_var, grad, s))) return rc;
-          rc = gbsgmc_sgld_update(chains, P, x, grad, aux, integ.alpha, integ.lmbd, &sj,
-                                  &noise, nullptr, s);
+          if ((rc = gbsgmc_sgld_update(chains, P, x, grad, aux, integ.alpha, integ.lmbd, &su,
+                                       &noise, nullptr, s)))
+            return rc;
+          rc = keep(nullptr, -1.0, sj, s);
           break;
         default:  // SGHMC
           if (j % integ.leapfrog_steps == 0 &&
-              (rc = gbsgmc_sghmc_resample(chains, P, aux, integ.mass_dev, &sj, &noise, s)))
+              (rc = gbsgmc_sghmc_resample(chains, P, aux, integ.mass_dev, &su, &noise, s)))
             return rc;
           if ((rc = gbsgmc_sghmc_position(chains, P, x, aux, integ.mass_dev, nullptr,
-                                          integ.friction, &sj, s)))
+                                          integ.friction, &su, s)))
             return rc;
           if ((rc = grad_fn(ij, per, U, lk_var, grad, s))) return rc;
-          rc = gbsgmc_sghmc_momentum(chains, P, aux, grad, nullptr, integ.friction, &sj,
-                                     &noise, s);
+          if ((rc = gbsgmc_sghmc_momentum(chains, P, aux, grad, nullptr, integ.friction, &su,
+                                          &noise, s)))
+            return rc;
+          rc = keep(nullptr, 1.0, sj, s);
           break;
       }
       if (rc != GBSGMC_OK) return rc;
@@ -277,8 +290,9 @@ int NetPlan::enqueue_obabo(int g, const UpdateFusion& moving, const UpdateFusion
   for (int j = 0; j + 1 < g; ++j) {
     const int32_t* ij = idx + j * cn;
     if ((rc = grad_fn(ij + n, per, U2, nullptr, grad2, s))) return rc;
-    if ((rc = grad_fn(ij + cn, per, U, nullptr, grad, s))) return rc;
     sj.offset = j;
+    if ((rc = keep(U2, 1.0, sj, s))) return rc;   // x is the step's, U its first value
+    if ((rc = grad_fn(ij + cn, per, U, nullptr, grad, s))) return rc;
     if ((rc = obabo_second_first_fused(chains, P, x, aux, grad2, grad, integ.mass_dev,
                                        integ.friction, ke_end, ke_start, &sj, &noise, moving,
                                        s)))
@@ -286,6 +300,7 @@ int NetPlan::enqueue_obabo(int g, const UpdateFusion& moving, const UpdateFusion
   }
   sj.offset = g - 1;
   if ((rc = grad_fn(idx + (g - 1) * cn + n, per, U2, lk_var, grad2, s))) return rc;
+  if ((rc = keep(U2, 1.0, sj, s))) return rc;
   if ((rc = obabo_second_fused(chains, P, x, aux, grad2, integ.mass_dev, integ.friction,
                                ke_end, &sj, &noise, last, s)))
     return rc;
@@ -372,7 +387,7 @@ struct ResgldPlan final : gbsgmc_plan {
                                                 nullptr, s)))
         return rc;
       if (samples != nullptr &&
-          (rc = keep_row(P, x, U, &sj, samples, sample_lik, s)))
+          (rc = keep_rows(1, P, x, U, nullptr, -1.0, &sj, samples, sample_lik, s)))
         return rc;
     }
     return plan_advance(this, g, s);
@@ -832,11 +847,12 @@ extern "C" int gbsgmc_glm_plan_create_keep(
                         noise, isrc, U_dev, block_steps, status_dev);
   if (rc != GBSGMC_OK) return rc;
   if (model == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: null model");
-  if (gbsgmc_glm_workspace_bytes(chains, n, model->d) == 0)
-    return set_error(GBSGMC_ERR_SHAPE, "glm_plan_create: bad shape");
+  const size_t ws = gbsgmc_glm_workspace_bytes(chains, n, model->d);
+  if (ws == 0) return set_error(GBSGMC_ERR_SHAPE, "glm_plan_create: bad shape");
   NetPlan* p = new (std::nothrow) NetPlan();
   if (p == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: out of memory");
-  p->loop = true;
+  // Injected normals are one step's: glm_loop would need a block's.
+  p->loop = noise->noise_dev == nullptr;
   p->glm = *model;
   p->chains = chains;
   p->n = n;
@@ -860,7 +876,24 @@ extern "C" int gbsgmc_glm_plan_create_keep(
                           p->draws() * n;
     if ((rc = plan_alloc(p, &p->idx, ibytes, "glm_plan_create: index buffer"))) break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(chains, 1, n);
+    if (p->loop) {
+      p->ctas = glm_loop_ctas(chains, 1, n);
+    } else {
+      if ((rc = p->alloc_grads("glm_plan_create: gradient"))) break;
+      if ((rc = plan_alloc(p, &p->U2, sizeof(double) * chains, "glm_plan_create: U"))) break;
+      // The workspace's tickets start at zero, as plan_alloc leaves it.
+      if ((rc = plan_alloc(p, &p->ws, ws, "glm_plan_create: workspace"))) break;
+      p->ws_size = ws;
+      const gbsgmc_glm m = *model;
+      void* wsp = p->ws;
+      const float* x = x_dev;
+      p->grad_fn = [m, chains, n, x, wsp, ws, status_dev](
+                       const int32_t* idx, int64_t stride, double* U, double* var, float* grad,
+                       cudaStream_t s) {
+        return gbsgmc_glm_value_and_grad(&m, chains, n, idx, stride, nullptr, x, U, grad, nullptr,
+                                         var, wsp, ws, status_dev, s);
+      };
+    }
     if ((rc = p->setup_external("glm_plan_create: index memset"))) break;
     rc = plan_capture(p);
   } while (false);

@@ -441,8 +441,12 @@ namespace {
 int autotune(GlmPlan* p) {
   const char* env = std::getenv("GBSGMC_AUTOTUNE");
   if (env != nullptr && env[0] == '0') return GBSGMC_OK;
-  if (glm_tune_lookup(p->chains, p->n, p->model.d, p->model.ld, &p->tune))
+  // Injected normals are one step's: no form that runs several a launch.
+  const bool injected = p->noise.noise_dev != nullptr;
+  if (glm_tune_lookup(p->chains, p->n, p->model.d, p->model.ld, &p->tune)) {
+    if (injected && p->tune.loop > 0) p->tune.loop = p->tune.multistep = 0;
     return GBSGMC_OK;
+  }
   const int C = p->chains, n = p->n, d = p->model.d;
   const size_t wbytes = sizeof(float) * static_cast<size_t>(C) * d;
   float* w = nullptr;
@@ -458,7 +462,7 @@ int autotune(GlmPlan* p) {
   GlmTune loop;
   loop.loop = glm_loop_ctas(C, 1, n);
   loop.multistep = 1;
-  if (2 * C <= glm_sm_count()) {
+  if (2 * C <= glm_sm_count() && !injected) {
     p->tune = loop;
     return GBSGMC_OK;
   }
@@ -497,7 +501,7 @@ int autotune(GlmPlan* p) {
         cands.push_back(t);
       }
     }
-    if (p->G >= 6) cands.push_back(loop);
+    if (p->G >= 6 && !injected) cands.push_back(loop);
   }
   if (cands.size() <= 1) {
     if (!cands.empty()) p->tune = cands[0];

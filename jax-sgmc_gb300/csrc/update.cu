@@ -995,27 +995,31 @@ namespace gbsgmc {
 
 int update_blocks(int chains, int64_t P) { return static_cast<int>(grid4(chains, P).grid.x); }
 
-// At kept steps (the schedule's keep slot >= 0) row 0 of x [., P] is copied to
-// samples [slot, P] and -U[0] to sample_lik[slot].
-__global__ void keep_row_kernel(int64_t P, const float* __restrict__ x,
-                                const double* __restrict__ U, Sched sched, float* samples,
-                                double* sample_lik) {
+// At kept steps (the schedule's keep slot >= 0) the rows of x [rows, P] are
+// copied to samples [slot, rows, P] and sign U, of two potentials their mean,
+// to sample_lik [slot, rows].
+__global__ void keep_rows_kernel(int rows, int64_t P, const float* __restrict__ x,
+                                 const double* __restrict__ U, const double* __restrict__ U2,
+                                 double sign, Sched sched, float* samples, double* sample_lik) {
   pdl_trigger();
   pdl_wait();
   const int slot = sched.keep_slot(sched.step());
   if (slot < 0) return;
+  const int64_t at = static_cast<int64_t>(slot) * rows + blockIdx.y;
   for (int64_t j = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; j < P;
        j += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    samples[static_cast<int64_t>(slot) * P + j] = x[j];
+    samples[at * P + j] = x[blockIdx.y * P + j];
   if (blockIdx.x == 0 && threadIdx.x == 0 && sample_lik != nullptr)
-    sample_lik[slot] = -U[0];
+    sample_lik[at] =
+        sign * (U2 != nullptr ? 0.5 * (U[blockIdx.y] + U2[blockIdx.y]) : U[blockIdx.y]);
 }
 
-int keep_row(int64_t P, const float* x, const double* U, const gbsgmc_sched* sched,
-             float* samples, double* sample_lik, cudaStream_t st) {
-  const int blocks = static_cast<int>(std::min<int64_t>((P + 1023) / 1024, 1024));
-  launch_pdl(keep_row_kernel, blocks, 256, 0, st, P, x, U, to_sched(sched), samples, sample_lik);
-  return check_launch("keep_row");
+int keep_rows(int rows, int64_t P, const float* x, const double* U, const double* U2, double sign,
+              const gbsgmc_sched* sched, float* samples, double* sample_lik, cudaStream_t st) {
+  const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((P + 1023) / 1024, 1024));
+  launch_pdl(keep_rows_kernel, dim3(blocks, static_cast<unsigned>(rows)), 256, 0, st, rows, P, x,
+             U, U2, sign, to_sched(sched), samples, sample_lik);
+  return check_launch("keep_rows");
 }
 
 int sgld_update_fused(int chains, int64_t P, float* x, const float* g, float* v,

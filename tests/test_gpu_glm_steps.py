@@ -1,0 +1,127 @@
+"""GLM plans that launch every gradient and update by itself, against the
+oracle's trajectories on the same indices and normals.
+
+Tolerance (as for the other K-step trajectories): 1e-4 relative plus 1e-5
+absolute; U within 1e-5 relative plus 1e-3 absolute.
+"""
+
+import numpy as np
+import pytest
+
+from oracle import sgmc_oracle as O
+
+pytestmark = pytest.mark.gpu
+K = 6
+
+
+def _cuda(a):
+  import torch
+  return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def _words(C):
+  from gbsgmc.data.numpy_loader import pcg64_words
+  return np.array([pcg64_words(c) for c in range(C)], np.uint64).view(np.int64)
+
+
+def _setup(C, n, d, N=5003):
+  from gbsgmc import data, likelihoods as L, potential
+  rng = np.random.default_rng(100 * d + n)
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (rng.random(N) < 1 / (1 + np.exp(-(X @ rng.normal(size=d) / np.sqrt(d))))).astype(np.float32)
+  pot = potential.minibatch_potential(L.GaussianPrior(3.0), L.Logistic())
+  x0 = (0.1 * rng.normal(size=(C, d))).astype(np.float32)
+  return X, y, data.NumpyDataLoader(x=X, y=y).device_dataset(), pot, x0, N
+
+
+def _schedule(kind, n, d, N):
+  curvature = N * 0.25 * max(1.0, 2.0 * d / n)
+  h0 = 0.02 / curvature if kind == "langevin" else 0.02 / np.sqrt(curvature)
+  return (h0 * 0.9 ** np.arange(K)).astype(np.float32)
+
+
+def _trajectory(kind, X, y, x0, idx, xi, h, leapfrog, N):
+  """Positions, momenta, kept positions and potentials of every step; xi(tag,
+  k) gives the normals."""
+  w, p, xs, Us = x0.copy(), np.zeros_like(x0), [], []
+  at = lambda w, j: O.glm_potential(w, X, y, idx[j], N, O.LOGISTIC, 1.0, 3.0)  # noqa: E731
+  for k in range(K):
+    if kind == "langevin":
+      r = at(w, k)
+      w, _ = O.sgld_step(w, r.grad.astype(np.float32), None, xi(0, k), h[k], 1.0, rms_prop=False)
+      U = -r.U
+    elif kind == "obabo":
+      a = at(w, 2 * k)
+      w, p, _ = O.obabo_first(w, p, a.grad.astype(np.float32), xi(1, k), h[k], 1.0, 2.0)
+      b = at(w, 2 * k + 1)
+      p, _ = O.obabo_second(p, b.grad.astype(np.float32), xi(2, k), h[k], 1.0, 2.0)
+      U = 0.5 * (a.U + b.U)
+    else:
+      if k % leapfrog == 0:
+        p = O.sghmc_resample(xi(3, k))
+      w, p = O.sghmc_position(w, p, h[k], 2.0)
+      r = at(w, k)
+      p = O.sghmc_momentum(p, r.grad.astype(np.float32), xi(4, k), h[k], 2.0)
+      U = r.U
+    xs.append(w)
+    Us.append(U)
+  return w, p, np.stack(xs), np.stack(Us)
+
+
+def _draws(C, n, N, count):
+  return np.stack([O.loader_draws(O.loader_rng(c), N, n, count) for c in range(C)], 1)
+
+
+@pytest.mark.parametrize("C,n,d", [(1, 33, 1), (3, 200, 129), (170, 40, 6)])
+@pytest.mark.parametrize("kind", ["langevin", "obabo", "sghmc"])
+def test_injected_normals(lib, monkeypatch, kind, C, n, d):
+  """A plan whose caller gives the normals, with kept samples."""
+  from gbsgmc import _lib, engine
+  X, y, ds, pot, x0, N = _setup(C, n, d)
+  z = np.random.default_rng(5).normal(size=(C, d)).astype(np.float32)
+  zd, make = _cuda(z), _lib.noise
+  monkeypatch.setattr(_lib, "noise", lambda *a: make(*a, noise_dev=zd, noise_stride=d))
+  h = _schedule(kind, n, d, N)
+  keep = np.array([-1, 0, -1, 1, -1, 2], np.int32)
+  draws = 2 if kind == "obabo" else 1
+  pcg, x = _cuda(_words(C)), _cuda(x0)
+  aux = None if kind == "langevin" else _cuda(np.zeros_like(x0))
+  kw = {} if kind == "langevin" else dict(friction=2.0, leapfrog_steps=3)
+  plan = engine.NetPlan(pot, ds, x, aux, n, kind, _cuda(h), _cuda(np.ones(K, np.float32)),
+                        engine.IndexSource(pcg=pcg), 11, block_steps=3, keep_tab=_cuda(keep),
+                        n_kept=3, **kw)
+  plan.run(0, K)
+  plan.check_status()
+  w, p, xs, Us = _trajectory(kind, X, y, x0, _draws(C, n, N, K * draws), lambda tag, k: z, h, 3, N)
+  tol = dict(rtol=1e-4, atol=1e-5)
+  np.testing.assert_allclose(x.cpu().numpy(), w, **tol)
+  np.testing.assert_allclose(plan.samples.cpu().numpy(), xs[keep >= 0], **tol)
+  np.testing.assert_allclose(plan.sample_lik.cpu().numpy(), Us[keep >= 0], rtol=1e-5, atol=1e-3)
+  if aux is not None:
+    np.testing.assert_allclose(aux.cpu().numpy(), p, rtol=1e-4, atol=1e-4 * np.abs(p).max())
+
+
+@pytest.mark.parametrize("C,n,d,block", [(2, 1100, 40, 6), (2, 90, 12, 3)])
+def test_injected_normals_sgld_plan(lib, monkeypatch, C, n, d, block):
+  """The SGLD plan of few chains: minibatches above 1,024 rows or blocks below
+  six steps, also where a plan with its own normals has made its choice."""
+  from gbsgmc import _lib, engine
+  monkeypatch.delenv("GBSGMC_AUTOTUNE", raising=False)
+  X, y, ds, pot, x0, N = _setup(C, n, d)
+  h = _schedule("langevin", n, d, N)
+  z = np.random.default_rng(6).normal(size=(C, d)).astype(np.float32)
+  zd, make = _cuda(z), _lib.noise
+
+  def run():
+    x = _cuda(x0)
+    plan = engine.SgldGlmPlan(pot, ds, x, None, 0.9, 1e-5, n, _cuda(h),
+                              _cuda(np.ones(K, np.float32)), _cuda(np.full(K, -1, np.int32)), 0,
+                              engine.IndexSource(pcg=_cuda(_words(C))), 11, 0, block)
+    plan.run(0, K)
+    plan.check_status()
+    return x.cpu().numpy()
+
+  run()
+  monkeypatch.setattr(_lib, "noise", lambda *a: make(*a, noise_dev=zd, noise_stride=d))
+  w, _, _, _ = _trajectory("langevin", X, y, x0, _draws(C, n, N, K), lambda tag, k: z, h, 3, N)
+  np.testing.assert_allclose(run(), w, rtol=1e-4, atol=1e-5)
