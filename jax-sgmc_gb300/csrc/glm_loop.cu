@@ -1043,6 +1043,39 @@ int glm_loop_ctas(int units, int chains_per_unit, int n) {
   return s;
 }
 
+// A CTA streams its rows at 11 to 47 GB/s (12 ns a row of up to 128 features,
+// 21 of 256, 110 of 1,000), so that few CTAs with many rows each take longer
+// than launches per gradient, which spread a chain over up to 64 CTAs.  The
+// line between them by the rows of a CTA, the width (float4 columns per lane)
+// and the share of the SMs that the clusters keep busy over their waves; us
+// an OBABO step, this form and the other: one chain of 16,384 rows of 256
+// features 90 and 130, of 65,536 353 and 212, of 65,536 x 1,000 1,858 and 413;
+// 16 of 8,192 x 256 83 and 97, of 16,384 164 and 155; 100 of 4,096 x 256 150
+// and 200, of 16,384 598 and 557; 64 of 2,048 x 1,000 206 and 256, of 8,192
+// 797 and 786.  One table serves SGHMC and the pairs too, whose lines lie up to
+// a third lower: over some 2,300 shapes of 1 to 600 chains, 256 to 65,536 rows
+// and 8 to 1,000 features this form is nowhere taken where it is more than 5 %
+// slower, and nowhere left where it is more than a third faster.
+bool glm_loop_pays(int units, int chains_per_unit, int n, int d) {
+  struct Line {
+    double busy;
+    int rows[4];   // 1, 2, 4, 8 float4 columns per lane
+  };
+  constexpr int kAny = 1 << 30;
+  constexpr Line kLines[] = {{0.25, {5000, 3000, 1000, 350}},
+                             {0.5, {8200, 4000, 1000, 400}},
+                             {0.8, {20000, 6000, 2500, 1000}},
+                             {0.95, {kAny, 20000, 8000, 1400}},
+                             {1.0, {kAny, kAny, kAny, 12000}}};
+  const int ctas = glm_loop_ctas(units, chains_per_unit, n);
+  const int64_t used = static_cast<int64_t>(units) * chains_per_unit * ctas, sms = glm_sm_count();
+  const double busy = static_cast<double>(used) / (sms * ((used + sms - 1) / sms));
+  const int qpl = glm_qpl((d + 3) / 4), width = qpl == 1 ? 0 : qpl == 2 ? 1 : qpl == 4 ? 2 : 3;
+  for (const Line& l : kLines)
+    if (busy <= l.busy) return ceil_div(n, ctas) <= l.rows[width];
+  return true;
+}
+
 namespace {
 
 // Rows a warp takes at once: its whole share of the slice where the registers

@@ -61,6 +61,8 @@ struct GlmLoopCall {
   int* status = nullptr;
 };
 int glm_loop_ctas(int units, int chains_per_unit, int n);
+// Whether that is faster than launches per gradient and update.
+bool glm_loop_pays(int units, int chains_per_unit, int n, int d);
 int glm_loop_prepare();
 int glm_loop(const GlmLoopCall& c, cudaStream_t st);
 // glm.cu: the float4 columns per lane of a row of dq float4, and the device's

@@ -852,7 +852,7 @@ extern "C" int gbsgmc_glm_plan_create_keep(
   NetPlan* p = new (std::nothrow) NetPlan();
   if (p == nullptr) return set_error(GBSGMC_ERR_ARG, "glm_plan_create: out of memory");
   // Injected normals are one step's: glm_loop would need a block's.
-  p->loop = noise->noise_dev == nullptr;
+  p->loop = noise->noise_dev == nullptr && glm_loop_pays(chains, 1, n, model->d);
   p->glm = *model;
   p->chains = chains;
   p->n = n;

@@ -125,3 +125,33 @@ def test_injected_normals_sgld_plan(lib, monkeypatch, C, n, d, block):
   monkeypatch.setattr(_lib, "noise", lambda *a: make(*a, noise_dev=zd, noise_stride=d))
   w, _, _, _ = _trajectory("langevin", X, y, x0, _draws(C, n, N, K), lambda tag, k: z, h, 3, N)
   np.testing.assert_allclose(run(), w, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("C,n,d,block", [(1, 8100, 260, False), (1, 7000, 260, True),
+                                         (2, 2900, 1000, False), (96, 50, 3, True)])
+@pytest.mark.parametrize("kind", ["obabo", "sghmc"])
+def test_long_minibatches_of_few_chains(lib, kind, C, n, d, block):
+  """Few chains with long minibatches get launches of their own for every
+  gradient, which spread a chain over more CTAs than a cluster has; others run
+  a block of steps in one launch."""
+  from gbsgmc import engine
+  X, y, ds, pot, x0, N = _setup(C, n, d, N=9001)
+  h = _schedule(kind, n, d, N)
+  keep = np.array([0, -1, 1, -1, -1, 2], np.int32)
+  draws = 2 if kind == "obabo" else 1
+  x, aux = _cuda(x0), _cuda(np.zeros_like(x0))
+  plan = engine.NetPlan(pot, ds, x, aux, n, kind, _cuda(h), _cuda(np.ones(K, np.float32)),
+                        engine.IndexSource(pcg=_cuda(_words(C))), 11, block_steps=3,
+                        keep_tab=_cuda(keep), n_kept=3, friction=2.0, leapfrog_steps=3)
+  plan.run(0, K)
+  plan.check_status()
+  per_block = engine._plan_launches(plan.handle, 2 * 3) - engine._plan_launches(plan.handle, 3)
+  assert (per_block == 3) == block   # index draw, block, counter
+  xi = lambda tag, k: np.stack([O.philox_normals(11, c, k, tag, d)  # noqa: E731
+                                for c in range(C)]).astype(np.float32)
+  w, p, xs, Us = _trajectory(kind, X, y, x0, _draws(C, n, N, K * draws), xi, h, 3, N)
+  tol = dict(rtol=1e-4, atol=1e-5)
+  np.testing.assert_allclose(x.cpu().numpy(), w, **tol)
+  np.testing.assert_allclose(plan.samples.cpu().numpy(), xs[keep >= 0], **tol)
+  np.testing.assert_allclose(plan.sample_lik.cpu().numpy(), Us[keep >= 0], rtol=1e-5, atol=1e-3)
+  np.testing.assert_allclose(aux.cpu().numpy(), p, rtol=1e-4, atol=1e-4 * np.abs(p).max())
