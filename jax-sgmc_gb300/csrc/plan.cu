@@ -455,14 +455,16 @@ int autotune(GlmPlan* p) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   int rc = GBSGMC_OK;
   std::vector<GlmTune> cands;
-  // With no more chains than half the SMs, blocks run as one glm_loop launch
-  // with a cluster per chain: every other form leaves SMs idle or pays a
-  // launch per step (one chain, n = 128, d = 32: 10.9 us a step against 1.5;
-  // 24 chains, n = 500, d = 101: 18.8 us a gradient against 3.0).
+  // Few chains and minibatches well below glm_loop_pays' line: blocks run as
+  // one glm_loop launch with a cluster per chain, untimed; every other form
+  // leaves SMs idle or pays a launch per step (one chain, n = 128, d = 32: 10.9
+  // us a step against 1.5; 16 of 4,096 x 256: 33 against 22).  From half that
+  // line on it is one of the forms that are timed (one chain of 65,536 x 256:
+  // 178 us a step against glm_kernel's 91).
   GlmTune loop;
   loop.loop = glm_loop_ctas(C, 1, n);
   loop.multistep = 1;
-  if (2 * C <= glm_sm_count() && !injected) {
+  if (2 * C <= glm_sm_count() && !injected && glm_loop_pays(C, 1, 2 * n, d)) {
     p->tune = loop;
     return GBSGMC_OK;
   }

@@ -6,6 +6,8 @@ and report to a scratch status word.
 import numpy as np
 import pytest
 
+from oracle import sgmc_oracle as O
+
 pytestmark = pytest.mark.gpu
 
 
@@ -102,3 +104,33 @@ def test_forced_launch_form(lib, monkeypatch, multi, steps):
   shape = plan.launch_shape()
   assert shape[5] == steps
   assert multi == "0" or shape[0] == 1
+
+
+@pytest.mark.parametrize("n,d,block", [(400, 1000, True), (30000, 1000, False)])
+def test_few_chains_with_long_minibatches(lib, monkeypatch, n, d, block):
+  """One chain: a cluster and one launch a block for short minibatches, a
+  launch a step over more CTAs for one that takes a cluster six times as long,
+  against the oracle (1e-4 relative plus 1e-5 absolute)."""
+  from gbsgmc import engine
+  monkeypatch.delenv("GBSGMC_AUTOTUNE", raising=False)
+  N, K = 30011, 6
+  _, ds, pot, x0, N = _setup(1, d, N)
+  rng = np.random.default_rng(d)   # as _setup draws them
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (rng.random(N) < 0.5).astype(np.float32)
+  h = (0.02 / (0.25 * N * max(1.0, 2.0 * d / n)) * 0.9 ** np.arange(K)).astype(np.float32)
+  x = _cuda(x0)
+  plan = engine.SgldGlmPlan(pot, ds, x, None, 0.9, 1e-5, n, _cuda(h),
+                            _cuda(np.ones(K, np.float32)), _cuda(np.full(K, -1, np.int32)), 0,
+                            engine.IndexSource(pcg=_cuda(_words(1))), 11, 0, K)
+  plan.run(0, K)
+  plan.check_status()
+  assert (plan.launch_shape()[5] == K) == block
+  idx = O.loader_draws(O.loader_rng(0), N, n, K)
+  w = x0
+  for k in range(K):
+    r = O.glm_potential(w, X, y, idx[k][None], N, O.LOGISTIC, 1.0, 3.0)
+    w, _ = O.sgld_step(w, r.grad.astype(np.float32), None,
+                       O.philox_normals(11, 0, k, 0, d)[None].astype(np.float32), h[k], 1.0,
+                       rms_prop=False)
+  np.testing.assert_allclose(x.cpu().numpy(), w, rtol=1e-4, atol=1e-5)
