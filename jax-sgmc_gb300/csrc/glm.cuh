@@ -55,6 +55,9 @@ struct GlmArgs {
   int dyn_fixed;      // 1: dynamically scheduled kernel, -1: not, 0: library choice
   int* status;
   int vec4;   // rows are 16-byte aligned: 128-bit loads
+  // Replica exchange: chain c's index row and noise stream belong to chain
+  // ident[c] (the states that moved into c with an exchange); NULL: c itself.
+  const int32_t* ident;
 };
 
 // Checks a model and its minibatches and fills the arguments common to every
@@ -62,6 +65,11 @@ struct GlmArgs {
 int glm_fill_args(GlmArgs& a, const gbsgmc_glm* m, int chains, int n, const int32_t* idx,
                   int64_t idx_stride, const float* mask, void* ws, size_t ws_size, int* status,
                   GlmTune tune);
+
+// The chain whose index row and noise stream chain (slot) c uses.
+__device__ __forceinline__ int ident_of(const GlmArgs& a, int c) {
+  return a.ident != nullptr ? __ldg(a.ident + c) : c;
+}
 
 // Bernoulli-logit log-likelihood y z - softplus(z) and its derivative
 // y - sigmoid(z), from one exponential: e = exp(-|z|),

@@ -82,7 +82,8 @@ int glm_sgld_step(const gbsgmc_glm* model, int chains, int n,
                   double* U_dev, double* lk_var_dev, float* samples_dev,
                   double* sample_lik_dev, void* ws, size_t ws_size,
                   int* status_dev, cudaStream_t stream, GlmTune tune,
-                  int steps = 1, int64_t idx_step_stride = 0);
+                  int steps = 1, int64_t idx_step_stride = 0,
+                  const int32_t* ident_dev = nullptr);
 // The exchange of reSGLD (normal, hot) pairs on the device after a step of
 // all 2 * pairs chains (normal chain p in slot p, its hot partner in slot
 // pairs + p): solver.parallel_tempering's rule per pair in FP64, and for a

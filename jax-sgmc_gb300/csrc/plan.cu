@@ -709,7 +709,8 @@ namespace {
 // belong to chain identities that travel with exchanged states: identity i
 // draws its own indices (buffer [G, 2P, n] by identity) and its own noise
 // (chain id chain_base + i), and slot s runs identity ident[s].  A block of
-// steps is one glm_loop launch, a cluster per pair.
+// steps is one glm_loop launch, a cluster per pair, or beyond its line
+// (glm_loop_pays) a launch per step and exchange.
 struct GlmPairsPlan final : gbsgmc_plan {
   gbsgmc_glm model;
   int pairs = 0, n = 0;
@@ -727,15 +728,22 @@ struct GlmPairsPlan final : gbsgmc_plan {
   float* samples = nullptr;
   double* sample_lik = nullptr;
   int* status = nullptr;
-  int ctas = 1;  // CTAs per chain
+  bool loop = true;
+  int ctas = 1;  // loop: CTAs per chain
+  gbsgmc::GlmTune tune;   // steps: their launch shape and workspace
+  void* ws = nullptr;
+  size_t ws_size = 0;
   int32_t* idx = nullptr;
 
   ~GlmPairsPlan() override {
     if (stream != nullptr) cudaStreamSynchronize(stream);
+    gbsgmc::plan_free(this, ws);
     gbsgmc::plan_free(this, idx);
   }
-  // The index draw, the block's steps, the step counter.
-  int64_t launches_per_block(int) const override { return 3; }
+  // The index draw, the block's steps (and exchanges), the step counter.
+  int64_t launches_per_block(int g) const override {
+    return loop ? 3 : 2 + 2 * static_cast<int64_t>(g);
+  }
   int enqueue(int g, cudaStream_t s) override {
     using namespace gbsgmc;
     const int chains = 2 * pairs;
@@ -744,6 +752,22 @@ struct GlmPairsPlan final : gbsgmc_plan {
     int rc = gbsgmc_index_draw_pcg64(isrc.pcg_dev, chains, rows, static_cast<int64_t>(g) * n,
                                      n, idx, n, cn, status, s);
     if (rc != GBSGMC_OK) return rc;
+    for (int j = 0; !loop && j < g; ++j) {
+      gbsgmc_sched sj = sched;
+      sj.base_dev = base;
+      sj.offset = j;
+      gbsgmc_sched step_sched = sj;
+      step_sched.keep_slot_dev = nullptr;  // the exchange stores the samples
+      rc = glm_sgld_step(&model, chains, n, idx + j * cn, n, w, v, alpha, lmbd, &step_sched,
+                         &noise, U, lk_var, nullptr, nullptr, ws, ws_size, status, s, tune, 1, 0,
+                         ident);
+      if (rc != GBSGMC_OK) return rc;
+      rc = resgld_pairs_exchange(pairs, model.d, w, v, U, lk_var, ident, &sj, temp.F, temp.seed,
+                                 pair_chain, temp.ssq_dev, temp.k_dev, temp.counts_dev, samples,
+                                 sample_lik, s);
+      if (rc != GBSGMC_OK) return rc;
+    }
+    if (!loop) return plan_advance(this, g, s);
     gbsgmc_sched s0 = sched;
     s0.base_dev = base;
     s0.offset = 0;
@@ -839,7 +863,16 @@ extern "C" int gbsgmc_glm_resgld_plan_create(
                          "glm_resgld_plan_create: index buffer")))
       break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(pairs, 2, n);
+    p->loop = glm_loop_pays(pairs, 2, n, model->d);
+    if (p->loop) {
+      p->ctas = glm_loop_ctas(pairs, 2, n);
+    } else {
+      p->ws_size = glm_ws_bytes(chains, n, model->d);
+      if ((rc = plan_alloc(p, &p->ws, p->ws_size, "glm_resgld_plan_create: workspace"))) break;
+      // The cached launch shape of this problem, or the library's default.
+      glm_tune_lookup(chains, n, model->d, model->ld, &p->tune);
+      p->tune.multistep = 0;
+    }
     rc = plan_capture(p);
   } while (false);
   if (rc != GBSGMC_OK) {

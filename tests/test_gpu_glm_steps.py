@@ -155,3 +155,36 @@ def test_long_minibatches_of_few_chains(lib, kind, C, n, d, block):
   np.testing.assert_allclose(plan.samples.cpu().numpy(), xs[keep >= 0], **tol)
   np.testing.assert_allclose(plan.sample_lik.cpu().numpy(), Us[keep >= 0], rtol=1e-5, atol=1e-3)
   np.testing.assert_allclose(aux.cpu().numpy(), p, rtol=1e-4, atol=1e-4 * np.abs(p).max())
+
+
+@pytest.mark.parametrize("n,d,block", [(5000, 300, False), (1600, 1000, False), (900, 300, True)])
+def test_long_minibatches_of_pairs(lib, monkeypatch, n, d, block):
+  """alias.re_sgld of one pair on both sides of the line between the block
+  launch and launches per step, against one chain at a time (other launch
+  shapes, so other summation orders: 1e-4 relative)."""
+  from gbsgmc import alias, data, engine, likelihoods as L, potential
+  rng = np.random.default_rng(d)
+  N = 6000
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (X @ rng.normal(size=d) / np.sqrt(d) + 0.5 * rng.normal(size=N)).astype(np.float32)
+  pot = potential.minibatch_potential(L.GaussianPrior(10.0), L.LinearGaussian(sigma=0.5))
+  inits = [({"w": (0.1 * rng.normal(size=d)).astype(np.float32)},
+            {"w": (0.1 * rng.normal(size=d)).astype(np.float32)}) for _ in range(2)]
+  first = 0.05 / (4 * N * max(1.0, 2.0 * d / n))
+  blocks = []
+  run_plan = engine.ResgldPairsPlan.run
+  monkeypatch.setattr(engine.ResgldPairsPlan, "run", lambda p, *a: (
+      blocks.append(p.launches(2 * 7) - p.launches(7)), run_plan(p, *a))[1])
+  outs = []
+  for fused in (True, False):
+    run = alias.re_sgld(pot, data.NumpyDataLoader(x=X, y=y), cache_size=7, batch_size=n,
+                        temperature=50.0, first_step_size=first,
+                        last_step_size=0.5 * first, burn_in=6, accepted_samples=6)
+    monkeypatch.setattr(engine, "FUSED_ENABLED", fused)
+    outs.append(run(*inits, iterations=12))
+  assert [b == 3 for b in blocks] == [block]   # index draw, block, counter
+  for a, b in zip(*outs):
+    np.testing.assert_allclose(a["samples"]["variables"]["w"], b["samples"]["variables"]["w"],
+                               rtol=1e-4, atol=1e-5)
+    np.testing.assert_allclose(a["samples"]["likelihood"], b["samples"]["likelihood"],
+                               rtol=1e-5, atol=1e-3)
