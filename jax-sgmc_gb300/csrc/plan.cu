@@ -710,7 +710,7 @@ namespace {
 // draws its own indices (buffer [G, 2P, n] by identity) and its own noise
 // (chain id chain_base + i), and slot s runs identity ident[s].  A block of
 // steps is one glm_loop launch, a cluster per pair, or beyond its line
-// (glm_loop_pays) a launch per step and exchange.
+// (glm_loop_pays) and with injected normals a launch per step and exchange.
 struct GlmPairsPlan final : gbsgmc_plan {
   gbsgmc_glm model;
   int pairs = 0, n = 0;
@@ -863,7 +863,7 @@ extern "C" int gbsgmc_glm_resgld_plan_create(
                          "glm_resgld_plan_create: index buffer")))
       break;
     if ((rc = glm_prepare())) break;
-    p->loop = glm_loop_pays(pairs, 2, n, model->d);
+    p->loop = noise->noise_dev == nullptr && glm_loop_pays(pairs, 2, n, model->d);
     if (p->loop) {
       p->ctas = glm_loop_ctas(pairs, 2, n);
     } else {

@@ -188,3 +188,32 @@ def test_long_minibatches_of_pairs(lib, monkeypatch, n, d, block):
                                rtol=1e-4, atol=1e-5)
     np.testing.assert_allclose(a["samples"]["likelihood"], b["samples"]["likelihood"],
                                rtol=1e-5, atol=1e-3)
+
+
+def test_injected_normals_of_pairs(lib, monkeypatch):
+  """A pairs plan given its first step's Philox normals makes that step."""
+  import torch
+  from gbsgmc import _lib, engine
+  P, n, d = 3, 200, 33
+  X, y, ds, pot, _, N = _setup(2 * P, n, d)
+  x0 = (0.1 * np.random.default_rng(1).normal(size=(2 * P, d))).astype(np.float32)
+  z = _cuda(np.stack([O.philox_normals(11, c, 0, 0, d) for c in range(2 * P)]).astype(np.float32))
+  make, outs = _lib.noise, []
+  for injected in (False, True):
+    if injected:
+      monkeypatch.setattr(_lib, "noise", lambda *a: make(*a, noise_dev=z, noise_stride=d))
+    x = _cuda(x0)
+    ident = torch.arange(2 * P, dtype=torch.int32, device="cuda").view(P, 2).T.reshape(-1)
+    ladder = torch.tensor([1.0] * P + [50.0] * P, device="cuda")
+    plan = engine.ResgldPairsPlan(
+        pot, ds, x, None, 0.9, 1e-5, n, _cuda(np.full(1, 1e-5, np.float32)),
+        _cuda(np.ones(1, np.float32)), _cuda(np.full(1, -1, np.int32)), ladder, 0,
+        _cuda(_words(2 * P)), ident.contiguous(),
+        torch.arange(0, 2 * P, 2, dtype=torch.int32, device="cuda"),
+        torch.zeros(P, dtype=torch.float64, device="cuda"),
+        torch.zeros(P, dtype=torch.int64, device="cuda"), 1.0, 5, 11, 0, 1)
+    plan.run(0, 1)
+    plan.check_status()
+    outs.append([a.cpu().numpy() for a in (x, plan.U, plan.lk_var, plan.ident)])
+  for a, b in zip(*outs):
+    np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-6)
