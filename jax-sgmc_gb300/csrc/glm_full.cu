@@ -2,7 +2,7 @@
 //   U_c = (-sum_i lk_i(w_c) - log p(w_c)) / T over every observation
 // (potential.py:219-293), and the Metropolis-Hastings samplers built on it:
 // AMAGOLD and SGGMC (solver.py:301-577) with the proposals' trajectories as
-// glm_loop launches.
+// glm_loop launches, or as launches per gradient and update beyond its line.
 //
 // glm_full_kernel is a tall matrix product (rows x chains over d) whose
 // outputs never leave the registers: thread t of a 128-thread CTA owns rows t
@@ -313,6 +313,7 @@ int full_args(GlmArgs& a, const gbsgmc_glm* m, int chains, const float* w, int* 
 struct GlmMhPlan final : gbsgmc_plan {
   gbsgmc_glm model, full;
   int chains = 0, n = 0, steps = 0, ctas = 1;
+  bool loop = true;
   gbsgmc_integrator integ{};
   gbsgmc_sched sched{};
   gbsgmc_noise noise{};
@@ -323,6 +324,12 @@ struct GlmMhPlan final : gbsgmc_plan {
   float* old = nullptr;     // owned [2, chains, d]
   double* acc = nullptr;    // owned: energy [C], ke [2 C], U [C], lk_var [C]
   double* part = nullptr;   // owned
+  // Trajectories by launches: gradient [chains, d], the second minibatch's
+  // potential, workspace of the gradient calls (all owned).
+  float* grad = nullptr;
+  double* U2 = nullptr;
+  void* ws = nullptr;
+  size_t ws_size = 0;
 
   bool amagold() const { return mh.kind == GBSGMC_MH_AMAGOLD; }
   int draws() const { return amagold() ? 1 : 2; }
@@ -332,11 +339,56 @@ struct GlmMhPlan final : gbsgmc_plan {
     plan_free(this, old);
     plan_free(this, acc);
     plan_free(this, part);
+    plan_free(this, grad);
+    plan_free(this, U2);
+    plan_free(this, ws);
   }
   int step_multiple() const override { return steps; }
   // Index draw and step counter, and per iteration the trajectory, the
   // full-data pass and the decision.
-  int64_t launches_per_block(int g) const override { return 2 + 3 * (g / steps); }
+  int64_t launches_per_block(int g) const override {
+    const int64_t traj = loop ? 1 : amagold() ? 3 * int64_t{steps} + 1 : 4 * int64_t{steps} + 1;
+    return 2 + (traj + 2) * (g / steps);
+  }
+
+  int gradient(const int32_t* ix, int64_t stride, double* U, cudaStream_t s) const {
+    return gbsgmc_glm_value_and_grad(&model, chains, n, ix, stride, nullptr, mh.x, U, grad,
+                                     nullptr, nullptr, ws, ws_size, status, s);
+  }
+
+  // The trajectory of the iteration whose first step is j, a launch at a time:
+  // the reversible leapfrog (integrator.py:349-560; half a position step at
+  // both ends) or OBABO (integrator.py:138-346).
+  int trajectory(int j, int64_t cn, int per, cudaStream_t s) const {
+    const int d = model.d;
+    const float f = integ.friction;
+    gbsgmc_sched sj = sched;
+    sj.base_dev = base;
+    sj.keep_slot_dev = nullptr;
+    int rc;
+    for (int i = 0; i < steps; ++i) {
+      const int32_t* ix = idx + (j + i) * cn;
+      sj.offset = j + i;
+      if (amagold()) {
+        if ((rc = gbsgmc_leapfrog_position(chains, d, mh.x, mh.p, nullptr, i == 0 ? 0.5f : 1.0f,
+                                           &sj, s)) ||
+            (rc = gradient(ix, per, mh.U_mean, s)) ||
+            (rc = gbsgmc_amagold_momentum(chains, d, mh.p, grad, nullptr, f, mh.energy, &sj, &noise,
+                                          s)))
+          return rc;
+      } else {
+        if ((rc = gradient(ix, per, mh.U_mean, s)) ||
+            (rc = gbsgmc_obabo_first(chains, d, mh.x, mh.p, grad, nullptr, f, mh.ke, &sj, &noise,
+                                     s)) ||
+            (rc = gradient(ix + n, per, U2, s)) ||
+            (rc = gbsgmc_obabo_second(chains, d, mh.p, grad, nullptr, f, mh.ke + chains, &sj,
+                                      &noise, s)))
+          return rc;
+      }
+    }
+    if (amagold()) return gbsgmc_leapfrog_position(chains, d, mh.x, mh.p, nullptr, 0.5f, &sj, s);
+    return mean_pair(chains, mh.U_mean, U2, s);
+  }
 
   int enqueue(int g, cudaStream_t s) override {
     const int per = draws() * n;
@@ -372,7 +424,7 @@ struct GlmMhPlan final : gbsgmc_plan {
       c.ke = mh.ke;
       c.energy = mh.energy;
       c.status = status;
-      if ((rc = glm_loop(c, s))) return rc;
+      if ((rc = loop ? glm_loop(c, s) : trajectory(j, cn, per, s))) return rc;
       if ((rc = launch_full(a, part, s))) return rc;
       a.sched = to_sched(&sj);
       glm_mh_finish_kernel<<<chains, 128, 0, s>>>(a, mh);
@@ -491,7 +543,15 @@ extern "C" int gbsgmc_glm_mh_plan_create(
                                        p->stream), "glm_mh_plan_create: copy")))
       break;
     if ((rc = glm_prepare())) break;
-    p->ctas = glm_loop_ctas(chains, 1, n);
+    p->loop = glm_loop_pays(chains, 1, n, model->d);
+    if (p->loop) {
+      p->ctas = glm_loop_ctas(chains, 1, n);
+    } else {
+      p->ws_size = glm_ws_bytes(chains, n, model->d);
+      if ((rc = plan_alloc(p, &p->grad, xbytes, "glm_mh_plan_create: gradient"))) break;
+      if ((rc = plan_alloc(p, &p->U2, sizeof(double) * chains, "glm_mh_plan_create: U"))) break;
+      if ((rc = plan_alloc(p, &p->ws, p->ws_size, "glm_mh_plan_create: workspace"))) break;
+    }
     rc = plan_capture(p);
   } while (false);
   if (rc != GBSGMC_OK) {

@@ -116,6 +116,8 @@ struct UpdateFusion {
                                    //   c draws as chain ident[c]); null: c
 };
 int update_blocks(int chains, int64_t P);
+// a[c] = (a[c] + b[c]) / 2.
+int mean_pair(int chains, double* a, const double* b, cudaStream_t st);
 // At the schedule's kept steps: the first `rows` (at most 65,535) rows of x to
 // samples[slot], sign U (with U2: sign times the mean of the two) to
 // sample_lik[slot] (may be null).

@@ -18,13 +18,6 @@
 namespace gbsgmc {
 namespace {
 
-__global__ void mean_pair_kernel(int chains, double* a, const double* b) {
-  pdl_trigger();
-  pdl_wait();
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c < chains) a[c] = 0.5 * (a[c] + b[c]);
-}
-
 // Value and gradient over all chains:
 // (idx, idx_stride, U, lk_var, gradient out [chains, P], stream).
 using GradFn =
@@ -304,8 +297,7 @@ int NetPlan::enqueue_obabo(int g, const UpdateFusion& moving, const UpdateFusion
   if ((rc = obabo_second_fused(chains, P, x, aux, grad2, integ.mass_dev, integ.friction,
                                ke_end, &sj, &noise, last, s)))
     return rc;
-  launch_pdl(mean_pair_kernel, (chains + 127) / 128, 128, 0, s, chains, U, U2);
-  return check_launch("plan: potential mean");
+  return mean_pair(chains, U, U2, s);
 }
 
 // 1 / (s^2 T) of the prior, 0 for a flat one, as the gradient's kernels take it.

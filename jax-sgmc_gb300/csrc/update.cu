@@ -995,6 +995,18 @@ namespace gbsgmc {
 
 int update_blocks(int chains, int64_t P) { return static_cast<int>(grid4(chains, P).grid.x); }
 
+__global__ void mean_pair_kernel(int chains, double* a, const double* b) {
+  pdl_trigger();
+  pdl_wait();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < chains) a[c] = 0.5 * (a[c] + b[c]);
+}
+
+int mean_pair(int chains, double* a, const double* b, cudaStream_t st) {
+  launch_pdl(mean_pair_kernel, (chains + 127) / 128, 128, 0, st, chains, a, b);
+  return check_launch("mean_pair");
+}
+
 // At kept steps (the schedule's keep slot >= 0) the rows of x [rows, P] are
 // copied to samples [slot, rows, P] and sign U, of two potentials their mean,
 // to sample_lik [slot, rows].

@@ -217,3 +217,47 @@ def test_injected_normals_of_pairs(lib, monkeypatch):
     outs.append([a.cpu().numpy() for a in (x, plan.U, plan.lk_var, plan.ident)])
   for a, b in zip(*outs):
     np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("n,block", [(2000, False), (1200, True)])
+@pytest.mark.parametrize("name", ["amagold", "sggmc"])
+def test_long_minibatches_of_mh_chains(lib, monkeypatch, name, n, block):
+  """AMAGOLD and SGGMC of a few chains on both sides of the line between
+  trajectories of one launch and of launches per gradient and update.  With
+  four slices a minibatch everywhere, the latter are the per-chain path's
+  arithmetic: the same bits; the former: 1e-4 relative plus 1e-5 absolute."""
+  from gbsgmc import alias, data, engine, likelihoods as L, potential
+  monkeypatch.setenv("GBSGMC_GLM_SLICES", "4")
+  rng = np.random.default_rng(n)
+  N, d, C = 2500, 1000, 2
+  X = rng.normal(size=(N, d)).astype(np.float32)
+  y = (rng.random(N) < 0.5).astype(np.float32)
+  pot = potential.minibatch_potential(L.GaussianPrior(2.0), L.Logistic())
+  full = potential.full_potential(L.GaussianPrior(2.0), L.Logistic())
+  inits = [{"w": (0.01 * rng.normal(size=d)).astype(np.float32)} for _ in range(C)]
+  loops, make = [], engine._lib.call
+
+  def call(fn, *args):
+    if fn == "gbsgmc_plan_run":
+      per = [int(engine._lib.load().gbsgmc_plan_launches(args[0], 3 * k)) for k in (1, 2)]
+      loops.append(per[1] - per[0] == 3)   # trajectory, full pass, decision
+    return make(fn, *args)
+
+  monkeypatch.setattr(engine._lib, "call", call)
+  outs = []
+  for fused in (True, False):
+    monkeypatch.setattr(engine, "FUSED_ENABLED", fused)
+    sampler = alias.amagold if name == "amagold" else alias.sggmc
+    run = sampler(pot, full, data.NumpyDataLoader(x=X, y=y), cache_size=8, batch_size=n,
+                  integration_steps=3, first_step_size=0.004, last_step_size=0.002, burn_in=2)
+    outs.append(run(*inits, iterations=6))
+  assert loops == [block]
+  for a, b in zip(*outs):
+    for key in ("energy", "variables"):
+      va, vb = (np.asarray(r["samples"][key]["w"] if key == "variables" else r["samples"][key])
+                for r in (a, b))
+      if block:
+        np.testing.assert_allclose(va, vb, rtol=1e-4, atol=1e-5 if key == "variables" else 1e-3)
+      else:
+        np.testing.assert_array_equal(va, vb)
+    assert np.isfinite(va).all()
