@@ -893,6 +893,18 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
                                {"likelihood": lik}, model_states)
 
 
+# The most integrator steps a plan takes as one block.
+MAX_BLOCK_STEPS = 100_000
+
+
+def mh_block_iterations(steps, chains, n, draws) -> int:
+  """Iterations that one block of an :class:`MhPlan` runs; 0 when the plan does
+  not take the run (an iteration is one block at least)."""
+  if steps > MAX_BLOCK_STEPS or steps * chains * n > 1 << 28:
+    return 0
+  return max(1, DEFAULT_BLOCK_STEPS // steps)
+
+
 class MhPlan:
   """Owns a ``gbsgmc_glm_mh_plan``: C AMAGOLD or SGGMC chains on a GLM
   potential, per iteration one trajectory launch, one full-data pass and one
@@ -901,7 +913,7 @@ class MhPlan:
 
   def __init__(self, potential, full, dataset, X, PM, U, n, kind, steps, friction,
                h_tab, t_tab, keep_tab, n_kept, pcg, mh_seed, noise_seed, chain_base,
-               observation_count):
+               observation_count, block_iterations):
     import torch
     C, P = X.shape
     self.steps = int(steps)
@@ -923,7 +935,7 @@ class MhPlan:
               self.integ, _lib.ptr(X), _lib.ptr(PM), _lib.ptr(U), self.sched, self.noise,
               self.isrc, int(mh_seed) & (2**64 - 1), _lib.ptr(keep_tab),
               _lib.ptr(self.samples), _lib.ptr(self.stat),
-              max(1, DEFAULT_BLOCK_STEPS // self.steps), _lib.ptr(self.status))
+              int(block_iterations), _lib.ptr(self.status))
     self.handle = handle
 
   def run(self, iterations):
@@ -1037,14 +1049,14 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
   status = torch.zeros(1, dtype=torch.int32, device="cuda")
   noise = _lib.noise(noise_key, chain_base)
   h, t, keep, n_kept, _ = sched_mod.tables(scheduler, iterations)
-  if not pot.is_network and isinstance(full, FullPotential) and \
-      steps * C * n <= 1 << 28:
+  block = mh_block_iterations(steps, C, n, 2 if kind == "sggmc" else 1)
+  if not pot.is_network and isinstance(full, FullPotential) and block > 0:
     # GLM chains: trajectories, full-data passes and decisions on the device.
     tabs = [torch.from_numpy(np.repeat(np.asarray(a, np.float32), steps)).cuda()
             for a in (h, t)]
     plan = MhPlan(pot, full, ds, X, Pm, U_old.contiguous(), n, kind, steps, f, *tabs,
                   torch.from_numpy(np.asarray(keep, np.int32)).cuda(), n_kept, pcg,
-                  seed, noise_key, chain_base, N)
+                  seed, noise_key, chain_base, N, block)
     try:
       if iterations:
         plan.run(iterations)
