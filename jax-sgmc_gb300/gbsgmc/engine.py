@@ -893,16 +893,19 @@ def try_fused_resgld(solver, scheduler, states, schedulers, iterations, saving):
                                {"likelihood": lik}, model_states)
 
 
-# The most integrator steps a plan takes as one block.
+# The most integrator steps a plan takes as one block, and the most indices (4
+# bytes each) that a block of an MH plan holds.
 MAX_BLOCK_STEPS = 100_000
+MAX_BLOCK_INDICES = 1 << 28
 
 
 def mh_block_iterations(steps, chains, n, draws) -> int:
   """Iterations that one block of an :class:`MhPlan` runs; 0 when the plan does
   not take the run (an iteration is one block at least)."""
-  if steps > MAX_BLOCK_STEPS or steps * chains * n > 1 << 28:
+  indices = steps * chains * n * draws
+  if steps > MAX_BLOCK_STEPS or indices > MAX_BLOCK_INDICES:
     return 0
-  return max(1, DEFAULT_BLOCK_STEPS // steps)
+  return max(1, min(DEFAULT_BLOCK_STEPS // steps, MAX_BLOCK_INDICES // max(indices, 1)))
 
 
 class MhPlan:
