@@ -53,6 +53,7 @@ constexpr int kClerkWarp = kRowWarps;
 constexpr int kNoiseWarp = kRowWarps + 1;
 constexpr int kLoopThreads = kRowThreads + 64 + kCopyThreads;  // 168 registers a thread
 constexpr int kMaxCtas = 8;                     // portable cluster size
+constexpr uint64_t kLingerNs = 1000000;         // copies and sends in flight land in microseconds
 constexpr int kMaxDepth = 4;
 
 struct LoopArgs {
@@ -72,6 +73,8 @@ struct LoopArgs {
   int cp_async;    // some copies are made by cp.async
   int gather;      // rows are copied four at a time
   int row_cols;    // floats of a row that are read (16-byte words)
+  uint64_t wait_ns;  // bound of each wait
+  int missing;     // arrivals that a chunk waits for and that never come
   // pairs
   int pairs;
   double F;
@@ -160,13 +163,20 @@ __device__ __forceinline__ void send16(uint32_t dst, uint32_t bar, uint32_t x, u
       ::"r"(dst), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
       : "memory");
 }
-// Bounded wait for phase `phase` of a barrier.
-__device__ __forceinline__ void wait_phase(LoopBars* b, uint64_t* bar, int phase, int* status) {
-  if (mbar_try_wait(bar, phase & 1)) return;
-  if (!mbar_wait_bounded(bar, phase & 1, &b->stop)) {
-    b->stop = 1;
-    raise_status(status, GBSGMC_ERR_TIMEOUT);
-  }
+// Bounded wait for phase `phase` of a barrier; false when it ran out.  The caller
+// then takes no further part in any barrier exchange (no copies, sends or
+// arrivals: the phases are no longer those that it counts) and runs through to
+// the kernel's end, so that the named barriers stay matched.
+__device__ __forceinline__ bool wait_phase(const LoopArgs& L, LoopBars* b, uint64_t* bar,
+                                           int phase) {
+  if (mbar_try_wait(bar, phase & 1)) return true;
+  if (mbar_wait_bounded(bar, phase & 1, &b->stop, L.wait_ns)) return true;
+  b->stop = 1;
+  raise_status(L.g.status, GBSGMC_ERR_TIMEOUT);
+  return false;
+}
+__device__ __forceinline__ bool stopped(const LoopBars* b) {
+  return *static_cast<const volatile int*>(&b->stop) != 0;
 }
 __device__ __forceinline__ void cluster_arrive() {
   asm volatile("barrier.cluster.arrive.release;" ::: "memory");
@@ -234,9 +244,8 @@ __device__ __forceinline__ double slice_total(const SliceSums* s, int ctas, int 
 }
 
 template <int QPL, int RW>
-__global__ void __launch_bounds__(kLoopThreads, 1)
-    glm_loop_kernel(const __grid_constant__ LoopArgs L, const __grid_constant__ CUtensorMap map) {
-  extern __shared__ __align__(128) unsigned char smem[];
+__device__ __forceinline__ void loop_roles(const LoopArgs& L, const CUtensorMap& map,
+                                           unsigned char* smem) {
   constexpr int LOG = Log2<RW>::v;
   constexpr int GROUP = 32 >> LOG;
   constexpr int kStride = kRowWarps * RW;
@@ -275,7 +284,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
 
   if (tid == 0) {
     for (int i = 0; i < depth; ++i) {
-      mbar_init(bars->full + i, kCopyWarps + (L.cp_async ? kCopyThreads : 0));
+      mbar_init(bars->full + i, kCopyWarps + (L.cp_async ? kCopyThreads : 0) + L.missing);
       mbar_init(bars->empty + i, kRowWarps);
     }
     for (int i = 0; i < 2; ++i) {
@@ -305,7 +314,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     const int vec4 = a.vec4, y_inline = a.y_inline, chunks = L.chunks;
     const uint32_t row_bytes = static_cast<uint32_t>(rq) * 16;
     int buf = 0, use = 0;  // ring position, times round the ring
-    for (int e = 0; e < events; ++e) {
+    bool live = true;      // no wait has run out
+    for (int e = 0; live && e < events; ++e) {
       const int32_t* src = a.idx + (L.draws == 2 ? e >> 1 : e) * a.idx_step_stride +
                            static_cast<int64_t>(who) * a.idx_stride +
                            (L.draws == 2 ? (e & 1) * a.n : 0) + row0;
@@ -326,7 +336,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
             for (int j = 0; j < 4; ++j) o[j] = r + j < r_end ? __ldg(at + r + j) : -1;
           };
           fetch(cw * share + 4 * lane);
-          if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
+          if (use > 0)
+            live = __all_sync(0xffffffffu,
+                              wait_phase(L, bars, bars->empty + buf, use - 1));
+          if (!live) break;
           for (int r0 = cw * share; r0 < r_end; r0 += 128) {
             const int r = r0 + 4 * lane;
             if (r0 > cw * share) fetch(r);
@@ -355,7 +368,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
           }
         } else {
           int o = cw * share + lane < r_end ? __ldg(at + cw * share + lane) : -1;
-          if (use > 0) wait_phase(bars, bars->empty + buf, use - 1, a.status);
+          if (use > 0)
+            live = __all_sync(0xffffffffu,
+                              wait_phase(L, bars, bars->empty + buf, use - 1));
+          if (!live) break;
           for (int r0 = cw * share; r0 < r_end; r0 += 32) {
             const int r = r0 + lane;
             if (r0 > cw * share) o = r < r_end ? __ldg(at + r) : -1;
@@ -394,10 +410,12 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
         }
       }
     }
-    // No copy is in flight when the CTA ends, even if a wait has run out.
+    // No copy is in flight when the CTA ends, even if a wait has run out (the
+    // other copy warp may then have left its part out: a short bound).
     for (int i = 0; i < depth; ++i) {
       const int last = use - (i < buf ? 0 : 1);
-      if (last >= 0) mbar_wait_bounded(bars->full + i, last & 1, nullptr);
+      if (last >= 0)
+        mbar_wait_bounded(bars->full + i, last & 1, nullptr, live ? kWaitLimitNs : kLingerNs);
     }
     return;
   }
@@ -455,6 +473,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     double ssq = pairs ? L.ssq[unit] : 0.0;
     int exchanges = 0, role = half, wants = 0;
     int done_slot = -1;  // pairs: sample slot of the step last decided
+    bool live = true;    // no wait has run out
     const bool energies = L.energy != nullptr || L.ke != nullptr;
     StepInfo in = {};
     auto wanted = [&](int j, int slot) {
@@ -534,7 +553,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
         double t[3];
         reduce_lane_sums(lsum + (e & 1) * kRowWarps * RW, kRowWarps * RW, lane, t);
         SliceSums* all = sums + (wants & 1) * ncta;
-        if (lane < ncta) {
+        if (live && lane < ncta) {
           const uint32_t dst = cluster_addr(all + rank, lane);
           const uint32_t bar = cluster_addr(bars->sums + (wants & 1), lane);
           const double v[4] = {t[0], t[1], t[2], ww};
@@ -543,8 +562,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
             send16(dst + 16 * i, bar, __double2loint(v[2 * i]), __double2hiint(v[2 * i]),
                    __double2loint(v[2 * i + 1]), __double2hiint(v[2 * i + 1]));
         }
-        wait_phase(bars, bars->sums + (wants & 1), wants >> 1, a.status);
-        if (lane == 0 && e + 1 < events)
+        live &= __all_sync(0xffffffffu,
+                           wait_phase(L, bars, bars->sums + (wants & 1), wants >> 1)) != 0;
+        if (live && lane == 0 && e + 1 < events)
           mbar_arrive_expect_tx(bars->sums + (wants & 1),
                                 static_cast<uint32_t>(ncta) * sizeof(SliceSums));
         ++wants;
@@ -695,6 +715,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
   int want = pairs || (L.kind != kLoopLeapfrog &&
                        (a.steps == 1 || a.sched.keep_slot(k0) >= 0));
   int buf = 0, use = 0;
+  bool live = true;   // no wait of this thread has run out
   for (int e = 0; e < events; ++e) {
     const int j = L.draws == 2 ? e >> 1 : e;
     const int par = e & 1;
@@ -709,7 +730,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
     A.mlk = A.mlk_c = A.K = A.s1 = A.s2 = 0.0f;
     A.cnt = 0;
     for (int q = 0; q < L.chunks; ++q) {
-      wait_phase(bars, bars->full + buf, use, a.status);
+      live &= wait_phase(L, bars, bars->full + buf, use);
       const int cnt = min(CH, R - q * CH);
       const float4* rows = rows_s + buf * CH * rq;
       const int32_t* ix = idx_s + buf * CH;
@@ -733,7 +754,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
                               A);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(bars->empty + buf);
+      if (live && lane == 0) mbar_arrive(bars->empty + buf);
       if (++buf == depth) {
         buf = 0;
         ++use;
@@ -771,7 +792,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
         gl[i] = t[0];
 #pragma unroll
         for (int w = 1; w < kRowWarps; ++w) gl[i] += t[w];
-        if (S > 1) {
+        if (S > 1 && live) {
           const uint32_t at = smem_addr(partf + slice * 4 * dq + p) - here;
           const uint32_t bar = smem_addr(bars->part + par) - here;
 #pragma unroll
@@ -780,8 +801,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
         }
       }
       if (S > 1) {
-        wait_phase(bars, bars->part + par, e >> 1, a.status);
-        if (tid == 0 && e + 2 < events)
+        live &= wait_phase(L, bars, bars->part + par, e >> 1);
+        if (live && tid == 0 && e + 2 < events)
           mbar_arrive_expect_tx(bars->part + par, static_cast<uint32_t>(S) * d * 4);
 #pragma unroll
         for (int i = 0; i < kMaxOwned; ++i) {
@@ -877,6 +898,31 @@ __global__ void __launch_bounds__(kLoopThreads, 1)
       if (i >= owned) continue;
       xo[tid + i * kRowThreads] = xs[i];
       if (ao != nullptr) ao[tid + i * kRowThreads] = as[i];
+    }
+  }
+}
+
+template <int QPL, int RW>
+__global__ void __launch_bounds__(kLoopThreads, 1)
+    glm_loop_kernel(const __grid_constant__ LoopArgs L, const __grid_constant__ CUtensorMap map) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  loop_roles<QPL, RW>(L, map, smem);
+  // No CTA ends while another of its cluster may send to it.  In a run without
+  // a timeout each CTA's own waits have seen every send land.  After one they
+  // have not: the cluster waits for its last sender, tells all of its CTAs of
+  // the timeout, and they wait for the sends (and their own copies) to land.
+  LoopBars* bars = reinterpret_cast<LoopBars*>(smem + L.o_bar);
+  const int ncta = L.kind == kLoopPairs ? 2 * L.ctas : L.ctas;
+  if (ncta > 1) {
+    if (stopped(bars) && threadIdx.x < ncta)
+      asm volatile("st.shared::cluster.u32 [%0], 1;" ::"r"(cluster_addr(&bars->stop, threadIdx.x))
+                   : "memory");
+    cluster_arrive();
+    cluster_wait();
+  }
+  if (stopped(bars)) {
+    const uint64_t t0 = global_ns();
+    while (global_ns() - t0 < kLingerNs) {
     }
   }
 }
@@ -1148,6 +1194,11 @@ int glm_loop(const GlmLoopCall& c, cudaStream_t st) {
   L.ke = c.kind == kLoopObabo ? c.ke : nullptr;
   L.energy = c.kind == kLoopLeapfrog ? c.energy : nullptr;
   L.ctas = c.ctas;
+  // The waits' bound.  With 0 they are sure to run out: every chunk waits for
+  // one arrival that never comes.
+  const char* wait = std::getenv("GBSGMC_LOOP_WAIT_NS");
+  L.wait_ns = wait != nullptr ? std::strtoull(wait, nullptr, 10) : kWaitLimitNs;
+  L.missing = L.wait_ns == 0 ? 1 : 0;
   const bool y_in_row = L.g.vec4 && L.g.y_inline;
   L.row_quads = (L.g.d + (y_in_row ? 1 : 0) + 3) / 4;
   L.cp_y = !y_in_row && (L.g.y_inline || L.g.y != nullptr) ? 1 : 0;

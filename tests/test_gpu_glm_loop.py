@@ -249,3 +249,39 @@ def test_pairs_match_the_per_pair_path(lib, pairs, n, d):
                                rtol=1e-4, atol=1e-5)
     np.testing.assert_allclose(a["samples"]["likelihood"], b["samples"]["likelihood"],
                                rtol=1e-5, atol=1e-3)
+
+
+@pytest.mark.parametrize("kind,C,n,d", [("obabo", 1, 4000, 200), ("sghmc", 5, 700, 33),
+                                        ("langevin", 40, 300, 101), ("langevin", 200, 90, 6)])
+def test_a_wait_that_runs_out_ends_cleanly(lib, monkeypatch, kind, C, n, d):
+  """The block launch's bounded waits are its failure detection.  With a bound
+  of 0 the first chunks also wait for a copy that never comes, with 1 ns a wait
+  may run out anywhere in the run: the launch reports GBSGMC_ERR_TIMEOUT and
+  ends, its CTAs staying until no other can send to them.  The device stays
+  usable: the same run with the default bound then gives what an untouched one
+  gives."""
+  from gbsgmc import _lib, engine
+  X, y, ds, pot, x0, N = _setup(C, n, d, O.LOGISTIC)
+  steps = 24
+  h = np.full(steps, 1e-7 if kind == "langevin" else 1e-4, np.float32)
+  kw = {} if kind == "langevin" else dict(friction=2.0, leapfrog_steps=3)
+
+  def run():
+    x = _cuda(x0)
+    plan = engine.NetPlan(pot, ds, x, None if kind == "langevin" else _cuda(np.zeros_like(x0)), n,
+                          kind, _cuda(h), _cuda(np.ones(steps, np.float32)),
+                          engine.IndexSource(pcg=_cuda(_words(C))), 11, block_steps=12, **kw)
+    plan.run(0, steps)
+    code = int(plan.status.item())
+    plan.close()
+    return code, x.cpu().numpy()
+
+  code, want = run()
+  assert code == 0
+  for limit in ("0", "1", "0"):
+    with monkeypatch.context() as m:
+      m.setenv("GBSGMC_LOOP_WAIT_NS", limit)
+      assert run()[0] in ([_lib.ERR_TIMEOUT] if limit == "0" else [0, _lib.ERR_TIMEOUT])
+    code, x = run()
+    assert code == 0
+    np.testing.assert_array_equal(x, want)
