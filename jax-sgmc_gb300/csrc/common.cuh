@@ -350,8 +350,8 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// An unevaluated sum of two floats, hi + lo (48 bits or more): exact sums and
-// products by the error-free transformations of Knuth and Dekker (FMA form).
+// Exact sums and products as an unevaluated pair of floats, hi + lo (the
+// error-free transformations of Knuth and Dekker, FMA form).
 struct Float2Sum {
   float hi, lo;
 };
@@ -364,23 +364,43 @@ __device__ __forceinline__ Float2Sum two_prod(float a, float b) {
   const float p = __fmul_rn(a, b);
   return {p, __fmaf_rn(a, b, -p)};
 }
-__device__ __forceinline__ Float2Sum add2(Float2Sum a, Float2Sum b) {
-  const Float2Sum s = two_sum(a.hi, b.hi);
-  const Float2Sum t = two_sum(a.lo, b.lo);
-  const Float2Sum u = two_sum(s.hi, __fadd_rn(s.lo, t.hi));
-  return two_sum(u.hi, __fadd_rn(u.lo, t.lo));
-}
-// Sum over the warp of pairs of floats, the same in every lane.
-__device__ __forceinline__ Float2Sum warp_sum(Float2Sum f) {
-  const int lane = threadIdx.x & 31;
+// A sum of floats held in three, hi + mid + lo: what rounding takes from hi is
+// carried exactly into mid and from there into lo, so that only lo rounds, at
+// 2^-48 of the terms: 70 bits, where an FP64 sum keeps 53 (compensated
+// summation of third order; T. Ogita, S. Rump, S. Oishi 2005).
+struct Float3Sum {
+  float hi, mid, lo;
+  __device__ __forceinline__ void add_mid(float v) {
+    const Float2Sum m = two_sum(mid, v);
+    mid = m.hi;
+    lo = __fadd_rn(lo, m.lo);
+  }
+  __device__ __forceinline__ void add(float v) {
+    const Float2Sum h = two_sum(hi, v);
+    hi = h.hi;
+    add_mid(h.lo);
+  }
+  __device__ __forceinline__ void add(Float2Sum v) {
+    add(v.hi);
+    add_mid(v.lo);
+  }
+};
+// Sum over the warp, the same in every lane (each operation's result is the
+// same for either order of its operands).
+__device__ __forceinline__ Float3Sum warp_sum(Float3Sum f) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const Float2Sum u{__shfl_xor_sync(0xffffffffu, f.hi, o),
-                      __shfl_xor_sync(0xffffffffu, f.lo, o)};
-    // The same operand order in both lanes of a pair: the same bits.
-    f = (lane & o) ? add2(u, f) : add2(f, u);
+    const float hi = __shfl_xor_sync(0xffffffffu, f.hi, o);
+    const float mid = __shfl_xor_sync(0xffffffffu, f.mid, o);
+    const float lo = __shfl_xor_sync(0xffffffffu, f.lo, o);
+    const Float2Sum h = two_sum(f.hi, hi), m = two_sum(f.mid, mid);
+    f = Float3Sum{h.hi, m.hi, __fadd_rn(__fadd_rn(f.lo, lo), m.lo)};
+    f.add_mid(h.lo);
   }
   return f;
+}
+__device__ __forceinline__ double widen(Float3Sum f) {
+  return static_cast<double>(f.hi) + (static_cast<double>(f.mid) + f.lo);
 }
 
 // Sum over the block; every thread receives the result.  `scratch` holds at

@@ -257,33 +257,37 @@ __device__ __forceinline__ LaneSums lane_sums(const Accum<QPL>& A) {
 // Totals of `count` lanes' sums by one warp: t[0] = sum m lk, t[1] = sum lk,
 // t[2] = sum lk^2 (every lane gets them).  The widening restores sum(lk) =
 // s1 + n K and sum(lk^2) = s2 + 2 K s1 + n K^2.  A warp's FP64 instruction
-// takes some 64 cycles here, so the lanes add pairs of floats and only the
-// totals become FP64 (16 tiles of 4 rows: 3,280 cycles in FP64); sums that
-// are not finite take the FP64 path, which keeps infinities what they are.
+// takes some 64 cycles here, so the lanes add floats in three parts, to more
+// bits than FP64 has, and only the totals become FP64, a lane each (16 tiles of
+// 4 rows: 3,280 cycles in FP64); sums that are not finite take the FP64 path,
+// which keeps infinities what they are.
 __device__ __forceinline__ void reduce_lane_sums(const LaneSums* v, int count, int lane,
                                                  double (&t)[3]) {
-  Float2Sum f[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+  Float3Sum f[3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
   bool fine = true;
   for (int i = lane; i < count; i += 32) {
     const LaneSums s = v[i];
     const float n_l = static_cast<float>(s.cnt);   // exact: a lane's rows are few
-    const Float2Sum nk = two_prod(n_l, s.K);
-    const Float2Sum ks = two_prod(2.0f * s.K, s.s1);
-    Float2Sum nkk = two_prod(nk.hi, s.K);
-    nkk.lo = __fmaf_rn(nk.lo, s.K, nkk.lo);
-    f[0] = add2(f[0], two_sum(s.mlk, s.mlk_c));
-    f[1] = add2(f[1], add2(two_sum(s.s1, nk.hi), Float2Sum{nk.lo, 0.f}));
-    f[2] = add2(f[2], add2(add2(two_sum(s.s2, ks.hi), Float2Sum{ks.lo, 0.f}), nkk));
+    const Float2Sum nk = two_prod(n_l, s.K), ks = two_prod(2.0f * s.K, s.s1);
+    const Float2Sum nkk = two_prod(nk.hi, s.K), rest = two_prod(nk.lo, s.K);
+    f[0].add(Float2Sum{s.mlk, s.mlk_c});
+    f[1].add(nk);
+    f[1].add(s.s1);
+    f[2].add(nkk);
+    f[2].add(ks);
+    f[2].add(s.s2);
+    f[2].add_mid(rest.hi);
+    f[2].lo = __fadd_rn(f[2].lo, rest.lo);
     // Far from overflow: |values| below 2^96.
     fine = fine && fabsf(s.mlk) < 7.9e28f && fabsf(nkk.hi) < 7.9e28f && fabsf(s.s2) < 7.9e28f &&
            fabsf(ks.hi) < 7.9e28f;
   }
   if (__all_sync(0xffffffffu, fine)) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      f[k] = warp_sum(f[k]);
-      t[k] = static_cast<double>(f[k].hi) + f[k].lo;
-    }
+    for (int k = 0; k < 3; ++k) f[k] = warp_sum(f[k]);
+    const double mine = widen(lane == 1 ? f[1] : lane == 2 ? f[2] : f[0]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t[k] = __shfl_sync(0xffffffffu, mine, k);
     return;
   }
   t[0] = t[1] = t[2] = 0.0;

@@ -12,9 +12,9 @@
 // chains' weights are broadcast reads.  Each x is read from memory once per
 // CB chains; evaluating the chains one by one through the minibatch kernel
 // read all rows once per chain and computed gradients that no caller used.
-// Likelihoods are added compensated per thread and chain, reduced as pairs of
-// floats, and the CTAs' FP64 partials summed in a fixed order, so a chain's U
-// does not depend on the other chains of the call.
+// Likelihoods are added compensated per thread and chain, reduced as floats in
+// three parts, and the CTAs' FP64 partials summed in a fixed order, so a
+// chain's U does not depend on the other chains of the call.
 #include <algorithm>
 #include <cmath>
 #include <new>
@@ -165,8 +165,7 @@ __global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a,
   for (int c = 0; c < CB; ++c) {
     double s;
     if (__all_sync(0xffffffffu, fabsf(sum[c]) < 7.9e28f)) {
-      const Float2Sum f = warp_sum(two_sum(sum[c], comp[c]));
-      s = static_cast<double>(f.hi) + f.lo;
+      s = widen(warp_sum(Float3Sum{sum[c], comp[c], 0.0f}));
     } else {  // keeps infinities what they are
       s = warp_sum(static_cast<double>(sum[c]));
     }

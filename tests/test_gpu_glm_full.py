@@ -53,3 +53,24 @@ def test_infinite_likelihoods_stay_infinite(lib):
   ds = data.NumpyDataLoader(x=X, y=np.zeros(300, np.float32)).device_dataset()
   U = full.value_all(torch.tensor([[1.0, 0.0], [0.0, 0.0]], device="cuda"), ds).cpu().numpy()
   assert U[0] == np.inf and np.isfinite(U[1])
+
+
+@pytest.mark.parametrize("C", [1, 5])
+def test_sums_keep_every_bit_of_fp64(lib, C):
+  """Whole likelihoods of three sizes (2^51; 36 bits; below 1,000) whose sum
+  FP64 holds exactly: every partial sum does, and so does U (no prior,
+  temperature 1)."""
+  import torch
+  from gbsgmc import data, likelihoods as L, potential
+  rng = np.random.default_rng(C)
+  N = 256 * 40   # a tile a CTA, two observations a thread
+  lk = (rng.integers(2**23, 2**24, N) << 12).astype(np.int64)
+  small = rng.random(N) < 0.5
+  lk[small] = rng.integers(1, 1000, small.sum())
+  lk[[77, 5000]] = 2**51
+  x = lk.astype(np.float32)
+  assert (x.astype(np.int64) == lk).all() and lk.sum() < 2**53
+  full = potential.full_potential(L.FlatPrior(), L.Linear())
+  U = full.value_all(torch.ones((C, 1), device="cuda"),
+                     data.NumpyDataLoader(x=x[:, None]).device_dataset()).cpu().numpy()
+  assert (-U == float(lk.sum())).all()

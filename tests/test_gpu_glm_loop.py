@@ -285,3 +285,39 @@ def test_a_wait_that_runs_out_ends_cleanly(lib, monkeypatch, kind, C, n, d):
     code, x = run()
     assert code == 0
     np.testing.assert_array_equal(x, want)
+
+
+@pytest.mark.parametrize("C,n", [(1, 900), (3, 333), (170, 700)])
+@pytest.mark.parametrize("form", ["evaluate", "block"])
+def test_variance_of_large_likelihoods(lib, form, C, n):
+  """var(lk) = E[lk^2] - E[lk]^2 where it cancels most: whole likelihoods of
+  about 2^20 that differ by a few hundred, whose sums over a lane are exact and
+  whose totals FP64 holds exactly.  What may then differ from the exact
+  variance is the rounding of the means, their square and its subtraction,
+  2.5 2^-52 E[lk^2] in all; U: two roundings."""
+  import torch
+  from gbsgmc import data, engine, likelihoods as L, potential
+  N = 3000
+  rng = np.random.default_rng(n)
+  lk = (2**20 + rng.integers(-300, 300, N)).astype(np.float32)
+  ds = data.NumpyDataLoader(x=lk[:, None]).device_dataset()
+  pot = potential.minibatch_potential(L.FlatPrior(), L.Linear())
+  W = torch.ones((C, 1), device="cuda")
+  if form == "evaluate":
+    idx = rng.integers(0, N, (C, n)).astype(np.int32)
+    r = pot.evaluate(W, _cuda(idx), ds)
+    U, var = r.U.cpu().numpy(), r.lk_var.cpu().numpy()
+  else:
+    idx = np.stack([O.loader_draws(O.loader_rng(c), N, n, 1)[0] for c in range(C)])
+    plan = engine.NetPlan(pot, ds, W, None, n, "langevin", _cuda(np.zeros(1, np.float32)),
+                          _cuda(np.ones(1, np.float32)), engine.IndexSource(pcg=_cuda(_words(C))),
+                          11, block_steps=1)
+    plan.run(0, 1)
+    plan.check_status()
+    U, var = plan.U.cpu().numpy(), plan.lk_var.cpu().numpy()
+  for c in range(C):
+    v = [int(a) for a in lk[idx[c]]]
+    s1, s2 = sum(v), sum(a * a for a in v)
+    exact = (n * s2 - s1 * s1) / (n * n)
+    assert abs(var[c] - exact) <= 2.5 * 2.0**-52 * s2 / n
+    assert abs(U[c] + N * s1 / n) <= 2 * 2.0**-53 * N * s1 / n
