@@ -5,13 +5,24 @@
 // glm_loop launches, or as launches per gradient and update beyond its line.
 //
 // glm_full_kernel is a tall matrix product (rows x chains over d) whose
-// outputs never leave the registers: thread t of a 128-thread CTA owns rows t
-// and t + 128 of a 256-row tile for CB chains, X passes through shared memory
-// in panels of 16 features (cp.async, double buffered, rows padded to an odd
-// number of 16-byte words so that a warp's 32 rows touch every bank), and the
-// chains' weights are broadcast reads.  Each x is read from memory once per
-// CB chains; evaluating the chains one by one through the minibatch kernel
-// read all rows once per chain and computed gradients that no caller used.
+// outputs never leave the registers: a CTA takes 256 rows for 2 CB chains, each
+// of its halves CB of the chains, thread t of a half the rows t and t + 128.  X
+// passes through shared memory in panels of 16 features (cp.async, double
+// buffered, rows padded to an odd number of 16-byte words so that a warp's 32
+// rows touch every bank), and the chains' weights are broadcast reads.  Each x
+// is read from memory once per 2 CB chains; evaluating the chains one by one
+// through the minibatch kernel read all rows once per chain and computed
+// gradients that no caller used.
+//
+// A dot product may be no further from the exact one than the minibatch
+// kernel's (chains of four to 32 products a lane, then a tree over the lanes):
+// chains of four, a tree over a panel, and the panels added with their
+// rounding carried along.  One chain of FMAs over d had 2.1 times that kernel's
+// rms error at 64 features and 4.7 times at 1,000; this has 0.9 and 0.5 times
+// (equal up to 32).  It takes 26.0 us for 100,000 rows of 64 features and 16
+// chains where that took 24.2 (1,000,000 rows: 137 and 112; 20,000: 15.9 and
+// 18.0, the chains now being split over more warps).
+//
 // Likelihoods are added compensated per thread and chain, reduced as floats in
 // three parts, and the CTAs' FP64 partials summed in a fixed order, so a
 // chain's U does not depend on the other chains of the call.
@@ -27,22 +38,22 @@
 namespace gbsgmc {
 namespace {
 
-constexpr int kFullThreads = 128;
-constexpr int kFullRows = 2 * kFullThreads;   // rows of a tile
+constexpr int kHalf = 128;                 // threads of a half: two rows each
+constexpr int kFullThreads = 2 * kHalf;
+constexpr int kFullRows = 2 * kHalf;       // rows of a tile
 constexpr int kPanel = 4;                     // float4 columns of a panel
 constexpr int kPanelStride = kPanel + 1;
 
-size_t full_smem(int dq, int cb) {
-  return sizeof(float4) * (2ull * kFullRows * kPanelStride + static_cast<size_t>(cb) * dq);
+size_t full_smem(int dq, int cb) {   // cb: chains of a half
+  return sizeof(float4) * (2ull * kFullRows * kPanelStride + 2ull * cb * dq);
 }
 
-// Row CTAs of a launch, up to four per SM, whose warps fill the issue slots
-// that a thread's chain of links and sums leaves (100,000 rows of 64 features,
-// 16 chains: 25.8 us with one CTA per SM and panels of 32 features, 23.2 so).
-// Depends on the data alone (see above).
+// Row CTAs of a launch: as many as run at once, two per SM (twice as many, for
+// 100,000 rows of 64 features and 16 chains: 31.5 us against 26.0).  Depends on
+// the data alone (see above).
 int full_ctas(int64_t n_rows) {
   const int64_t tiles = (n_rows + kFullRows - 1) / kFullRows;
-  return static_cast<int>(std::min<int64_t>(tiles, 4 * glm_sm_count()));
+  return static_cast<int>(std::min<int64_t>(tiles, 2 * glm_sm_count()));
 }
 
 __device__ __forceinline__ void full_copy(const GlmArgs& a, float4* buf, int64_t row0, int q0,
@@ -72,17 +83,22 @@ __device__ __forceinline__ void full_copy(const GlmArgs& a, float4* buf, int64_t
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Grid (full_ctas, chain groups of CB).  part[cta][chain] gets the CTA's sum
+__device__ __forceinline__ float dot4(const float4& x, const float4& k) {
+  return fmaf(x.w, k.w, fmaf(x.z, k.z, fmaf(x.y, k.y, x.x * k.x)));
+}
+
+// Grid (full_ctas, chain groups of 2 CB).  part[cta][chain] gets the CTA's sum
 // of the chain's likelihoods.
 template <int CB>
-__global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a, double* part) {
+__global__ void __launch_bounds__(kFullThreads, 2) glm_full_kernel(const GlmArgs a, double* part) {
   extern __shared__ __align__(128) unsigned char smem[];
   float4* xs = reinterpret_cast<float4*>(smem);
   float4* ws = xs + 2 * kFullRows * kPanelStride;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int c0 = blockIdx.y * CB, dq = a.dq;
+  const int tid = threadIdx.x, lane = tid & 31, half = tid / kHalf, row = tid % kHalf;
+  const int warp = row >> 5, c0 = blockIdx.y * 2 * CB, dq = a.dq;
+  const bool active = c0 + half * CB < a.chains;   // this half has a chain
   // Weights of the group, zero past d and past the last chain.
-  for (int i = tid; i < CB * 4 * dq; i += kFullThreads) {
+  for (int i = tid; i < 2 * CB * 4 * dq; i += kFullThreads) {
     const int c = i / (4 * dq), j = i % (4 * dq);
     reinterpret_cast<float*>(ws)[i] =
         c0 + c < a.chains && j < a.d ? a.w[static_cast<int64_t>(c0 + c) * a.d + j] : 0.0f;
@@ -96,18 +112,18 @@ __global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a,
   if (first < tiles) full_copy(a, xs, first * kFullRows, 0, tid);
   int buf = 0;
   for (int64_t t = first; t < tiles; t += gridDim.x) {
-    const int64_t row0 = t * kFullRows;
+    const int64_t row0 = t * kFullRows + row;
     float y[2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int64_t r = row0 + tid + i * kFullThreads;
+      const int64_t r = row0 + i * kHalf;
       y[i] = 0.0f;
       if (r < a.n_rows)
         y[i] = a.y_inline ? __ldg(a.X + r * a.ld + a.d) : (a.y != nullptr ? __ldg(a.y + r) : 0.0f);
     }
-    float z[2][CB];
+    float z[2][CB], z_lo[2][CB];
 #pragma unroll
-    for (int c = 0; c < CB; ++c) z[0][c] = z[1][c] = 0.0f;
+    for (int c = 0; c < CB; ++c) z[0][c] = z[1][c] = z_lo[0][c] = z_lo[1][c] = 0.0f;
     for (int p = 0; p < panels; ++p) {
       // The next panel: of this tile, or the first of the CTA's next tile.
       const int64_t tn = p + 1 < panels ? t : t + gridDim.x;
@@ -118,49 +134,70 @@ __global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a,
         asm volatile("cp.async.commit_group;" ::: "memory");
       asm volatile("cp.async.wait_group 1;" ::: "memory");
       __syncthreads();
-      const float4* xa = xs + (buf * kFullRows + tid) * kPanelStride;
-      const float4* xb = xa + kFullThreads * kPanelStride;
+      const float4* xa = xs + (buf * kFullRows + row) * kPanelStride;
+      const float4* xb = xa + kHalf * kPanelStride;
+      const float4* wp = ws + half * CB * dq + p * kPanel;
       const int cols = min(kPanel, dq - p * kPanel);
-      const float4* wp = ws + p * kPanel;
-#pragma unroll 2
-      for (int v = 0; v < cols; ++v) {
-        const float4 u = xa[v], w = xb[v];
+      // A panel's 16 products: chains of four, added pairwise.
+      float pa[2][CB];
 #pragma unroll
-        for (int c = 0; c < CB; ++c) {
-          const float4 k = wp[c * dq + v];
-          z[0][c] = fmaf(u.x, k.x, z[0][c]);
-          z[1][c] = fmaf(w.x, k.x, z[1][c]);
-          z[0][c] = fmaf(u.y, k.y, z[0][c]);
-          z[1][c] = fmaf(w.y, k.y, z[1][c]);
-          z[0][c] = fmaf(u.z, k.z, z[0][c]);
-          z[1][c] = fmaf(w.z, k.z, z[1][c]);
-          z[0][c] = fmaf(u.w, k.w, z[0][c]);
-          z[1][c] = fmaf(w.w, k.w, z[1][c]);
+      for (int h = 0; h < 2; ++h) {
+        if (active && 2 * h < cols) {
+          const bool two = 2 * h + 1 < cols;
+          const float4 u0 = xa[2 * h], w0 = xb[2 * h];
+          const float4 u1 = two ? xa[2 * h + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 w1 = two ? xb[2 * h + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+          for (int c = 0; c < CB; ++c) {
+            const float4 k0 = wp[c * dq + 2 * h];
+            float a0 = dot4(u0, k0), a1 = dot4(w0, k0);
+            if (two) {
+              const float4 k1 = wp[c * dq + 2 * h + 1];
+              a0 += dot4(u1, k1);
+              a1 += dot4(w1, k1);
+            }
+            pa[0][c] = h ? pa[0][c] + a0 : a0;
+            pa[1][c] = h ? pa[1][c] + a1 : a1;
+          }
         }
       }
+#pragma unroll
+      for (int c = 0; c < CB; ++c)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          if (!active) continue;
+          const Float2Sum s = two_sum(z[r][c], pa[r][c]);
+          z[r][c] = s.hi;
+          z_lo[r][c] = __fadd_rn(z_lo[r][c], s.lo);
+        }
       __syncthreads();  // the buffer is free for the panel after the next
       buf ^= 1;
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      if (row0 + tid + i * kFullThreads >= a.n_rows) continue;
+      if (!active || row0 + i * kHalf >= a.n_rows) continue;
 #pragma unroll
       for (int c = 0; c < CB; ++c) {
+        // z_lo is no number once z has overflowed.
+        const float zi = z[i][c] + (isfinite(z_lo[i][c]) ? z_lo[i][c] : 0.0f);
         float lk, dz;
         if (a.family == GBSGMC_GLM_LOGISTIC) {
-          logistic_link(z[i][c], y[i], true, lk, dz);
+          logistic_link(zi, y[i], true, lk, dz);
         } else if (a.family == GBSGMC_GLM_LINEAR) {
-          lk = z[i][c];
+          lk = zi;
         } else {
-          const float res = y[i] - z[i][c];
+          const float res = y[i] - zi;
           lk = -0.5f * res * res * a.inv_s2 - a.log_norm;
         }
-        neumaier_add(sum[c], comp[c], lk);
+        // (comp is of no account once sum has overflowed.)
+        const Float2Sum s = two_sum(sum[c], lk);
+        sum[c] = s.hi;
+        comp[c] = __fadd_rn(comp[c], s.lo);
       }
     }
   }
   // Sums of the CTA's threads, chain by chain.
-  __shared__ double red[kFullThreads / 32][CB];
+  __shared__ double red[2][kHalf / 32][CB];
 #pragma unroll
   for (int c = 0; c < CB; ++c) {
     double s;
@@ -169,13 +206,14 @@ __global__ void __launch_bounds__(kFullThreads) glm_full_kernel(const GlmArgs a,
     } else {  // keeps infinities what they are
       s = warp_sum(static_cast<double>(sum[c]));
     }
-    if (lane == 0) red[warp][c] = s;
+    if (lane == 0) red[half][warp][c] = s;
   }
   __syncthreads();
-  if (tid < CB && c0 + tid < a.chains) {
-    double s = red[0][tid];
+  if (tid < 2 * CB && c0 + tid < a.chains) {
+    const int g = tid / CB, c = tid % CB;
+    double s = red[g][0][c];
 #pragma unroll
-    for (int w = 1; w < kFullThreads / 32; ++w) s += red[w][tid];
+    for (int w = 1; w < kHalf / 32; ++w) s += red[g][w][c];
     part[static_cast<int64_t>(blockIdx.x) * a.chains + c0 + tid] = s;
   }
 }
@@ -281,14 +319,15 @@ int launch_full_cb(const GlmArgs& a, double* part, cudaStream_t st) {
     done = 1;
   }
   const dim3 grid(static_cast<unsigned>(full_ctas(a.n_rows)),
-                  static_cast<unsigned>(ceil_div(a.chains, CB)));
+                  static_cast<unsigned>(ceil_div(a.chains, 2 * CB)));
   glm_full_kernel<CB><<<grid, kFullThreads, full_smem(a.dq, CB), st>>>(a, part);
   return check_launch("glm_full");
 }
 
 int launch_full(const GlmArgs& a, double* part, cudaStream_t st) {
-  // Groups of 16 chains when there are that many: x is read once per group.
-  return a.chains > 4 ? launch_full_cb<16>(a, part, st) : launch_full_cb<4>(a, part, st);
+  // Groups of 16 chains (eight a half) when there are more than four: x is read
+  // once per group.
+  return a.chains > 4 ? launch_full_cb<8>(a, part, st) : launch_full_cb<2>(a, part, st);
 }
 
 size_t full_ws_bytes(const gbsgmc_glm* m, int chains) {
