@@ -90,7 +90,8 @@ def re_sgld(potential_fn, data_loader, cache_size: int = 512,
 
   def run_fn(*init_samples, init_model_state: Pytree = None, iterations=1000):
     init = partial(resgld_solver[0], init_model_state=init_model_state)
-    states = _init_states(resgld_solver[0], lambda pair: init(*pair), init_samples,
+    states = _init_states(resgld_solver[0], lambda pair: init(*pair),
+                          [tuple(pair) for pair in init_samples],
                           init_model_state=init_model_state)
     return mcmc.run_chains(states, iterations=iterations,
                            schedulers=[{'temperature': {'tau': temperature}}])

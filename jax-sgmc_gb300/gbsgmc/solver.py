@@ -143,8 +143,7 @@ def parallel_tempering(integrator, sa_schedule=None):
         float(F), torch.zeros(1, dtype=torch.int64, device="cuda"),
         key_to_seed((seed, normal.chain)), seed, int(normal.chain))
 
-  def init_many(pairs, ssq_init=0.0, key=0, F=1.0, **kwargs):
-    """``[init(*pair, ...) for pair in pairs]`` in bulk."""
+  def init_pairs(pairs, ssq_init=0.0, key=0, F=1.0, **kwargs):
     from .integrator import LangevinChains
     seed = int(np.asarray(key).ravel()[-1]) if key is not None else 0
     chains = init_integrator.many([s for pair in pairs for s in pair], key=seed,
@@ -154,8 +153,16 @@ def parallel_tempering(integrator, sa_schedule=None):
       return [make(n, h) for n, h in zip(chains[0::2], chains[1::2])]
     return PairChains(chains, float(ssq_init), float(F), seed, make)
 
-  if getattr(init_integrator, "many", None) is not None:
-    init.many = init_many
+  def init_many(pairs, **kwargs):
+    """``[init(*pair, ...) for pair in pairs]``, in bulk where every pair is
+    two samples (a pair may also bring its own ssq_init, key and F)."""
+    pairs = [tuple(pair) for pair in pairs]
+    if any(len(pair) != 2 for pair in pairs):
+      return [init(*pair, **kwargs) for pair in pairs]
+    return init_pairs(pairs, **kwargs)
+
+  init_any = init if getattr(init_integrator, "many", None) is None else \
+      util.with_many(init, init_many)
 
   def update(state: TemperingState, normal_schedule, hot_schedule,
              uniform=None):
@@ -184,7 +191,7 @@ def parallel_tempering(integrator, sa_schedule=None):
   def get(state: TemperingState):
     return get_integrator(state.normal)
 
-  return SolverTriplet(init, update, get, kind="parallel_tempering",
+  return SolverTriplet(init_any, update, get, kind="parallel_tempering",
                        integrator=integrator)
 
 
