@@ -1063,6 +1063,7 @@ def try_fused_mh(solver, scheduler, states, schedulers, iterations, saving):
     try:
       if iterations:
         plan.run(iterations)
+      full._unit.check_status()   # the starts' potentials
       plan.check_status()
       samples, extra = plan.samples, plan.stat
     finally:
