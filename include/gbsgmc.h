@@ -810,8 +810,10 @@ int gbsgmc_cnn_plan_create(gbsgmc_plan** plan, const gbsgmc_cnn* model,
 
 /* As gbsgmc_mlp_plan_create for the generalised-linear families (P = d): a
  * block of steps, gradients and updates, is one launch in which a cluster of
- * CTAs owns each chain.  Meant for OBABO and SGHMC; SGLD on these families
- * has its own plan (gbsgmc_sgld_glm_plan_create). */
+ * CTAs owns each chain; where that would leave SMs idle over long minibatches,
+ * and with injected normals (noise_dev), every gradient and update is a launch
+ * of its own.  Meant for OBABO and SGHMC; SGLD on these families has its own
+ * plan (gbsgmc_sgld_glm_plan_create). */
 int gbsgmc_glm_plan_create(gbsgmc_plan** plan, const gbsgmc_glm* model,
                            int chains, int n, const gbsgmc_integrator* integrator,
                            float* x_dev, float* aux_dev,
@@ -936,9 +938,11 @@ int gbsgmc_mlp_resgld_plan_create_keep(gbsgmc_plan** plan, const gbsgmc_mlp* mod
  * | pair_chain_dev[p]).  At kept steps the normal slots' x and -U go to
  * samples_dev [slot, pairs, d] and sample_lik_dev [slot, pairs]; swap counts
  * are added to tempering->counts_dev [pairs] when it is not NULL
- * (tempering->every and flags_dev are not used).  Per step: one fused SGLD
- * launch for all 2 pairs chains and one exchange launch; per block one
- * index-draw launch, replayed from a CUDA graph.
+ * (tempering->every and flags_dev are not used).  A block of steps is an index
+ * draw and one launch in which a cluster of CTAs owns each pair, exchanges
+ * included; where that would leave SMs idle over long minibatches, and with
+ * injected normals (noise_dev), each step is one fused SGLD launch for all 2
+ * pairs chains and one exchange launch.  Replayed from a CUDA graph.
  * Replaces alias.re_sgld (jax_sgmc/alias.py:122-208) through solver.mcmc. */
 int gbsgmc_glm_resgld_plan_create(gbsgmc_plan** plan, const gbsgmc_glm* model,
                                   int pairs, int n, float* x_dev, float* v_dev,

@@ -168,8 +168,9 @@ __device__ __forceinline__ float bf(bf16 v) { return __bfloat162float(v); }
 // the second tap pair and the other kernel rows.  Nothing is copied per tap.
 // Core matrices start on 16-byte boundaries, as that layout allows.
 // For 8 x 256 images the forward pass took 128 us as three launches (weights,
-// gather, GEMM) and takes 36; the output gradient with the weight GEMM took
-// 137 and takes 55 (32 splits of 8 chains leave a third of the SMs one CTA).
+// gather, GEMM) and takes 36; the output gradient with the weight GEMM took 137
+// and, as a launch of its own, 55.  It now shares cnn_weight_grads_kernel with
+// the other layers' (all three and the routing: 85).
 // ---------------------------------------------------------------------------
 constexpr int kStripThreads = 128;
 constexpr int kPlaneRow = 9 * 16, kPlane = 34 * kPlaneRow;   // bytes
@@ -848,7 +849,8 @@ __device__ __forceinline__ int pool_windows(const float (&x)[32], uint4& p, uint
 // address of the same box: conv2's box of 128 pixels is 72 rows of 160 bytes
 // for TMA instead of 9 boxes, or an im2col of 9 times the map, written and read
 // back.  2,048 images: 25 us against 147 with the im2col (335 MB), dP1 26
-// against 115 with a box per tap, dW2 25 against 95.  W2 lies in shared memory,
+// against 115 with a box per tap, dW2, while it had a launch of its own, 25
+// against 95 (now part of cnn_weight_grads_kernel).  W2 lies in shared memory,
 // [output octet][tap, input][8], for a run of strips of one chain: MN-major B
 // of the forward GEMM, K-major B of the transposed one.
 // ---------------------------------------------------------------------------
@@ -1990,8 +1992,8 @@ int run_cnn(CnnArgs& a, const CnnLayout& L, void* ws, cudaStream_t st) {
     return launched("cnn_dense_kernel");
   };
   // Sixteen images share a block's copy of Wd once that fills the SMs.
-  rc = int64_t(C) * n >= 16 * 152 / 2 ? dense(cnn_dense_kernel<16, 2>, 16, 2)
-                                      : dense(cnn_dense_kernel<4, 1>, 4, 1);
+  rc = int64_t(C) * n >= 16 * (sms / 2) ? dense(cnn_dense_kernel<16, 2>, 16, 2)
+                                        : dense(cnn_dense_kernel<4, 1>, 4, 1);
   if (rc) return rc;
 
   if (a.want_grad) {

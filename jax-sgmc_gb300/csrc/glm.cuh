@@ -146,9 +146,9 @@ __device__ __forceinline__ float transposed_warp_sum(float (&p)[RW], int lane) {
 }
 
 // Per-lane accumulators of one CTA row stream.  The likelihood sums stay in
-// fp32 per lane (a lane sees a few dozen rows); they are widened to fp64 for
-// the warp and block reductions.  GB300's fp64 pipe runs at a small fraction
-// of the fp32 rate, so per-row fp64 arithmetic would throttle the kernel.
+// fp32 per lane (a lane sees a few dozen rows); reduce_lane_sums makes fp64
+// totals of them.  GB300's fp64 pipe runs at a small fraction of the fp32 rate,
+// so per-row fp64 arithmetic would throttle the kernel.
 //
 // The sum of the (masked) likelihoods that makes U is compensated: each
 // addition's rounding error is carried in mlk_c (Neumaier's variant of

@@ -18,9 +18,10 @@
 //     us; 64 chains of 512 rows of 32 features 299 to 136 us a 50 steps, 64
 //     of 128 features 307 to 153; never slower);
 //   * the row warps do what nothing else can do earlier: row tiles of the
-//     chunk exactly as glm_kernel takes them (same slices, warps, tiles and
-//     summation orders: the same bits), the reduction, the exchange and the
-//     update.  CTA s holds rows [s R, (s + 1) R) of every minibatch; it sends
+//     chunk by glm_kernel's code, the reduction, the exchange and the update.
+//     The slices (glm_loop_ctas) and rows per warp (loop_rows_per_warp) are this
+//     kernel's own, so its sums have other orders than glm_kernel's unless these
+//     coincide, and a chain's bits depend on how many chains run beside it.  CTA s holds rows [s R, (s + 1) R) of every minibatch; it sends
 //     its partial gradient into all CTAs of the cluster (st.async, counted on
 //     the receivers' mbarriers), and every CTA adds the partials in slice
 //     order and updates its own copy of x, held in registers, so no second

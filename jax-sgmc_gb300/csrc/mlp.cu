@@ -717,8 +717,9 @@ __global__ void __launch_bounds__(256, kFisher ? 2 : 3) mlp_out_kernel(const Mlp
 // 9. Bias and output-layer gradients, U and var(lk).  Grid (ceil(H1/256) +
 //    ceil(H2/256) + 1, chains) with a gradient, (1, chains) without: blocks of
 //    the first layer's columns, of the second's, and one of the values, whose
-//    loads would otherwise follow one another (64 chains of 2,048 rows: 22 ->
-//    11 us behind the last GEMM).
+//    loads would otherwise follow one another.  The launch by itself, for 64
+//    chains of 2,048 rows: 29.2 us with block-wide sums in turn, 14.3 with the
+//    sums side by side (below) and the layers in one block, 9.5 so.
 // ---------------------------------------------------------------------------
 // Adds rows r .. of a column of partials (ld apart) in order, K loads in
 // flight, while K are left before n.
@@ -803,8 +804,7 @@ __global__ void __launch_bounds__(256) mlp_finalize_kernel(const MlpArgs a, int 
   }
   if (blockIdx.x + 1 != gridDim.x) return;
   // Five FP64 sums, a warp each: as block-wide sums one after the other they
-  // held the launch (64 chains of 2,048 rows: 28.8 -> 13.8 us, with the
-  // column loads above in flight together).
+  // held the launch.
   const int warp = t >> 5, lane = t & 31;
   if (warp < 5) {
     double v = 0.0;

@@ -304,8 +304,10 @@ def minibatch_potential(prior, likelihood, strategy="map", has_state=False,
 
 class FullPotential:
   """Potential over the complete dataset (potential.py:219-293):
-  ``U = (-sum_{all i} lk_i - log p(sample)) / temperature``, evaluated in
-  ordered chunks of observations with the GLM kernel."""
+  ``U = (-sum_{all i} lk_i - log p(sample)) / temperature``.  The value alone
+  of the GLM families is one pass of ``glm_full_kernel`` over all rows for all
+  chains; gradients, and the networks, go through the minibatch kernels in
+  ordered chunks of observations."""
 
   CHUNK = 65536
 

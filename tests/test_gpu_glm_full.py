@@ -1,5 +1,5 @@
 """The full-data potential of many chains (glm_full.cu) at the edges of its
-row tiles (256), feature panels (32) and chain groups (4 and 16), against the
+row tiles (256), feature panels (16) and chain groups (4 and 16), against the
 oracle in float64.
 
 Tolerance: each likelihood is an fp32 value of relative error about 1e-6 (its
